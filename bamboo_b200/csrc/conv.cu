@@ -188,13 +188,47 @@ bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, cons
   }
 }
 
-// mean / rstd per channel from the partial rows (biased variance, as batch norm normalises with)
-__global__ void bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv_rows, float eps,
-                                       float* __restrict__ mean, float* __restrict__ rstd) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+// Column sums over the partial rows: a block owns 32 channels and splits the rows over its 32 warps
+// (coalesced 128-byte reads, four rows in flight per warp), then adds the warps' sums in warp order, so
+// the result does not depend on scheduling.  A thread per channel walking all (up to 592) partial rows is
+// a chain of that many L2 latencies: 26-28 us per call at 592 rows, against about 3 us this way.
+// Valid in warp 0 only: t1, t2 of channel blockIdx.x * 32 + lane.
+__device__ __forceinline__ void bn_sum_partials(const float* __restrict__ ws, int parts, int C, float& t1, float& t2) {
+  __shared__ float sm1[32][33], sm2[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s1 = 0.f, s2 = 0.f;
-  for (int p = 0; p < parts; ++p) { s1 += ws[(long long)p * 2 * C + c]; s2 += ws[(long long)p * 2 * C + C + c]; }
+  if (c < C) {
+    int p = w;
+    for (; p + 96 < parts; p += 128) {
+      float a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float* row = ws + (long long)(p + 32 * u) * 2 * C + c;
+        a[u] = __ldg(row); b[u] = __ldg(row + C);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { s1 += a[u]; s2 += b[u]; }
+    }
+    for (; p < parts; p += 32) { const float* row = ws + (long long)p * 2 * C + c; s1 += __ldg(row); s2 += __ldg(row + C); }
+  }
+  sm1[w][lane] = s1; sm2[w][lane] = s2;
+  __syncthreads();
+  t1 = 0.f; t2 = 0.f;
+  if (w == 0) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) { t1 += sm1[j][lane]; t2 += sm2[j][lane]; }
+  }
+}
+
+// mean / rstd per channel from the partial rows (biased variance, as batch norm normalises with)
+__global__ void __launch_bounds__(1024)
+bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv_rows, float eps,
+                       float* __restrict__ mean, float* __restrict__ rstd) {
+  float s1, s2;
+  bn_sum_partials(ws, parts, C, s1, s2);
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x >= 32 || c >= C) return;
   const float m = s1 * inv_rows;
   const float var = fmaxf(s2 * inv_rows - m * m, 0.f);
   mean[c] = m;
@@ -202,12 +236,13 @@ __global__ void bn_finish_stats_kernel(const float* __restrict__ ws, int parts, 
 }
 
 // sums[0][c] = sum dz', sums[1][c] = sum dz' * yhat; dbeta += sums[0], dgamma += sums[1]
-__global__ void bn_finish_bwd_kernel(const float* __restrict__ ws, int parts, int C, float* __restrict__ sums,
-                                     float* __restrict__ dgamma, float* __restrict__ dbeta) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s1 = 0.f, s2 = 0.f;
-  for (int p = 0; p < parts; ++p) { s1 += ws[(long long)p * 2 * C + c]; s2 += ws[(long long)p * 2 * C + C + c]; }
+__global__ void __launch_bounds__(1024)
+bn_finish_bwd_kernel(const float* __restrict__ ws, int parts, int C, float* __restrict__ sums,
+                     float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  float s1, s2;
+  bn_sum_partials(ws, parts, C, s1, s2);
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x >= 32 || c >= C) return;
   sums[c] = s1; sums[C + c] = s2;
   dbeta[c] += s1; dgamma[c] += s2;
 }
@@ -313,7 +348,7 @@ extern "C" int bb_bn_stats(const void* y, long long rows, int C, float eps, floa
   const int grid = bn_grid(rows, C);
   float* ws = static_cast<float*>(workspace);
   bn_reduce_kernel<RED_STATS><<<grid, 256, 0, s>>>((const uint4*)y, nullptr, nullptr, nullptr, nullptr, 0, rows, C, ws);
-  bn_finish_stats_kernel<<<(C + 127) / 128, 128, 0, s>>>(ws, grid, C, 1.0f / (float)rows, eps, mean, rstd);
+  bn_finish_stats_kernel<<<(C + 31) / 32, 1024, 0, s>>>(ws, grid, C, 1.0f / (float)rows, eps, mean, rstd);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -346,7 +381,7 @@ extern "C" int bb_bn_bwd(const void* dz, const void* z, const void* y, const flo
   float* ws = static_cast<float*>(workspace);
   float* sums = ws + (long long)grid * 2 * C;
   bn_reduce_kernel<RED_BWD><<<grid, 256, 0, s>>>((const uint4*)dz, (const uint4*)z, (const uint4*)y, mean, rstd, relu, rows, C, ws);
-  bn_finish_bwd_kernel<<<(C + 127) / 128, 128, 0, s>>>(ws, grid, C, sums, dgamma, dbeta);
+  bn_finish_bwd_kernel<<<(C + 31) / 32, 1024, 0, s>>>(ws, grid, C, sums, dgamma, dbeta);
   bn_bwd_apply_kernel<<<grid, 256, 0, s>>>((const uint4*)dz, (const uint4*)z, (const uint4*)y, mean, rstd,
                                            (const __nv_bfloat16*)gamma, sums, (uint4*)dy, (uint4*)dres, rows, C, relu,
                                            1.0f / (float)rows);

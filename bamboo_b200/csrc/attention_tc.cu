@@ -1,4 +1,4 @@
-// Fused attention on the 5th-generation tensor cores: head dimension 64 (forward and backward) and 128 (forward).
+// Fused attention on the 5th-generation tensor cores: head dimensions 64 and 128, forward and backward.
 //
 // Every contraction (Q.K^T, P.V, dO.V^T, dS.K, P^T.dO, dS^T.Q) is a tcgen05.mma with fp32
 // accumulators in tensor memory; tiles arrive by TMA into 128-byte-swizzled shared memory;
@@ -11,11 +11,12 @@
 // lane quarter each) do the softmax / element-wise work and the final stores.  Kernels:
 //   forward          : CTA owns 256 query rows as two tiles in ping-pong (one softmax group per tile),
 //                      the output row accumulates in tensor memory; templated on the head dimension;
-//   fused backward   : CTA owns 128 key rows, streams 64-row query / dO sub-tiles, computes the scores
-//                      once and produces dK, dV (fixed summation order) and dQ (fp32 add-reductions
-//                      into an accumulator that a small kernel scales and converts);
+//   fused backward   : (head dimension 64) CTA owns 128 key rows, streams 64-row query / dO sub-tiles,
+//                      computes the scores once and produces dK, dV (fixed summation order) and dQ (fp32
+//                      add-reductions into an accumulator that a small kernel scales and converts);
 //   two-role backward: dK/dV CTAs and dQ CTAs in one launch, scores computed by both roles, every
-//                      sum in a fixed order (no reductions) - selected by BB_ATTENTION_BWD=split.
+//                      sum in a fixed order (no reductions); templated on the head dimension - the
+//                      backward at 128, and at 64 when BB_ATTENTION_BWD=split asks for fixed-order sums.
 #include "tma_host.cuh"
 #include <math.h>
 #include <stdlib.h>
@@ -119,13 +120,15 @@ struct Ctl {
 };
 
 
-// delta[b, h, s] = sum_d dO * O.  Eight lanes per (token, head): each loads 16 bytes of O and dO
-// (a warp reads four consecutive heads of a token: 512 contiguous bytes per operand), two
+// delta[b, h, s] = sum_d dO * O.  D / 8 lanes per (token, head): each loads 16 bytes of O and dO
+// (a warp reads consecutive heads of a token: 512 contiguous bytes per operand), two
 // independent units per thread for memory-level parallelism.  The same pass clears the fp32
 // accumulator of the fused backward kernel, when there is one.
+template <int D>
 __global__ void __launch_bounds__(256)
 attn_tc_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const TcParams p) {
-  const int per_tok = p.H * 8;                                 // 16-byte chunks per token row
+  constexpr int LANES = D / 8;                                 // lanes of one (token, head)
+  const int per_tok = p.H * LANES;                             // 16-byte chunks per token row
   const long long total = (long long)p.B * p.S * per_tok;
   const long long stride = (long long)gridDim.x * blockDim.x;
   if (p.dq_acc) {
@@ -157,12 +160,13 @@ attn_tc_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* _
       t += __shfl_xor_sync(0xffffffffu, t, 1);
       t += __shfl_xor_sync(0xffffffffu, t, 2);
       t += __shfl_xor_sync(0xffffffffu, t, 4);
+      if (D == 128) t += __shfl_xor_sync(0xffffffffu, t, 8);
       s[u] = t;
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      if (cc[u] < total && (threadIdx.x & 7) == 0) {
-        const long long tok = cc[u] / per_tok; const int head = (int)(cc[u] % per_tok) >> 3;
+      if (cc[u] < total && (threadIdx.x & (LANES - 1)) == 0) {
+        const long long tok = cc[u] / per_tok; const int head = (int)(cc[u] % per_tok) / LANES;
         p.delta[((tok / p.S) * p.H + head) * p.S + (tok % p.S)] = s[u];
       }
     }
@@ -182,22 +186,42 @@ constexpr int SUB_BYTES = SUB * HD * 2;          // 8 KiB: [64 x 64] bf16
 // two could not (issue slots were 35 % busy with 4-warp groups).
 constexpr int GROUP_THREADS = 256;
 constexpr int NT2 = 64 + 2 * GROUP_THREADS;
-constexpr int NST = 6;                           // streamed sub-tile ring depth
-constexpr int NSB = 3;                           // score buffers in tensor memory
+
+// Geometry of the two-role backward at head dimension D.  A [rows x 128] operand is two [rows x 64] atoms of
+// 128-byte rows, one after the other (two TMA boxes), exactly as in the forward kernel.
+// Tensor memory (512 columns): NSB score and NSB dP buffers of 64 columns, then the accumulators - dV and dK
+// (D columns each) or dQ (D columns): 3 buffers at D = 64, 2 at D = 128, where dV + dK alone take half of it.
+// Shared memory at D = 128: K and V (64 KiB), three stages of query and dO sub-tiles (96 KiB), P^T and dS^T for
+// two groups (64 KiB) - 224 of 227 KiB, so the ring cannot be deeper.
+template <int D> struct Bwd2 {
+  static constexpr int NA = D / 64;                          // 64-column atoms per row
+  static constexpr int NST = (D == 64) ? 6 : 3;              // streamed sub-tile ring depth
+  static constexpr int NSB = (D == 64) ? 3 : 2;              // score buffers in tensor memory
+  static constexpr int OWN_BYTES = NA * TILE_BYTES;          // one of the CTA's own [128 x D] operands
+  static constexpr int STREAM_BYTES = NA * SUB_BYTES;        // one streamed [64 x D] sub-tile
+  static constexpr int ACC = 2 * NSB * 64;                   // first accumulator column
+};
+// k-step k (16 columns) of a K-major [rows x D] operand whose 64-column atoms lie `atom` bytes apart
+__device__ __forceinline__ uint64_t desc_kmajor_atoms(uint64_t d0, int k, int atom) {
+  return desc_kmajor(d0 + (uint64_t)((k >> 2) * (atom >> 4)), k & 3);
+}
 
 // ------------------------------------------------------------------ dQ (pipelined)
-// smem: Q, dO [128 x 64] | K, V sub-tiles [64 x 64] x 3 stages | dS [128 q x 64 kv] x 2
-// TMEM: S 2 x 64 | dP 2 x 64 | dQ 64
+// smem: Q, dO [128 x D] | K, V sub-tiles [64 x D] x NST stages | dS [128 q x 64 kv] x 2
+// TMEM: S NSB x 64 | dP NSB x 64 | dQ D
+template <int D>
 __device__ __forceinline__ void
 attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtensorMap& tm_do, const TcParams& p,
                  const int bx, const int nbx) {
+  using G = Bwd2<D>;
+  constexpr int NA = G::NA, NST = G::NST, NSB = G::NSB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sDO = sQ + TILE_BYTES;
-  uint8_t* sK = sDO + TILE_BYTES;              // NST stages x 8 KiB
-  uint8_t* sV = sK + NST * SUB_BYTES;          // NST stages x 8 KiB
-  uint8_t* sDS = sV + NST * SUB_BYTES;         // 2 x 16 KiB
+  uint8_t* sDO = sQ + G::OWN_BYTES;
+  uint8_t* sK = sDO + G::OWN_BYTES;            // NST stages
+  uint8_t* sV = sK + NST * G::STREAM_BYTES;    // NST stages
+  uint8_t* sDS = sV + NST * G::STREAM_BYTES;   // 2 x 16 KiB
   Ctl* ctl = reinterpret_cast<Ctl*>(sDS + 2 * TILE_BYTES);
   uint64_t* q_full = &ctl->bars[0];
   uint64_t* kv_full = &ctl->bars[1];           // [NST]
@@ -212,7 +236,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   const int qb = nbx - 1 - bx, head = blockIdx.y, batch = blockIdx.z;
   const int q0 = qb * TQ;
   const int row_base = batch * p.S;
-  const int colq = head * HD, colk = p.hidden + head * HD, colv = 2 * p.hidden + head * HD;
+  const int colq = head * D, colk = p.hidden + head * D, colv = 2 * p.hidden + head * D;
   int nblk = (p.S + SUB - 1) / SUB;
   if (p.causal) nblk = min(nblk, (q0 + TQ) / SUB);
 
@@ -231,26 +255,32 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
-  const uint32_t tDQ = tmem + 384;             // S[b] at tmem + 64 b, dP[b] at tmem + 192 + 64 b (b < 3)
+  const uint32_t tDQ = tmem + G::ACC;          // S[b] at tmem + 64 b, dP[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
     if (lane == 0) {
-      bb::mbar_arrive_expect_tx(q_full, 2 * TILE_BYTES);
-      bb::tma_load_2d(sQ, &tm_q, q_full, colq, row_base + q0);
-      bb::tma_load_2d(sDO, &tm_do, q_full, colq, row_base + q0);
+      bb::mbar_arrive_expect_tx(q_full, 2 * G::OWN_BYTES);
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        bb::tma_load_2d(sQ + a * TILE_BYTES, &tm_q, q_full, colq + 64 * a, row_base + q0);
+        bb::tma_load_2d(sDO + a * TILE_BYTES, &tm_do, q_full, colq + 64 * a, row_base + q0);
+      }
       for (int j = 0; j < nblk; ++j) {
         const int s = j % NST;
         if (!bb::mbar_wait(&kv_empty[s], ((j / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
-        bb::mbar_arrive_expect_tx(&kv_full[s], 2 * SUB_BYTES);
-        bb::tma_load_2d(sK + s * SUB_BYTES, &tm_kv, &kv_full[s], colk, row_base + j * SUB);
-        bb::tma_load_2d(sV + s * SUB_BYTES, &tm_kv, &kv_full[s], colv, row_base + j * SUB);
+        bb::mbar_arrive_expect_tx(&kv_full[s], 2 * G::STREAM_BYTES);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          bb::tma_load_2d(sK + s * G::STREAM_BYTES + a * SUB_BYTES, &tm_kv, &kv_full[s], colk + 64 * a, row_base + j * SUB);
+          bb::tma_load_2d(sV + s * G::STREAM_BYTES + a * SUB_BYTES, &tm_kv, &kv_full[s], colv + 64 * a, row_base + j * SUB);
+        }
       }
     }
   } else if (warp == 1) {
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));
-    const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));     // stage 0; stage s: + s * SUB_BYTES / 16
+    const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));     // stage 0; stage s: + s * STREAM_BYTES / 16
     const uint64_t dKm0 = desc_mn0(bb::smem_u32(sK)), dDS0 = desc_k0(bb::smem_u32(sDS));
-    const uint32_t i_s = idesc(64, 0, 0), i_dq = idesc(64, 0, 1);
+    const uint32_t i_s = idesc(64, 0, 0), i_dq = idesc(D, 0, 1);
     bool alive = bb::mbar_wait(q_full, 0, &ctl->abort_flag, p.status);
     // software pipeline: the scores run two sub-blocks ahead of the dQ updates
     for (int j = 0; j < nblk + 2 && alive; ++j) {
@@ -260,11 +290,11 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
         if (!bb::mbar_wait(&s_empty[b], ((j / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
         if (lane == 0) {
-          const uint64_t dK = dK0 + (uint64_t)(s * (SUB_BYTES >> 4)), dV = dV0 + (uint64_t)(s * (SUB_BYTES >> 4));
+          const uint64_t dK = dK0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dV = dV0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            bb::umma_f16(tmem + 64 * b, desc_kmajor(dQ0, k), desc_kmajor(dK, k), i_s, k > 0);
-            bb::umma_f16(tmem + 192 + 64 * b, desc_kmajor(dDO0, k), desc_kmajor(dV, k), i_s, k > 0);
+          for (int k = 0; k < D / 16; ++k) {
+            bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dQ0, k, TILE_BYTES), desc_kmajor_atoms(dK, k, SUB_BYTES), i_s, k > 0);
+            bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dDO0, k, TILE_BYTES), desc_kmajor_atoms(dV, k, SUB_BYTES), i_s, k > 0);
           }
           bb::umma_commit(&s_full[b]);
         }
@@ -275,7 +305,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
         if (!bb::mbar_wait(&ds_full[b2], (jj >> 1) & 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
         if (lane == 0) {
-          const uint64_t dK2 = dKm0 + (uint64_t)(s2 * (SUB_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
+          const uint64_t dK2 = dKm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < 4; ++k) bb::umma_f16(tDQ, desc_kmajor(dDS, k), desc_mnmajor64(dK2, k), i_dq, (jj > 0 || k > 0));
           bb::umma_commit(&ds_empty[b2]);
@@ -302,7 +332,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
     int n = 0;                                               // this group's iteration count
     for (int j = g; j < nblk && alive; j += 2, ++n) {
       const int sb = j % NSB;
-      const uint32_t tS = tmem + 64 * sb, tDP = tmem + 192 + 64 * sb;
+      const uint32_t tS = tmem + 64 * sb, tDP = tmem + 64 * (NSB + sb);
       const bool ok = bb::mbar_wait(&s_full[sb], (j / NSB) & 1, &ctl->abort_flag, p.status);
       if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) { alive = false; break; }
       bb::tc_fence_after_sync();
@@ -340,11 +370,13 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
       if (lane == 0) bb::mbar_arrive(&ds_full[g]);
     }
     const bool fin = alive && bb::mbar_wait(acc_full, 0, &ctl->abort_flag, p.status);
-    if (bb::named_bar_all(3 + g, GROUP_THREADS, fin) && g == 0) {
+    if (bb::named_bar_all(3 + g, GROUP_THREADS, fin) && g < NA) {
+      // group g stores the g-th 64 columns
       bb::tc_fence_after_sync();
       float v[32];
-      ld32(tDQ + lane_addr + hf * 32, v);
-      if (qrow < p.S) store_row32(p.dq + (long long)(row_base + qrow) * p.stride_dqkv + colq + hf * 32, v, p.scale);
+      const int c = 64 * g + hf * 32;
+      ld32(tDQ + lane_addr + c, v);
+      if (qrow < p.S) store_row32(p.dq + (long long)(row_base + qrow) * p.stride_dqkv + colq + c, v, p.scale);
     }
   }
   bb::tc_fence_before_sync();
@@ -352,21 +384,26 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   if (warp == 1) bb::tmem_dealloc(tmem, 512);
 }
 
-constexpr int DQ2_SMEM = 2 * TILE_BYTES + 2 * NST * SUB_BYTES + 2 * TILE_BYTES + (int)sizeof(Ctl) + 1024;
+template <int D> constexpr int dq2_smem() {
+  return 2 * Bwd2<D>::OWN_BYTES + 2 * Bwd2<D>::NST * Bwd2<D>::STREAM_BYTES + 2 * TILE_BYTES + (int)sizeof(Ctl) + 1024;
+}
 
 // ------------------------------------------------------------------ dK, dV (pipelined)
-// smem: K, V [128 x 64] | Q, dO sub-tiles [64 x 64] x 3 stages | P^T, dS^T [128 kv x 64 q] x 2 each
+// smem: K, V [128 x D] | Q, dO sub-tiles [64 x D] x NST stages | P^T, dS^T [128 kv x 64 q] x 2 each
 //       | per-group lse / delta of the sub-block's 64 query columns
-// TMEM: S^T 2 x 64 | dP^T 2 x 64 | dV 64 | dK 64
+// TMEM: S^T NSB x 64 | dP^T NSB x 64 | dV D | dK D
+template <int D>
 __device__ __forceinline__ void
 attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUtensorMap& tm_do64, const TcParams& p, const int bx) {
+  using G = Bwd2<D>;
+  constexpr int NA = G::NA, NST = G::NST, NSB = G::NSB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
-  uint8_t* sV = sK + TILE_BYTES;
-  uint8_t* sQ = sV + TILE_BYTES;               // NST stages x 8 KiB
-  uint8_t* sDO = sQ + NST * SUB_BYTES;         // NST stages x 8 KiB
-  uint8_t* sP = sDO + NST * SUB_BYTES;         // 2 x 16 KiB
+  uint8_t* sV = sK + G::OWN_BYTES;
+  uint8_t* sQ = sV + G::OWN_BYTES;             // NST stages
+  uint8_t* sDO = sQ + NST * G::STREAM_BYTES;   // NST stages
+  uint8_t* sP = sDO + NST * G::STREAM_BYTES;   // 2 x 16 KiB
   uint8_t* sDS = sP + 2 * TILE_BYTES;          // 2 x 16 KiB
   float* s_lse = reinterpret_cast<float*>(sDS + 2 * TILE_BYTES);   // [2][64]
   float* s_delta = s_lse + 2 * SUB;                                // [2][64]
@@ -384,7 +421,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   const int kb = bx, head = blockIdx.y, batch = blockIdx.z;
   const int k0 = kb * TQ;
   const int row_base = batch * p.S;
-  const int colq = head * HD, colk = p.hidden + head * HD, colv = 2 * p.hidden + head * HD;
+  const int colq = head * D, colk = p.hidden + head * D, colv = 2 * p.hidden + head * D;
   const int nq = (p.S + SUB - 1) / SUB;
   const int qstart = p.causal ? (k0 / SUB) : 0;
   const int nblk = nq - qstart;
@@ -404,27 +441,33 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
-  const uint32_t tDV = tmem + 384, tDK = tmem + 448;   // S^T[b] at tmem + 64 b, dP^T[b] at tmem + 192 + 64 b (b < 3)
+  const uint32_t tDV = tmem + G::ACC, tDK = tDV + D;   // S^T[b] at tmem + 64 b, dP^T[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
     if (lane == 0) {
-      bb::mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
-      bb::tma_load_2d(sK, &tm128, kv_full, colk, row_base + k0);
-      bb::tma_load_2d(sV, &tm128, kv_full, colv, row_base + k0);
+      bb::mbar_arrive_expect_tx(kv_full, 2 * G::OWN_BYTES);
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        bb::tma_load_2d(sK + a * TILE_BYTES, &tm128, kv_full, colk + 64 * a, row_base + k0);
+        bb::tma_load_2d(sV + a * TILE_BYTES, &tm128, kv_full, colv + 64 * a, row_base + k0);
+      }
       for (int i = 0; i < nblk; ++i) {
         const int s = i % NST;
         if (!bb::mbar_wait(&q_empty[s], ((i / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
-        bb::mbar_arrive_expect_tx(&q_full[s], 2 * SUB_BYTES);
-        bb::tma_load_2d(sQ + s * SUB_BYTES, &tm64, &q_full[s], colq, row_base + (qstart + i) * SUB);
-        bb::tma_load_2d(sDO + s * SUB_BYTES, &tm_do64, &q_full[s], colq, row_base + (qstart + i) * SUB);
+        bb::mbar_arrive_expect_tx(&q_full[s], 2 * G::STREAM_BYTES);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          bb::tma_load_2d(sQ + s * G::STREAM_BYTES + a * SUB_BYTES, &tm64, &q_full[s], colq + 64 * a, row_base + (qstart + i) * SUB);
+          bb::tma_load_2d(sDO + s * G::STREAM_BYTES + a * SUB_BYTES, &tm_do64, &q_full[s], colq + 64 * a, row_base + (qstart + i) * SUB);
+        }
       }
     }
   } else if (warp == 1) {
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));
-    const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));   // stage 0; stage s: + s * SUB_BYTES / 16
+    const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));   // stage 0; stage s: + s * STREAM_BYTES / 16
     const uint64_t dQm0 = desc_mn0(bb::smem_u32(sQ)), dDOm0 = desc_mn0(bb::smem_u32(sDO));
     const uint64_t dP0 = desc_k0(bb::smem_u32(sP)), dDS0 = desc_k0(bb::smem_u32(sDS));
-    const uint32_t i_s = idesc(64, 0, 0), i_acc = idesc(64, 0, 1);
+    const uint32_t i_s = idesc(64, 0, 0), i_acc = idesc(D, 0, 1);
     bool alive = bb::mbar_wait(kv_full, 0, &ctl->abort_flag, p.status);
     // the score products run two sub-blocks ahead of the dV / dK updates
     for (int i = 0; i < nblk + 2 && alive; ++i) {
@@ -434,11 +477,11 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         if (!bb::mbar_wait(&s_empty[b], ((i / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
         if (lane == 0) {
-          const uint64_t dQ = dQ0 + (uint64_t)(s * (SUB_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (SUB_BYTES >> 4));
+          const uint64_t dQ = dQ0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            bb::umma_f16(tmem + 64 * b, desc_kmajor(dK0, k), desc_kmajor(dQ, k), i_s, k > 0);
-            bb::umma_f16(tmem + 192 + 64 * b, desc_kmajor(dV0, k), desc_kmajor(dDO, k), i_s, k > 0);
+          for (int k = 0; k < D / 16; ++k) {
+            bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dK0, k, TILE_BYTES), desc_kmajor_atoms(dQ, k, SUB_BYTES), i_s, k > 0);
+            bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dV0, k, TILE_BYTES), desc_kmajor_atoms(dDO, k, SUB_BYTES), i_s, k > 0);
           }
           bb::umma_commit(&s_full[b]);
         }
@@ -449,7 +492,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         if (!bb::mbar_wait(&p_full[b2], (ii >> 1) & 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
         if (lane == 0) {
-          const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (SUB_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (SUB_BYTES >> 4));
+          const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4));
           const uint64_t dP = dP0 + (uint64_t)(b2 * (TILE_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -498,7 +541,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         nx_delta = (q < p.S) ? delta_g[q] : 0.f;
       }
       const int sb = i % NSB;
-      const uint32_t tS = tmem + 64 * sb, tDP = tmem + 192 + 64 * sb;
+      const uint32_t tS = tmem + 64 * sb, tDP = tmem + 64 * (NSB + sb);
       const bool ok = bb::mbar_wait(&s_full[sb], (i / NSB) & 1, &ctl->abort_flag, p.status);
       if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) { alive = false; break; }
       bb::tc_fence_after_sync();
@@ -542,12 +585,16 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
     const bool fin = alive && nblk > 0 && bb::mbar_wait(acc_full, 0, &ctl->abort_flag, p.status);
     if (bb::named_bar_all(3 + g, GROUP_THREADS, fin)) {
       bb::tc_fence_after_sync();
-      float v[32];
       // the two groups split the final stores: group 0 writes dV, group 1 writes dK
       const uint32_t src = (g == 0) ? tDV : tDK;
-      ld32(src + lane_addr + hf * 32, v);
       __nv_bfloat16* dst = (g == 0) ? p.dv : p.dk;
-      if (krow < p.S) store_row32(dst + (long long)(row_base + krow) * p.stride_dqkv + colq + hf * 32, v, g == 0 ? 1.f : p.scale);
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        float v[32];
+        const int c = 64 * a + hf * 32;
+        ld32(src + lane_addr + c, v);
+        if (krow < p.S) store_row32(dst + (long long)(row_base + krow) * p.stride_dqkv + colq + c, v, g == 0 ? 1.f : p.scale);
+      }
     }
   }
   bb::tc_fence_before_sync();
@@ -555,18 +602,22 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   if (warp == 1) bb::tmem_dealloc(tmem, 512);
 }
 
-constexpr int DKV2_SMEM = 2 * TILE_BYTES + 2 * NST * SUB_BYTES + 4 * TILE_BYTES + 4 * SUB * (int)sizeof(float) + (int)sizeof(Ctl) + 1024;
+template <int D> constexpr int dkv2_smem() {
+  return 2 * Bwd2<D>::OWN_BYTES + 2 * Bwd2<D>::NST * Bwd2<D>::STREAM_BYTES + 4 * TILE_BYTES + 4 * SUB * (int)sizeof(float) + (int)sizeof(Ctl) + 1024;
+}
 
 // Both backward roles in one launch: of the 2 * nbx CTAs of a (batch, head), the first nbx own a
 // key tile (dK, dV) and the rest a query tile (dQ).  The two roles are independent, so the tail
 // of one fills with CTAs of the other instead of leaving SMs idle between two launches.
-constexpr int BWD2_SMEM = DKV2_SMEM > DQ2_SMEM ? DKV2_SMEM : DQ2_SMEM;
+template <int D> constexpr int bwd2_smem() { return dkv2_smem<D>() > dq2_smem<D>() ? dkv2_smem<D>() : dq2_smem<D>(); }
+static_assert(bwd2_smem<64>() <= 232448 && bwd2_smem<128>() <= 232448, "227 KiB of shared memory per CTA");
+template <int D>
 __global__ void __launch_bounds__(NT2, 1)
 attn_tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_constant__ CUtensorMap tm64,
                     const __grid_constant__ CUtensorMap tm_do128, const __grid_constant__ CUtensorMap tm_do64, const TcParams p) {
   const int nbx = gridDim.x >> 1;
-  if ((int)blockIdx.x < nbx) attn_tc_dkv2_body(tm128, tm64, tm_do64, p, blockIdx.x);
-  else attn_tc_dq2_body(tm128, tm64, tm_do128, p, blockIdx.x - nbx, nbx);
+  if ((int)blockIdx.x < nbx) attn_tc_dkv2_body<D>(tm128, tm64, tm_do64, p, blockIdx.x);
+  else attn_tc_dq2_body<D>(tm128, tm64, tm_do128, p, blockIdx.x - nbx, nbx);
 }
 
 // ------------------------------------------------------------------ fused backward: dK, dV and dQ from one pass
@@ -1201,37 +1252,49 @@ int bb_attention_tc_fwd(const void* qkv_q, void* out, float* lse, int B, int H, 
   return BB_ERR_UNSUPPORTED;
 }
 
+namespace {
+// the two-role kernel (see attn_tc_bwd2_kernel): delta pre-pass, then dK / dV and dQ tiles in one launch
+template <int D>
+int launch_bwd2(const CUtensorMap& tm_qkv, const CUtensorMap& tm_qkv64, const CUtensorMap& tm_do, const CUtensorMap& tm_do64,
+                const void* out, const void* d_out, const TcParams& p, int dgrid, cudaStream_t stream) {
+  BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd2_kernel<D>, bwd2_smem<D>())) return rc; });
+  attn_tc_delta_kernel<D><<<dgrid, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
+  dim3 grid(2 * ((p.S + TQ - 1) / TQ), p.H, p.B);
+  attn_tc_bwd2_kernel<D><<<grid, NT2, bwd2_smem<D>(), stream>>>(tm_qkv, tm_qkv64, tm_do, tm_do64, p);
+  BB_CUDA_CHECK(cudaGetLastError());
+  return BB_OK;
+}
+}  // namespace
+
 int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, const float* lse, void* dq, void* dk, void* dv,
-                        float* delta, float* dq_acc, int B, int H, int S, long long stride_qkv, long long stride_o,
+                        float* delta, float* dq_acc, int B, int H, int S, int D, long long stride_qkv, long long stride_o,
                         long long stride_dqkv, int causal, float scale, cudaStream_t stream) {
+  if (D != 64 && D != 128) return BB_ERR_UNSUPPORTED;
   if (int rc = bbhost::bind_context()) return rc;
-  CUtensorMap tm_qkv, tm_do;
+  // boxes of 64 columns: [128 rows] for the CTA's own tiles, [64 rows] for the streamed sub-tiles
+  CUtensorMap tm_qkv, tm_do, tm_qkv64, tm_do64;
   const long long T = (long long)B * S;
-  if (int rc = bbhost::encode_2d(&tm_qkv, qkv_q, T, 3LL * H * HD, stride_qkv, HD, TQ)) return rc;
-  if (int rc = bbhost::encode_2d(&tm_do, d_out, T, (long long)H * HD, stride_o, HD, TQ)) return rc;
+  if (int rc = bbhost::encode_2d(&tm_qkv, qkv_q, T, 3LL * H * D, stride_qkv, 64, TQ)) return rc;
+  if (int rc = bbhost::encode_2d(&tm_do, d_out, T, (long long)H * D, stride_o, 64, TQ)) return rc;
+  if (int rc = bbhost::encode_2d(&tm_qkv64, qkv_q, T, 3LL * H * D, stride_qkv, 64, SUB)) return rc;
+  if (int rc = bbhost::encode_2d(&tm_do64, d_out, T, (long long)H * D, stride_o, 64, SUB)) return rc;
   TcParams p = {};
   p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.lse = const_cast<float*>(lse); p.delta = delta; p.stride_o = stride_o; p.stride_dqkv = stride_dqkv;
-  p.B = B; p.H = H; p.S = S; p.hidden = H * HD; p.causal = causal; p.scale = scale; p.status = bb_device_status_word();
-  CUtensorMap tm_qkv64, tm_do64;
-  if (int rc = bbhost::encode_2d(&tm_qkv64, qkv_q, T, 3LL * H * HD, stride_qkv, HD, SUB)) return rc;
-  if (int rc = bbhost::encode_2d(&tm_do64, d_out, T, (long long)H * HD, stride_o, HD, SUB)) return rc;
+  p.B = B; p.H = H; p.S = S; p.hidden = H * D; p.causal = causal; p.scale = scale; p.status = bb_device_status_word();
+  const long long chunks = T * H * (D / 8);
+  long long dgrid = (chunks + 511) / 512, cap = (long long)bb_num_sms() * 8;
+  if (dgrid > cap) dgrid = cap;
+  // Head dimension 128: the two-role kernel.  The fused kernel's tensor-memory map (scores, dP, dV, dK and two dQ
+  // tiles) would need 768 columns there.
+  if (D == 128) return launch_bwd2<128>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
   // BB_ATTENTION_BWD=split in the environment selects the two-role kernel (dK/dV and dQ computed by
   // different CTAs, every sum in a fixed order); the default is the fused kernel
   static const bool split = [] { const char* e = getenv("BB_ATTENTION_BWD"); return e && e[0] == 's'; }();
-  const long long chunks = T * H * 8;
-  long long dgrid = (chunks + 511) / 512, cap = (long long)bb_num_sms() * 8;
-  if (split) {
-    BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd2_kernel, BWD2_SMEM)) return rc; });
-    attn_tc_delta_kernel<<<(int)(dgrid < cap ? dgrid : cap), 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
-    dim3 grid(2 * ((S + TQ - 1) / TQ), H, B);
-    attn_tc_bwd2_kernel<<<grid, NT2, BWD2_SMEM, stream>>>(tm_qkv, tm_qkv64, tm_do, tm_do64, p);
-    BB_CUDA_CHECK(cudaGetLastError());
-    return BB_OK;
-  }
+  if (split) return launch_bwd2<64>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
   p.dq_acc = dq_acc;
   BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd3_kernel, BWD3_SMEM)) return rc; });
-  attn_tc_delta_kernel<<<(int)(dgrid < cap ? dgrid : cap), 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
+  attn_tc_delta_kernel<64><<<(int)dgrid, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
   dim3 grid((S + TQ - 1) / TQ, H, B);
   // the accumulator as [B * H * S rows, 64] fp32; a reduction moves [128 rows x 32 columns]
   CUtensorMap tm_acc;

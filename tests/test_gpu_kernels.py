@@ -441,3 +441,28 @@ def test_ping_counter_may_run_ahead_of_the_receiver(L):
 def test_status_word_is_clean(L):
     torch.cuda.synchronize()
     assert L.read_status() == 0
+
+
+# Head dimension 128 backward on the tensor cores, at the edges of its 128-row tiles and 64-row sub-blocks: one row, one
+# short of / one past a sub-block and a tile, several batches (a partial tile reads the next batch's rows, masked).
+# Tolerance: bf16 P and dS carry 2^-9 relative error each, sums are fp32 - the 2e-2 of `close` is an order above.
+@pytest.mark.parametrize("B,H,S,causal", [(2, 1, 1, True), (2, 2, 63, False), (2, 2, 65, True), (3, 1, 127, True),
+                                          (2, 3, 129, False), (2, 1, 257, True), (1, 2, 385, False)])
+def test_attention_backward_head_dim_128_tile_edges(L, B, H, S, causal):
+    D = 128
+    torch.manual_seed(21)
+    qkv = torch.randn(B * S, 3 * H * D, device="cuda").bfloat16()
+    out = torch.empty(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(B, H, S, device="cuda")
+    L.attention_fwd(qkv, out, lse, B, H, S, D, causal)
+    qf = qkv.float().requires_grad_(True)
+    ref = _attn_ref(qf, B, H, S, D, causal)
+    do = torch.randn_like(out)
+    ref.backward(do.float())
+    dqkv = torch.full_like(qkv, float("nan"))
+    L.attention_bwd(qkv, out, do, lse, dqkv, B, H, S, D, causal)
+    again = torch.full_like(qkv, float("nan"))
+    L.attention_bwd(qkv, out, do, lse, again, B, H, S, D, causal)
+    close(dqkv, qf.grad)
+    assert torch.equal(dqkv, again)                     # every sum in a fixed order
+    assert L.read_status() == 0

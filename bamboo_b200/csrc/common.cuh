@@ -43,6 +43,26 @@ int bb_current_device();
     }                                                     \
   } while (0)
 
+// One product of a k x k convolution whose patch matrix is never stored: the GEMM's producer gathers the
+// patches with im2col TMA loads (gemm_tcgen05.cu).  `x` is the NHWC tensor the patches come from.
+//   BB_CONV_FWD    D[P, Cout] = patches(x) * W^T                   x = input, channels C = Cin
+//   BB_CONV_WGRAD  D[Cout, k*k*C] += dy^T * patches(x)             x = input, other = dy [P, Cout]
+//   BB_CONV_DGRAD  D[P, C_in] = patches(x) * (W turned by 180 deg) x = dy, stride 1, channels C = Cout
+enum { BB_CONV_FWD = 0, BB_CONV_WGRAD = 1, BB_CONV_DGRAD = 2 };
+struct bb_conv_gemm_args {
+  int mode;
+  const void* x; int N, H, W, C;        // patch source
+  int k, stride, pad, Ho, Wo;           // window over it; N * Ho * Wo patches
+  const void* other;                    // weights [Cout, k*k*Cin], or dy for BB_CONV_WGRAD
+  int other_channels;                   // Cout (FWD, WGRAD) or Cin (DGRAD)
+  void* D;
+  int max_ctas;
+};
+// True when the im2col loads can express the convolution's patches (64-channel blocks, window within the
+// tensor map's limits).
+bool bb_conv_gemm_supported(int C, int k, int stride, int pad);
+int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream);
+
 namespace bb {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -147,6 +167,17 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       : : "r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
+}
+// im2col load of an NHWC tensor: consecutive output pixels from input position (c, w, h, n) on (the first
+// tap's corner of the first pixel's window), all shifted by the tap's (off_w, off_h).  The tensor map holds
+// the window's range, the stride and the zero fill outside the image.
+__device__ __forceinline__ void tma_load_im2col(void* smem_dst, const void* tmap, uint64_t* bar, int c, int w, int h, int n,
+                                                uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], "
+      "{%7, %8};"
+      : : "r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
+      : "memory");
 }
 // shared -> global tile store / fp32 add-reduction through a tensor map (clips at the edges)
 __device__ __forceinline__ void tma_store_2d(const void* tmap, const void* smem_src, int c0, int c1) {
@@ -283,6 +314,14 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tma
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       : : "r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int c, int w,
+                                                     int h, int n, uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+      : : "r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)

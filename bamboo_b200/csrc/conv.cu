@@ -4,7 +4,9 @@
 // global average pooling.  All of these are HBM-bound: 16-byte vectors over the channel
 // dimension, consecutive threads on consecutive channel chunks of a pixel, fp32 arithmetic.
 // A convolution itself is the library's GEMM: output pixels x (taps * input channels) times the
-// [Cout, k, k, Cin] weight matrix.
+// [Cout, k, k, Cin] weight matrix.  With channels in blocks of 64 the GEMM gathers the patches itself
+// (im2col TMA loads, bb_conv_gemm); the patch kernels below serve the other channel counts (the stem, narrow
+// networks) and the input gradient of strided convolutions.
 #include "common.cuh"
 #include "bamboo_b200.h"
 
@@ -566,6 +568,12 @@ struct ConvSizes {
   int Ho, Wo;
   long long P, K;
   bool direct;                       // 1 x 1 / stride 1: the activation tensor is the patch matrix
+  // Patches gathered by the GEMM's own loads (bb_conv_gemm) instead of a stored patch matrix: needs 64-channel blocks.
+  // Forward and weight gradient read windows of x, the input gradient windows of dy; with a stride the latter would
+  // need dy spread out with zeros, so it keeps the patch-gradient matrix and its adjoint gather.
+  // A 3 x 3 layer's patch matrix is nine times its input, written and read once per product: 128 channels, 32 images
+  // of 28 x 28, forward + backward 181 -> 89 us of device time (gathers 80 us, GEMMs 63 -> 55 us) without it.
+  bool implicit_x, implicit_dx;
   long long col_bytes, dy_bytes, dcol_bytes, bn_bytes;
 };
 
@@ -579,11 +587,13 @@ bool conv_sizes(const bb_conv_desc* d, ConvSizes* s) {
   s->P = (long long)d->N * s->Ho * s->Wo;
   s->K = (long long)d->k * d->k * d->Cin;
   s->direct = d->k == 1 && d->stride == 1;
+  s->implicit_x = !s->direct && bb_conv_gemm_supported(d->Cin, d->k, d->stride, d->pad);
+  s->implicit_dx = !s->direct && d->stride == 1 && d->pad < d->k && bb_conv_gemm_supported(d->Cout, d->k, 1, d->k - 1 - d->pad);
   s->bn_bytes = bb_bn_workspace_bytes(s->P, d->Cout);
   if (s->bn_bytes < 0) return false;
-  s->col_bytes = s->direct ? 0 : up256(s->P * s->K * 2);
+  s->col_bytes = s->direct || s->implicit_x ? 0 : up256(s->P * s->K * 2);
   s->dy_bytes = up256(s->P * d->Cout * 2);
-  s->dcol_bytes = s->direct ? 0 : up256(s->P * s->K * 2);
+  s->dcol_bytes = s->direct || s->implicit_dx ? 0 : up256(s->P * s->K * 2);
   s->bn_bytes = up256(s->bn_bytes);
   return true;
 }
@@ -594,6 +604,18 @@ int conv_gemm(const bb_conv_desc* d, int M, int N, int K, const void* A, long lo
   g.M = M; g.N = N; g.K = K; g.A = A; g.lda = lda; g.a_mn_major = a_mn; g.B = B; g.ldb = ldb; g.b_mn_major = b_mn;
   g.D = D; g.ldd = ldd; g.epilogue = epi; g.max_ctas = d->max_ctas;
   return bb_gemm_bf16(&g, stream);
+}
+
+// products over patches of x [N, H, W, Cin]
+int conv_implicit(const bb_conv_desc* d, const ConvSizes& s, int mode, const void* x, const void* other, void* D, void* stream) {
+  const bb_conv_gemm_args a = {mode, x, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, other, d->Cout, D, d->max_ctas};
+  return bb_conv_gemm(&a, stream);
+}
+// dx: a stride-1 convolution over dy [N, Ho, Wo, Cout] with the window turned by 180 degrees and the complementary padding
+int conv_implicit_dx(const bb_conv_desc* d, const ConvSizes& s, const void* dy, void* dx, void* stream) {
+  const bb_conv_gemm_args a = {BB_CONV_DGRAD, dy, d->N, s.Ho, s.Wo, d->Cout, d->k, 1, d->k - 1 - d->pad, d->H, d->W,
+                               d->w, d->Cin, dx, d->max_ctas};
+  return bb_conv_gemm(&a, stream);
 }
 
 #define BB_TRY(expr) do { int _rc = (expr); if (_rc != BB_OK) return _rc; } while (0)
@@ -615,12 +637,16 @@ extern "C" int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* 
     return BB_ERR_INVALID_ARG;
   }
   uint8_t* sc = static_cast<uint8_t*>(scratch);
-  const void* col = x;
-  if (!s.direct) {
-    BB_TRY(bb_im2col_nhwc(x, sc, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
-    col = sc;
+  if (s.implicit_x) {
+    BB_TRY(conv_implicit(d, s, BB_CONV_FWD, x, d->w, y, stream));
+  } else {
+    const void* col = x;
+    if (!s.direct) {
+      BB_TRY(bb_im2col_nhwc(x, sc, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
+      col = sc;
+    }
+    BB_TRY(conv_gemm(d, (int)s.P, d->Cout, (int)s.K, col, s.K, 0, d->w, s.K, 0, y, d->Cout, BB_EPI_STORE, stream));
   }
-  BB_TRY(conv_gemm(d, (int)s.P, d->Cout, (int)s.K, col, s.K, 0, d->w, s.K, 0, y, d->Cout, BB_EPI_STORE, stream));
   BB_TRY(bb_bn_stats(y, s.P, d->Cout, d->eps, mean, rstd, sc + s.col_bytes, s.bn_bytes, stream));
   BB_TRY(bb_bn_apply(y, mean, rstd, d->gamma, d->beta, residual, z, s.P, d->Cout, d->relu, stream));
   return BB_OK;
@@ -641,18 +667,26 @@ extern "C" int bb_conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* 
   uint8_t* dcolbuf = colbuf + s.col_bytes;
   uint8_t* bnws = dcolbuf + (dx ? s.dcol_bytes : 0);
   BB_TRY(bb_bn_bwd(dz, z, y, mean, rstd, d->gamma, dy, dres, d->g_gamma, d->g_beta, s.P, d->Cout, d->relu, bnws, s.bn_bytes, stream));
-  const void* col = x;
-  if (!s.direct) {
-    BB_TRY(bb_im2col_nhwc(x, colbuf, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
-    col = colbuf;
-  }
   // dW[Cout, K] += dy^T patches
-  BB_TRY(conv_gemm(d, d->Cout, (int)s.K, (int)s.P, dy, d->Cout, 1, col, s.K, 1, d->g_w, s.K, BB_EPI_ACCUM_F32, stream));
+  if (s.implicit_x) {
+    BB_TRY(conv_implicit(d, s, BB_CONV_WGRAD, x, dy, d->g_w, stream));
+  } else {
+    const void* col = x;
+    if (!s.direct) {
+      BB_TRY(bb_im2col_nhwc(x, colbuf, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
+      col = colbuf;
+    }
+    BB_TRY(conv_gemm(d, d->Cout, (int)s.K, (int)s.P, dy, d->Cout, 1, col, s.K, 1, d->g_w, s.K, BB_EPI_ACCUM_F32, stream));
+  }
   if (dx) {
-    void* dcol = s.direct ? dx : (void*)dcolbuf;
-    BB_TRY(conv_gemm(d, (int)s.P, (int)s.K, d->Cout, dy, d->Cout, 0, d->w, s.K, 1, dcol, s.K, BB_EPI_STORE, stream));
-    if (!s.direct)
-      BB_TRY(bb_col2im_nhwc(dcol, dx, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
+    if (s.implicit_dx) {
+      BB_TRY(conv_implicit_dx(d, s, dy, dx, stream));
+    } else {
+      void* dcol = s.direct ? dx : (void*)dcolbuf;
+      BB_TRY(conv_gemm(d, (int)s.P, (int)s.K, d->Cout, dy, d->Cout, 0, d->w, s.K, 1, dcol, s.K, BB_EPI_STORE, stream));
+      if (!s.direct)
+        BB_TRY(bb_col2im_nhwc(dcol, dx, d->N, d->H, d->W, d->Cin, d->k, d->stride, d->pad, s.Ho, s.Wo, s.K, stream));
+    }
   }
   return BB_OK;
 }

@@ -68,6 +68,24 @@ struct GemmParams {
   int* status;
 };
 
+// Geometry of a convolution product (template parameter CONV): which operand the im2col loads gather.
+struct ConvParams {
+  int mode;                   // BB_CONV_FWD / BB_CONV_WGRAD / BB_CONV_DGRAD
+  int k, stride, pad;
+  int cblocks;                // 64-channel blocks per tap of the patch source
+  int wcols;                  // columns of one tap in the weight matrix (Cin)
+  unsigned Wo, Ho;            // windows per image row / rows of windows per image
+  unsigned long long magic_w, magic_h;
+};
+struct NoConv {};
+template <bool CONV> struct ConvArg { typedef NoConv type; };
+template <> struct ConvArg<true> { typedef ConvParams type; };
+
+// n / d for n < 2^32 with magic = floor(2^64 / d) + 1 (0 for d = 1): the error n * d / 2^64 stays below 1
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
+  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
+}
+
 __device__ __forceinline__ void unpack8(const uint4& q, float* f) {
   f[0] = bb::bf16_lo(q.x); f[1] = bb::bf16_hi(q.x); f[2] = bb::bf16_lo(q.y); f[3] = bb::bf16_hi(q.y);
   f[4] = bb::bf16_lo(q.z); f[5] = bb::bf16_hi(q.z); f[6] = bb::bf16_lo(q.w); f[7] = bb::bf16_hi(q.w);
@@ -243,10 +261,10 @@ __device__ __forceinline__ void add_bias(const GemmParams& p, int n0, float* v) 
   }
 }
 
-template <int BN, bool PAIR, int EW>
+template <int BN, bool PAIR, int EW, bool CONV>
 __global__ void __launch_bounds__(num_threads(EW), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const GemmParams p) {
+                         const GemmParams p, const typename ConvArg<CONV>::type cv) {
   using C = Cfg<BN, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   // 128-byte swizzle atoms need 1024-byte aligned stage buffers
@@ -329,43 +347,109 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         const int m0 = mi * C::TILE_M + (int)rank * BM;                    // this CTA's A rows
         const int n0 = ni * BN + (int)rank * C::B_ROWS;                    // this CTA's share of B (pairs: half)
         const int kb0 = ks * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) { alive = false; break; }
-          uint8_t* a = sA + s * A_STAGE_BYTES;
-          uint8_t* b = sB + s * C::B_STAGE_BYTES;
-          const int k0 = kb * BK;
-          if constexpr (PAIR) {
-            // both CTAs' copies complete on rank 0's barrier, where the MMA issuer waits
-            if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
-            const uint32_t fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), 0);
-            if (!p.a_mn) {
-              bb::tma_load_2d_pair(a, &tmA, fb, k0, m0);
-            } else {
+        if constexpr (CONV) {
+          // Patches of a convolution: a stage's patch tile is 64 channels of one tap for a run of windows, one
+          // im2col load (the hardware walks the windows, applies the stride and fills with zeros outside the
+          // image).  FWD / DGRAD gather A (windows = output rows, k-blocks run over taps x channel blocks),
+          // WGRAD gathers B (windows = the reduction, columns = taps x channels).
+          auto window = [&](unsigned px, int& w, int& h, int& n) {
+            const unsigned row = fast_div(px, cv.magic_w), img = fast_div(row, cv.magic_h);
+            w = (int)(px - row * cv.Wo) * cv.stride - cv.pad;
+            h = (int)(row - img * cv.Ho) * cv.stride - cv.pad;
+            n = (int)img;
+          };
+          auto patches = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int c, int w, int h, int n, int ow, int oh) {
+            if constexpr (PAIR) bb::tma_load_im2col_pair(dst, tm, fb, c, w, h, n, (uint16_t)ow, (uint16_t)oh);
+            else bb::tma_load_im2col(dst, tm, &full_bar[s], c, w, h, n, (uint16_t)ow, (uint16_t)oh);
+          };
+          auto plain = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int x, int y) {
+            if constexpr (PAIR) bb::tma_load_2d_pair(dst, tm, fb, x, y);
+            else bb::tma_load_2d(dst, tm, &full_bar[s], x, y);
+          };
+          constexpr int BJ = C::B_ROWS / 64;
+          int w, h, n;
+          int cj[BJ], rj[BJ], sj[BJ];          // WGRAD: channel and tap of each 64-column block of B
+          if (cv.mode == BB_CONV_WGRAD) {
 #pragma unroll
-              for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d_pair(a + j * 8192, &tmA, fb, m0 + 64 * j, k0);
-            }
-            if (!p.b_mn) {
-              bb::tma_load_2d_pair(b, &tmB, fb, k0, n0);
-            } else {
-#pragma unroll
-              for (int j = 0; j < C::B_ROWS / 64; ++j) bb::tma_load_2d_pair(b + j * 8192, &tmB, fb, n0 + 64 * j, k0);
+            for (int j = 0; j < BJ; ++j) {
+              const int cb = min((n0 >> 6) + j, cv.k * cv.k * cv.cblocks - 1);     // past the last tap: never stored
+              const int tap = cb / cv.cblocks;
+              cj[j] = (cb - tap * cv.cblocks) * 64; rj[j] = tap / cv.k; sj[j] = tap - rj[j] * cv.k;
             }
           } else {
-            bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-            if (!p.a_mn) {
-              bb::tma_load_2d(a, &tmA, &full_bar[s], k0, m0);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d(a + j * 8192, &tmA, &full_bar[s], m0 + 64 * j, k0);
-            }
-            if (!p.b_mn) {
-              bb::tma_load_2d(b, &tmB, &full_bar[s], k0, n0);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j) bb::tma_load_2d(b + j * 8192, &tmB, &full_bar[s], n0 + 64 * j, k0);
-            }
+            window((unsigned)m0, w, h, n);
           }
-          if (++s == C::STAGES) { s = 0; phase ^= 1; }
+          int tap = kb0 / cv.cblocks, cb = kb0 - tap * cv.cblocks;
+          int tr = tap / cv.k, ts = tap - tr * cv.k;
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) { alive = false; break; }
+            uint8_t* a = sA + s * A_STAGE_BYTES;
+            uint8_t* b = sB + s * C::B_STAGE_BYTES;
+            uint32_t fb = 0;
+            if constexpr (PAIR) {
+              if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+              fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), 0);
+            } else {
+              bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
+            }
+            if (cv.mode == BB_CONV_WGRAD) {
+              window((unsigned)kb * BK, w, h, n);
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j) plain(a + j * 8192, &tmA, fb, m0 + 64 * j, kb * BK);
+#pragma unroll
+              for (int j = 0; j < BJ; ++j) patches(b + j * 8192, &tmB, fb, cj[j], w, h, n, sj[j], rj[j]);
+            } else {
+              patches(a, &tmA, fb, cb * 64, w, h, n, ts, tr);
+              if (cv.mode == BB_CONV_FWD) {
+                plain(b, &tmB, fb, kb * BK, n0);
+              } else {
+                const int col = ((cv.k - 1 - tr) * cv.k + (cv.k - 1 - ts)) * cv.wcols + n0;   // the tap turned by 180 degrees
+#pragma unroll
+                for (int j = 0; j < BJ; ++j) plain(b + j * 8192, &tmB, fb, col + 64 * j, cb * 64);
+              }
+              if (++cb == cv.cblocks) { cb = 0; if (++ts == cv.k) { ts = 0; ++tr; } }
+            }
+            if (++s == C::STAGES) { s = 0; phase ^= 1; }
+          }
+        } else {
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) { alive = false; break; }
+            uint8_t* a = sA + s * A_STAGE_BYTES;
+            uint8_t* b = sB + s * C::B_STAGE_BYTES;
+            const int k0 = kb * BK;
+            if constexpr (PAIR) {
+              // both CTAs' copies complete on rank 0's barrier, where the MMA issuer waits
+              if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+              const uint32_t fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), 0);
+              if (!p.a_mn) {
+                bb::tma_load_2d_pair(a, &tmA, fb, k0, m0);
+              } else {
+#pragma unroll
+                for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d_pair(a + j * 8192, &tmA, fb, m0 + 64 * j, k0);
+              }
+              if (!p.b_mn) {
+                bb::tma_load_2d_pair(b, &tmB, fb, k0, n0);
+              } else {
+#pragma unroll
+                for (int j = 0; j < C::B_ROWS / 64; ++j) bb::tma_load_2d_pair(b + j * 8192, &tmB, fb, n0 + 64 * j, k0);
+              }
+            } else {
+              bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
+              if (!p.a_mn) {
+                bb::tma_load_2d(a, &tmA, &full_bar[s], k0, m0);
+              } else {
+#pragma unroll
+                for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d(a + j * 8192, &tmA, &full_bar[s], m0 + 64 * j, k0);
+              }
+              if (!p.b_mn) {
+                bb::tma_load_2d(b, &tmB, &full_bar[s], k0, n0);
+              } else {
+#pragma unroll
+                for (int j = 0; j < BN / 64; ++j) bb::tma_load_2d(b + j * 8192, &tmB, &full_bar[s], n0 + 64 * j, k0);
+              }
+            }
+            if (++s == C::STAGES) { s = 0; phase ^= 1; }
+          }
         }
       };
       if (rank == 0) {
@@ -699,17 +783,29 @@ TicketTable* ticket_table() {
   return t;
 }
 
-template <int BN, bool PAIR, int EW>
-int launch(const bb_gemm_desc* g, cudaStream_t stream) {
+// `cv`: convolution product (CONV); the descriptor then holds the sizes and the operand that is no patch matrix
+template <int BN, bool PAIR, int EW, bool CONV>
+int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* cv = nullptr) {
   using C = Cfg<BN, PAIR>;
   CUtensorMap tmA, tmB;
   int rc;
-  if (!g->a_mn_major) rc = encode_2d(&tmA, g->A, g->M, g->K, g->lda, BK, BM);
+  if (CONV && cv->mode != BB_CONV_WGRAD) rc = bbhost::encode_im2col(&tmA, cv->x, cv->N, cv->H, cv->W, cv->C, cv->k, cv->stride, cv->pad, BM);
+  else if (!g->a_mn_major) rc = encode_2d(&tmA, g->A, g->M, g->K, g->lda, BK, BM);
   else rc = encode_2d(&tmA, g->A, g->K, g->M, g->lda, 64, BK);
   if (rc) return rc;
-  if (!g->b_mn_major) rc = encode_2d(&tmB, g->B, g->N, g->K, g->ldb, BK, C::B_ROWS);
+  if (CONV && cv->mode == BB_CONV_WGRAD) rc = bbhost::encode_im2col(&tmB, cv->x, cv->N, cv->H, cv->W, cv->C, cv->k, cv->stride, cv->pad, BK);
+  else if (CONV && cv->mode == BB_CONV_DGRAD) rc = encode_2d(&tmB, g->B, cv->C, g->ldb, g->ldb, 64, BK);
+  else if (!g->b_mn_major) rc = encode_2d(&tmB, g->B, g->N, g->K, g->ldb, BK, C::B_ROWS);
   else rc = encode_2d(&tmB, g->B, g->K, g->N, g->ldb, 64, BK);
   if (rc) return rc;
+  typename ConvArg<CONV>::type cp;
+  if constexpr (CONV) {
+    cp.mode = cv->mode; cp.k = cv->k; cp.stride = cv->stride; cp.pad = cv->pad; cp.cblocks = cv->C / 64;
+    cp.wcols = cv->mode == BB_CONV_DGRAD ? cv->other_channels : cv->C;
+    cp.Wo = cv->Wo; cp.Ho = cv->Ho;
+    cp.magic_w = cv->Wo == 1 ? 0 : ~0ull / (unsigned long long)cv->Wo + 1;
+    cp.magic_h = cv->Ho == 1 ? 0 : ~0ull / (unsigned long long)cv->Ho + 1;
+  }
   GemmParams p;
   p.M = g->M; p.N = g->N; p.K = g->K; p.a_mn = g->a_mn_major; p.b_mn = g->b_mn_major; p.epi = g->epilogue;
   p.D = g->D; p.D2 = g->D2; p.bias = g->bias; p.aux = g->aux; p.ldd = g->ldd; p.ld_aux = g->ld_aux ? g->ld_aux : g->ldd;
@@ -742,7 +838,7 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream) {
   if (ksplit < 1) ksplit = 1;
   p.kb_per_split = (total_kb + ksplit - 1) / ksplit;
   p.ksplit = (total_kb + p.kb_per_split - 1) / p.kb_per_split;   // no empty splits
-  BB_ONCE_PER_DEVICE(BB_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, PAIR, EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES)));
+  BB_ONCE_PER_DEVICE(BB_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, PAIR, EW, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES)));
   const int tiles = mn_tiles * p.ksplit;
   int workers = workers_max;
   if (g->max_ctas > 0 && g->max_ctas / (PAIR ? 2 : 1) < workers) workers = g->max_ctas / (PAIR ? 2 : 1);
@@ -771,14 +867,14 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<BN, true, EW>, tmA, tmB, p);
+    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<BN, true, EW, CONV>, tmA, tmB, p, cp);
     if (le != cudaSuccess) {
       if (tt) tt->base[slot] -= (unsigned)tiles;     // nothing ran: the counter keeps its value
       bb_set_last_error("gemm_bf16_tcgen05_kernel (pair) launch", le);
       return BB_ERR_CUDA;
     }
   } else {
-    gemm_bf16_tcgen05_kernel<BN, false, EW><<<workers, num_threads(EW), C::SMEM_BYTES, stream>>>(tmA, tmB, p);
+    gemm_bf16_tcgen05_kernel<BN, false, EW, CONV><<<workers, num_threads(EW), C::SMEM_BYTES, stream>>>(tmA, tmB, p, cp);
   }
   {
     cudaError_t le = cudaGetLastError();
@@ -789,6 +885,28 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream) {
     }
   }
   return BB_OK;
+}
+
+// Tile width, and whether CTA pairs / sixteen epilogue warps are used.
+int choose_tile(const bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
+  const int e = g->epilogue;
+  // CTA pairs (256 x 256 per pair) pay off on long reductions and on long runs of tiles per
+  // CTA; short problems are quicker to start and drain as single CTAs (measured on B200:
+  // K >= 3072 or >= 40 tiles per CTA 2-6 % faster as pairs, K = 1024 with <= 7 tiles 4-8 % slower)
+  const long long tiles_single = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
+  *pair_out = g->cta_pair > 0 ||
+                    (g->cta_pair == 0 && g->tile_n == 0 && g->M > BM && g->N > 128 &&
+                     (g->K >= 2048 || tiles_single >= 16LL * bb_num_sms()));
+  // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant)
+  *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048);
+  int bn = g->tile_n;
+  if (bn == 0) {
+    // 256-wide tiles halve the A re-reads; use them when they still fill the machine
+    const long long tiles256 = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
+    // the add-reduction epilogue can split K to fill the machine, so it always takes wide tiles
+    bn = (g->N > 128 && (tiles256 >= bb_num_sms() || e == BB_EPI_ACCUM_F32)) ? 256 : 128;
+  }
+  return bn;
 }
 
 }  // namespace
@@ -820,25 +938,45 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   // cuTensorMapEncodeTiled is a driver call and needs a context bound to the calling thread;
   // a thread that has only ever set its device (autograd worker threads) has none yet.
   if (int rc = bbhost::bind_context()) return rc;
-  // CTA pairs (256 x 256 per pair) pay off on long reductions and on long runs of tiles per
-  // CTA; short problems are quicker to start and drain as single CTAs (measured on B200:
-  // K >= 3072 or >= 40 tiles per CTA 2-6 % faster as pairs, K = 1024 with <= 7 tiles 4-8 % slower)
-  const long long tiles_single = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
-  const bool pair = g->cta_pair > 0 ||
-                    (g->cta_pair == 0 && g->tile_n == 0 && g->M > BM && g->N > 128 &&
-                     (g->K >= 2048 || tiles_single >= 16LL * bb_num_sms()));
-  // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant)
-  const bool wide_epi = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048);
-  if (pair) return wide_epi ? launch<256, true, 4>(g, s) : launch<256, true, 2>(g, s);
-  int bn = g->tile_n;
-  if (bn == 0) {
-    // 256-wide tiles halve the A re-reads; use them when they still fill the machine
-    const long long tiles256 = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
-    // the add-reduction epilogue can split K to fill the machine, so it always takes wide tiles
-    bn = (g->N > 128 && (tiles256 >= bb_num_sms() || e == BB_EPI_ACCUM_F32)) ? 256 : 128;
-  }
-  if (bn == 256) return wide_epi ? launch<256, false, 4>(g, s) : launch<256, false, 2>(g, s);
-  if (bn == 128) return wide_epi ? launch<128, false, 4>(g, s) : launch<128, false, 2>(g, s);
+  bool pair, wide_epi;
+  const int bn = choose_tile(g, &pair, &wide_epi);
+  if (pair) return wide_epi ? launch<256, true, 4, false>(g, s) : launch<256, true, 2, false>(g, s);
+  if (bn == 256) return wide_epi ? launch<256, false, 4, false>(g, s) : launch<256, false, 2, false>(g, s);
+  if (bn == 128) return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);
   bb_set_last_error_msg("bb_gemm_bf16: tile_n must be 0, 128 or 256");
   return BB_ERR_INVALID_ARG;
+}
+
+bool bb_conv_gemm_supported(int C, int k, int stride, int pad) {
+  // tensor map limits of a rank-4 im2col load: window corners in [-128, 127], traversal stride <= 8
+  return C > 0 && C % 64 == 0 && k >= 1 && k <= 64 && stride >= 1 && stride <= 8 && pad >= 0 && pad < k;
+}
+
+int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream) {
+  const long long P = (long long)a->N * a->Ho * a->Wo;
+  if (!a->x || !a->other || !a->D || P <= 0 || P >= (1LL << 31) || !bb_conv_gemm_supported(a->C, a->k, a->stride, a->pad) ||
+      a->other_channels <= 0 || (a->other_channels & 7) || (a->mode == BB_CONV_DGRAD && a->stride != 1) ||
+      (((uintptr_t)a->x | (uintptr_t)a->other | (uintptr_t)a->D) & 15)) {
+    bb_set_last_error_msg("bb_conv_gemm: null or unaligned operand, or a geometry the im2col loads cannot express");
+    return BB_ERR_INVALID_ARG;
+  }
+  const int taps = a->k * a->k;
+  bb_gemm_desc g = {};
+  g.D = a->D; g.max_ctas = a->max_ctas;
+  if (a->mode == BB_CONV_WGRAD) {
+    g.M = a->other_channels; g.N = taps * a->C; g.K = (int)P;
+    g.A = a->other; g.lda = a->other_channels; g.a_mn_major = 1; g.b_mn_major = 1;
+    g.ldd = g.N; g.epilogue = BB_EPI_ACCUM_F32;
+  } else {
+    g.M = (int)P; g.N = a->other_channels; g.K = taps * a->C;
+    g.B = a->other; g.ldb = a->mode == BB_CONV_FWD ? g.K : (long long)taps * a->other_channels;
+    g.b_mn_major = a->mode == BB_CONV_DGRAD;
+    g.ldd = a->other_channels; g.epilogue = BB_EPI_STORE;
+  }
+  if (int rc = bbhost::bind_context()) return rc;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  bool pair, wide_epi;
+  const int bn = choose_tile(&g, &pair, &wide_epi);
+  if (pair) return launch<256, true, 2, true>(&g, s, a);
+  return bn == 256 ? launch<256, false, 2, true>(&g, s, a) : launch<128, false, 2, true>(&g, s, a);
 }

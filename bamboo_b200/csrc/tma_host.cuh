@@ -59,4 +59,40 @@ inline int encode_2d(CUtensorMap* tm, const void* base, long long rows, long lon
   return BB_OK;
 }
 
+typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const int*, const int*, cuuint32_t, cuuint32_t, const cuuint32_t*,
+                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// im2col tensor map over an NHWC bf16 tensor: `pixels` consecutive output positions of a k x k window with the
+// given stride and padding, 64 channels each (128-byte swizzle).  The windows' first taps run over
+// [-pad, size + pad - k] in steps of `stride`; a tap is chosen per load by its offset.
+inline int encode_im2col(CUtensorMap* tm, const void* base, int N, int H, int W, int C, int k, int stride, int pad, int pixels) {
+  static EncodeIm2colFn fn = nullptr;
+  if (!fn) {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &sym, cudaEnableDefault, &qres) != cudaSuccess ||
+        qres != cudaDriverEntryPointSuccess) {
+      bb_set_last_error_msg("cuTensorMapEncodeIm2col entry point not available");
+      return BB_ERR_CUDA;
+    }
+    fn = reinterpret_cast<EncodeIm2colFn>(sym);
+  }
+  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+  cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
+  int lower[2] = {-pad, -pad}, upper[2] = {pad - (k - 1), pad - (k - 1)};
+  cuuint32_t estr[4] = {1, (cuuint32_t)stride, (cuuint32_t)stride, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, lower, upper, 64, (cuuint32_t)pixels,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    char msg[256];
+    snprintf(msg, sizeof(msg), "cuTensorMapEncodeIm2col failed with CUresult %d (base %p, NHWC %d x %d x %d x %d, k %d, stride %d, pad %d)",
+             (int)r, base, N, H, W, C, k, stride, pad);
+    bb_set_last_error_msg(msg);
+    return BB_ERR_INVALID_ARG;
+  }
+  return BB_OK;
+}
+
 }  // namespace bbhost

@@ -467,9 +467,18 @@ def avgpool_bwd(dy, dx):
     return dx
 
 
+def _conv_route(desc):
+    """(direct, implicit_x, implicit_dx) as bb_conv_bn_fwd / bb_conv_bn_bwd choose it (launch accounting)."""
+    direct = desc.k == 1 and desc.stride == 1
+    small = desc.k <= 64 and desc.pad < desc.k
+    return direct, not direct and small and desc.Cin % 64 == 0 and desc.stride <= 8, \
+        not direct and small and desc.Cout % 64 == 0 and desc.stride == 1
+
+
 def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch):
     global LAUNCHES
-    LAUNCHES += 4 + (0 if (desc.k == 1 and desc.stride == 1) else 1)
+    direct, implicit_x, _ = _conv_route(desc)
+    LAUNCHES += 4 + (0 if direct or implicit_x else 1)
     check(load().bb_conv_bn_fwd(ctypes.byref(desc), _ptr(x), _ptr(residual), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd),
                                 _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_fwd")
     return z
@@ -477,8 +486,8 @@ def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch):
 
 def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch):
     global LAUNCHES
-    direct = desc.k == 1 and desc.stride == 1
-    LAUNCHES += 4 + (0 if direct else 1) + (0 if dx is None else (1 if direct else 2))
+    direct, implicit_x, implicit_dx = _conv_route(desc)
+    LAUNCHES += 4 + (0 if direct or implicit_x else 1) + (0 if dx is None else (1 if direct or implicit_dx else 2))
     check(load().bb_conv_bn_bwd(ctypes.byref(desc), _ptr(x), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd), _ptr(dz), _ptr(dx),
                                 _ptr(dres), _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_bwd")
     return dx

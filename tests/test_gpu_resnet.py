@@ -138,6 +138,50 @@ def test_conv_bn_layer_without_relu(L, cin, cout, k, stride, hw):
     assert L.read_status() == 0
 
 
+# (channels in / out, window, stride, image side): reductions of one to several 64-channel blocks, output rows that no
+# 128-row tile divides, images smaller than the window, an even window (asymmetric turned padding), both tile widths and
+# CTA pairs (256 x 256 outputs with reductions of 2048 and more), channel counts that only one direction can gather
+@pytest.mark.parametrize("cin,cout,k,stride,hw", [(64, 64, 3, 1, 1), (64, 64, 3, 1, 2), (64, 16, 3, 1, 5), (192, 64, 3, 1, 11),
+                                                  (64, 64, 2, 1, 6), (64, 64, 7, 1, 9), (64, 128, 7, 2, 13), (128, 64, 3, 2, 15),
+                                                  (64, 128, 1, 2, 7), (256, 256, 3, 1, 14), (256, 256, 3, 2, 29), (512, 128, 3, 1, 7),
+                                                  (8, 64, 3, 1, 10), (64, 8, 3, 1, 9), (128, 512, 3, 1, 35)])
+def test_convolution_with_gathered_patches(L, cin, cout, k, stride, hw):
+    """The convolution alone (what the layer feeds into batch norm, and the gradients that come out of it) against
+    conv2d in fp32 on the same bf16 operands.  One bf16 rounding of each result: 2^-9 of the value, so 4e-3 in the
+    2-norm; the weight gradient is summed and kept in fp32 (1e-4: order of the sums)."""
+    from bamboo_b200 import resnet
+    from bamboo_b200.arena import ParamArena
+    N = 9
+    m = resnet.ConvBN(cin, cout, k, stride=stride, relu=False, generator=torch.Generator().manual_seed(11))
+    ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(12)
+    x = torch.randn(N, hw, hw, cin, device="cuda", generator=g).bfloat16()
+    ho = (hw + 2 * m.pad - k) // stride + 1
+    P = N * ho * ho
+    y = torch.empty(P, cout, dtype=torch.bfloat16, device="cuda")
+    z = torch.empty(N, ho, ho, cout, dtype=torch.bfloat16, device="cuda")
+    stats = torch.empty(2, cout, device="cuda")
+    d = resnet._conv_desc(m, N, hw, hw, cin, True)
+    scratch = torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device="cuda")
+    L.conv_bn_fwd(d, x, None, y, z, stats[0], stats[1], scratch)
+    w = m.weight.detach().float().view(cout, k, k, cin).permute(0, 3, 1, 2).contiguous().requires_grad_(True)
+    xr = x.float().permute(0, 3, 1, 2).contiguous().requires_grad_(True)
+    with torch.backends.cudnn.flags(allow_tf32=False):
+        want = F.conv2d(xr, w, None, stride=stride, padding=m.pad)
+        assert _rel(y.view(N, ho, ho, cout), want.detach().permute(0, 2, 3, 1)) <= 4e-3
+        dz = torch.randn(N, ho, ho, cout, device="cuda", generator=g).bfloat16()
+        dx = torch.empty_like(x)
+        bwd = torch.empty(d._bwd_scratch[1], dtype=torch.uint8, device="cuda")
+        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, None, bwd)
+        dy = bwd[:P * cout * 2].view(torch.bfloat16).view(N, ho, ho, cout)      # the scratch starts with dy
+        want.backward(dy.float().permute(0, 3, 1, 2).contiguous())
+    # a strided layer rounds every tap's contribution to bf16 before they are summed: k * k roundings instead of one
+    assert _rel(dx, xr.grad.permute(0, 2, 3, 1)) <= 8e-3
+    assert _rel(m.weight.main_grad.view(cout, k, k, cin).permute(0, 3, 1, 2), w.grad) <= 1e-4
+    torch.cuda.synchronize()
+    assert L.read_status() == 0
+
+
 def _block_params(blk, prefix):
     out = {}
     for name in ("conv1", "conv2", "conv3", "down"):

@@ -258,7 +258,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   const uint32_t tDQ = tmem + G::ACC;          // S[b] at tmem + 64 b, dP[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (bb::elect_one()) {
       bb::mbar_arrive_expect_tx(q_full, 2 * G::OWN_BYTES);
 #pragma unroll
       for (int a = 0; a < NA; ++a) {
@@ -281,15 +281,15 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));     // stage 0; stage s: + s * STREAM_BYTES / 16
     const uint64_t dKm0 = desc_mn0(bb::smem_u32(sK)), dDS0 = desc_k0(bb::smem_u32(sDS));
     const uint32_t i_s = idesc(64, 0, 0), i_dq = idesc(D, 0, 1);
-    bool alive = bb::mbar_wait(q_full, 0, &ctl->abort_flag, p.status);
+    bool alive = bb::mbar_wait_warp(q_full, 0, &ctl->abort_flag, p.status);
     // software pipeline: the scores run two sub-blocks ahead of the dQ updates
     for (int j = 0; j < nblk + 2 && alive; ++j) {
       if (j < nblk) {
         const int s = j % NST, b = j % NSB;
-        if (!bb::mbar_wait(&kv_full[s], (j / NST) & 1, &ctl->abort_flag, p.status)) break;
-        if (!bb::mbar_wait(&s_empty[b], ((j / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&kv_full[s], (j / NST) & 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&s_empty[b], ((j / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint64_t dK = dK0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dV = dV0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
@@ -302,9 +302,9 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
       }
       if (j >= 2) {
         const int jj = j - 2, s2 = jj % NST, b2 = jj & 1;
-        if (!bb::mbar_wait(&ds_full[b2], (jj >> 1) & 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&ds_full[b2], (jj >> 1) & 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint64_t dK2 = dKm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < 4; ++k) bb::umma_f16(tDQ, desc_kmajor(dDS, k), desc_mnmajor64(dK2, k), i_dq, (jj > 0 || k > 0));
@@ -444,7 +444,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   const uint32_t tDV = tmem + G::ACC, tDK = tDV + D;   // S^T[b] at tmem + 64 b, dP^T[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (bb::elect_one()) {
       bb::mbar_arrive_expect_tx(kv_full, 2 * G::OWN_BYTES);
 #pragma unroll
       for (int a = 0; a < NA; ++a) {
@@ -468,15 +468,15 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
     const uint64_t dQm0 = desc_mn0(bb::smem_u32(sQ)), dDOm0 = desc_mn0(bb::smem_u32(sDO));
     const uint64_t dP0 = desc_k0(bb::smem_u32(sP)), dDS0 = desc_k0(bb::smem_u32(sDS));
     const uint32_t i_s = idesc(64, 0, 0), i_acc = idesc(D, 0, 1);
-    bool alive = bb::mbar_wait(kv_full, 0, &ctl->abort_flag, p.status);
+    bool alive = bb::mbar_wait_warp(kv_full, 0, &ctl->abort_flag, p.status);
     // the score products run two sub-blocks ahead of the dV / dK updates
     for (int i = 0; i < nblk + 2 && alive; ++i) {
       if (i < nblk) {
         const int s = i % NST, b = i % NSB;
-        if (!bb::mbar_wait(&q_full[s], (i / NST) & 1, &ctl->abort_flag, p.status)) break;
-        if (!bb::mbar_wait(&s_empty[b], ((i / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&q_full[s], (i / NST) & 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&s_empty[b], ((i / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint64_t dQ = dQ0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
@@ -489,9 +489,9 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
       }
       if (i >= 2) {
         const int ii = i - 2, s2 = ii % NST, b2 = ii & 1;
-        if (!bb::mbar_wait(&p_full[b2], (ii >> 1) & 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&p_full[b2], (ii >> 1) & 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4));
           const uint64_t dP = dP0 + (uint64_t)(b2 * (TILE_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
@@ -698,7 +698,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
   const uint32_t tDV = tmem + 256, tDK = tmem + 320, tDQ = tmem + 384;    // dQ[b] at tDQ + 64 b
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (bb::elect_one()) {
       bb::mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
       bb::tma_load_2d(sK, &tm128, kv_full, colk, row_base + k0);
       bb::tma_load_2d(sV, &tm128, kv_full, colv, row_base + k0);
@@ -716,13 +716,13 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));   // stage 0; stage s: + s * SUB_BYTES / 16
     const uint32_t i_s = idesc(64, 0, 0);
-    bool alive = bb::mbar_wait(kv_full, 0, &ctl->abort_flag, p.status);
+    bool alive = bb::mbar_wait_warp(kv_full, 0, &ctl->abort_flag, p.status);
     for (int i = 0; i < nblk && alive; ++i) {
       const int s = i % NST3, b = i & 1;
-      if (!bb::mbar_wait(&q_full[s], (i / NST3) & 1, &ctl->abort_flag, p.status)) break;
-      if (!bb::mbar_wait(&s_empty[b], ((i >> 1) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      if (!bb::mbar_wait_warp(&q_full[s], (i / NST3) & 1, &ctl->abort_flag, p.status)) break;
+      if (!bb::mbar_wait_warp(&s_empty[b], ((i >> 1) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
       bb::tc_fence_after_sync();
-      if (lane == 0) {
+      if (bb::elect_one()) {
         const uint64_t dQ = dQ0 + (uint64_t)(s * (SUB_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (SUB_BYTES >> 4));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -742,14 +742,14 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
     const uint64_t dDSm0 = bb::make_smem_desc_sw128(bb::smem_u32(sDS), TILE_BYTES, 1024);
     const uint64_t dKm0 = desc_mn0(bb::smem_u32(sK));
     const uint32_t i_acc = idesc(64, 0, 1), i_dq = idesc(64, 1, 1);
-    bool alive = bb::mbar_wait(kv_full, 0, &ctl->abort_flag, p.status);
+    bool alive = bb::mbar_wait_warp(kv_full, 0, &ctl->abort_flag, p.status);
     for (int ii = 0; ii < nblk && alive; ++ii) {
       const int s2 = ii % NST3, g2 = ii & 1, pair = ii >> 1, ps = pair & 1;
       // (the sub-tiles landed long ago - the score products read them; the wait makes them visible to this thread)
-      if (!bb::mbar_wait(&q_full[s2], (ii / NST3) & 1, &ctl->abort_flag, p.status)) break;
-      if (!bb::mbar_wait(&p_full[g2], pair & 1, &ctl->abort_flag, p.status)) break;
+      if (!bb::mbar_wait_warp(&q_full[s2], (ii / NST3) & 1, &ctl->abort_flag, p.status)) break;
+      if (!bb::mbar_wait_warp(&p_full[g2], pair & 1, &ctl->abort_flag, p.status)) break;
       bb::tc_fence_after_sync();
-      if (lane == 0) {
+      if (bb::elect_one()) {
         const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (SUB_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (SUB_BYTES >> 4));
         const uint64_t dP = dP0 + (uint64_t)(g2 * (TILE_BYTES >> 4));
         const uint64_t dDS = dDS0 + (uint64_t)((ps * 2 + g2) * (TILE_BYTES >> 4));
@@ -764,9 +764,9 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       __syncwarp();
       if (g2 == 1) {
         // both halves of the pair are staged: dQ[pair] = dS . K over the tile's 128 keys
-        if (!bb::mbar_wait(&dq_empty[pair & 1], ((pair >> 1) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+        if (!bb::mbar_wait_warp(&dq_empty[pair & 1], ((pair >> 1) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint64_t dA = dDSm0 + (uint64_t)(ps * 2 * (TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < 8; ++k)
@@ -1028,7 +1028,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t tmem = ctl->tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (bb::elect_one()) {
       bb::mbar_arrive_expect_tx(q_full, 2 * Q_BYTES);
 #pragma unroll
       for (int a = 0; a < NA; ++a) {
@@ -1050,7 +1050,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ));
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK));   // stage 0; stage s: + s * KV_BYTES / 16
     const uint32_t i_s = idesc(64, 0, 0);
-    bool alive = bb::mbar_wait(q_full, 0, &ctl->abort_flag, p.status);
+    bool alive = bb::mbar_wait_warp(q_full, 0, &ctl->abort_flag, p.status);
     // scores of sub-block jj for group g into score buffer jj & 1
     auto issue_scores = [&](int g, int jj) {
       const uint64_t dK = dK0 + (uint64_t)((jj % NKV) * (KV_BYTES >> 4)), dQ = dQ0 + (uint64_t)(g * (Q_BYTES >> 4));
@@ -1063,9 +1063,9 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     };
     // prologue: the first two score products of each group
     for (int jj = 0; jj < 2 && jj <= jmax && alive; ++jj) {
-      if (!bb::mbar_wait(&kv_full[jj % NKV], 0, &ctl->abort_flag, p.status)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&kv_full[jj % NKV], 0, &ctl->abort_flag, p.status)) { alive = false; break; }
       bb::tc_fence_after_sync();
-      if (lane == 0) {
+      if (bb::elect_one()) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) if (jj <= BB_LAST(g)) issue_scores(g, jj);
       }
@@ -1077,10 +1077,10 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int g = 0; g < 2; ++g) {
         if (jj + 2 > BB_LAST(g)) continue;
         // group g is done reading S_g(jj): its buffer is free
-        if (!bb::mbar_wait(&s_free[2 * g + (jj & 1)], (jj >> 1) & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
-        if (!bb::mbar_wait(&kv_full[(jj + 2) % NKV], ((jj + 2) / NKV) & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
+        if (!bb::mbar_wait_warp(&s_free[2 * g + (jj & 1)], (jj >> 1) & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
+        if (!bb::mbar_wait_warp(&kv_full[(jj + 2) % NKV], ((jj + 2) / NKV) & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
         bb::tc_fence_after_sync();
-        if (lane == 0) issue_scores(g, jj + 2);
+        if (bb::elect_one()) issue_scores(g, jj + 2);
         __syncwarp();
       }
     }
@@ -1094,13 +1094,13 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int s = jj % NKV;
       const uint64_t dV = dVm0 + (uint64_t)(s * (KV_BYTES >> 4));
       // (V_jj landed before the scores of this sub-block were issued; the wait makes it visible to this thread)
-      if (!bb::mbar_wait(&kv_full[s], (jj / NKV) & 1, &ctl->abort_flag, p.status)) break;
+      if (!bb::mbar_wait_warp(&kv_full[s], (jj / NKV) & 1, &ctl->abort_flag, p.status)) break;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         if (jj > BB_LAST(g)) continue;
-        if (!bb::mbar_wait(&p_full[g], jj & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
+        if (!bb::mbar_wait_warp(&p_full[g], jj & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           const uint32_t tO = tmem + 256 + 128 * g;
           const uint64_t dPg = dP0 + (uint64_t)((2 * g + (jj & 1)) * (TILE_BYTES >> 4));
 #pragma unroll
@@ -1110,7 +1110,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
       }
       // K_jj, V_jj: the score products that read K_jj retired before P(jj) existed, the P V products are issued
-      if (alive && lane == 0) bb::umma_commit(&kv_empty[s]);
+      if (alive && bb::elect_one()) bb::umma_commit(&kv_empty[s]);
       __syncwarp();
     }
   } else if (warp >= 3) {

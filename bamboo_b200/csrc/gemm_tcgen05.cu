@@ -337,7 +337,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (bb::elect_one()) {
       int s = 0; uint32_t phase = 0;
       bool alive = true;
       // operand loads of one work unit
@@ -523,15 +523,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       int tile;
       if (!next_unit(it, tile, true)) { alive = false; break; }
       if (tile < 0) break;
-      if (!bb::mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status)) { alive = false; break; }
       bb::tc_fence_after_sync();
       const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
       const int ks = tile / num_mn;
       const int num_kb = min(total_kb, (ks + 1) * p.kb_per_split) - ks * p.kb_per_split;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!bb::mbar_wait(&full_bar[s], phase, abort_flag, p.status)) { alive = false; break; }
+        if (!bb::mbar_wait_warp(&full_bar[s], phase, abort_flag, p.status)) { alive = false; break; }
         bb::tc_fence_after_sync();
-        if (lane == 0) {
+        if (bb::elect_one()) {
           // one descriptor per stage; a k-step only adds to its address field (16-byte units)
           const uint64_t ad0 = bb::make_smem_desc_sw128(bb::smem_u32(sA + s * A_STAGE_BYTES), a_lbo, 1024u);
           const uint64_t bd0 = bb::make_smem_desc_sw128(bb::smem_u32(sB + s * C::B_STAGE_BYTES), b_lbo, 1024u);

@@ -484,10 +484,15 @@ def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch):
     return z
 
 
-def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch):
+def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch, residual=True):
+    """``residual=False``: the forward call added none, so the ReLU mask may come from y instead of z."""
     global LAUNCHES
     direct, implicit_x, implicit_dx = _conv_route(desc)
     LAUNCHES += 4 + (0 if direct or implicit_x else 1) + (0 if dx is None else (1 if direct or implicit_dx else 2))
+    if not residual:
+        check(load().bb_conv_bn_bwd_no_residual(ctypes.byref(desc), _ptr(x), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd), _ptr(dz),
+                                                _ptr(dx), _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_bwd")
+        return dx
     check(load().bb_conv_bn_bwd(ctypes.byref(desc), _ptr(x), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd), _ptr(dz), _ptr(dx),
                                 _ptr(dres), _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_bwd")
     return dx

@@ -91,7 +91,7 @@ class _ConvBNNativeFn(torch.autograd.Function):
         dx = torch.empty(N, H, W, Cin, dtype=torch.bfloat16, device=dev) if need_dx else None
         dres = torch.empty_like(z) if ctx.has_res else None
         scratch = torch.empty(d._bwd_scratch[1 if need_dx else 0], dtype=torch.uint8, device=dev)
-        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, dres, scratch)
+        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, dres, scratch, residual=ctx.has_res)
         return dx, dres, None, None, None, None
 
 

@@ -138,6 +138,47 @@ def test_conv_bn_layer_without_relu(L, cin, cout, k, stride, hw):
     assert L.read_status() == 0
 
 
+# rows: fewer than one per thread group, around a thread's four rows in flight, many; channels: the narrowest (one
+# 16-byte chunk), ordinary, the widest (a row per block)
+@pytest.mark.parametrize("rows,C", [(1, 8), (255, 8), (3, 64), (129, 64), (1025, 256), (7, 2048), (50, 2048), (40000, 64)])
+def test_batch_norm_backward_mask_from_y_equals_mask_from_z(L, rows, C):
+    """bb_conv_bn_bwd_no_residual takes the ReLU mask from y: the same values as the general entry point, which reads the
+    stored output, in every bit (same kernels, same order of sums), a channel that
+    is zero throughout included."""
+    from bamboo_b200 import resnet
+    from bamboo_b200.arena import ParamArena
+    m = resnet.ConvBN(8, C, 1, relu=True, generator=torch.Generator().manual_seed(5))
+    with torch.no_grad():
+        m.bn_weight.copy_(torch.linspace(-1.0, 1.5, C)); m.bn_bias.copy_(torch.linspace(0.5, -0.5, C))
+        m.bn_weight[0] = 0.0; m.bn_bias[0] = 0.0                  # z = 0 everywhere: nothing passes
+    ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(1, 1, rows, 8, device="cuda", generator=g).bfloat16()
+    x[..., 0] = 0.0
+    d = resnet._conv_desc(m, 1, 1, rows, 8, True)
+    y, z = torch.empty(rows, C, dtype=torch.bfloat16, device="cuda"), torch.empty(1, 1, rows, C, dtype=torch.bfloat16, device="cuda")
+    stats = torch.empty(2, C, device="cuda")
+    L.conv_bn_fwd(d, x, None, y, z, stats[0], stats[1], torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device="cuda"))
+    dz = torch.randn(1, 1, rows, C, device="cuda", generator=g).bfloat16()
+    out = []
+    for residual in (True, False):
+        for p in (m.weight, m.bn_weight, m.bn_bias):
+            p.main_grad.zero_()
+        dx = torch.empty_like(x)
+        scratch = torch.zeros(d._bwd_scratch[1], dtype=torch.uint8, device="cuda")
+        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, None, scratch, residual=residual)
+        out.append((scratch[:rows * C * 2].view(torch.bfloat16).clone(), m.bn_weight.main_grad.clone(), m.bn_bias.main_grad.clone()))
+    for a, b in zip(*out):
+        assert torch.equal(a.nan_to_num(), b.nan_to_num()) and torch.equal(a.isnan(), b.isnan())
+    # (the values themselves, against fp32: masked gradient through batch norm)
+    yf = y.float().requires_grad_(True)
+    if rows > 3:
+        ga, be = m.bn_weight.detach().float().requires_grad_(True), m.bn_bias.detach().float().requires_grad_(True)
+        zf = F.batch_norm(yf, None, None, ga, be, training=True, eps=m.eps)
+        zf.backward(torch.where(z.view(rows, C) > 0, dz.view(rows, C).float(), torch.zeros((), device="cuda")))
+        assert _rel(out[1][0].view(rows, C), yf.grad) <= TOL and _rel(out[1][1], ga.grad) <= TOL
+
+
 # (channels in / out, window, stride, image side): reductions of one to several 64-channel blocks, output rows that no
 # 128-row tile divides, images smaller than the window, an even window (asymmetric turned padding), both tile widths and
 # CTA pairs (256 x 256 outputs with reductions of 2048 and more), channel counts that only one direction can gather

@@ -783,6 +783,21 @@ TicketTable* ticket_table() {
   return t;
 }
 
+// Too few output tiles to fill the machine: split the reduction; partial sums meet in the fp32 add-reduction of the
+// epilogue.  Cost model: waves x (k-blocks + fixed overhead).
+int wave_split(int mn_tiles, int workers, int total_kb) {
+  int ksplit = 1;
+  long long best = -1;
+  for (int s = 1; s <= 16; ++s) {
+    const int kbs = (total_kb + s - 1) / s;
+    if (s > 1 && kbs < 8) break;
+    const long long waves = ((long long)mn_tiles * s + workers - 1) / workers;
+    const long long cost = waves * (kbs + 8);
+    if (best < 0 || cost < best) { best = cost; ksplit = s; }
+  }
+  return ksplit;
+}
+
 // `cv`: convolution product (CONV); the descriptor then holds the sizes and the operand that is no patch matrix
 template <int BN, bool PAIR, int EW, bool CONV>
 int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* cv = nullptr) {
@@ -821,17 +836,7 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
     if (g->split_k > 0) {
       ksplit = g->split_k;
     } else {
-      // too few output tiles to fill the machine: split the reduction; partial sums meet in
-      // the fp32 add-reduction of the epilogue.  Cost model: waves x (k-blocks + fixed overhead).
-      const int sms = workers_max;
-      long long best = -1;
-      for (int s = 1; s <= 16; ++s) {
-        const int kbs = (total_kb + s - 1) / s;
-        if (s > 1 && kbs < 8) break;
-        const long long waves = ((long long)mn_tiles * s + sms - 1) / sms;
-        const long long cost = waves * (kbs + 8);
-        if (best < 0 || cost < best) { best = cost; ksplit = s; }
-      }
+      ksplit = wave_split(mn_tiles, workers_max, total_kb);
     }
   }
   if (ksplit > total_kb) ksplit = total_kb;
@@ -887,16 +892,70 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   return BB_OK;
 }
 
+// Whether a problem runs as CTA pairs (see choose_tile)
+bool pairs_pay(int M, int N, int K) {
+  const long long tiles_single = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);
+  return M > BM && N > 128 && (K >= 2048 || tiles_single >= 16LL * bb_num_sms());
+}
+
+// Weight gradients (fp32 add-reduction): few output tiles and a long reduction, so tile, pairing and the split of the
+// reduction are chosen together.  A unit's time is counted in 16 KiB operand loads: two per k-block for a 128 x 128
+// tile, three for 128 x 256, a little less for each CTA of a 256 x 256 pair, plus a tile's start and its add-reduction
+// (EPI per 128 columns); a plan costs waves x that.  Splits go as far as one wave of the machine (or 16, as more
+// than one wave evens out ragged ones) and leave at least eight k-blocks per unit (short reductions stay whole, with one
+// order of additions).  No unit sums more k-blocks than wave_split gives the widest tile: the accumulator's rounding
+// grows with their number (256 x 2304 x 6272 against fp64: 13 k-blocks 7.8e-7, 25 k-blocks 1.6e-6).
+// Measured (us, before: at most 16 splits and always 256 columns): 64 x 64 x 100352 41 -> 14.4, 64 x 576 x 100352
+// 57 -> 37, 256 x 64 x 100352 41 -> 22.5, 256 x 512 x 25088 24.6 -> 18.4, 64 x 392 x 401408 186 -> 84, 128 x 128 x 800
+// 14.3 -> 12.3; 1024 x 1024 x 8192 and larger as before.
+struct AccumPlan { int bn; bool pair; int ksplit; };
+AccumPlan plan_accum(int M, int N, int K) {
+  constexpr double EPI = 14.0;
+  const long long kb = (K + BK - 1) / BK;
+  long long longest;
+  {
+    const bool pair = pairs_pay(M, N, K);
+    const int tm = pair ? 2 * BM : BM, bn = N > 128 ? 256 : 128;
+    const int s = wave_split(((M + tm - 1) / tm) * ((N + bn - 1) / bn), pair ? bb_num_sms() / 2 : bb_num_sms(), (int)kb);
+    longest = (kb + s - 1) / s;
+  }
+  AccumPlan best = {128, false, 1};
+  double best_cost = -1;
+  for (int c = 0; c < 3; ++c) {
+    const bool pair = c == 0;
+    const int bn = c == 2 ? 128 : 256;
+    if (bn == 256 && N <= 128) continue;
+    if (pair && !pairs_pay(M, N, K)) continue;
+    const long long tm = pair ? 2 * BM : BM;
+    const long long tiles = ((M + tm - 1) / tm) * ((N + bn - 1) / bn);
+    const long long workers = pair ? bb_num_sms() / 2 : bb_num_sms();
+    const double per_kb = pair ? 2.9 : (bn == 256 ? 3.0 : 2.0), fixed = bn == 256 ? 2 * EPI : EPI;
+    const long long smax = workers / tiles > 16 ? workers / tiles : 16;
+    for (long long s = 1; s <= smax; ++s) {
+      const long long kbs = (kb + s - 1) / s;
+      if (s > 1 && kbs < 8) break;
+      if (kbs > longest) continue;
+      const long long units = tiles * ((kb + kbs - 1) / kbs);
+      const double cost = (double)((units + workers - 1) / workers) * ((double)kbs * per_kb + fixed);
+      if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, pair, (int)s}; }
+    }
+  }
+  return best;
+}
+
 // Tile width, and whether CTA pairs / sixteen epilogue warps are used.
-int choose_tile(const bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
+int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
   const int e = g->epilogue;
+  if (e == BB_EPI_ACCUM_F32 && g->split_k <= 0 && g->tile_n == 0 && g->cta_pair == 0) {
+    const AccumPlan pl = plan_accum(g->M, g->N, g->K);
+    g->split_k = pl.ksplit;
+    *pair_out = pl.pair; *wide_out = false;
+    return pl.bn;
+  }
   // CTA pairs (256 x 256 per pair) pay off on long reductions and on long runs of tiles per
   // CTA; short problems are quicker to start and drain as single CTAs (measured on B200:
   // K >= 3072 or >= 40 tiles per CTA 2-6 % faster as pairs, K = 1024 with <= 7 tiles 4-8 % slower)
-  const long long tiles_single = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
-  *pair_out = g->cta_pair > 0 ||
-                    (g->cta_pair == 0 && g->tile_n == 0 && g->M > BM && g->N > 128 &&
-                     (g->K >= 2048 || tiles_single >= 16LL * bb_num_sms()));
+  *pair_out = g->cta_pair > 0 || (g->cta_pair == 0 && g->tile_n == 0 && pairs_pay(g->M, g->N, g->K));
   // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant)
   *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048);
   int bn = g->tile_n;
@@ -939,7 +998,9 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   // a thread that has only ever set its device (autograd worker threads) has none yet.
   if (int rc = bbhost::bind_context()) return rc;
   bool pair, wide_epi;
-  const int bn = choose_tile(g, &pair, &wide_epi);
+  bb_gemm_desc planned = *g;
+  const int bn = choose_tile(&planned, &pair, &wide_epi);
+  g = &planned;
   if (pair) return wide_epi ? launch<256, true, 4, false>(g, s) : launch<256, true, 2, false>(g, s);
   if (bn == 256) return wide_epi ? launch<256, false, 4, false>(g, s) : launch<256, false, 2, false>(g, s);
   if (bn == 128) return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);

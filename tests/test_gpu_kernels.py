@@ -147,6 +147,28 @@ def test_gemm_split_k_accumulation(L, split, cta_pair):
     assert torch.equal(acc, want)                                    # small integers: exact
 
 
+# (output channels, columns, rows of the reduction): one to many output tiles, reductions of one k-block, of a few (left
+# whole), and of so many that a single tile is split over the whole machine; ragged last splits and pairs
+@pytest.mark.parametrize("M,N,K", [(64, 64, 40), (8, 72, 130), (128, 128, 800), (64, 392, 4097), (64, 64, 100352), (256, 2304, 1000),
+                                   (1024, 256, 64), (256, 512, 25088), (512, 4608, 2100)])
+def test_gemm_planned_weight_gradients(L, M, N, K):
+    """The add-reduction epilogue with tile, pairing and split left to the library, on top of existing gradients,
+    against fp64.  Products of bf16 values are exact in fp32; what differs is the fp32 rounding of the sums: with
+    random signs about sqrt(K) additions of 2^-24 each, 2e-5 at the longest reduction."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(K, M, device="cuda", generator=g).bfloat16()
+    b = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    start = torch.randn(M, N, device="cuda", generator=g)
+    d = start.clone()
+    for _ in range(2):
+        L.gemm(a, b, d, a_mn=True, b_mn=True, epilogue=L.EPI_ACCUM_F32, M=M, N=N, K=K)
+    want = start.double() + 2 * (a.double().t() @ b.double())
+    err = ((d.double() - want).norm() / want.norm()).item()
+    print(f"weight gradient {M}x{N}x{K}: relative error {err:.2e}")
+    assert err <= 2e-5
+    assert L.read_status() == 0
+
+
 def test_gemm_rejects_bad_arguments(L):
     A = torch.zeros(16, 12, device="cuda", dtype=torch.bfloat16)   # leading dimension not a multiple of 8
     B = torch.zeros(16, 12, device="cuda", dtype=torch.bfloat16)

@@ -279,17 +279,38 @@ class _MLPHalfFn(torch.autograd.Function):
 NATIVE_BLOCKS = True
 
 
+_HALF_PARAMS = {L.HALF_ATTENTION: ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "proj_w", "proj_b"),
+                L.HALF_MLP: ("ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")}
+
+
+def _anchor(mod, half):
+    """The parameter that stands for a half block in the autograd graph: the first that takes a gradient.  The kernels
+    add weight gradients to the arena themselves, so a parameter's edge carries nothing but the fact that the output
+    depends on trained values; one edge per half costs the engine one empty accumulation instead of six."""
+    params = mod._parameters
+    for name in _HALF_PARAMS[half]:
+        p = params.get(name)
+        if p is None:
+            p = getattr(mod, name)
+        if p.requires_grad:
+            return p
+    return p
+
+
+def _half(x, mod, half):
+    return _HalfFn.apply(x, mod, half, _anchor(mod, half))
+
+
 def _half_desc(mod, half, T, B, S, need_grads):
     """The module's cached bb_block_desc for this geometry; rebuilt when its parameters moved
     (another arena) or the GEMM CTA budget changed."""
-    names = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "proj_w", "proj_b") if half == L.HALF_ATTENTION else \
-            ("ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")
-    params = [getattr(mod, n) for n in names]
-    key = (half, T, B, S, L.GEMM_MAX_CTAS, params[2].data_ptr(), need_grads)
+    weight = getattr(mod, _HALF_PARAMS[half][2])
+    key = (half, T, B, S, L.GEMM_MAX_CTAS, weight.data_ptr(), need_grads)
     cache = mod.__dict__.setdefault("_desc_cache", {})
     d = cache.get(key)
     if d is not None:
         return d
+    params = [getattr(mod, n) for n in _HALF_PARAMS[half]]
     h = params[2].shape[1]
     heads = getattr(mod, "heads", 1)
     d = L.BlockDesc(tokens=T, batch=B, seq=S, heads=heads, head_dim=h // heads, hidden=h,
@@ -316,43 +337,38 @@ class _HalfFn(torch.autograd.Function):
     x + fc2(gelu(fc1(LN2(x))))."""
 
     @staticmethod
-    def forward(ctx, x, mod, half, *params):
+    def forward(ctx, x, mod, half, anchor):
         _require_cuda(x, "transformer block")
+        if not x.is_contiguous():
+            x = x.contiguous()
         shape = x.shape
-        h = shape[-1]
-        x2 = x.reshape(-1, h)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        T = x2.shape[0]
-        B, S = (shape[0], shape[1]) if x.dim() == 3 else (1, T)
+        T = x.numel() // shape[-1]
+        B, S = (shape[0], shape[1]) if len(shape) == 3 else (1, T)
         d = _half_desc(mod, half, T, B, S, False)
         saved = torch.empty(d._saved_bytes, dtype=torch.uint8, device=x.device)
-        out = torch.empty(T, h, dtype=torch.bfloat16, device=x.device)
-        L.block_half_fwd(d, half, x2, saved, out)
-        ctx.mod, ctx.half, ctx.geom, ctx.shape = mod, half, (T, B, S), shape
-        ctx.save_for_backward(x2, saved)
-        return out.view(shape)
+        out = torch.empty(shape, dtype=torch.bfloat16, device=x.device)
+        L.block_half_fwd(d, half, x, saved, out)
+        ctx.mod, ctx.half, ctx.geom = mod, half, (T, B, S)
+        ctx.save_for_backward(x, saved)
+        return out
 
     @staticmethod
     def backward(ctx, dout):
-        x2, saved = ctx.saved_tensors
-        T, B, S = ctx.geom
-        h = x2.shape[1]
-        d2 = dout.reshape(-1, h)
-        if not d2.is_contiguous():
-            d2 = d2.contiguous()
-        d = _half_desc(ctx.mod, ctx.half, T, B, S, True)
-        scratch = torch.empty(d._scratch_bytes, dtype=torch.uint8, device=x2.device)
-        dx = torch.empty(T, h, dtype=torch.bfloat16, device=x2.device)
+        x, saved = ctx.saved_tensors
+        if not dout.is_contiguous():
+            dout = dout.contiguous()
+        d = _half_desc(ctx.mod, ctx.half, *ctx.geom, True)
+        scratch = torch.empty(d._scratch_bytes, dtype=torch.uint8, device=x.device)
+        dx = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
         side = None
         if WGRAD_SIDE_STREAM:
-            st = _wgrad_stream(x2.device)
+            st = _wgrad_stream(x.device)
             side = st.cuda_stream
             # operands of the weight-gradient kernels: not to be handed out again before that stream is done
-            for t in (d2, saved, scratch):
+            for t in (dout, saved, scratch):
                 t.record_stream(st)
-        L.block_half_bwd(d, ctx.half, x2, saved, d2, dx, scratch, side)
-        return (dx.view(ctx.shape), None, None) + (None,) * 6
+        L.block_half_bwd(d, ctx.half, x, saved, dout, dx, scratch, side)
+        return dx, None, None, None
 
 
 def _use_native_blocks():
@@ -540,10 +556,7 @@ class TransformerBlock(nn.Module):
 
     def forward(self, x):
         if _use_native_blocks():
-            x1 = _HalfFn.apply(x, self, L.HALF_ATTENTION, self.ln1_w, self.ln1_b, self.qkv_w, self.qkv_b, self.proj_w,
-                               self.proj_b)
-            return _HalfFn.apply(x1, self, L.HALF_MLP, self.ln2_w, self.ln2_b, self.fc1_w, self.fc1_b, self.fc2_w,
-                                 self.fc2_b)
+            return _half(_half(x, self, L.HALF_ATTENTION), self, L.HALF_MLP)
         return _BlockFn.apply(x, self, self.ln1_w, self.ln1_b, self.qkv_w, self.qkv_b, self.proj_w, self.proj_b,
                               self.ln2_w, self.ln2_b, self.fc1_w, self.fc1_b, self.fc2_w, self.fc2_b)
 
@@ -564,8 +577,7 @@ class AttentionHalf(nn.Module):
 
     def forward(self, x):
         if _use_native_blocks():
-            return _HalfFn.apply(x, self, L.HALF_ATTENTION, self.ln1_w, self.ln1_b, self.qkv_w, self.qkv_b, self.proj_w,
-                                 self.proj_b)
+            return _half(x, self, L.HALF_ATTENTION)
         return _AttnHalfFn.apply(x, self, self.ln1_w, self.ln1_b, self.qkv_w, self.qkv_b, self.proj_w, self.proj_b)
 
 
@@ -583,7 +595,7 @@ class MLPHalf(nn.Module):
 
     def forward(self, x):
         if _use_native_blocks():
-            return _HalfFn.apply(x, self, L.HALF_MLP, self.ln2_w, self.ln2_b, self.fc1_w, self.fc1_b, self.fc2_w, self.fc2_b)
+            return _half(x, self, L.HALF_MLP)
         return _MLPHalfFn.apply(x, self, self.ln2_w, self.ln2_b, self.fc1_w, self.fc1_b, self.fc2_w, self.fc2_b)
 
 

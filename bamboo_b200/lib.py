@@ -91,6 +91,13 @@ def load():
         lib.bb_block_saved_bytes.restype = ctypes.c_longlong
         lib.bb_block_scratch_bytes.restype = ctypes.c_longlong
         lib.bb_conv_bn_scratch_bytes.restype = ctypes.c_longlong
+        # calls made once per layer and micro-batch: with declared argument types plain integers are passed as they are
+        vp, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+        lib.bb_block_half_fwd.argtypes = [vp, i, vp, vp, vp, vp]
+        lib.bb_block_half_bwd.argtypes = [vp, i, vp, vp, vp, vp, vp, ll, vp, vp]
+        lib.bb_conv_bn_fwd.argtypes = [vp] * 8 + [ll, vp]
+        lib.bb_conv_bn_bwd.argtypes = [vp] * 10 + [ll, vp]
+        lib.bb_conv_bn_bwd_no_residual.argtypes = [vp] * 9 + [ll, vp]
         _lib = lib
     return _lib
 
@@ -111,6 +118,10 @@ def read_status():
 
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def _addr(t):
+    return t if t is None or type(t) is int else t.data_ptr()
 
 
 def _stream(raw=None):
@@ -359,11 +370,17 @@ def cast_f32_to_bf16(src, dst):
     return dst
 
 
+def _raw_stream():
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def block_half_fwd(desc, half, x, saved, out):
     global LAUNCHES
     LAUNCHES += HALF_FWD_LAUNCHES[half]
-    check(load().bb_block_half_fwd(ctypes.byref(desc), _I(half), _ptr(x), _ptr(saved), _ptr(out), _stream()),
-          "bb_block_half_fwd")
+    rc = (_lib or load()).bb_block_half_fwd(ctypes.byref(desc), half, x.data_ptr(), saved.data_ptr(), out.data_ptr(), _raw_stream())
+    if rc < 0:
+        check(rc, "bb_block_half_fwd")
     return out
 
 
@@ -371,10 +388,11 @@ def block_half_bwd(desc, half, x, saved, dout, dx, scratch, side_stream=None):
     """``side_stream``: raw handle of the stream for the weight gradients (None: the current stream)."""
     global LAUNCHES
     LAUNCHES += HALF_BWD_LAUNCHES[half]
-    main = _stream()
-    side = main if side_stream is None else ctypes.c_void_p(side_stream)
-    check(load().bb_block_half_bwd(ctypes.byref(desc), _I(half), _ptr(x), _ptr(saved), _ptr(dout), _ptr(dx), _ptr(scratch),
-                                   _LL(scratch.numel()), main, side), "bb_block_half_bwd")
+    main = _raw_stream()
+    rc = (_lib or load()).bb_block_half_bwd(ctypes.byref(desc), half, x.data_ptr(), saved.data_ptr(), dout.data_ptr(), dx.data_ptr(),
+                                            scratch.data_ptr(), scratch.numel(), main, main if side_stream is None else side_stream)
+    if rc < 0:
+        check(rc, "bb_block_half_bwd")
     return dx
 
 
@@ -476,23 +494,27 @@ def _conv_route(desc):
 
 
 def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch):
+    """``mean`` / ``rstd``: fp32 tensors, or their device addresses."""
     global LAUNCHES
     direct, implicit_x, _ = _conv_route(desc)
     LAUNCHES += 4 + (0 if direct or implicit_x else 1)
-    check(load().bb_conv_bn_fwd(ctypes.byref(desc), _ptr(x), _ptr(residual), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd),
-                                _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_fwd")
+    rc = (_lib or load()).bb_conv_bn_fwd(ctypes.byref(desc), x.data_ptr(), _addr(residual), y.data_ptr(), z.data_ptr(), _addr(mean),
+                                         _addr(rstd), scratch.data_ptr(), scratch.numel(), _raw_stream())
+    if rc < 0:
+        check(rc, "bb_conv_bn_fwd")
     return z
 
 
 def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch, residual=True):
-    """``residual=False``: the forward call added none, so the ReLU mask may come from y instead of z."""
+    """``residual=False``: the forward call added none, so the ReLU mask may come from y instead of z.
+    ``mean`` / ``rstd``: fp32 tensors, or their device addresses."""
     global LAUNCHES
     direct, implicit_x, implicit_dx = _conv_route(desc)
     LAUNCHES += 4 + (0 if direct or implicit_x else 1) + (0 if dx is None else (1 if direct or implicit_dx else 2))
-    if not residual:
-        check(load().bb_conv_bn_bwd_no_residual(ctypes.byref(desc), _ptr(x), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd), _ptr(dz),
-                                                _ptr(dx), _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_bwd")
-        return dx
-    check(load().bb_conv_bn_bwd(ctypes.byref(desc), _ptr(x), _ptr(y), _ptr(z), _ptr(mean), _ptr(rstd), _ptr(dz), _ptr(dx),
-                                _ptr(dres), _ptr(scratch), _LL(scratch.numel()), _stream()), "bb_conv_bn_bwd")
+    lib = _lib or load()
+    head = (ctypes.byref(desc), x.data_ptr(), y.data_ptr(), z.data_ptr(), _addr(mean), _addr(rstd), dz.data_ptr(), _addr(dx))
+    tail = (scratch.data_ptr(), scratch.numel(), _raw_stream())
+    rc = lib.bb_conv_bn_bwd(*head, _addr(dres), *tail) if residual else lib.bb_conv_bn_bwd_no_residual(*head, *tail)
+    if rc < 0:
+        check(rc, "bb_conv_bn_bwd")
     return dx

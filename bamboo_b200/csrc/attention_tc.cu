@@ -137,6 +137,7 @@ struct Ctl {
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_tc_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const TcParams p) {
+  bb::pdl_sync();
   constexpr int LANES = D / 8;                                 // lanes of one (token, head)
   const int per_tok = p.H * LANES;                             // 16-byte chunks per token row
   const long long total = (long long)p.B * p.S * per_tok;
@@ -265,6 +266,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
+  bb::pdl_sync();
   const uint32_t tDQ = tmem + G::ACC;          // S[b] at tmem + 64 b, dP[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
@@ -451,6 +453,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
+  bb::pdl_sync();
   const uint32_t tDV = tmem + G::ACC, tDK = tDV + D;   // S^T[b] at tmem + 64 b, dP^T[b] at tmem + 64 (NSB + b)
 
   if (warp == 0) {
@@ -711,6 +714,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
+  bb::pdl_sync();
   // S^T[b] at tmem + 64 b, dP^T[b] at tmem + 128 + 64 b (b < 2)
   const uint32_t tDV = tmem + 256, tDK = tmem + 320, tDQ = tmem + 384;    // dQ[b] at tDQ + 64 b
 
@@ -936,6 +940,7 @@ constexpr int BWD3_SMEM = 2 * TILE_BYTES + 2 * NST3 * SUB_BYTES + 2 * TILE_BYTES
 // dq (bf16, packed projection layout) = scale * accumulator; eight values per thread
 __global__ void __launch_bounds__(256)
 attn_tc_dq_convert_kernel(const TcParams p) {
+  bb::pdl_sync();
   const int per_tok = p.H * 8;
   const long long total = (long long)p.B * p.S * per_tok;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (long long)gridDim.x * blockDim.x) {
@@ -1044,6 +1049,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
+  bb::pdl_sync();
 
   if (warp == 0) {
     if (bb::elect_one()) {
@@ -1291,6 +1297,7 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_slot;
+  bb::pdl_sync();
 
   if (warp == 0) {
     auto load_k = [&](int j) {
@@ -1466,10 +1473,10 @@ int launch_fwd2(const void* qkv_q, void* out, float* lse, int B, int H, int S, l
   // columns, allocated in powers of two), and the two-tile kernel keeps the softmax groups on the SM instead.
   if constexpr (D == 64) {
     BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_fwd3_kernel, FWD3_SMEM)) return rc; });
-    attn_tc_fwd3_kernel<<<(S + TQ - 1) / TQ * H * B, FWD3_THREADS, FWD3_SMEM, stream>>>(tm_q, tm_kv, p);
+    bb_launch(attn_tc_fwd3_kernel, (S + TQ - 1) / TQ * H * B, FWD3_THREADS, FWD3_SMEM, stream, tm_q, tm_kv, p);
   } else {
     BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_fwd2_kernel<D>, Fwd2<D>::SMEM)) return rc; });
-    attn_tc_fwd2_kernel<D><<<(S + 2 * TQ - 1) / (2 * TQ) * H * B, FWD2_THREADS, Fwd2<D>::SMEM, stream>>>(tm_q, tm_kv, p);
+    bb_launch(attn_tc_fwd2_kernel<D>, (S + 2 * TQ - 1) / (2 * TQ) * H * B, FWD2_THREADS, Fwd2<D>::SMEM, stream, tm_q, tm_kv, p);
   }
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
@@ -1490,9 +1497,9 @@ template <int D>
 int launch_bwd2(const CUtensorMap& tm_qkv, const CUtensorMap& tm_qkv64, const CUtensorMap& tm_do, const CUtensorMap& tm_do64,
                 const void* out, const void* d_out, const TcParams& p, int dgrid, cudaStream_t stream) {
   BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd2_kernel<D>, bwd2_smem<D>())) return rc; });
-  attn_tc_delta_kernel<D><<<dgrid, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
+  bb_launch(attn_tc_delta_kernel<D>, dgrid, 256, 0, stream, (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
   const int grid = 2 * ((p.S + TQ - 1) / TQ) * p.H * p.B;
-  attn_tc_bwd2_kernel<D><<<grid, NT2, bwd2_smem<D>(), stream>>>(tm_qkv, tm_qkv64, tm_do, tm_do64, p);
+  bb_launch(attn_tc_bwd2_kernel<D>, grid, NT2, bwd2_smem<D>(), stream, tm_qkv, tm_qkv64, tm_do, tm_do64, p);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -1526,14 +1533,14 @@ int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, c
   if (split) return launch_bwd2<64>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
   p.dq_acc = dq_acc;
   BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd3_kernel, BWD3_SMEM)) return rc; });
-  attn_tc_delta_kernel<64><<<(int)dgrid, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
+  bb_launch(attn_tc_delta_kernel<64>, (int)dgrid, 256, 0, stream, (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
   const int grid = (S + TQ - 1) / TQ * H * B;
   // the accumulator as [B * H * S rows, 64] fp32; a reduction moves [128 rows x 32 columns]
   CUtensorMap tm_acc;
   if (int rc = bbhost::encode_2d(&tm_acc, dq_acc, (long long)B * H * S, HD, HD, 32, TQ, 1)) return rc;
-  attn_tc_bwd3_kernel<<<grid, NT3, BWD3_SMEM, stream>>>(tm_qkv, tm_qkv64, tm_do64, tm_acc, p);
+  bb_launch(attn_tc_bwd3_kernel, grid, NT3, BWD3_SMEM, stream, tm_qkv, tm_qkv64, tm_do64, tm_acc, p);
   long long cgrid = (chunks + 255) / 256;
-  attn_tc_dq_convert_kernel<<<(int)(cgrid < cap ? cgrid : cap), 256, 0, stream>>>(p);
+  bb_launch(attn_tc_dq_convert_kernel, (int)(cgrid < cap ? cgrid : cap), 256, 0, stream, p);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }

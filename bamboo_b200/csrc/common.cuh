@@ -43,6 +43,29 @@ int bb_current_device();
     }                                                     \
   } while (0)
 
+// Kernels that one entry point issues back to back (half a transformer block, a convolution layer) are launched so that
+// each may become resident while the kernel in front of it in its stream still drains (programmatic stream
+// serialization): launch, barrier set-up and tensor-memory allocation then cost nothing on the stream.  A kernel waits
+// for that predecessor - complete, its memory visible - in bb::pdl_sync() before it touches global memory, and only
+// then lets its own successor in, so a kernel never overlaps more than its direct neighbours and everything before the
+// predecessor is complete too.
+extern thread_local int bb_back_to_back;
+struct BackToBack {
+  const int n;
+  explicit BackToBack(bool on = true) : n(on ? 1 : 0) { bb_back_to_back += n; }
+  ~BackToBack() { bb_back_to_back -= n; }
+};
+template <typename... P, typename... A>
+inline cudaError_t bb_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = bb_back_to_back > 0 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
+}
+
 // One product of a k x k convolution whose patch matrix is never stored: the GEMM's producer gathers the
 // patches with im2col TMA loads (gemm_tcgen05.cu).  `x` is the NHWC tensor the patches come from.
 //   BB_CONV_FWD    D[P, Cout] = patches(x) * W^T                   x = input, channels C = Cin
@@ -88,6 +111,12 @@ __device__ __forceinline__ bool elect_one() {
       "selp.b32 %0, 1, 0, P;\n\t}"
       : "=r"(pred));
   return pred != 0;
+}
+
+// Called by every thread before its first access to global memory (see bb_launch).
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- mbarrier

@@ -50,6 +50,7 @@ constexpr int PATCH_U = 4;             // chunks per thread of the gather
 // col[(n, ho, wo), (r, s, c)] = x[n, ho*stride - pad + r, wo*stride - pad + s, c]  (0 outside)
 __global__ void __launch_bounds__(256)
 im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGeom g, const ConvMagic m) {
+  bb::pdl_sync();
   const unsigned chunks = g.C >> 3;                       // 16-byte chunks per pixel
   const unsigned row_chunks = g.k * g.k * chunks;
   const unsigned total = g.Wo * row_chunks;
@@ -83,6 +84,7 @@ im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGe
 // The taps that reach a pixel are every stride-th one; along them the output pixel moves back by one.
 __global__ void __launch_bounds__(256)
 col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const ConvGeom g, const ConvMagic m) {
+  bb::pdl_sync();
   const unsigned chunks = g.C >> 3;
   const unsigned total = g.W * chunks;
   const long long ld16 = g.ld_col >> 3;
@@ -135,8 +137,7 @@ extern "C" int bb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int
   }
   const int chunks = C >> 3, row_chunks = k * k * chunks;
   const ConvMagic m = {div_magic(row_chunks), div_magic(chunks), div_magic(k), div_magic(Ho)};
-  im2col_kernel<<<patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream>>>(
-      (const uint4*)x, (uint4*)col, g, m);
+  bb_launch(im2col_kernel, patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream, (const uint4*)x, (uint4*)col, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -150,8 +151,7 @@ extern "C" int bb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, i
   }
   const int chunks = C >> 3;
   const ConvMagic m = {0, div_magic(chunks), 0, div_magic(H)};
-  col2im_kernel<<<patch_grid((long long)W * chunks, 256, (long long)N * H), 256, 0, (cudaStream_t)stream>>>(
-      (const uint4*)dcol, (uint4*)dx, g, m);
+  bb_launch(col2im_kernel, patch_grid((long long)W * chunks, 256, (long long)N * H), 256, 0, (cudaStream_t)stream, (const uint4*)dcol, (uint4*)dx, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(256, BN_CTAS)
 bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, const uint4* __restrict__ yy,
                  const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma,
                  const __nv_bfloat16* __restrict__ beta, long long rows, int C, float* __restrict__ ws) {
+  bb::pdl_sync();
   __shared__ float sm[256 * 16];
   const int chunks = C >> 3;
   const long long gthreads = (long long)gridDim.x * blockDim.x;
@@ -295,6 +296,7 @@ __device__ __forceinline__ void bn_sum_partials(const float* __restrict__ ws, in
 __global__ void __launch_bounds__(1024)
 bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv_rows, float eps,
                        float* __restrict__ mean, float* __restrict__ rstd) {
+  bb::pdl_sync();
   float s1, s2;
   bn_sum_partials(ws, parts, C, s1, s2);
   const int c = blockIdx.x * 32 + threadIdx.x;
@@ -309,6 +311,7 @@ bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv
 __global__ void __launch_bounds__(1024)
 bn_finish_bwd_kernel(const float* __restrict__ ws, int parts, int C, float* __restrict__ sums,
                      float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  bb::pdl_sync();
   float s1, s2;
   bn_sum_partials(ws, parts, C, s1, s2);
   const int c = blockIdx.x * 32 + threadIdx.x;
@@ -325,6 +328,7 @@ __global__ void __launch_bounds__(256, BN_CTAS)
 bn_apply_kernel(const uint4* __restrict__ y, const float* __restrict__ mean, const float* __restrict__ rstd,
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
                 const uint4* __restrict__ residual, uint4* __restrict__ z, long long rows, int C, int relu) {
+  bb::pdl_sync();
   const int chunks = C >> 3;
   const long long gthreads = (long long)gridDim.x * blockDim.x;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -372,6 +376,7 @@ bn_bwd_apply_kernel(const uint4* __restrict__ dz, const uint4* __restrict__ zz, 
                     const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma,
                     const __nv_bfloat16* __restrict__ beta, const float* __restrict__ sums, uint4* __restrict__ dy,
                     uint4* __restrict__ dres, long long rows, int C, float inv_rows) {
+  bb::pdl_sync();
   constexpr int U = 2;         // four rows would take 128 registers
   const int chunks = C >> 3;
   const long long gthreads = (long long)gridDim.x * blockDim.x;
@@ -442,9 +447,9 @@ int bn_bwd(const void* dz, const void* z, const void* y, const float* mean, cons
   const __nv_bfloat16 *ga = (const __nv_bfloat16*)gamma, *be = (const __nv_bfloat16*)beta;
   const float inv = 1.0f / (float)rows;
 #define BB_BN_BWD(MASK)                                                                                               \
-  bn_reduce_kernel<RED_BWD, MASK><<<grid, 256, 0, s>>>(qd, qz, qy, mean, rstd, ga, be, rows, C, ws);                  \
-  bn_finish_bwd_kernel<<<(C + 31) / 32, 1024, 0, s>>>(ws, grid, C, sums, dgamma, dbeta);                             \
-  bn_bwd_apply_kernel<MASK><<<grid, 256, 0, s>>>(qd, qz, qy, mean, rstd, ga, be, sums, (uint4*)dy, (uint4*)dres, rows, C, inv)
+  bb_launch(bn_reduce_kernel<RED_BWD, MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, ga, be, rows, C, ws);                  \
+  bb_launch(bn_finish_bwd_kernel, (C + 31) / 32, 1024, 0, s, ws, grid, C, sums, dgamma, dbeta);                             \
+  bb_launch(bn_bwd_apply_kernel<MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, ga, be, sums, (uint4*)dy, (uint4*)dres, rows, C, inv)
   if (!relu) { BB_BN_BWD(MASK_NONE); }
   else if (be) { BB_BN_BWD(MASK_Y); }
   else { BB_BN_BWD(MASK_Z); }
@@ -471,9 +476,9 @@ extern "C" int bb_bn_stats(const void* y, long long rows, int C, float eps, floa
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = bn_grid(rows, C);
   float* ws = static_cast<float*>(workspace);
-  bn_reduce_kernel<RED_STATS, MASK_NONE><<<grid, 256, 0, s>>>((const uint4*)y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+  bb_launch(bn_reduce_kernel<RED_STATS, MASK_NONE>, grid, 256, 0, s, (const uint4*)y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                                                               rows, C, ws);
-  bn_finish_stats_kernel<<<(C + 31) / 32, 1024, 0, s>>>(ws, grid, C, 1.0f / (float)rows, eps, mean, rstd);
+  bb_launch(bn_finish_stats_kernel, (C + 31) / 32, 1024, 0, s, ws, grid, C, 1.0f / (float)rows, eps, mean, rstd);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -486,7 +491,7 @@ extern "C" int bb_bn_apply(const void* y, const float* mean, const float* rstd, 
     return BB_ERR_INVALID_ARG;
   }
   auto kernel = residual ? bn_apply_kernel<true> : bn_apply_kernel<false>;
-  kernel<<<bn_grid(rows, C), 256, 0, (cudaStream_t)stream>>>((const uint4*)y, mean, rstd, (const __nv_bfloat16*)gamma,
+  bb_launch(kernel, bn_grid(rows, C), 256, 0, (cudaStream_t)stream, (const uint4*)y, mean, rstd, (const __nv_bfloat16*)gamma,
                                                              (const __nv_bfloat16*)beta, (const uint4*)residual, (uint4*)z, rows, C, relu);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
@@ -750,6 +755,7 @@ extern "C" int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* 
     bb_set_last_error_msg("bb_conv_bn_fwd: bad descriptor, null buffer or scratch smaller than bb_conv_bn_scratch_bytes");
     return BB_ERR_INVALID_ARG;
   }
+  const BackToBack scope;
   uint8_t* sc = static_cast<uint8_t*>(scratch);
   if (s.implicit_x) {
     BB_TRY(conv_implicit(d, s, BB_CONV_FWD, x, d->w, y, stream));
@@ -775,6 +781,7 @@ int conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void*
     bb_set_last_error_msg("bb_conv_bn_bwd: bad descriptor, null buffer, missing gradient pointer or scratch too small");
     return BB_ERR_INVALID_ARG;
   }
+  const BackToBack scope;
   uint8_t* sc = static_cast<uint8_t*>(scratch);
   void* dy = sc;
   uint8_t* colbuf = sc + s.dy_bytes;

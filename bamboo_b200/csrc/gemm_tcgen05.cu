@@ -316,6 +316,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   else __syncthreads();
   bb::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  bb::pdl_sync();
 
   // Next work unit of this CTA as announced by the scheduling thread (-1: no more).  Called by a
   // whole warp (`warp_wide`) or by a single thread; the entry is handed back once it has been read.
@@ -868,10 +869,11 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * workers); cfg.blockDim = dim3(num_threads(EW));
     cfg.dynamicSmemBytes = C::SMEM_BYTES; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = bb_back_to_back > 0 ? 2 : 1;
     cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<BN, true, EW, CONV>, tmA, tmB, p, cp);
     if (le != cudaSuccess) {
       if (tt) tt->base[slot] -= (unsigned)tiles;     // nothing ran: the counter keeps its value
@@ -879,7 +881,7 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
       return BB_ERR_CUDA;
     }
   } else {
-    gemm_bf16_tcgen05_kernel<BN, false, EW, CONV><<<workers, num_threads(EW), C::SMEM_BYTES, stream>>>(tmA, tmB, p, cp);
+    bb_launch(gemm_bf16_tcgen05_kernel<BN, false, EW, CONV>, workers, num_threads(EW), C::SMEM_BYTES, stream, tmA, tmB, p, cp);
   }
   {
     cudaError_t le = cudaGetLastError();

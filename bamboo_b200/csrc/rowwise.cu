@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                      const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int h, float eps) {
+  bb::pdl_sync();
   const int lane = threadIdx.x & 31;
   const int warp_global = blockIdx.x * WARPS + (threadIdx.x >> 5);
   const int warp_stride = gridDim.x * WARPS;
@@ -81,6 +82,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                      const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows, int h) {
+  bb::pdl_sync();
   extern __shared__ float acc[];  // [warps][2][h], each lane owns its own columns
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
@@ -141,6 +143,7 @@ layernorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
                          const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                          const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows) {
+  bb::pdl_sync();
   constexpr int h = NCH * 256;
   extern __shared__ float acc[];  // [warps][2][h]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -237,6 +240,7 @@ layernorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
                           const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                           const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                           __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows, int h, int slots) {
+  bb::pdl_sync();
   extern __shared__ float sm[];
   using V = ColVec<CW>;
   using VT = typename V::T;
@@ -355,6 +359,7 @@ layernorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
 __global__ void __launch_bounds__(1024)
 reduce_partials_kernel(const float* __restrict__ partials, float* __restrict__ out0, float* __restrict__ out1,
                        float* __restrict__ out2, long long pair_offset, int nparts, int n, long long stride) {
+  bb::pdl_sync();
   __shared__ float red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + tx;
@@ -392,6 +397,7 @@ __device__ unsigned int g_colsum_tickets[COLSUM_TICKET_SLOTS];
 __global__ void __launch_bounds__(256)
 colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ partials, float* __restrict__ out, int rows, int n,
               long long ld, int rows_per_split, unsigned int* __restrict__ tickets) {
+  bb::pdl_sync();
   __shared__ float red[8][256];
   __shared__ int s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -525,8 +531,8 @@ extern "C" int bb_layernorm_fwd(const void* x, const void* gamma, const void* be
     bb_set_last_error_msg("bb_layernorm_fwd: null pointer or hidden size not a multiple of 8");
     return BB_ERR_INVALID_ARG;
   }
-  layernorm_fwd_kernel<<<row_grid(rows), WARPS * 32, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, mean, rstd, rows, h, eps);
+  bb_launch(layernorm_fwd_kernel, row_grid(rows), WARPS * 32, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma,
+            (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, mean, rstd, rows, h, eps);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -590,8 +596,8 @@ int ln_bwd_cols_launch(const void* dy, const void* x, const void* gamma, const f
   });
 #define BB_LNC_ARGS (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, mean, rstd, \
                     (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, rows, h, slots
-  if (sum_res) layernorm_bwd_cols_kernel<MAXT, CW, R, MINB, PF, true><<<grid, threads, sm_bytes, s>>>(BB_LNC_ARGS);
-  else layernorm_bwd_cols_kernel<MAXT, CW, R, MINB, PF, false><<<grid, threads, sm_bytes, s>>>(BB_LNC_ARGS);
+  if (sum_res) bb_launch(layernorm_bwd_cols_kernel<MAXT, CW, R, MINB, PF, true>, grid, threads, sm_bytes, s, BB_LNC_ARGS);
+  else bb_launch(layernorm_bwd_cols_kernel<MAXT, CW, R, MINB, PF, false>, grid, threads, sm_bytes, s, BB_LNC_ARGS);
 #undef BB_LNC_ARGS
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
@@ -622,11 +628,11 @@ int ln_bwd_main(const void* dy, const void* x, const void* gamma, const float* m
   });
 #define BB_LN_ARGS (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, mean, rstd, \
                    (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, rows
-  if (h == 256) layernorm_bwd_reg_kernel<1><<<grid, warps * 32, smem, s>>>(BB_LN_ARGS);
-  else if (h == 512) layernorm_bwd_reg_kernel<2><<<grid, warps * 32, smem, s>>>(BB_LN_ARGS);
-  else if (h == 768) layernorm_bwd_reg_kernel<3><<<grid, warps * 32, smem, s>>>(BB_LN_ARGS);
-  else if (h == 1024) layernorm_bwd_reg_kernel<4><<<grid, warps * 32, smem, s>>>(BB_LN_ARGS);
-  else layernorm_bwd_kernel<<<grid, warps * 32, smem, s>>>(BB_LN_ARGS, h);
+  if (h == 256) bb_launch(layernorm_bwd_reg_kernel<1>, grid, warps * 32, smem, s, BB_LN_ARGS);
+  else if (h == 512) bb_launch(layernorm_bwd_reg_kernel<2>, grid, warps * 32, smem, s, BB_LN_ARGS);
+  else if (h == 768) bb_launch(layernorm_bwd_reg_kernel<3>, grid, warps * 32, smem, s, BB_LN_ARGS);
+  else if (h == 1024) bb_launch(layernorm_bwd_reg_kernel<4>, grid, warps * 32, smem, s, BB_LN_ARGS);
+  else bb_launch(layernorm_bwd_kernel, grid, warps * 32, smem, s, BB_LN_ARGS, h);
 #undef BB_LN_ARGS
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
@@ -668,7 +674,7 @@ extern "C" int bb_layernorm_bwd(const void* dy, const void* x, const void* gamma
   const int grid = ln_bwd_grid(rows, h);
   float* ws = (float*)workspace;
   if (int rc = ln_bwd_main(dy, x, gamma, mean, rstd, dres, dx, ws, false, rows, h, grid, ln_bwd_warps(h), s)) return rc;
-  reduce_partials_kernel<<<dim3((h + 31) / 32, 2), 1024, 0, s>>>(ws, dgamma, dbeta, nullptr, (long long)h, grid, h, 2LL * h);
+  bb_launch(reduce_partials_kernel, dim3((h + 31) / 32, 2), 1024, 0, s, ws, dgamma, dbeta, nullptr, (long long)h, grid, h, 2LL * h);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -726,7 +732,7 @@ extern "C" int bb_layernorm_bwd_static(const void* dy, const void* x, const void
   // every partial row that the reduction reads is rewritten by this launch, so the scratch
   // needs no clearing although it still holds the previous call's sums
   if (int rc = ln_bwd_main(dy, x, gamma, mean, rstd, dres, dx, ws, false, rows, h, grid, warps, s)) return rc;
-  reduce_partials_kernel<<<dim3((h + 31) / 32, 2), 1024, 0, s>>>(ws, dgamma, dbeta, nullptr, (long long)h, grid, h, 2LL * h);
+  bb_launch(reduce_partials_kernel, dim3((h + 31) / 32, 2), 1024, 0, s, ws, dgamma, dbeta, nullptr, (long long)h, grid, h, 2LL * h);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -796,7 +802,7 @@ extern "C" int bb_colsum_accum(const void* dy, long long ld, float* out, void* w
   dim3 grid((n + 255) / 256, splits);
   unsigned int* tickets = colsum_tickets((int)grid.x);
   if (!tickets) { bb_set_last_error_msg("bb_colsum_accum: ticket counters unavailable on this device"); return BB_ERR_CUDA; }
-  colsum_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)dy, (float*)workspace, out, rows, n, ld, rps, tickets);
+  bb_launch(colsum_kernel, grid, 256, 0, s, (const __nv_bfloat16*)dy, (float*)workspace, out, rows, n, ld, rps, tickets);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }
@@ -829,7 +835,7 @@ extern "C" int bb_layernorm_bwd_res(const void* dy, const void* x, const void* g
   }
   const int grid = ln_bwd_grid(rows, h);
   if (int rc = ln_bwd_main(dy, x, gamma, mean, rstd, dres, dx, ws, true, rows, h, grid, ln_bwd_warps(h), s)) return rc;
-  reduce_partials_kernel<<<dim3((h + 31) / 32, 3), 1024, 0, s>>>(ws, dgamma, dbeta, dres_sum, (long long)h, grid, h, 3LL * h);
+  bb_launch(reduce_partials_kernel, dim3((h + 31) / 32, 3), 1024, 0, s, ws, dgamma, dbeta, dres_sum, (long long)h, grid, h, 3LL * h);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
 }

@@ -9,6 +9,8 @@ thread_local char g_err[512] = "";
 __device__ int g_status_word = 0;
 }  // namespace
 
+thread_local int bb_back_to_back = 0;
+
 void bb_set_last_error(const char* what, cudaError_t e) {
   snprintf(g_err, sizeof(g_err), "%s: %s", what, cudaGetErrorString(e));
 }

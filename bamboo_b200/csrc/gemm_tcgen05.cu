@@ -894,7 +894,7 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   return BB_OK;
 }
 
-// Whether a problem runs as CTA pairs (see choose_tile)
+// Whether a weight gradient of the widest tile would run as CTA pairs
 bool pairs_pay(int M, int N, int K) {
   const long long tiles_single = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);
   return M > BM && N > 128 && (K >= 2048 || tiles_single >= 16LL * bb_num_sms());
@@ -945,29 +945,56 @@ AccumPlan plan_accum(int M, int N, int K) {
   return best;
 }
 
-// Tile width, and whether CTA pairs / sixteen epilogue warps are used.
+// Products that are stored: tile width and pairing by the time that they are expected to take, in microseconds.  A tile
+// costs a rate per k-block (128 x 128, 128 x 256, and 128 x 256 for each CTA of a pair, the cheapest per output because
+// it loads least) and, wave after wave, what its epilogue leaves uncovered; once per launch its start and its last
+// epilogue.  Fitted on 8 shapes each of 12 problem sizes between 512 x 256 x 256 and 4096 x 16384 x 4096, where it is
+// within a tenth of the measured times; what the choice gained where it changed (us, with a fixed rule before):
+// 513 x 2048 x 2048 26.6 -> 20.5 (128 wide instead of a quarter-filled wave of pairs), 999 x 1024 x 4096 34.8 -> 28.7,
+// 4096 x 1024 x 1024 20.4 -> 16.4 and 8192 x 512 x 1536 24.6 -> 20.5 (one wave of 256 wide tiles instead of two).
+struct StorePlan { int bn; bool pair; };
+StorePlan plan_store(int M, int N, int K, int max_ctas, bool pairs_allowed) {
+  static const struct { int bn; bool pair; double kblock, wave, once; } kinds[3] = {
+      {256, true, 0.34, 2.3, 10.5}, {256, false, 0.41, 1.2, 8.5}, {128, false, 0.30, 1.2, 8.0}};
+  const double kb = (double)((K + BK - 1) / BK);
+  StorePlan best = {128, false};
+  double best_us = -1;
+  for (const auto& k : kinds) {
+    if ((k.bn == 256 && N <= 128) || (k.pair && (!pairs_allowed || M <= BM))) continue;
+    const long long tm = k.pair ? 2 * BM : BM;
+    const long long tiles = ((M + tm - 1) / tm) * ((N + k.bn - 1) / k.bn);
+    long long workers = bb_num_sms();
+    if (max_ctas > 0 && max_ctas < workers) workers = max_ctas;
+    if (k.pair) workers = workers > 1 ? workers / 2 : 1;
+    const double us = (double)((tiles + workers - 1) / workers) * (kb * k.kblock + k.wave) + k.once;
+    if (best_us < 0 || us < best_us) { best_us = us; best = {k.bn, k.pair}; }
+  }
+  return best;
+}
+
+// Tile width (0: the descriptor names none that exists), pairing, epilogue warps, and the split of a weight gradient
 int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
   const int e = g->epilogue;
+  *wide_out = false;
   if (e == BB_EPI_ACCUM_F32 && g->split_k <= 0 && g->tile_n == 0 && g->cta_pair == 0) {
     const AccumPlan pl = plan_accum(g->M, g->N, g->K);
     g->split_k = pl.ksplit;
-    *pair_out = pl.pair; *wide_out = false;
+    *pair_out = pl.pair;
     return pl.bn;
   }
-  // CTA pairs (256 x 256 per pair) pay off on long reductions and on long runs of tiles per
-  // CTA; short problems are quicker to start and drain as single CTAs (measured on B200:
-  // K >= 3072 or >= 40 tiles per CTA 2-6 % faster as pairs, K = 1024 with <= 7 tiles 4-8 % slower)
-  *pair_out = g->cta_pair > 0 || (g->cta_pair == 0 && g->tile_n == 0 && pairs_pay(g->M, g->N, g->K));
   // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant)
   *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048);
-  int bn = g->tile_n;
-  if (bn == 0) {
-    // 256-wide tiles halve the A re-reads; use them when they still fill the machine
-    const long long tiles256 = (long long)((g->M + BM - 1) / BM) * ((g->N + 255) / 256);
-    // the add-reduction epilogue can split K to fill the machine, so it always takes wide tiles
-    bn = (g->N > 128 && (tiles256 >= bb_num_sms() || e == BB_EPI_ACCUM_F32)) ? 256 : 128;
+  *pair_out = g->cta_pair > 0;
+  if (g->cta_pair > 0) return 256;
+  if (g->tile_n != 0) return g->tile_n;
+  // an add-reduction whose split was given takes wide tiles: the split fills the machine
+  if (e == BB_EPI_ACCUM_F32) {
+    *pair_out = g->cta_pair == 0 && pairs_pay(g->M, g->N, g->K);
+    return g->N > 128 ? 256 : 128;
   }
-  return bn;
+  const StorePlan pl = plan_store(g->M, g->N, g->K, g->max_ctas, g->cta_pair == 0);
+  *pair_out = pl.pair;
+  return pl.bn;
 }
 
 }  // namespace

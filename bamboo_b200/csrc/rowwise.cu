@@ -73,6 +73,60 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
   }
 }
 
+// The same for hidden sizes up to 1024, a row in registers: one read with all of a row's loads in flight, where the loop
+// above goes three times through L1 with one load in flight each time.  Same sums in the same order.  8192 x 1024 10.9 ->
+// 9.9 us, 8192 x 768 10.6 -> 8.8 us; wider rows lose more to the registers than they win (4096 x 4096: 17.8 -> 24.7 us).
+template <int NCH>
+__global__ void __launch_bounds__(WARPS * 32)
+layernorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+                         const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+                         float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int h, float eps) {
+  bb::pdl_sync();
+  const int lane = threadIdx.x & 31;
+  const int warp_stride = gridDim.x * WARPS;
+  const int nch = h >> 3;
+  for (int row = blockIdx.x * WARPS + (threadIdx.x >> 5); row < rows; row += warp_stride) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
+    uint4 q[NCH];
+#pragma unroll
+    for (int u = 0; u < NCH; ++u) {
+      const int c = lane + 32 * u;
+      q[u] = c < nch ? __ldg(xr + c) : make_uint4(0, 0, 0, 0);
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < NCH; ++u) {
+      float f[8]; unpack8(q[u], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += f[i];
+    }
+    const float mean = warp_sum(s) / (float)h;
+    float v = 0.f;
+#pragma unroll
+    for (int u = 0; u < NCH; ++u) {
+      if (lane + 32 * u >= nch) break;
+      float f[8]; unpack8(q[u], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { float d = f[i] - mean; v += d * d; }
+    }
+    const float rstd = rsqrtf(warp_sum(v) / (float)h + eps);
+    uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * h);
+#pragma unroll
+    for (int u = 0; u < NCH; ++u) {
+      const int c = lane + 32 * u;
+      if (c >= nch) break;
+      float f[8], g[8], b[8];
+      unpack8(q[u], f);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(beta) + c), b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = (f[i] - mean) * rstd * g[i] + b[i];
+      yr[c] = pack8(f);
+    }
+    if (lane == 0) { mean_out[row] = mean; rstd_out[row] = rstd; }
+  }
+}
+
 // ------------------------------------------------------------------ LayerNorm backward
 // dx = rstd * (dy*gamma - mean(dy*gamma) - xhat * mean(dy*gamma*xhat)) [+ dres]
 // Per-CTA partial sums of dgamma = sum dy*xhat and dbeta = sum dy go to `partials`
@@ -531,7 +585,10 @@ extern "C" int bb_layernorm_fwd(const void* x, const void* gamma, const void* be
     bb_set_last_error_msg("bb_layernorm_fwd: null pointer or hidden size not a multiple of 8");
     return BB_ERR_INVALID_ARG;
   }
-  bb_launch(layernorm_fwd_kernel, row_grid(rows), WARPS * 32, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma,
+  const int per_lane = (h / 8 + 31) / 32;            // 16-byte chunks of a row per lane
+  auto kernel = per_lane <= 1 ? layernorm_fwd_reg_kernel<1> : per_lane <= 2 ? layernorm_fwd_reg_kernel<2>
+                : per_lane <= 4 ? layernorm_fwd_reg_kernel<4> : layernorm_fwd_kernel;
+  bb_launch(kernel, row_grid(rows), WARPS * 32, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma,
             (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, mean, rstd, rows, h, eps);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;

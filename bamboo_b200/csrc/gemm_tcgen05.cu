@@ -932,8 +932,12 @@ AccumPlan plan_accum(int M, int N, int K) {
     const long long tiles = ((M + tm - 1) / tm) * ((N + bn - 1) / bn);
     const long long workers = pair ? bb_num_sms() / 2 : bb_num_sms();
     const double per_kb = pair ? 2.9 : (bn == 256 ? 3.0 : 2.0), fixed = bn == 256 ? 2 * EPI : EPI;
-    const long long smax = workers / tiles > 16 ? workers / tiles : 16;
-    for (long long s = 1; s <= smax; ++s) {
+    // up to 16, then the largest that stays within one wave: between the two a larger split only shortens the units
+    long long widest = workers / tiles;
+    if (widest > (kb - 1) / 7) widest = (kb - 1) / 7;        // (the largest with eight k-blocks per unit)
+    for (int i = 1; i <= 17; ++i) {
+      const long long s = i <= 16 ? i : widest;
+      if (i == 17 && widest <= 16) break;
       const long long kbs = (kb + s - 1) / s;
       if (s > 1 && kbs < 8) break;
       if (kbs > longest) continue;

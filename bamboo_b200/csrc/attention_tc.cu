@@ -955,7 +955,7 @@ attn_tc_dq_convert_kernel(const TcParams p) {
   }
 }
 
-// ------------------------------------------------------------------ forward (two query tiles in ping-pong)
+// ------------------------------------------------------------------ forward at head dimension 128 (two query tiles in ping-pong)
 // A CTA owns 256 query rows of one (batch, head) as two 128-row tiles; compute group g (4 warps,
 // one query row per thread) runs the online softmax of tile g.  Keys/values stream in 64-row
 // sub-tiles that serve both query tiles.  Per sub-block jj and group g:
@@ -970,7 +970,7 @@ attn_tc_dq_convert_kernel(const TcParams p) {
 // fp32 / bf16 range; the final division by the row sum makes the choice of reference immaterial.
 // smem: Q_0, Q_1 [128 x D] | K, V sub-tiles [64 x D] x NKV stages | P_g,b [128 x 64] x 4
 // TMEM: S_g,b at 128 g + 64 b | O_g at 256 + 128 g (D columns)
-// Head dimension D = 64 or 128.  A [rows x 128] operand lies in shared memory as two [rows x 64] atoms of
+// (The template also fits D = 64, where the kernel after this one is faster.)  A [rows x 128] operand lies in shared memory as two [rows x 64] atoms of
 // 128-byte rows, one after the other (two TMA boxes): the score product walks its eight 16-column k-steps
 // through both atoms; V as the B operand of P V (N = D, its columns) names the distance between the atoms in
 // the descriptor's leading-dimension field.  The whole tensor memory is in use at D = 128 (2 x 2 score

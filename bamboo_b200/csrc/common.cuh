@@ -86,7 +86,15 @@ struct bb_conv_gemm_args {
 bool bb_conv_gemm_supported(int C, int k, int stride, int pad);
 int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream);
 
+// Division by a number known at launch: n / d = high word of n * magic with magic = floor(2^64 / d) + 1 (0 stands for
+// d = 1); for n < 2^32 the error n * d / 2^64 stays below 1.
+inline unsigned long long bb_div_magic(int d) { return d == 1 ? 0 : ~0ull / (unsigned long long)d + 1; }
+
 namespace bb {
+
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
+  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -39,11 +39,6 @@ struct ConvGeom {
 // then take three multiplications by reciprocals.  With a 64-bit division per index, the 7 x 7 / stride 2 gather of
 // 32 x 224 x 224 x 8 took 144 us for its 315 MB (arithmetic, not memory; now 72 us), the fourteen adjoint gathers of an
 // image-network step 574 us (now 442 us).
-// n / d for n < 2^32 with magic = floor(2^64 / d) + 1 (0 for d = 1): the error n * d / 2^64 stays below 1
-__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
-  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
-}
-unsigned long long div_magic(int d) { return d == 1 ? 0 : ~0ull / (unsigned long long)d + 1; }
 struct ConvMagic { unsigned long long row_chunks, chunks, k, rows; };
 constexpr int PATCH_U = 4;             // chunks per thread of the gather
 
@@ -57,7 +52,7 @@ im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGe
   const long long ld16 = g.ld_col >> 3;
   const unsigned e0 = blockIdx.x * (256 * PATCH_U) + threadIdx.x;
   for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.Ho; row += gridDim.y) {
-    const unsigned n = fast_div(row, m.rows);
+    const unsigned n = bb::fast_div(row, m.rows);
     const int h0 = (int)(row - n * g.Ho) * g.stride - g.pad;
     const uint4* xi = x + (long long)n * g.H * g.W * chunks;
     uint4* out = col + (long long)row * g.Wo * ld16;
@@ -66,9 +61,9 @@ im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGe
 #pragma unroll
     for (int u = 0; u < PATCH_U; ++u) {
       const unsigned e = e0 + u * 256;
-      const unsigned wo = fast_div(e, m.row_chunks), within = e - wo * row_chunks;
-      const unsigned tap = fast_div(within, m.chunks), cc = within - tap * chunks;
-      const unsigned r = fast_div(tap, m.k), s = tap - r * g.k;
+      const unsigned wo = bb::fast_div(e, m.row_chunks), within = e - wo * row_chunks;
+      const unsigned tap = bb::fast_div(within, m.chunks), cc = within - tap * chunks;
+      const unsigned r = bb::fast_div(tap, m.k), s = tap - r * g.k;
       const int h = h0 + (int)r, w = (int)wo * g.stride - g.pad + (int)s;
       dst[u] = e < total ? (long long)wo * ld16 + within : -1;
       v[u] = make_uint4(0, 0, 0, 0);
@@ -90,10 +85,10 @@ col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const Conv
   const long long ld16 = g.ld_col >> 3;
   const unsigned e = blockIdx.x * 256 + threadIdx.x;
   if (e >= total) return;
-  const unsigned w = fast_div(e, m.chunks), cc = e - w * chunks;
+  const unsigned w = bb::fast_div(e, m.chunks), cc = e - w * chunks;
   const int s0 = (int)(w + g.pad) % g.stride, wo0 = (int)(w + g.pad) / g.stride;
   for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.H; row += gridDim.y) {
-    const unsigned n = fast_div(row, m.rows);
+    const unsigned n = bb::fast_div(row, m.rows);
     const int h = (int)(row - n * g.H);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int ho = (h + g.pad) / g.stride;
@@ -136,7 +131,7 @@ extern "C" int bb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int
     return BB_ERR_INVALID_ARG;
   }
   const int chunks = C >> 3, row_chunks = k * k * chunks;
-  const ConvMagic m = {div_magic(row_chunks), div_magic(chunks), div_magic(k), div_magic(Ho)};
+  const ConvMagic m = {bb_div_magic(row_chunks), bb_div_magic(chunks), bb_div_magic(k), bb_div_magic(Ho)};
   bb_launch(im2col_kernel, patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream, (const uint4*)x, (uint4*)col, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
@@ -150,7 +145,7 @@ extern "C" int bb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, i
     return BB_ERR_INVALID_ARG;
   }
   const int chunks = C >> 3;
-  const ConvMagic m = {0, div_magic(chunks), 0, div_magic(H)};
+  const ConvMagic m = {0, bb_div_magic(chunks), 0, bb_div_magic(H)};
   bb_launch(col2im_kernel, patch_grid((long long)W * chunks, 256, (long long)N * H), 256, 0, (cudaStream_t)stream, (const uint4*)dcol, (uint4*)dx, g, m);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;

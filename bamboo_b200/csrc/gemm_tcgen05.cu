@@ -22,7 +22,8 @@
 //   a_mn = 0 : A is [M, K] (K contiguous)     a_mn = 1 : A is stored [K, M] (M contiguous)
 //   b_mn = 0 : B is [N, K] (K contiguous)     b_mn = 1 : B is stored [K, N] (N contiguous)
 // which covers a linear layer's forward (0,0), input gradient (0,1) and weight gradient
-// (1,1) without a transpose pass.
+// (1,1) without a transpose pass.  A convolution's patch matrix as A or B is gathered by the producer
+// (template parameter CONV, bb_conv_gemm).
 #include "common.cuh"
 #include "bamboo_b200.h"
 #include "tma_host.cuh"
@@ -80,11 +81,6 @@ struct ConvParams {
 struct NoConv {};
 template <bool CONV> struct ConvArg { typedef NoConv type; };
 template <> struct ConvArg<true> { typedef ConvParams type; };
-
-// n / d for n < 2^32 with magic = floor(2^64 / d) + 1 (0 for d = 1): the error n * d / 2^64 stays below 1
-__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
-  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
-}
 
 __device__ __forceinline__ void unpack8(const uint4& q, float* f) {
   f[0] = bb::bf16_lo(q.x); f[1] = bb::bf16_hi(q.x); f[2] = bb::bf16_lo(q.y); f[3] = bb::bf16_hi(q.y);
@@ -354,7 +350,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           // image).  FWD / DGRAD gather A (windows = output rows, k-blocks run over taps x channel blocks),
           // WGRAD gathers B (windows = the reduction, columns = taps x channels).
           auto window = [&](unsigned px, int& w, int& h, int& n) {
-            const unsigned row = fast_div(px, cv.magic_w), img = fast_div(row, cv.magic_h);
+            const unsigned row = bb::fast_div(px, cv.magic_w), img = bb::fast_div(row, cv.magic_h);
             w = (int)(px - row * cv.Wo) * cv.stride - cv.pad;
             h = (int)(row - img * cv.Ho) * cv.stride - cv.pad;
             n = (int)img;
@@ -819,8 +815,8 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
     cp.mode = cv->mode; cp.k = cv->k; cp.stride = cv->stride; cp.pad = cv->pad; cp.cblocks = cv->C / 64;
     cp.wcols = cv->mode == BB_CONV_DGRAD ? cv->other_channels : cv->C;
     cp.Wo = cv->Wo; cp.Ho = cv->Ho;
-    cp.magic_w = cv->Wo == 1 ? 0 : ~0ull / (unsigned long long)cv->Wo + 1;
-    cp.magic_h = cv->Ho == 1 ? 0 : ~0ull / (unsigned long long)cv->Ho + 1;
+    cp.magic_w = bb_div_magic(cv->Wo);
+    cp.magic_h = bb_div_magic(cv->Ho);
   }
   GemmParams p;
   p.M = g->M; p.N = g->N; p.K = g->K; p.a_mn = g->a_mn_major; p.b_mn = g->b_mn_major; p.epi = g->epilogue;

@@ -7,9 +7,9 @@ blocks, avgpool, flatten, fc).  Here the list is ``ResNetStem`` (conv1 + bn1 + r
 50 x ``Bottleneck``, ``ResNetHead`` (avgpool + flatten + fc): the same boundaries between blocks,
 with the stem's four and the head's three entries each fused into one layer.
 
-Every convolution is the library's tcgen05 GEMM over a patch matrix (rows = output pixels,
-columns = taps x input channels; a 1 x 1 / stride 1 convolution reads the activation tensor
-itself), followed by batch norm with batch statistics, the residual add and ReLU in one
+Every convolution is the library's tcgen05 GEMM over a patch matrix (rows = output pixels, columns = taps x input
+channels) that is never stored where channels come in blocks of 64: the GEMM's loads gather the patches (a 1 x 1 /
+stride 1 convolution reads the activation tensor itself). The products are followed by batch norm with batch statistics, the residual add and ReLU in one
 element-wise pass.  Weights are stored ``[Cout, k, k, Cin]`` (flattened to 2-D), activations
 ``[N, H, W, C]``; channel counts are multiples of 8, so the 3-channel input is carried in 8
 channels with five zero planes.  Batch-norm running statistics are not kept: they do not enter a

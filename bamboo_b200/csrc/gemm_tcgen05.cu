@@ -982,8 +982,11 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     *pair_out = pl.pair;
     return pl.bn;
   }
-  // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant)
-  *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048);
+  // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant), and for the residual add,
+  // whose operand comes from memory: twice the warps have twice the loads in flight
+  // (2331 x 1024 x 1024 16.1 -> 14.9 us, 4096 x 1024 x 1024 16.9 -> 15.1 us, 8192 x 1024 x 4096 56.7 -> 55.8 us; none slower)
+  *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_RESIDUAL ||
+                                                          ((e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048)));
   *pair_out = g->cta_pair > 0;
   if (g->cta_pair > 0) return 256;
   if (g->tile_n != 0) return g->tile_n;

@@ -1379,7 +1379,7 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int c0 = j * SUB;
       // only sub-blocks that touch the causal diagonal or the end of the sequence need masks
       const bool need_mask = (c0 + SUB > p.S) || (p.causal && c0 + SUB - 1 > q0);
-      uint32_t sc[64];                                       // the row's scores, then its probabilities
+      uint32_t sc[64];                                       // the row's scores
       bb::tmem_ld_32x32b_x32(tS, sc);
       bb::tmem_ld_32x32b_x32(tS + 32, sc + 32);
       bb::tmem_ld_wait();
@@ -1404,14 +1404,20 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         l_i *= alpha;
       }
       const float nm = (m_ref == -INFINITY) ? 0.f : -m_ref;
-      float rs[4] = {0.f, 0.f, 0.f, 0.f};
+      // exp2(-inf) = 0 covers the masked entries.  The row sum takes columns i and i + 32 together, i ascending: the
+      // two-tile kernel's order, so that a row's result does not depend on which kernel computed it
+      float rs = 0.f;
+      uint32_t pk[32];
 #pragma unroll
-      for (int i = 0; i < 64; i += 2) {                      // exp2(-inf) = 0 covers the masked entries
-        const float x = ex2(fmaf(__uint_as_float(sc[i]), sl, nm)), y = ex2(fmaf(__uint_as_float(sc[i + 1]), sl, nm));
-        rs[(i >> 1) & 3] += x + y;
-        sc[i >> 1] = bb::pack_bf16x2(x, y);
+      for (int i = 0; i < 32; i += 2) {
+        const float x0 = ex2(fmaf(__uint_as_float(sc[i]), sl, nm)), y0 = ex2(fmaf(__uint_as_float(sc[i + 32]), sl, nm));
+        const float x1 = ex2(fmaf(__uint_as_float(sc[i + 1]), sl, nm)), y1 = ex2(fmaf(__uint_as_float(sc[i + 33]), sl, nm));
+        rs += x0 + y0;
+        rs += x1 + y1;
+        pk[i >> 1] = bb::pack_bf16x2(x0, x1);
+        pk[16 + (i >> 1)] = bb::pack_bf16x2(y0, y1);
       }
-      l_i += (rs[0] + rs[1]) + (rs[2] + rs[3]);
+      l_i += rs;
       if (j > 0) {
         // the previous product has retired: its P buffer is free and the accumulator is at rest
         if (!bb::mbar_wait_warp(pv_full, (j - 1) & 1, &ctl->abort_flag, p.status)) { alive = false; break; }
@@ -1430,8 +1436,8 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           bb::tmem_st_wait();
         }
       }
-      atom_store_half_row(sP, row, 0, sc);
-      atom_store_half_row(sP, row, 1, sc + 16);
+      atom_store_half_row(sP, row, 0, pk);
+      atom_store_half_row(sP, row, 1, pk + 16);
       bb::tc_fence_before_sync();
       bb::fence_proxy_async();
       __syncwarp();

@@ -524,3 +524,21 @@ def test_attention_head_dim_64_tile_edges(L, B, H, S, causal, grow):
     L.attention_bwd(qkv, out, do, lse, dqkv, B, H, S, D, causal)
     close(dqkv, qf.grad)
     assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("B,H,S,causal,want_out,want_lse",
+                         [(2, 3, 257, False, "9a5419f9f8e4b22c", "28ec0ae142d23f85"), (1, 2, 1000, True, "17536437b67bc51e", "0507974505271b4a"),
+                          (3, 1, 64, True, "30ae10657d9dc1ad", "2a728876a08dc590")])
+def test_attention_head_dim_64_keeps_its_summation_order(L, B, H, S, causal, want_out, want_lse):
+    """Output and log-sum-exp in every bit: digests of what the two-tile kernel (one CTA per 256 query rows), which had this
+    head dimension before, gives for the same inputs.  A row's sum takes columns i and i + 32 of a sub-block together,
+    i ascending; any other order changes last bits of the log-sum-exp and, after a few layers, every activation."""
+    import hashlib
+    D = 64
+    i = torch.arange(B * S * 3 * H * D)
+    qkv = ((i * 2654435761 % 65521).float() / 65521 * 4 - 2).view(B * S, 3 * H * D).bfloat16().cuda()
+    out = torch.empty(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(B, H, S, device="cuda")
+    L.attention_fwd(qkv, out, lse, B, H, S, D, causal)
+    digest = [hashlib.sha256(t.cpu().view(torch.uint8).numpy().tobytes()).hexdigest()[:16] for t in (out, lse)]
+    assert digest == [want_out, want_lse]

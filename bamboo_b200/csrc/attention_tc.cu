@@ -136,7 +136,7 @@ struct Ctl {
 // accumulator of the fused backward kernel, when there is one.
 template <int D>
 __global__ void __launch_bounds__(256)
-attn_tc_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const TcParams p) {
+attn_tc_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const TcParams p) {
   bb::pdl_sync();
   constexpr int LANES = D / 8;                                 // lanes of one (token, head)
   const int per_tok = p.H * LANES;                             // 16-byte chunks per token row
@@ -158,8 +158,8 @@ attn_tc_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* _
       a[u] = make_uint4(0, 0, 0, 0); b[u] = a[u];
       if (cc[u] < total) {
         const long long tok = cc[u] / per_tok; const int within = (int)(cc[u] % per_tok);
-        a[u] = __ldg(reinterpret_cast<const uint4*>(o + tok * p.stride_o + within * 8));
-        b[u] = __ldg(reinterpret_cast<const uint4*>(d_o + tok * p.stride_o + within * 8));
+        a[u] = __ldca(reinterpret_cast<const uint4*>(o + tok * p.stride_o + within * 8));
+        b[u] = __ldca(reinterpret_cast<const uint4*>(d_o + tok * p.stride_o + within * 8));
       }
     }
 #pragma unroll

@@ -122,7 +122,11 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
-// Called by every thread before its first access to global memory (see bb_launch).
+// Called by every thread before its first access to global memory (see bb_launch).  A kernel that calls it may be
+// resident while its predecessor still writes, so what a kernel may have written is not constant for its successor's
+// lifetime and must not be read through the read-only path: no __ldg and no `const T* __restrict__` (which lets the
+// compiler choose that path, and move the load) on anything but parameters (gamma, beta, bias), and no __restrict__ on
+// what is added to.  __ldca and __ldcg are coherent and stay behind the wait, as do plain loads through other pointers.
 __device__ __forceinline__ void pdl_sync() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -44,7 +44,7 @@ constexpr int PATCH_U = 4;             // chunks per thread of the gather
 
 // col[(n, ho, wo), (r, s, c)] = x[n, ho*stride - pad + r, wo*stride - pad + s, c]  (0 outside)
 __global__ void __launch_bounds__(256)
-im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGeom g, const ConvMagic m) {
+im2col_kernel(const uint4* x, uint4* __restrict__ col, const ConvGeom g, const ConvMagic m) {
   bb::pdl_sync();
   const unsigned chunks = g.C >> 3;                       // 16-byte chunks per pixel
   const unsigned row_chunks = g.k * g.k * chunks;
@@ -67,7 +67,7 @@ im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGe
       const int h = h0 + (int)r, w = (int)wo * g.stride - g.pad + (int)s;
       dst[u] = e < total ? (long long)wo * ld16 + within : -1;
       v[u] = make_uint4(0, 0, 0, 0);
-      if (e < total && h >= 0 && h < g.H && w >= 0 && w < g.W) v[u] = __ldg(xi + ((long long)h * g.W + w) * chunks + cc);
+      if (e < total && h >= 0 && h < g.H && w >= 0 && w < g.W) v[u] = __ldca(xi + ((long long)h * g.W + w) * chunks + cc);
     }
 #pragma unroll
     for (int u = 0; u < PATCH_U; ++u) if (dst[u] >= 0) out[dst[u]] = v[u];
@@ -78,7 +78,7 @@ im2col_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, const ConvGe
 // Gather form (one thread owns an input pixel's chunk): no atomics, fixed summation order (r, then s, ascending).
 // The taps that reach a pixel are every stride-th one; along them the output pixel moves back by one.
 __global__ void __launch_bounds__(256)
-col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const ConvGeom g, const ConvMagic m) {
+col2im_kernel(const uint4* dcol, uint4* __restrict__ dx, const ConvGeom g, const ConvMagic m) {
   bb::pdl_sync();
   const unsigned chunks = g.C >> 3;
   const unsigned total = g.W * chunks;
@@ -100,7 +100,7 @@ col2im_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, const Conv
       for (int s = s0; s < g.k; s += g.stride, --wo) {
         if (wo < 0 || wo >= g.Wo) continue;
         float f[8];
-        unpack8(__ldg(src + (long long)wo * ld16 + s * chunks), f);
+        unpack8(__ldca(src + (long long)wo * ld16 + s * chunks), f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] += f[i];
       }
@@ -180,8 +180,8 @@ __device__ __forceinline__ bool bn_positive(float v) { return v > 4.5917748e-41f
 
 template <int MODE, int MASK>
 __global__ void __launch_bounds__(256, BN_CTAS)
-bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, const uint4* __restrict__ yy,
-                 const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma,
+bn_reduce_kernel(const uint4* a, const uint4* zz, const uint4* yy,
+                 const float* mean, const float* rstd, const __nv_bfloat16* __restrict__ gamma,
                  const __nv_bfloat16* __restrict__ beta, long long rows, int C, float* __restrict__ ws) {
   bb::pdl_sync();
   __shared__ float sm[256 * 16];
@@ -196,7 +196,7 @@ bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, cons
   if (MODE == RED_BWD) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      mu[i] = mean[cc * 8 + i]; rs[i] = rstd[cc * 8 + i];
+      mu[i] = __ldca(mean + cc * 8 + i); rs[i] = __ldca(rstd + cc * 8 + i);
       if (MASK == MASK_Y) bn_scale_shift(__bfloat162float(gamma[cc * 8 + i]), __bfloat162float(beta[cc * 8 + i]), mu[i], rs[i], sc[i], sh[i]);
     }
   }
@@ -208,9 +208,9 @@ bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, cons
     for (int u = 0; u < BN_U; ++u) {
       const long long ru = r + u * row_step;
       const bool in = ru < rows;
-      qa[u] = in ? __ldg(a + ru * chunks + cc) : zero;
-      if (MODE == RED_BWD) qy[u] = in ? __ldg(yy + ru * chunks + cc) : zero;
-      if (MASK == MASK_Z) qz[u] = in ? __ldg(zz + ru * chunks + cc) : zero;
+      qa[u] = in ? __ldca(a + ru * chunks + cc) : zero;
+      if (MODE == RED_BWD) qy[u] = in ? __ldca(yy + ru * chunks + cc) : zero;
+      if (MASK == MASK_Z) qz[u] = in ? __ldca(zz + ru * chunks + cc) : zero;
     }
 #pragma unroll
     for (int u = 0; u < BN_U; ++u) {
@@ -259,7 +259,7 @@ bn_reduce_kernel(const uint4* __restrict__ a, const uint4* __restrict__ zz, cons
 // the result does not depend on scheduling.  A thread per channel walking all (up to 592) partial rows is
 // a chain of that many L2 latencies: 26-28 us per call at 592 rows, against about 3 us this way.
 // Valid in warp 0 only: t1, t2 of channel blockIdx.x * 32 + lane.
-__device__ __forceinline__ void bn_sum_partials(const float* __restrict__ ws, int parts, int C, float& t1, float& t2) {
+__device__ __forceinline__ void bn_sum_partials(const float* ws, int parts, int C, float& t1, float& t2) {
   __shared__ float sm1[32][33], sm2[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -271,12 +271,12 @@ __device__ __forceinline__ void bn_sum_partials(const float* __restrict__ ws, in
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float* row = ws + (long long)(p + 32 * u) * 2 * C + c;
-        a[u] = __ldg(row); b[u] = __ldg(row + C);
+        a[u] = __ldca(row); b[u] = __ldca(row + C);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) { s1 += a[u]; s2 += b[u]; }
     }
-    for (; p < parts; p += 32) { const float* row = ws + (long long)p * 2 * C + c; s1 += __ldg(row); s2 += __ldg(row + C); }
+    for (; p < parts; p += 32) { const float* row = ws + (long long)p * 2 * C + c; s1 += __ldca(row); s2 += __ldca(row + C); }
   }
   sm1[w][lane] = s1; sm2[w][lane] = s2;
   __syncthreads();
@@ -289,7 +289,7 @@ __device__ __forceinline__ void bn_sum_partials(const float* __restrict__ ws, in
 
 // mean / rstd per channel from the partial rows (biased variance, as batch norm normalises with)
 __global__ void __launch_bounds__(1024)
-bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv_rows, float eps,
+bn_finish_stats_kernel(const float* ws, int parts, int C, float inv_rows, float eps,
                        float* __restrict__ mean, float* __restrict__ rstd) {
   bb::pdl_sync();
   float s1, s2;
@@ -304,8 +304,8 @@ bn_finish_stats_kernel(const float* __restrict__ ws, int parts, int C, float inv
 
 // sums[0][c] = sum dz', sums[1][c] = sum dz' * yhat; dbeta += sums[0], dgamma += sums[1]
 __global__ void __launch_bounds__(1024)
-bn_finish_bwd_kernel(const float* __restrict__ ws, int parts, int C, float* __restrict__ sums,
-                     float* __restrict__ dgamma, float* __restrict__ dbeta) {
+bn_finish_bwd_kernel(const float* ws, int parts, int C, float* __restrict__ sums,
+                     float* dgamma, float* dbeta) {
   bb::pdl_sync();
   float s1, s2;
   bn_sum_partials(ws, parts, C, s1, s2);
@@ -320,9 +320,9 @@ bn_finish_bwd_kernel(const float* __restrict__ ws, int parts, int C, float* __re
 // z = (y - mean) * rstd * gamma + beta (+ residual) (ReLU)
 template <bool RES>
 __global__ void __launch_bounds__(256, BN_CTAS)
-bn_apply_kernel(const uint4* __restrict__ y, const float* __restrict__ mean, const float* __restrict__ rstd,
+bn_apply_kernel(const uint4* y, const float* mean, const float* rstd,
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
-                const uint4* __restrict__ residual, uint4* __restrict__ z, long long rows, int C, int relu) {
+                const uint4* residual, uint4* __restrict__ z, long long rows, int C, int relu) {
   bb::pdl_sync();
   const int chunks = C >> 3;
   const long long gthreads = (long long)gridDim.x * blockDim.x;
@@ -332,13 +332,14 @@ bn_apply_kernel(const uint4* __restrict__ y, const float* __restrict__ mean, con
   float sc[8], sh[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    bn_scale_shift(__bfloat162float(gamma[cc * 8 + i]), __bfloat162float(beta[cc * 8 + i]), mean[cc * 8 + i], rstd[cc * 8 + i], sc[i], sh[i]);
+    bn_scale_shift(__bfloat162float(gamma[cc * 8 + i]), __bfloat162float(beta[cc * 8 + i]), __ldca(mean + cc * 8 + i),
+                   __ldca(rstd + cc * 8 + i), sc[i], sh[i]);
   for (long long r = rows - 1 - g / chunks; r >= 0; r -= BN_U * row_step) {
     uint4 qy[BN_U], qr[BN_U];
 #pragma unroll
     for (int u = 0; u < BN_U; ++u) {
       const long long ru = r - u * row_step;
-      if (ru >= 0) { qy[u] = __ldg(y + ru * chunks + cc); if (RES) qr[u] = __ldg(residual + ru * chunks + cc); }
+      if (ru >= 0) { qy[u] = __ldca(y + ru * chunks + cc); if (RES) qr[u] = __ldca(residual + ru * chunks + cc); }
     }
 #pragma unroll
     for (int u = 0; u < BN_U; ++u) {
@@ -367,9 +368,9 @@ bn_apply_kernel(const uint4* __restrict__ y, const float* __restrict__ mean, con
 // also flows into the residual branch)
 template <int MASK>
 __global__ void __launch_bounds__(256, BN_CTAS)
-bn_bwd_apply_kernel(const uint4* __restrict__ dz, const uint4* __restrict__ zz, const uint4* __restrict__ yy,
-                    const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma,
-                    const __nv_bfloat16* __restrict__ beta, const float* __restrict__ sums, uint4* __restrict__ dy,
+bn_bwd_apply_kernel(const uint4* dz, const uint4* zz, const uint4* yy,
+                    const float* mean, const float* rstd, const __nv_bfloat16* __restrict__ gamma,
+                    const __nv_bfloat16* __restrict__ beta, const float* sums, uint4* __restrict__ dy,
                     uint4* __restrict__ dres, long long rows, int C, float inv_rows) {
   bb::pdl_sync();
   constexpr int U = 2;         // four rows would take 128 registers
@@ -382,10 +383,10 @@ bn_bwd_apply_kernel(const uint4* __restrict__ dz, const uint4* __restrict__ zz, 
   float k0[8], k1[8], k2[8], sc[8], sh[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const float rs = rstd[cc * 8 + i], ga = __bfloat162float(gamma[cc * 8 + i]), mu = mean[cc * 8 + i];
+    const float rs = __ldca(rstd + cc * 8 + i), ga = __bfloat162float(gamma[cc * 8 + i]), mu = __ldca(mean + cc * 8 + i);
     k0[i] = ga * rs;
-    k2[i] = rs * (sums[C + cc * 8 + i] * inv_rows);
-    k1[i] = fmaf(-mu, k2[i], sums[cc * 8 + i] * inv_rows);
+    k2[i] = rs * (__ldca(sums + C + cc * 8 + i) * inv_rows);
+    k1[i] = fmaf(-mu, k2[i], __ldca(sums + cc * 8 + i) * inv_rows);
     if (MASK == MASK_Y) bn_scale_shift(ga, __bfloat162float(beta[cc * 8 + i]), mu, rs, sc[i], sh[i]);
   }
   for (long long r = rows - 1 - g / chunks; r >= 0; r -= U * row_step) {
@@ -394,9 +395,9 @@ bn_bwd_apply_kernel(const uint4* __restrict__ dz, const uint4* __restrict__ zz, 
     for (int u = 0; u < U; ++u) {
       const long long ru = r - u * row_step;
       if (ru >= 0) {
-        qd[u] = __ldg(dz + ru * chunks + cc);
-        qy[u] = __ldg(yy + ru * chunks + cc);
-        if (MASK == MASK_Z) qz[u] = __ldg(zz + ru * chunks + cc);
+        qd[u] = __ldca(dz + ru * chunks + cc);
+        qy[u] = __ldca(yy + ru * chunks + cc);
+        if (MASK == MASK_Z) qz[u] = __ldca(zz + ru * chunks + cc);
       }
     }
 #pragma unroll

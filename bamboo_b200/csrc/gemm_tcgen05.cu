@@ -125,7 +125,7 @@ __device__ __forceinline__ void slab_fetch_bf16(const __nv_bfloat16* src, long l
     if (r < M) {
       const __nv_bfloat16* g = src + (long long)r * ld + c;
       if (c + 8 <= N) {
-        q = __ldg(reinterpret_cast<const uint4*>(g));
+        q = __ldca(reinterpret_cast<const uint4*>(g));
       } else {
         unsigned short e[8];
 #pragma unroll
@@ -206,7 +206,7 @@ __device__ __forceinline__ void slab64_fetch(uint8_t* slab, const __nv_bfloat16*
     if (r < M) {
       const __nv_bfloat16* g = src + (long long)r * ld + c;
       if (c + 8 <= N) {
-        q[i] = __ldg(reinterpret_cast<const uint4*>(g));
+        q[i] = __ldca(reinterpret_cast<const uint4*>(g));
       } else {
         unsigned short e[8];
 #pragma unroll

@@ -35,7 +35,7 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 // ------------------------------------------------------------------ LayerNorm forward
 // y = (x - mean) * rstd * gamma + beta ; statistics in fp32 (biased variance, eps inside sqrt)
 __global__ void __launch_bounds__(WARPS * 32)
-layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+layernorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
                      const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int h, float eps) {
   bb::pdl_sync();
@@ -47,14 +47,14 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
     float s = 0.f;
     for (int c = lane; c < nch; c += 32) {
-      float f[8]; unpack8(xr[c], f);
+      float f[8]; unpack8(__ldca(xr + c), f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) s += f[i];
     }
     const float mean = warp_sum(s) / (float)h;
     float v = 0.f;
     for (int c = lane; c < nch; c += 32) {   // second pass hits L1
-      float f[8]; unpack8(xr[c], f);
+      float f[8]; unpack8(__ldca(xr + c), f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) { float d = f[i] - mean; v += d * d; }
     }
@@ -62,7 +62,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
     uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * h);
     for (int c = lane; c < nch; c += 32) {
       float f[8], g[8], b[8];
-      unpack8(xr[c], f);
+      unpack8(__ldca(xr + c), f);
       unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
       unpack8(__ldg(reinterpret_cast<const uint4*>(beta) + c), b);
 #pragma unroll
@@ -78,7 +78,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 // 9.9 us, 8192 x 768 10.6 -> 8.8 us; wider rows lose more to the registers than they win (4096 x 4096: 17.8 -> 24.7 us).
 template <int NCH>
 __global__ void __launch_bounds__(WARPS * 32)
-layernorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+layernorm_fwd_reg_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
                          const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                          float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int h, float eps) {
   bb::pdl_sync();
@@ -91,7 +91,7 @@ layernorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 #pragma unroll
     for (int u = 0; u < NCH; ++u) {
       const int c = lane + 32 * u;
-      q[u] = c < nch ? __ldg(xr + c) : make_uint4(0, 0, 0, 0);
+      q[u] = c < nch ? __ldca(xr + c) : make_uint4(0, 0, 0, 0);
     }
     float s = 0.f;
 #pragma unroll
@@ -132,9 +132,9 @@ layernorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 // Per-CTA partial sums of dgamma = sum dy*xhat and dbeta = sum dy go to `partials`
 // ([gridDim.x][2][h] fp32); reduce_partials_kernel folds them into the fp32 gradients.
 __global__ void __launch_bounds__(WARPS * 32)
-layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                     const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                     const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                     const __nv_bfloat16* __restrict__ gamma, const float* mean_in,
+                     const float* rstd_in, const __nv_bfloat16* dres,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows, int h) {
   bb::pdl_sync();
   extern __shared__ float acc[];  // [warps][2][h], each lane owns its own columns
@@ -151,11 +151,11 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   for (int row = warp_global; row < rows; row += warp_stride) {
     const uint4* dyr = reinterpret_cast<const uint4*>(dy + (size_t)row * h);
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
-    const float mean = mean_in[row], rstd = rstd_in[row];
+    const float mean = __ldca(mean_in + row), rstd = __ldca(rstd_in + row);
     float s1 = 0.f, s2 = 0.f;
     for (int c = lane; c < nch; c += 32) {
       float d[8], f[8], g[8];
-      unpack8(dyr[c], d); unpack8(xr[c], f);
+      unpack8(__ldca(dyr + c), d); unpack8(__ldca(xr + c), f);
       unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
 #pragma unroll
       for (int i = 0; i < 8; ++i) { float t = d[i] * g[i]; s1 += t; s2 += t * (f[i] - mean) * rstd; }
@@ -165,10 +165,10 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
     const uint4* rr = dres ? reinterpret_cast<const uint4*>(dres + (size_t)row * h) : nullptr;
     for (int c = lane; c < nch; c += 32) {
       float d[8], f[8], g[8], o[8];
-      unpack8(dyr[c], d); unpack8(xr[c], f);
+      unpack8(__ldca(dyr + c), d); unpack8(__ldca(xr + c), f);
       unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
       float r[8];
-      if (rr) unpack8(rr[c], r);
+      if (rr) unpack8(__ldca(rr + c), r);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float xh = (f[i] - mean) * rstd;
@@ -193,9 +193,9 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 // once per CTA, when the warps' partials are combined.
 template <int NCH>
 __global__ void __launch_bounds__(WARPS * 32)
-layernorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                         const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                         const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+layernorm_bwd_reg_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                         const __nv_bfloat16* __restrict__ gamma, const float* mean_in,
+                         const float* rstd_in, const __nv_bfloat16* dres,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows) {
   bb::pdl_sync();
   constexpr int h = NCH * 256;
@@ -212,10 +212,10 @@ layernorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
   for (int row = blockIdx.x * nwarps + warp; row < rows; row += gridDim.x * nwarps) {
     const uint4* dyr = reinterpret_cast<const uint4*>(dy + (size_t)row * h);
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
-    const float mean = mean_in[row], rstd = rstd_in[row];
+    const float mean = __ldca(mean_in + row), rstd = __ldca(rstd_in + row);
     uint4 qd[NCH], qx[NCH];
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) { qd[j] = dyr[lane + 32 * j]; qx[j] = xr[lane + 32 * j]; }
+    for (int j = 0; j < NCH; ++j) { qd[j] = __ldca(dyr + lane + 32 * j); qx[j] = __ldca(xr + lane + 32 * j); }
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int j = 0; j < NCH; ++j) {
@@ -231,7 +231,7 @@ layernorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
     for (int j = 0; j < NCH; ++j) {
       float d[8], f[8], o[8], r[8];
       unpack8(qd[j], d); unpack8(qx[j], f);
-      if (rr) unpack8(rr[lane + 32 * j], r);
+      if (rr) unpack8(__ldca(rr + lane + 32 * j), r);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float xh = (f[i] - mean) * rstd;
@@ -290,9 +290,9 @@ template <> struct ColVec<4> {
 // (twice the operand registers, memory requests in flight all the time).
 template <int MAXT, int CW, int R, int MINB, bool PF, bool SUMRES>
 __global__ void __launch_bounds__(MAXT, MINB)
-layernorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                          const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                          const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+layernorm_bwd_cols_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                          const __nv_bfloat16* __restrict__ gamma, const float* mean_in,
+                          const float* rstd_in, const __nv_bfloat16* dres,
                           __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int rows, int h, int slots) {
   bb::pdl_sync();
   extern __shared__ float sm[];
@@ -318,10 +318,10 @@ layernorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
       const int row = first + r;
       ld[r] = V::zero(); lx[r] = ld[r]; lr[r] = ld[r]; lm[r] = 0.f; ls[r] = 0.f;
       if (row < rows) {
-        ld[r] = reinterpret_cast<const VT*>(dy + (size_t)row * h)[tc];
-        lx[r] = reinterpret_cast<const VT*>(x + (size_t)row * h)[tc];
-        if (dres) lr[r] = reinterpret_cast<const VT*>(dres + (size_t)row * h)[tc];
-        lm[r] = mean_in[row]; ls[r] = rstd_in[row];
+        ld[r] = __ldca(reinterpret_cast<const VT*>(dy + (size_t)row * h) + tc);
+        lx[r] = __ldca(reinterpret_cast<const VT*>(x + (size_t)row * h) + tc);
+        if (dres) lr[r] = __ldca(reinterpret_cast<const VT*>(dres + (size_t)row * h) + tc);
+        lm[r] = __ldca(mean_in + row); ls[r] = __ldca(rstd_in + row);
       }
     }
   };
@@ -411,8 +411,7 @@ layernorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
 // blockIdx.y selects one of up to three (partials, out) pairs, `pair_offset` floats apart in
 // `partials` (LayerNorm: dgamma, dbeta and the residual gradient's column sums in one launch).
 __global__ void __launch_bounds__(1024)
-reduce_partials_kernel(const float* __restrict__ partials, float* __restrict__ out0, float* __restrict__ out1,
-                       float* __restrict__ out2, long long pair_offset, int nparts, int n, long long stride) {
+reduce_partials_kernel(const float* partials, float* out0, float* out1, float* out2, long long pair_offset, int nparts, int n, long long stride) {
   bb::pdl_sync();
   __shared__ float red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -449,7 +448,7 @@ constexpr int COLSUM_TICKET_SLOTS = 1 << 16;
 __device__ unsigned int g_colsum_tickets[COLSUM_TICKET_SLOTS];
 
 __global__ void __launch_bounds__(256)
-colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ partials, float* __restrict__ out, int rows, int n,
+colsum_kernel(const __nv_bfloat16* dy, float* partials, float* out, int rows, int n,
               long long ld, int rows_per_split, unsigned int* __restrict__ tickets) {
   bb::pdl_sync();
   __shared__ float red[8][256];
@@ -467,7 +466,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ partials
       uint4 q[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        q[u] = (r + 8 * u < r1) ? *reinterpret_cast<const uint4*>(src + (size_t)(r + 8 * u) * ld) : make_uint4(0, 0, 0, 0);
+        q[u] = (r + 8 * u < r1) ? __ldca(reinterpret_cast<const uint4*>(src + (size_t)(r + 8 * u) * ld)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         float f[8];

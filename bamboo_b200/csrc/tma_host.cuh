@@ -1,4 +1,4 @@
-// Host-side helper shared by the TMA kernels: encode a 2-D tensor map (128-byte swizzle)
+// Host-side helpers shared by the TMA kernels: encode tensor maps (128-byte swizzle)
 // through the driver entry point, resolved at run time so the library has no link-time
 // dependency on libcuda.
 #pragma once
@@ -36,27 +36,42 @@ inline int bind_context() {
   return BB_OK;
 }
 
-// 2-D tensor map over a row-major [rows, cols] matrix (bf16, or fp32 when f32 != 0) with leading
-// dimension ld (elements); box = box_cols x box_rows; 128-byte swizzle.
-inline int encode_2d(CUtensorMap* tm, const void* base, long long rows, long long cols, long long ld, int box_cols,
-                     int box_rows, int f32 = 0) {
+// Tensor map of `rank` dimensions (innermost first, 128-byte swizzle) over bf16, or fp32 when f32 != 0; `pitch`: bytes
+// between neighbours of every dimension but the innermost.
+inline int encode_tiled(CUtensorMap* tm, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* pitch,
+                        const cuuint32_t* box, int f32) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) { bb_set_last_error_msg("cuTensorMapEncodeTiled entry point not available"); return BB_ERR_CUDA; }
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
-                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base),
+                  dims, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     char msg[256];
-    snprintf(msg, sizeof(msg), "cuTensorMapEncodeTiled failed with CUresult %d (base %p, rows %lld, cols %lld, ld %lld, box %dx%d, "
-             "f32 %d); operands need a 16-byte aligned base and row pitch", (int)r, base, rows, cols, ld, box_cols, box_rows, f32);
+    snprintf(msg, sizeof(msg), "cuTensorMapEncodeTiled failed with CUresult %d (base %p, rows %lld, cols %lld, row pitch %lld bytes, box %ux%u, "
+             "f32 %d); operands need a 16-byte aligned base and row pitch", (int)r, base, (long long)dims[1], (long long)dims[0],
+             (long long)pitch[0], box[0], box[1], f32);
     bb_set_last_error_msg(msg);
     return BB_ERR_INVALID_ARG;
   }
   return BB_OK;
+}
+
+// 2-D tensor map over a row-major [rows, cols] matrix with leading dimension ld (elements); box = box_cols x box_rows.
+inline int encode_2d(CUtensorMap* tm, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows,
+                     int f32 = 0) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, pitch[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  return encode_tiled(tm, base, 2, dims, pitch, box, f32);
+}
+
+// 3-D tensor map over `seqs` sequences of `rows` bf16 rows each, one after the other in a [seqs * rows, cols] matrix.  A box
+// ends with its sequence: rows past the end load as zeros.
+inline int encode_seqs(CUtensorMap* tm, const void* base, int seqs, int rows, long long cols, long long ld, int box_cols, int box_rows) {
+  const cuuint64_t row = (cuuint64_t)ld * 2;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)seqs}, pitch[2] = {row, row * (cuuint64_t)rows};
+  const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  return encode_tiled(tm, base, 3, dims, pitch, box, 0);
 }
 
 typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

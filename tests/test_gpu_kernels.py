@@ -542,3 +542,44 @@ def test_attention_head_dim_64_keeps_its_summation_order(L, B, H, S, causal, wan
     L.attention_fwd(qkv, out, lse, B, H, S, D, causal)
     digest = [hashlib.sha256(t.cpu().view(torch.uint8).numpy().tobytes()).hexdigest()[:16] for t in (out, lse)]
     assert digest == [want_out, want_lse]
+
+
+# lengths that end inside a 64-row sub-block, inside a 128-row tile, and one past a tile (the next tile of the machine then
+# lies almost wholly past the end); 384: no overhang, for the heads' own accumulator rows
+@pytest.mark.parametrize("S", [1, 50, 100, 129, 300, 384])
+@pytest.mark.parametrize("D,causal", [(64, True), (64, False), (128, True), (128, False)])
+def test_attention_non_finite_values_stay_in_their_sequence(L, D, causal, S):
+    """A tile that overhangs the end of a sequence must not let in its neighbour's rows, nor add to its neighbour's: zero
+    (a masked probability) times Inf is NaN.  One head of the middle sequence is Inf / NaN; every other (sequence, head)
+    has to come out as without it - the same bits, but for dQ at head dimension 64, whose additions have no fixed
+    order (bf16 result: 2^-8 of the largest value)."""
+    B, H = 3, 3
+    torch.manual_seed(31)
+    clean = torch.randn(B, S, 3, H, D, device="cuda").bfloat16()
+    dclean = torch.randn(B, S, H, D, device="cuda").bfloat16()
+    bad, dbad = clean.clone(), dclean.clone()
+    bad[1, :, 0, 1], bad[1, :, 1, 1], bad[1, :, 2, 1] = float("inf"), float("nan"), float("inf")
+    dbad[1, :, 1] = float("inf")
+
+    def passes(qkv, do):
+        qkv, do = qkv.reshape(B * S, 3 * H * D), do.reshape(B * S, H * D)
+        out = torch.empty(B * S, H * D, device="cuda", dtype=torch.bfloat16)
+        lse = torch.empty(B, H, S, device="cuda")
+        dqkv = torch.empty_like(qkv)
+        L.attention_fwd(qkv, out, lse, B, H, S, D, causal)
+        L.attention_bwd(qkv, out, do, lse, dqkv, B, H, S, D, causal)
+        return out.view(B, S, H, D), lse, dqkv.view(B, S, 3, H, D)
+
+    (o0, l0, g0), (o1, l1, g1) = passes(clean, dclean), passes(bad, dbad)
+    assert not torch.isfinite(o1[1, :, 1].float()).all()
+    for b in range(B):
+        for h in range(H):
+            if (b, h) == (1, 1):
+                continue
+            assert torch.equal(o0[b, :, h], o1[b, :, h]) and torch.equal(l0[b, h], l1[b, h]), (b, h)
+            assert torch.equal(g0[b, :, 1:, h], g1[b, :, 1:, h]), (b, h)
+            if D == 128:
+                assert torch.equal(g0[b, :, 0, h], g1[b, :, 0, h]), (b, h)
+            else:
+                assert ((g0[b, :, 0, h].float() - g1[b, :, 0, h].float()).abs().max() <= 2 ** -8 * g0[b, :, 0, h].float().abs().max()).item(), (b, h)
+    assert L.read_status() == 0

@@ -165,7 +165,8 @@ enum { RED_STATS = 0, RED_BWD = 1 };
 // y.  Image-network step (7 bottlenecks, 224 x 224, 2 x 32 images), all passes: reductions 1292 -> 1143 us,
 // element-wise 1305 -> 975 us.
 // Where the backward pass takes the ReLU mask from: nowhere, the stored output z > 0, or (no residual was added) the
-// normalised value itself, computed again from y with the forward pass's own arithmetic - one tensor less to read.
+// normalised value itself, computed again from y with the forward pass's own arithmetic and the scale and shift that the
+// forward pass kept (gamma and beta may have changed since) - one tensor less to read.
 enum { MASK_NONE = 0, MASK_Z = 1, MASK_Y = 2 };
 constexpr int BN_U = 4;              // rows in flight per thread
 constexpr int BN_CTAS = 3;           // blocks per SM (at most 85 registers a thread): the grid is one full wave
@@ -181,8 +182,7 @@ __device__ __forceinline__ bool bn_positive(float v) { return v > 4.5917748e-41f
 template <int MODE, int MASK>
 __global__ void __launch_bounds__(256, BN_CTAS)
 bn_reduce_kernel(const uint4* a, const uint4* zz, const uint4* yy,
-                 const float* mean, const float* rstd, const __nv_bfloat16* __restrict__ gamma,
-                 const __nv_bfloat16* __restrict__ beta, long long rows, int C, float* __restrict__ ws) {
+                 const float* mean, const float* rstd, const float* affine, long long rows, int C, float* __restrict__ ws) {
   bb::pdl_sync();
   __shared__ float sm[256 * 16];
   const int chunks = C >> 3;
@@ -197,7 +197,7 @@ bn_reduce_kernel(const uint4* a, const uint4* zz, const uint4* yy,
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       mu[i] = __ldca(mean + cc * 8 + i); rs[i] = __ldca(rstd + cc * 8 + i);
-      if (MASK == MASK_Y) bn_scale_shift(__bfloat162float(gamma[cc * 8 + i]), __bfloat162float(beta[cc * 8 + i]), mu[i], rs[i], sc[i], sh[i]);
+      if (MASK == MASK_Y) { sc[i] = __ldca(affine + cc * 8 + i); sh[i] = __ldca(affine + C + cc * 8 + i); }
     }
   }
   const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -287,10 +287,12 @@ __device__ __forceinline__ void bn_sum_partials(const float* ws, int parts, int 
   }
 }
 
-// mean / rstd per channel from the partial rows (biased variance, as batch norm normalises with)
+// mean / rstd per channel from the partial rows (biased variance, as batch norm normalises with); affine (or null):
+// scale and shift of the normalisation, [2, C]
 __global__ void __launch_bounds__(1024)
-bn_finish_stats_kernel(const float* ws, int parts, int C, float inv_rows, float eps,
-                       float* __restrict__ mean, float* __restrict__ rstd) {
+bn_finish_stats_kernel(const float* ws, int parts, int C, float inv_rows, float eps, const __nv_bfloat16* __restrict__ gamma,
+                       const __nv_bfloat16* __restrict__ beta, float* __restrict__ mean, float* __restrict__ rstd,
+                       float* __restrict__ affine) {
   bb::pdl_sync();
   float s1, s2;
   bn_sum_partials(ws, parts, C, s1, s2);
@@ -298,8 +300,14 @@ bn_finish_stats_kernel(const float* ws, int parts, int C, float inv_rows, float 
   if (threadIdx.x >= 32 || c >= C) return;
   const float m = s1 * inv_rows;
   const float var = fmaxf(s2 * inv_rows - m * m, 0.f);
+  const float rs = rsqrtf(var + eps);
   mean[c] = m;
-  rstd[c] = rsqrtf(var + eps);
+  rstd[c] = rs;
+  if (affine) {
+    float sc, sh;
+    bn_scale_shift(__bfloat162float(gamma[c]), __bfloat162float(beta[c]), m, rs, sc, sh);
+    affine[c] = sc; affine[C + c] = sh;
+  }
 }
 
 // sums[0][c] = sum dz', sums[1][c] = sum dz' * yhat; dbeta += sums[0], dgamma += sums[1]
@@ -370,7 +378,7 @@ template <int MASK>
 __global__ void __launch_bounds__(256, BN_CTAS)
 bn_bwd_apply_kernel(const uint4* dz, const uint4* zz, const uint4* yy,
                     const float* mean, const float* rstd, const __nv_bfloat16* __restrict__ gamma,
-                    const __nv_bfloat16* __restrict__ beta, const float* sums, uint4* __restrict__ dy,
+                    const float* affine, const float* sums, uint4* __restrict__ dy,
                     uint4* __restrict__ dres, long long rows, int C, float inv_rows) {
   bb::pdl_sync();
   constexpr int U = 2;         // four rows would take 128 registers
@@ -387,7 +395,7 @@ bn_bwd_apply_kernel(const uint4* dz, const uint4* zz, const uint4* yy,
     k0[i] = ga * rs;
     k2[i] = rs * (__ldca(sums + C + cc * 8 + i) * inv_rows);
     k1[i] = fmaf(-mu, k2[i], __ldca(sums + cc * 8 + i) * inv_rows);
-    if (MASK == MASK_Y) bn_scale_shift(ga, __bfloat162float(beta[cc * 8 + i]), mu, rs, sc[i], sh[i]);
+    if (MASK == MASK_Y) { sc[i] = __ldca(affine + cc * 8 + i); sh[i] = __ldca(affine + C + cc * 8 + i); }
   }
   for (long long r = rows - 1 - g / chunks; r >= 0; r -= U * row_step) {
     uint4 qd[U], qy[U], qz[U];
@@ -434,20 +442,20 @@ int bn_grid(long long rows, int C) {
   return (int)(blocks < 1 ? 1 : blocks);
 }
 
-// `beta`: non-null when the mask may come from y (the forward pass added no residual)
-int bn_bwd(const void* dz, const void* z, const void* y, const float* mean, const float* rstd, const void* gamma, const void* beta,
+// `affine`: the forward pass's scale and shift, non-null when the mask may come from y (no residual was added)
+int bn_bwd(const void* dz, const void* z, const void* y, const float* mean, const float* rstd, const void* gamma, const float* affine,
            void* dy, void* dres, float* dgamma, float* dbeta, long long rows, int C, int relu, float* ws, cudaStream_t s) {
   const int grid = bn_grid(rows, C);
   float* sums = ws + (long long)grid * 2 * C;
   const uint4 *qd = (const uint4*)dz, *qz = (const uint4*)z, *qy = (const uint4*)y;
-  const __nv_bfloat16 *ga = (const __nv_bfloat16*)gamma, *be = (const __nv_bfloat16*)beta;
+  const __nv_bfloat16* ga = (const __nv_bfloat16*)gamma;
   const float inv = 1.0f / (float)rows;
 #define BB_BN_BWD(MASK)                                                                                               \
-  bb_launch(bn_reduce_kernel<RED_BWD, MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, ga, be, rows, C, ws);                  \
+  bb_launch(bn_reduce_kernel<RED_BWD, MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, affine, rows, C, ws);                      \
   bb_launch(bn_finish_bwd_kernel, (C + 31) / 32, 1024, 0, s, ws, grid, C, sums, dgamma, dbeta);                             \
-  bb_launch(bn_bwd_apply_kernel<MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, ga, be, sums, (uint4*)dy, (uint4*)dres, rows, C, inv)
+  bb_launch(bn_bwd_apply_kernel<MASK>, grid, 256, 0, s, qd, qz, qy, mean, rstd, ga, affine, sums, (uint4*)dy, (uint4*)dres, rows, C, inv)
   if (!relu) { BB_BN_BWD(MASK_NONE); }
-  else if (be) { BB_BN_BWD(MASK_Y); }
+  else if (affine) { BB_BN_BWD(MASK_Y); }
   else { BB_BN_BWD(MASK_Z); }
 #undef BB_BN_BWD
   BB_CUDA_CHECK(cudaGetLastError());
@@ -462,8 +470,10 @@ extern "C" long long bb_bn_workspace_bytes(long long rows, int C) {
   return ((long long)bn_grid(rows, C) * 2 * C + 2 * C) * (long long)sizeof(float);
 }
 
-extern "C" int bb_bn_stats(const void* y, long long rows, int C, float eps, float* mean, float* rstd, void* workspace,
-                           long long workspace_bytes, void* stream) {
+namespace {
+// `affine` (or null): filled with the scale and shift that gamma and beta give with these statistics
+int bn_stats(const void* y, long long rows, int C, float eps, float* mean, float* rstd, const void* gamma, const void* beta,
+             float* affine, void* workspace, long long workspace_bytes, void* stream) {
   if (!y || !mean || !rstd || !workspace || bad_bn(rows, C) || workspace_bytes < bb_bn_workspace_bytes(rows, C) ||
       ((uintptr_t)y & 15)) {
     bb_set_last_error_msg("bb_bn_stats: null/unaligned pointer, workspace too small, or channels not 8 x a power of two <= 2048");
@@ -472,11 +482,17 @@ extern "C" int bb_bn_stats(const void* y, long long rows, int C, float eps, floa
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = bn_grid(rows, C);
   float* ws = static_cast<float*>(workspace);
-  bb_launch(bn_reduce_kernel<RED_STATS, MASK_NONE>, grid, 256, 0, s, (const uint4*)y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                              rows, C, ws);
-  bb_launch(bn_finish_stats_kernel, (C + 31) / 32, 1024, 0, s, ws, grid, C, 1.0f / (float)rows, eps, mean, rstd);
+  bb_launch(bn_reduce_kernel<RED_STATS, MASK_NONE>, grid, 256, 0, s, (const uint4*)y, nullptr, nullptr, nullptr, nullptr, nullptr, rows, C, ws);
+  bb_launch(bn_finish_stats_kernel, (C + 31) / 32, 1024, 0, s, ws, grid, C, 1.0f / (float)rows, eps, (const __nv_bfloat16*)gamma,
+            (const __nv_bfloat16*)beta, mean, rstd, affine);
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
+}
+}  // namespace
+
+extern "C" int bb_bn_stats(const void* y, long long rows, int C, float eps, float* mean, float* rstd, void* workspace,
+                           long long workspace_bytes, void* stream) {
+  return bn_stats(y, rows, C, eps, mean, rstd, nullptr, nullptr, nullptr, workspace, workspace_bytes, stream);
 }
 
 extern "C" int bb_bn_apply(const void* y, const float* mean, const float* rstd, const void* gamma, const void* beta,
@@ -744,8 +760,9 @@ extern "C" long long bb_conv_bn_scratch_bytes(const bb_conv_desc* d, int backwar
   return s.dy_bytes + s.col_bytes + (need_dx ? s.dcol_bytes : 0) + s.bn_bytes;
 }
 
-extern "C" int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void* y, void* z, float* mean,
-                              float* rstd, void* scratch, long long scratch_bytes, void* stream) {
+namespace {
+int conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void* y, void* z, float* mean, float* rstd, float* affine,
+                void* scratch, long long scratch_bytes, void* stream) {
   ConvSizes s;
   if (!conv_sizes(d, &s) || !x || !y || !z || !mean || !rstd || !scratch || scratch_bytes < s.col_bytes + s.bn_bytes) {
     bb_set_last_error_msg("bb_conv_bn_fwd: bad descriptor, null buffer or scratch smaller than bb_conv_bn_scratch_bytes");
@@ -763,16 +780,16 @@ extern "C" int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* 
     }
     BB_TRY(conv_gemm(d, (int)s.P, d->Cout, (int)s.K, col, s.K, 0, d->w, s.K, 0, y, d->Cout, BB_EPI_STORE, stream));
   }
-  BB_TRY(bb_bn_stats(y, s.P, d->Cout, d->eps, mean, rstd, sc + s.col_bytes, s.bn_bytes, stream));
+  BB_TRY(bn_stats(y, s.P, d->Cout, d->eps, mean, rstd, d->gamma, d->beta, affine, sc + s.col_bytes, s.bn_bytes, stream));
   BB_TRY(bb_bn_apply(y, mean, rstd, d->gamma, d->beta, residual, z, s.P, d->Cout, d->relu, stream));
   return BB_OK;
 }
 
-namespace {
+// the ReLU mask comes from y and affine, or from z when affine is null
 int conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean, const float* rstd,
-                const void* dz, void* dx, void* dres, int residual, void* scratch, long long scratch_bytes, void* stream) {
+                const float* affine, const void* dz, void* dx, void* dres, void* scratch, long long scratch_bytes, void* stream) {
   ConvSizes s;
-  if (!conv_sizes(d, &s) || !x || !y || !z || !mean || !rstd || !dz || !scratch || !d->g_w || !d->g_gamma || !d->g_beta ||
+  if (!conv_sizes(d, &s) || !x || !y || (!z && !affine) || !mean || !rstd || !dz || !scratch || !d->g_w || !d->g_gamma || !d->g_beta ||
       scratch_bytes < bb_conv_bn_scratch_bytes(d, 1, dx != nullptr)) {
     bb_set_last_error_msg("bb_conv_bn_bwd: bad descriptor, null buffer, missing gradient pointer or scratch too small");
     return BB_ERR_INVALID_ARG;
@@ -787,7 +804,7 @@ int conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void*
     bb_set_last_error_msg("bb_conv_bn_bwd: activations must be 16-byte aligned");
     return BB_ERR_INVALID_ARG;
   }
-  BB_TRY(bn_bwd(dz, z, y, mean, rstd, d->gamma, residual ? nullptr : d->beta, dy, dres, d->g_gamma, d->g_beta, s.P, d->Cout, d->relu,
+  BB_TRY(bn_bwd(dz, z, y, mean, rstd, d->gamma, affine, dy, dres, d->g_gamma, d->g_beta, s.P, d->Cout, d->relu,
                 reinterpret_cast<float*>(bnws), (cudaStream_t)stream));
   // dW[Cout, K] += dy^T patches
   if (s.implicit_x) {
@@ -814,14 +831,32 @@ int conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void*
 }
 }  // namespace
 
+extern "C" int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void* y, void* z, float* mean,
+                              float* rstd, void* scratch, long long scratch_bytes, void* stream) {
+  return conv_bn_fwd(d, x, residual, y, z, mean, rstd, nullptr, scratch, scratch_bytes, stream);
+}
+
 extern "C" int bb_conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean,
                               const float* rstd, const void* dz, void* dx, void* dres, void* scratch, long long scratch_bytes,
                               void* stream) {
-  return conv_bn_bwd(d, x, y, z, mean, rstd, dz, dx, dres, 1, scratch, scratch_bytes, stream);
+  return conv_bn_bwd(d, x, y, z, mean, rstd, nullptr, dz, dx, dres, scratch, scratch_bytes, stream);
 }
 
 extern "C" int bb_conv_bn_bwd_no_residual(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean,
                                           const float* rstd, const void* dz, void* dx, void* scratch, long long scratch_bytes,
                                           void* stream) {
-  return conv_bn_bwd(d, x, y, z, mean, rstd, dz, dx, nullptr, 0, scratch, scratch_bytes, stream);
+  return conv_bn_bwd(d, x, y, z, mean, rstd, nullptr, dz, dx, nullptr, scratch, scratch_bytes, stream);
+}
+
+extern "C" int bb_conv_bn_fwd_affine(const bb_conv_desc* d, const void* x, void* y, void* z, float* mean, float* rstd, float* affine,
+                                     void* scratch, long long scratch_bytes, void* stream) {
+  if (!affine) { bb_set_last_error_msg("bb_conv_bn_fwd_affine: null affine"); return BB_ERR_INVALID_ARG; }
+  return conv_bn_fwd(d, x, nullptr, y, z, mean, rstd, affine, scratch, scratch_bytes, stream);
+}
+
+extern "C" int bb_conv_bn_bwd_affine(const bb_conv_desc* d, const void* x, const void* y, const float* mean, const float* rstd,
+                                     const float* affine, const void* dz, void* dx, void* scratch, long long scratch_bytes,
+                                     void* stream) {
+  if (!affine) { bb_set_last_error_msg("bb_conv_bn_bwd_affine: null affine"); return BB_ERR_INVALID_ARG; }
+  return conv_bn_bwd(d, x, y, nullptr, mean, rstd, affine, dz, dx, nullptr, scratch, scratch_bytes, stream);
 }

@@ -98,6 +98,8 @@ def load():
         lib.bb_conv_bn_fwd.argtypes = [vp] * 8 + [ll, vp]
         lib.bb_conv_bn_bwd.argtypes = [vp] * 10 + [ll, vp]
         lib.bb_conv_bn_bwd_no_residual.argtypes = [vp] * 9 + [ll, vp]
+        lib.bb_conv_bn_fwd_affine.argtypes = [vp] * 8 + [ll, vp]
+        lib.bb_conv_bn_bwd_affine.argtypes = [vp] * 9 + [ll, vp]
         _lib = lib
     return _lib
 
@@ -493,28 +495,40 @@ def _conv_route(desc):
         not direct and small and desc.Cout % 64 == 0 and desc.stride == 1
 
 
-def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch):
-    """``mean`` / ``rstd``: fp32 tensors, or their device addresses."""
+def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch, affine=None):
+    """``mean`` / ``rstd`` / ``affine``: fp32 tensors, or their device addresses.  ``affine`` [2, Cout] (without a residual
+    only) keeps the scale and shift for ``conv_bn_bwd``."""
     global LAUNCHES
     direct, implicit_x, _ = _conv_route(desc)
     LAUNCHES += 4 + (0 if direct or implicit_x else 1)
-    rc = (_lib or load()).bb_conv_bn_fwd(ctypes.byref(desc), x.data_ptr(), _addr(residual), y.data_ptr(), z.data_ptr(), _addr(mean),
-                                         _addr(rstd), scratch.data_ptr(), scratch.numel(), _raw_stream())
+    lib = _lib or load()
+    tail = (scratch.data_ptr(), scratch.numel(), _raw_stream())
+    if affine is None:
+        rc = lib.bb_conv_bn_fwd(ctypes.byref(desc), x.data_ptr(), _addr(residual), y.data_ptr(), z.data_ptr(), _addr(mean), _addr(rstd), *tail)
+    else:
+        assert residual is None
+        rc = lib.bb_conv_bn_fwd_affine(ctypes.byref(desc), x.data_ptr(), y.data_ptr(), z.data_ptr(), _addr(mean), _addr(rstd),
+                                       _addr(affine), *tail)
     if rc < 0:
         check(rc, "bb_conv_bn_fwd")
     return z
 
 
-def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch, residual=True):
-    """``residual=False``: the forward call added none, so the ReLU mask may come from y instead of z.
-    ``mean`` / ``rstd``: fp32 tensors, or their device addresses."""
+def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch, residual=True, affine=None):
+    """``residual=False``: the forward call added none.  ``affine``: what that call kept; the ReLU mask then comes from y and
+    not from z.  ``mean`` / ``rstd`` / ``affine``: fp32 tensors, or their device addresses."""
     global LAUNCHES
     direct, implicit_x, implicit_dx = _conv_route(desc)
     LAUNCHES += 4 + (0 if direct or implicit_x else 1) + (0 if dx is None else (1 if direct or implicit_dx else 2))
     lib = _lib or load()
-    head = (ctypes.byref(desc), x.data_ptr(), y.data_ptr(), z.data_ptr(), _addr(mean), _addr(rstd), dz.data_ptr(), _addr(dx))
     tail = (scratch.data_ptr(), scratch.numel(), _raw_stream())
-    rc = lib.bb_conv_bn_bwd(*head, _addr(dres), *tail) if residual else lib.bb_conv_bn_bwd_no_residual(*head, *tail)
+    if affine is not None:
+        assert not residual
+        rc = lib.bb_conv_bn_bwd_affine(ctypes.byref(desc), x.data_ptr(), y.data_ptr(), _addr(mean), _addr(rstd), _addr(affine),
+                                       dz.data_ptr(), _addr(dx), *tail)
+    else:
+        head = (ctypes.byref(desc), x.data_ptr(), y.data_ptr(), z.data_ptr(), _addr(mean), _addr(rstd), dz.data_ptr(), _addr(dx))
+        rc = lib.bb_conv_bn_bwd(*head, _addr(dres), *tail) if residual else lib.bb_conv_bn_bwd_no_residual(*head, *tail)
     if rc < 0:
         check(rc, "bb_conv_bn_bwd")
     return dx

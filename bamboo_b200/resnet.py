@@ -70,12 +70,12 @@ class _ConvBNNativeFn(torch.autograd.Function):
         d = _conv_desc(mod, N, H, W, Cin, False)
         y = torch.empty(N * Ho * Wo, Cout, dtype=torch.bfloat16, device=dev)
         z = torch.empty(N, Ho, Wo, Cout, dtype=torch.bfloat16, device=dev)
-        stats = torch.empty(2, Cout, dtype=torch.float32, device=dev)
+        stats = torch.empty(4, Cout, dtype=torch.float32, device=dev)        # mean, rstd, scale, shift (no residual)
         scratch = torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device=dev)
         if residual is not None and not residual.is_contiguous():
             residual = residual.contiguous()
         mean = stats.data_ptr()
-        L.conv_bn_fwd(d, x, residual, y, z, mean, mean + 4 * Cout, scratch)
+        L.conv_bn_fwd(d, x, residual, y, z, mean, mean + 4 * Cout, scratch, mean + 8 * Cout if residual is None else None)
         ctx.mod, ctx.has_res = mod, residual is not None
         ctx.save_for_backward(x, y, z, stats)
         return z
@@ -93,7 +93,8 @@ class _ConvBNNativeFn(torch.autograd.Function):
         dres = torch.empty_like(z) if ctx.has_res else None
         scratch = torch.empty(d._bwd_scratch[1 if need_dx else 0], dtype=torch.uint8, device=dev)
         mean = stats.data_ptr()
-        L.conv_bn_bwd(d, x, y, z, mean, mean + 4 * stats.shape[1], dz, dx, dres, scratch, residual=ctx.has_res)
+        row = 4 * stats.shape[1]
+        L.conv_bn_bwd(d, x, y, z, mean, mean + row, dz, dx, dres, scratch, ctx.has_res, None if ctx.has_res else mean + 2 * row)
         return dx, dres, None, None
 
 

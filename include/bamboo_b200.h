@@ -260,9 +260,16 @@ int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, v
                    void* scratch, long long scratch_bytes, void* stream);
 int bb_conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean, const float* rstd,
                    const void* dz, void* dx, void* dres, void* scratch, long long scratch_bytes, void* stream);
-/* The same when the forward call added no residual: the ReLU mask then comes from y, mean and rstd, and z is not read. */
+/* The same without a residual gradient. */
 int bb_conv_bn_bwd_no_residual(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean,
                                const float* rstd, const void* dz, void* dx, void* scratch, long long scratch_bytes, void* stream);
+/* A layer without a residual, whose backward call does not read z: the forward call keeps the scale and shift that it
+ * normalised with (affine: fp32 [2, Cout]), and the backward call takes the ReLU mask from y and those.  The mask is that
+ * of the forward call even if gamma and beta have changed in between. */
+int bb_conv_bn_fwd_affine(const bb_conv_desc* d, const void* x, void* y, void* z, float* mean, float* rstd, float* affine,
+                          void* scratch, long long scratch_bytes, void* stream);
+int bb_conv_bn_bwd_affine(const bb_conv_desc* d, const void* x, const void* y, const float* mean, const float* rstd,
+                          const float* affine, const void* dz, void* dx, void* scratch, long long scratch_bytes, void* stream);
 /* 3 x 3 / stride 2 / padding 1 max pooling (argmax: 1 byte per output element, position 0..8 in
  * the window, first maximum wins) and global average pooling over HW pixels.
  * Replaces: model.maxpool / model.avgpool of the same layer list. */

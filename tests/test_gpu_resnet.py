@@ -142,7 +142,7 @@ def test_conv_bn_layer_without_relu(L, cin, cout, k, stride, hw):
 # 16-byte chunk), ordinary, the widest (a row per block)
 @pytest.mark.parametrize("rows,C", [(1, 8), (255, 8), (3, 64), (129, 64), (1025, 256), (7, 2048), (50, 2048), (40000, 64)])
 def test_batch_norm_backward_mask_from_y_equals_mask_from_z(L, rows, C):
-    """bb_conv_bn_bwd_no_residual takes the ReLU mask from y: the same values as the general entry point, which reads the
+    """bb_conv_bn_bwd_affine takes the ReLU mask from y: the same values as the general entry point, which reads the
     stored output, in every bit (same kernels, same order of sums), a channel that
     is zero throughout included."""
     from bamboo_b200 import resnet
@@ -157,8 +157,8 @@ def test_batch_norm_backward_mask_from_y_equals_mask_from_z(L, rows, C):
     x[..., 0] = 0.0
     d = resnet._conv_desc(m, 1, 1, rows, 8, True)
     y, z = torch.empty(rows, C, dtype=torch.bfloat16, device="cuda"), torch.empty(1, 1, rows, C, dtype=torch.bfloat16, device="cuda")
-    stats = torch.empty(2, C, device="cuda")
-    L.conv_bn_fwd(d, x, None, y, z, stats[0], stats[1], torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device="cuda"))
+    stats = torch.empty(4, C, device="cuda")
+    L.conv_bn_fwd(d, x, None, y, z, stats[0], stats[1], torch.empty(max(d._fwd_scratch, 16), dtype=torch.uint8, device="cuda"), stats[2:])
     dz = torch.randn(1, 1, rows, C, device="cuda", generator=g).bfloat16()
     out = []
     for residual in (True, False):
@@ -166,7 +166,7 @@ def test_batch_norm_backward_mask_from_y_equals_mask_from_z(L, rows, C):
             p.main_grad.zero_()
         dx = torch.empty_like(x)
         scratch = torch.zeros(d._bwd_scratch[1], dtype=torch.uint8, device="cuda")
-        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, None, scratch, residual=residual)
+        L.conv_bn_bwd(d, x, y, z, stats[0], stats[1], dz, dx, None, scratch, residual=residual, affine=None if residual else stats[2:])
         out.append((scratch[:rows * C * 2].view(torch.bfloat16).clone(), m.bn_weight.main_grad.clone(), m.bn_bias.main_grad.clone()))
     for a, b in zip(*out):
         assert torch.equal(a.nan_to_num(), b.nan_to_num()) and torch.equal(a.isnan(), b.isnan())
@@ -177,6 +177,29 @@ def test_batch_norm_backward_mask_from_y_equals_mask_from_z(L, rows, C):
         zf = F.batch_norm(yf, None, None, ga, be, training=True, eps=m.eps)
         zf.backward(torch.where(z.view(rows, C) > 0, dz.view(rows, C).float(), torch.zeros((), device="cuda")))
         assert _rel(out[1][0].view(rows, C), yf.grad) <= TOL and _rel(out[1][1], ga.grad) <= TOL
+
+
+@pytest.mark.parametrize("residual", [False, True])
+def test_relu_mask_is_that_of_the_forward_pass(L, residual):
+    """Gain and bias that change between a layer's forward and backward pass (an update while a micro-batch is in flight)
+    do not move the ReLU mask: the bias gradient stays the sum of dz over the positive outputs."""
+    from bamboo_b200 import resnet
+    from bamboo_b200.arena import ParamArena
+    C, rows = 64, 300
+    m = resnet.ConvBN(16, C, 1, relu=True, generator=torch.Generator().manual_seed(5))
+    ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(1, 1, rows, 16, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    res = torch.randn(1, 1, rows, C, device="cuda", generator=g).bfloat16() if residual else None
+    z = m(x, res)
+    with torch.no_grad():
+        m.bn_bias.add_(1.0)
+        m.bn_weight.mul_(-1.0)
+    dz = torch.randint(-8, 9, z.shape, device="cuda", generator=g).bfloat16()
+    z.backward(dz)
+    # whole numbers below 2^24: the sums are exact
+    want = torch.where(z > 0, dz.float(), torch.zeros((), device="cuda")).sum((0, 1, 2))
+    assert torch.equal(m.bn_bias.main_grad.view(-1), want)
 
 
 # (channels in / out, window, stride, image side): reductions of one to several 64-channel blocks, output rows that no

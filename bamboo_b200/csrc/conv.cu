@@ -130,6 +130,7 @@ extern "C" int bb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int
     bb_set_last_error_msg("bb_im2col_nhwc: null/unaligned pointer or inconsistent geometry (channels and ld_col multiples of 8)");
     return BB_ERR_INVALID_ARG;
   }
+  if (Ho <= 0 || Wo <= 0) return BB_OK;        // a window larger than the padded image: no patches
   const int chunks = C >> 3, row_chunks = k * k * chunks;
   const ConvMagic m = {bb_div_magic(row_chunks), bb_div_magic(chunks), bb_div_magic(k), bb_div_magic(Ho)};
   bb_launch(im2col_kernel, patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream, (const uint4*)x, (uint4*)col, g, m);

@@ -1,0 +1,23 @@
+"""Which route a convolution's geometry takes, and its limits, as far as the library decides them on the host."""
+import subprocess
+import sys
+
+import pytest
+
+
+# (H, k, stride): the output side is (H - k) / stride + 1 = 0 or below
+@pytest.mark.parametrize("H,k,stride", [(2, 3, 1), (1, 4, 1), (2, 4, 2), (1, 3, 2)])
+def test_patch_gather_without_windows_is_an_empty_call(H, k, stride):
+    """A window that does not fit makes an empty patch matrix: a call that does nothing, and no host fault (in a child
+    process: a division by zero ends the process that makes it)."""
+    side = int((H - k) / stride) + 1
+    code = f"""
+import ctypes
+from bamboo_b200 import lib as L
+i = ctypes.c_int
+rc = L.load().bb_im2col_nhwc(ctypes.c_void_p(1 << 20), ctypes.c_void_p(1 << 21), i(3), i({H}), i({H}), i(8), i({k}), i({stride}), i(0),
+                             i({side}), i({side}), ctypes.c_longlong({k * k * 8}), None)
+assert rc == 0, (rc, L.load().bb_last_error())
+"""
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, (done.returncode, done.stderr[-500:])

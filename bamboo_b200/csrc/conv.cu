@@ -719,7 +719,9 @@ bool conv_sizes(const bb_conv_desc* d, ConvSizes* s) {
   s->P = (long long)d->N * s->Ho * s->Wo;
   s->K = (long long)d->k * d->k * d->Cin;
   s->direct = d->k == 1 && d->stride == 1;
-  s->implicit_x = !s->direct && bb_conv_gemm_supported(d->Cin, d->k, d->stride, d->pad);
+  // (with a stride, Ho = 1 also stands for a window that overhangs the padded image, which has no im2col box)
+  s->implicit_x = !s->direct && bb_conv_gemm_supported(d->Cin, d->k, d->stride, d->pad) &&
+                  (d->H < d->W ? d->H : d->W) + 2 * d->pad >= d->k;
   s->implicit_dx = !s->direct && d->stride == 1 && d->pad < d->k && bb_conv_gemm_supported(d->Cout, d->k, 1, d->k - 1 - d->pad);
   s->bn_bytes = bb_bn_workspace_bytes(s->P, d->Cout);
   if (s->bn_bytes < 0) return false;

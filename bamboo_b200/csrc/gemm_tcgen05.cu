@@ -1048,6 +1048,7 @@ bool bb_conv_gemm_supported(int C, int k, int stride, int pad) {
 int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream) {
   const long long P = (long long)a->N * a->Ho * a->Wo;
   if (!a->x || !a->other || !a->D || P <= 0 || P >= (1LL << 31) || !bb_conv_gemm_supported(a->C, a->k, a->stride, a->pad) ||
+      a->H + 2 * a->pad < a->k || a->W + 2 * a->pad < a->k ||
       a->other_channels <= 0 || (a->other_channels & 7) || (a->mode == BB_CONV_DGRAD && a->stride != 1) ||
       (((uintptr_t)a->x | (uintptr_t)a->other | (uintptr_t)a->D) & 15)) {
     bb_set_last_error_msg("bb_conv_gemm: null or unaligned operand, or a geometry the im2col loads cannot express");

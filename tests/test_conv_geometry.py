@@ -1,4 +1,5 @@
 """Which route a convolution's geometry takes, and its limits, as far as the library decides them on the host."""
+import ctypes
 import subprocess
 import sys
 
@@ -21,3 +22,15 @@ assert rc == 0, (rc, L.load().bb_last_error())
 """
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, (done.returncode, done.stderr[-500:])
+
+
+# (H, W, k, stride, pad): Ho or Wo = 1 by rounding towards zero, although the window is larger than the padded image
+@pytest.mark.parametrize("H,W,k,stride,pad", [(2, 2, 4, 3, 0), (1, 9, 2, 2, 0), (9, 1, 2, 2, 0), (1, 1, 7, 8, 2)])
+def test_overhanging_windows_are_gathered_into_a_patch_matrix(H, W, k, stride, pad):
+    """The im2col loads have no box for them, so the layer's scratch has to hold the patch matrix."""
+    from bamboo_b200 import lib as L
+    N, cin, cout = 5, 64, 64
+    fake = 1 << 20
+    d = L.ConvDesc(N=N, H=H, W=W, Cin=cin, Cout=cout, k=k, stride=stride, pad=pad, relu=0, eps=1e-5, max_ctas=0, w=fake, gamma=fake, beta=fake)
+    windows = N * (int((H + 2 * pad - k) / stride) + 1) * (int((W + 2 * pad - k) / stride) + 1)
+    assert L.load().bb_conv_bn_scratch_bytes(ctypes.byref(d), 0, 0) >= windows * k * k * cin * 2

@@ -699,7 +699,7 @@ inline long long up256(long long n) { return (n + 255) & ~255LL; }
 struct ConvSizes {
   int Ho, Wo;
   long long P, K;
-  bool direct;                       // 1 x 1 / stride 1: the activation tensor is the patch matrix
+  bool direct;                       // 1 x 1 / stride 1 without padding: the activation tensor is the patch matrix
   // Patches gathered by the GEMM's own loads (bb_conv_gemm) instead of a stored patch matrix: needs 64-channel blocks.
   // Forward and weight gradient read windows of x, the input gradient windows of dy; with a stride the latter would
   // need dy spread out with zeros, so it keeps the patch-gradient matrix and its adjoint gather.
@@ -718,7 +718,7 @@ bool conv_sizes(const bb_conv_desc* d, ConvSizes* s) {
   if (s->Ho <= 0 || s->Wo <= 0) return false;
   s->P = (long long)d->N * s->Ho * s->Wo;
   s->K = (long long)d->k * d->k * d->Cin;
-  s->direct = d->k == 1 && d->stride == 1;
+  s->direct = d->k == 1 && d->stride == 1 && d->pad == 0;
   // (with a stride, Ho = 1 also stands for a window that overhangs the padded image, which has no im2col box)
   s->implicit_x = !s->direct && bb_conv_gemm_supported(d->Cin, d->k, d->stride, d->pad) &&
                   (d->H < d->W ? d->H : d->W) + 2 * d->pad >= d->k;

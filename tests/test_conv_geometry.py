@@ -34,3 +34,14 @@ def test_overhanging_windows_are_gathered_into_a_patch_matrix(H, W, k, stride, p
     d = L.ConvDesc(N=N, H=H, W=W, Cin=cin, Cout=cout, k=k, stride=stride, pad=pad, relu=0, eps=1e-5, max_ctas=0, w=fake, gamma=fake, beta=fake)
     windows = N * (int((H + 2 * pad - k) / stride) + 1) * (int((W + 2 * pad - k) / stride) + 1)
     assert L.load().bb_conv_bn_scratch_bytes(ctypes.byref(d), 0, 0) >= windows * k * k * cin * 2
+
+
+@pytest.mark.parametrize("pad", [1, 3])
+def test_padded_pointwise_convolution_is_not_read_from_the_activations(pad):
+    """A 1 x 1 convolution with padding has more output positions than input pixels: read as the patch matrix, the
+    activation tensor would end too early."""
+    from bamboo_b200 import lib as L
+    N, side, cin, cout = 2, 5, 64, 64
+    fake = 1 << 20
+    d = L.ConvDesc(N=N, H=side, W=side, Cin=cin, Cout=cout, k=1, stride=1, pad=pad, relu=0, eps=1e-5, max_ctas=0, w=fake, gamma=fake, beta=fake)
+    assert L.load().bb_conv_bn_scratch_bytes(ctypes.byref(d), 0, 0) >= N * (side + 2 * pad) ** 2 * cin * 2

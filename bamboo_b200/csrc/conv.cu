@@ -38,36 +38,42 @@ struct ConvGeom {
 // Both patch kernels walk image rows (blockIdx.y) and 16-byte chunks inside a row (blockIdx.x): the indices of a chunk
 // then take three multiplications by reciprocals.  With a 64-bit division per index, the 7 x 7 / stride 2 gather of
 // 32 x 224 x 224 x 8 took 144 us for its 315 MB (arithmetic, not memory; now 72 us), the fourteen adjoint gathers of an
-// image-network step 574 us (now 442 us).
+// image-network step 574 us (now 442 us).  Index type I: rows of 2^31 chunks (34 GB) and more take 64-bit divisions.
 struct ConvMagic { unsigned long long row_chunks, chunks, k, rows; };
 constexpr int PATCH_U = 4;             // chunks per thread of the gather
 
+template <typename I> __device__ __forceinline__ I chunk_div(I n, I d, unsigned long long magic) {
+  if constexpr (sizeof(I) == 4) return bb::fast_div(n, magic);
+  else return n / d;
+}
+
 // col[(n, ho, wo), (r, s, c)] = x[n, ho*stride - pad + r, wo*stride - pad + s, c]  (0 outside)
+template <typename I>
 __global__ void __launch_bounds__(256)
 im2col_kernel(const uint4* x, uint4* __restrict__ col, const ConvGeom g, const ConvMagic m) {
   bb::pdl_sync();
-  const unsigned chunks = g.C >> 3;                       // 16-byte chunks per pixel
-  const unsigned row_chunks = g.k * g.k * chunks;
-  const unsigned total = g.Wo * row_chunks;
+  const I chunks = g.C >> 3;                              // 16-byte chunks per pixel
+  const I row_chunks = (I)g.k * g.k * chunks;
+  const I total = g.Wo * row_chunks;
   const long long ld16 = g.ld_col >> 3;
-  const unsigned e0 = blockIdx.x * (256 * PATCH_U) + threadIdx.x;
+  const I e0 = (I)blockIdx.x * (256 * PATCH_U) + threadIdx.x;
   for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.Ho; row += gridDim.y) {
     const unsigned n = bb::fast_div(row, m.rows);
     const int h0 = (int)(row - n * g.Ho) * g.stride - g.pad;
-    const uint4* xi = x + (long long)n * g.H * g.W * chunks;
+    const uint4* xi = x + (long long)n * g.H * g.W * (long long)chunks;
     uint4* out = col + (long long)row * g.Wo * ld16;
     uint4 v[PATCH_U];
     long long dst[PATCH_U];
 #pragma unroll
     for (int u = 0; u < PATCH_U; ++u) {
-      const unsigned e = e0 + u * 256;
-      const unsigned wo = bb::fast_div(e, m.row_chunks), within = e - wo * row_chunks;
-      const unsigned tap = bb::fast_div(within, m.chunks), cc = within - tap * chunks;
-      const unsigned r = bb::fast_div(tap, m.k), s = tap - r * g.k;
+      const I e = e0 + u * 256;
+      const I wo = chunk_div<I>(e, row_chunks, m.row_chunks), within = e - wo * row_chunks;
+      const I tap = chunk_div<I>(within, chunks, m.chunks), cc = within - tap * chunks;
+      const I r = chunk_div<I>(tap, g.k, m.k), s = tap - r * g.k;
       const int h = h0 + (int)r, w = (int)wo * g.stride - g.pad + (int)s;
       dst[u] = e < total ? (long long)wo * ld16 + within : -1;
       v[u] = make_uint4(0, 0, 0, 0);
-      if (e < total && h >= 0 && h < g.H && w >= 0 && w < g.W) v[u] = __ldca(xi + ((long long)h * g.W + w) * chunks + cc);
+      if (e < total && h >= 0 && h < g.H && w >= 0 && w < g.W) v[u] = __ldca(xi + ((long long)h * g.W + w) * (long long)chunks + cc);
     }
 #pragma unroll
     for (int u = 0; u < PATCH_U; ++u) if (dst[u] >= 0) out[dst[u]] = v[u];
@@ -77,15 +83,16 @@ im2col_kernel(const uint4* x, uint4* __restrict__ col, const ConvGeom g, const C
 // Adjoint of the gather: dx[n, h, w, c] = sum over the (output pixel, tap) pairs that read it.
 // Gather form (one thread owns an input pixel's chunk): no atomics, fixed summation order (r, then s, ascending).
 // The taps that reach a pixel are every stride-th one; along them the output pixel moves back by one.
+template <typename I>
 __global__ void __launch_bounds__(256)
 col2im_kernel(const uint4* dcol, uint4* __restrict__ dx, const ConvGeom g, const ConvMagic m) {
   bb::pdl_sync();
-  const unsigned chunks = g.C >> 3;
-  const unsigned total = g.W * chunks;
+  const I chunks = g.C >> 3;
+  const I total = g.W * chunks;
   const long long ld16 = g.ld_col >> 3;
-  const unsigned e = blockIdx.x * 256 + threadIdx.x;
+  const I e = (I)blockIdx.x * 256 + threadIdx.x;
   if (e >= total) return;
-  const unsigned w = bb::fast_div(e, m.chunks), cc = e - w * chunks;
+  const I w = chunk_div<I>(e, chunks, m.chunks), cc = e - w * chunks;
   const int s0 = (int)(w + g.pad) % g.stride, wo0 = (int)(w + g.pad) / g.stride;
   for (unsigned row = blockIdx.y; row < (unsigned)g.N * g.H; row += gridDim.y) {
     const unsigned n = bb::fast_div(row, m.rows);
@@ -94,7 +101,7 @@ col2im_kernel(const uint4* dcol, uint4* __restrict__ dx, const ConvGeom g, const
     int ho = (h + g.pad) / g.stride;
     for (int r = (h + g.pad) % g.stride; r < g.k && ho >= 0; r += g.stride, --ho) {
       if (ho >= g.Ho) continue;
-      const uint4* src = dcol + ((long long)n * g.Ho + ho) * g.Wo * ld16 + (long long)r * g.k * chunks + cc;
+      const uint4* src = dcol + ((long long)n * g.Ho + ho) * g.Wo * ld16 + (long long)r * g.k * (long long)chunks + cc;
       int wo = wo0;
 #pragma unroll 4
       for (int s = s0; s < g.k; s += g.stride, --wo) {
@@ -112,11 +119,11 @@ col2im_kernel(const uint4* dcol, uint4* __restrict__ dx, const ConvGeom g, const
 bool bad_geom(const ConvGeom& g) {
   return g.N <= 0 || g.H <= 0 || g.W <= 0 || g.C <= 0 || (g.C & 7) || g.k <= 0 || g.stride <= 0 || g.pad < 0 ||
          g.Ho != (g.H + 2 * g.pad - g.k) / g.stride + 1 || g.Wo != (g.W + 2 * g.pad - g.k) / g.stride + 1 ||
-         g.ld_col < (long long)g.k * g.k * g.C || (g.ld_col & 7) ||
-         // 32-bit indices inside a row of windows (34 GB of patches) and over the rows
-         (long long)g.Wo * g.k * g.k * (g.C >> 3) >= (1LL << 31) || (long long)g.W * (g.C >> 3) >= (1LL << 31) ||
-         (long long)g.N * g.H >= (1LL << 31) || (long long)g.N * g.Ho >= (1LL << 31);
+         g.ld_col < (long long)g.k * g.k * g.C || (g.ld_col & 7);
 }
+constexpr long long PATCH_32BIT = 1LL << 31;       // chunks of a row, rows of a launch
+// images whose rows one launch can count
+int patch_images(int rows_per_image) { return (int)((PATCH_32BIT - 1) / rows_per_image); }
 dim3 patch_grid(long long chunks_per_row, int per_block, long long rows) {
   return dim3((unsigned)((chunks_per_row + per_block - 1) / per_block), (unsigned)(rows < 65535 ? rows : 65535));
 }
@@ -131,10 +138,19 @@ extern "C" int bb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int
     return BB_ERR_INVALID_ARG;
   }
   if (Ho <= 0 || Wo <= 0) return BB_OK;        // a window larger than the padded image: no patches
-  const int chunks = C >> 3, row_chunks = k * k * chunks;
-  const ConvMagic m = {bb_div_magic(row_chunks), bb_div_magic(chunks), bb_div_magic(k), bb_div_magic(Ho)};
-  bb_launch(im2col_kernel, patch_grid((long long)Wo * row_chunks, 256 * PATCH_U, (long long)N * Ho), 256, 0, (cudaStream_t)stream, (const uint4*)x, (uint4*)col, g, m);
-  BB_CUDA_CHECK(cudaGetLastError());
+  const int chunks = C >> 3;
+  const long long row_chunks = (long long)k * k * chunks, total = Wo * row_chunks;
+  const bool small = total < PATCH_32BIT;
+  const ConvMagic m = {small ? bb_div_magic((int)row_chunks) : 0, bb_div_magic(chunks), bb_div_magic(k), bb_div_magic(Ho)};
+  auto kernel = small ? im2col_kernel<unsigned> : im2col_kernel<unsigned long long>;
+  const int per = patch_images(Ho);
+  for (long long n = 0; n < N; n += per) {
+    ConvGeom part = g;
+    part.N = (int)(N - n < per ? N - n : per);
+    bb_launch(kernel, patch_grid(total, 256 * PATCH_U, (long long)part.N * Ho), 256, 0, (cudaStream_t)stream,
+              (const uint4*)x + n * H * W * chunks, (uint4*)col + n * Ho * Wo * (ld_col >> 3), part, m);
+    BB_CUDA_CHECK(cudaGetLastError());
+  }
   return BB_OK;
 }
 
@@ -146,9 +162,17 @@ extern "C" int bb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, i
     return BB_ERR_INVALID_ARG;
   }
   const int chunks = C >> 3;
+  const long long total = (long long)W * chunks, windows = Ho > 0 && Wo > 0 ? (long long)Ho * Wo : 0;
   const ConvMagic m = {0, bb_div_magic(chunks), 0, bb_div_magic(H)};
-  bb_launch(col2im_kernel, patch_grid((long long)W * chunks, 256, (long long)N * H), 256, 0, (cudaStream_t)stream, (const uint4*)dcol, (uint4*)dx, g, m);
-  BB_CUDA_CHECK(cudaGetLastError());
+  auto kernel = total < PATCH_32BIT ? col2im_kernel<unsigned> : col2im_kernel<unsigned long long>;
+  const int per = patch_images(H);
+  for (long long n = 0; n < N; n += per) {
+    ConvGeom part = g;
+    part.N = (int)(N - n < per ? N - n : per);
+    bb_launch(kernel, patch_grid(total, 256, (long long)part.N * H), 256, 0, (cudaStream_t)stream,
+              (const uint4*)dcol + n * windows * (ld_col >> 3), (uint4*)dx + n * H * W * chunks, part, m);
+    BB_CUDA_CHECK(cudaGetLastError());
+  }
   return BB_OK;
 }
 

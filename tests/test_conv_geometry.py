@@ -45,3 +45,18 @@ def test_padded_pointwise_convolution_is_not_read_from_the_activations(pad):
     fake = 1 << 20
     d = L.ConvDesc(N=N, H=side, W=side, Cin=cin, Cout=cout, k=1, stride=1, pad=pad, relu=0, eps=1e-5, max_ctas=0, w=fake, gamma=fake, beta=fake)
     assert L.load().bb_conv_bn_scratch_bytes(ctypes.byref(d), 0, 0) >= N * (side + 2 * pad) ** 2 * cin * 2
+
+
+# (N, H, W, C, k): a row of windows, a row of pixels, and the rows of all images beyond 31 bits
+@pytest.mark.parametrize("N,H,W,C,k", [(1, 64, (1 << 19) + 63, 8, 64), (1, 1, 1 << 22, 4096, 1), (1 << 16, 1 << 15, 1, 8, 1)])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_patch_kernels_accept_rows_beyond_31_bits(N, H, W, C, k, adjoint):
+    """34 GB of patches fit a GPU.  Without one the launch fails, but the geometry is not refused."""
+    import torch
+    from bamboo_b200 import lib as L
+    if torch.cuda.is_available():
+        pytest.skip("the pointers are no device memory")
+    i, fn = ctypes.c_int, L.load().bb_col2im_nhwc if adjoint else L.load().bb_im2col_nhwc
+    rc = fn(ctypes.c_void_p(1 << 20), ctypes.c_void_p(1 << 21), i(N), i(H), i(W), i(C), i(k), i(1), i(0), i(H - k + 1), i(W - k + 1),
+            ctypes.c_longlong(k * k * C), None)
+    assert rc == -2, (rc, L.load().bb_last_error())

@@ -108,7 +108,7 @@ extern "C" int bb_block_half_fwd(const bb_block_desc* d, int half, const void* x
     bb_set_last_error_msg("bb_block_half_fwd: bad descriptor or null buffer");
     return BB_ERR_INVALID_ARG;
   }
-  const BackToBack scope(d->max_ctas >= 0);
+  const BackToBack scope(d->max_ctas == 0);
   const int T = d->tokens, h = d->hidden;
   uint8_t* sv = static_cast<uint8_t*>(saved);
   if (half == BB_HALF_ATTENTION) {
@@ -149,7 +149,7 @@ extern "C" int bb_block_half_bwd(const bb_block_desc* d, int half, const void* x
   // successor that already waits there keeps them out.  So kernels overlap their predecessor only where that GEMM has no
   // more tiles than the GPU has SMs, and launches count for more than the tail (one step: 8192 tokens x 1024 33.4 ms
   // without, 34.4 ms with overlap; forward + backward of one block: 2331 tokens x 1024 406 us without, 398 us with).
-  const BackToBack scope(d->max_ctas >= 0 &&
+  const BackToBack scope(d->max_ctas == 0 &&
                          (side_stream == stream || (long long)((T + 127) / 128) * ((h + 255) / 256) <= bb_num_sms()));
   const uint8_t* sv = static_cast<const uint8_t*>(saved);
   uint8_t* sc = static_cast<uint8_t*>(scratch);

@@ -48,8 +48,8 @@ int bb_current_device();
 // serialization): launch, barrier set-up and tensor-memory allocation then cost nothing on the stream.  A kernel waits
 // for that predecessor - complete, its memory visible - in bb::pdl_sync() before it touches global memory, and only
 // then lets its own successor in, so a kernel never overlaps more than its direct neighbours and everything before the
-// predecessor is complete too.  Work that must hand its SMs back at once (max_ctas < 0: redundant computation beside the
-// main stream) is launched plainly: a kernel that waits keeps its SMs.
+// predecessor is complete too.  Work beside the main stream (max_ctas other than 0: redundant computation with short CTAs
+// or on a budget of them) is launched plainly: a kernel that waits keeps its SMs.
 extern thread_local int bb_back_to_back;
 struct BackToBack {
   const int n;

@@ -795,7 +795,7 @@ int conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void
     bb_set_last_error_msg("bb_conv_bn_fwd: bad descriptor, null buffer or scratch smaller than bb_conv_bn_scratch_bytes");
     return BB_ERR_INVALID_ARG;
   }
-  const BackToBack scope(d->max_ctas >= 0);
+  const BackToBack scope(d->max_ctas == 0);
   uint8_t* sc = static_cast<uint8_t*>(scratch);
   if (s.implicit_x) {
     BB_TRY(conv_implicit(d, s, BB_CONV_FWD, x, d->w, y, stream));
@@ -821,7 +821,7 @@ int conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void*
     bb_set_last_error_msg("bb_conv_bn_bwd: bad descriptor, null buffer, missing gradient pointer or scratch too small");
     return BB_ERR_INVALID_ARG;
   }
-  const BackToBack scope(d->max_ctas >= 0);
+  const BackToBack scope(d->max_ctas == 0);
   uint8_t* sc = static_cast<uint8_t*>(scratch);
   void* dy = sc;
   uint8_t* colbuf = sc + s.dy_bytes;

@@ -474,6 +474,7 @@ int bb_attention_tc_fwd(const void* qkv_q, void* out, float* lse, int B, int H, 
 int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, const float* lse, void* dq, void* dk, void* dv,
                         float* delta, float* dq_acc, int B, int H, int S, int D, long long stride_qkv, long long stride_o,
                         long long stride_dqkv, int causal, float scale, cudaStream_t stream);
+int bb_attention_tc_bwd_launches(int D);
 
 namespace {
 // The tcgen05 kernels (attention_tc.cu) read q, k, v through one tensor map over the packed
@@ -524,6 +525,13 @@ long long attn_ws_delta_bytes(int B, int H, int S) { return (((long long)B * H *
 extern "C" long long bb_attention_bwd_workspace_bytes(int B, int H, int S) {
   if (B <= 0 || H <= 0 || S <= 0) return 0;
   return attn_ws_delta_bytes(B, H, S) + (long long)B * H * S * 64 * (long long)sizeof(float);
+}
+
+extern "C" int bb_attention_bwd_launches(int H, int D) {
+  // (any address: q, k and v are slices of one packed projection)
+  const char* q = reinterpret_cast<const char*>(16);
+  const long long hb = (long long)H * D * 2;
+  return use_tc_path(q, q + hb, q + 2 * hb, H, D, 3LL * H * D) ? bb_attention_tc_bwd_launches(D) : 3;
 }
 
 extern "C" int bb_attention_bwd(const void* q, const void* k, const void* v, const void* out, const void* d_out, const float* lse,

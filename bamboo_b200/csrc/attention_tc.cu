@@ -1512,6 +1512,13 @@ int bb_attention_tc_fwd(const void* qkv_q, void* out, float* lse, int B, int H, 
 }
 
 namespace {
+// BB_ATTENTION_BWD=split in the environment selects the two-role kernel (dK/dV and dQ computed by
+// different CTAs, every sum in a fixed order) at head dimension 64; the default there is the fused kernel
+bool split_backward() {
+  static const bool split = [] { const char* e = getenv("BB_ATTENTION_BWD"); return e && e[0] == 's'; }();
+  return split;
+}
+
 // the two-role kernel (see attn_tc_bwd2_kernel): delta pre-pass, then dK / dV and dQ tiles in one launch
 template <int D>
 int launch_bwd2(const CUtensorMap& tm_qkv, const CUtensorMap& tm_qkv64, const CUtensorMap& tm_do, const CUtensorMap& tm_do64,
@@ -1524,6 +1531,9 @@ int launch_bwd2(const CUtensorMap& tm_qkv, const CUtensorMap& tm_qkv64, const CU
   return BB_OK;
 }
 }  // namespace
+
+// delta and the two-role kernel, or delta, the fused kernel and the conversion of dQ
+int bb_attention_tc_bwd_launches(int D) { return D == 128 || split_backward() ? 2 : 3; }
 
 int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, const float* lse, void* dq, void* dk, void* dv,
                         float* delta, float* dq_acc, int B, int H, int S, int D, long long stride_qkv, long long stride_o,
@@ -1548,10 +1558,7 @@ int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, c
   // Head dimension 128: the two-role kernel.  The fused kernel's tensor-memory map (scores, dP, dV, dK and two dQ
   // tiles) would need 768 columns there.
   if (D == 128) return launch_bwd2<128>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
-  // BB_ATTENTION_BWD=split in the environment selects the two-role kernel (dK/dV and dQ computed by
-  // different CTAs, every sum in a fixed order); the default is the fused kernel
-  static const bool split = [] { const char* e = getenv("BB_ATTENTION_BWD"); return e && e[0] == 's'; }();
-  if (split) return launch_bwd2<64>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
+  if (split_backward()) return launch_bwd2<64>(tm_qkv, tm_qkv64, tm_do, tm_do64, out, d_out, p, (int)dgrid, stream);
   p.dq_acc = dq_acc;
   BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd3_kernel, BWD3_SMEM)) return rc; });
   bb_launch(attn_tc_delta_kernel<64>, (int)dgrid, 256, 0, stream, (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);

@@ -787,6 +787,15 @@ extern "C" long long bb_conv_bn_scratch_bytes(const bb_conv_desc* d, int backwar
   return s.dy_bytes + s.col_bytes + (need_dx ? s.dcol_bytes : 0) + s.bn_bytes;
 }
 
+extern "C" int bb_conv_bn_launches(const bb_conv_desc* d, int backward, int need_dx) {
+  ConvSizes s;
+  if (!conv_sizes(d, &s)) return -1;
+  // the product with the input's patches (and their gather), three passes of batch norm; the input gradient (and its adjoint gather)
+  int n = 4 + (s.direct || s.implicit_x ? 0 : 1);
+  if (backward && need_dx) n += s.direct || s.implicit_dx ? 1 : 2;
+  return n;
+}
+
 namespace {
 int conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void* y, void* z, float* mean, float* rstd, float* affine,
                 void* scratch, long long scratch_bytes, void* stream) {

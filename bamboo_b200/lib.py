@@ -63,7 +63,7 @@ class ConvDesc(ctypes.Structure):
 HALF_ATTENTION, HALF_MLP = 0, 1
 # kernels behind one call of bb_block_half_fwd / bb_block_half_bwd, per half (launch accounting)
 HALF_FWD_LAUNCHES = {HALF_ATTENTION: 4, HALF_MLP: 3}
-HALF_BWD_LAUNCHES = {HALF_ATTENTION: 10, HALF_MLP: 7}   # attention backward: three launches for either head dimension
+HALF_BWD_LAUNCHES = {HALF_ATTENTION: 7, HALF_MLP: 7}   # and those of the attention backward (bb_attention_bwd_launches)
 
 _lib = None
 _lock = threading.Lock()
@@ -315,12 +315,12 @@ def attention_fwd(qkv, out, lse, B, H, S, D, causal, scale=None):
 
 def attention_bwd(qkv, out, dout, lse, dqkv, B, H, S, D, causal, scale=None):
     global LAUNCHES
-    LAUNCHES += 3
+    lib = load()
+    LAUNCHES += lib.bb_attention_bwd_launches(_I(H), _I(D))
     hd = H * D
     esz = qkv.element_size()
     base, dbase = qkv.data_ptr(), dqkv.data_ptr()
     scale = (1.0 / D ** 0.5) if scale is None else scale
-    lib = load()
     lib.bb_attention_bwd_workspace_bytes.restype = _LL
     need = lib.bb_attention_bwd_workspace_bytes(_I(B), _I(H), _I(S))
     ws = workspace(need, "attention")
@@ -389,10 +389,13 @@ def block_half_fwd(desc, half, x, saved, out):
 def block_half_bwd(desc, half, x, saved, dout, dx, scratch, side_stream=None):
     """``side_stream``: raw handle of the stream for the weight gradients (None: the current stream)."""
     global LAUNCHES
+    lib = _lib or load()
     LAUNCHES += HALF_BWD_LAUNCHES[half]
+    if half == HALF_ATTENTION:
+        LAUNCHES += lib.bb_attention_bwd_launches(desc.heads, desc.head_dim)
     main = _raw_stream()
-    rc = (_lib or load()).bb_block_half_bwd(ctypes.byref(desc), half, x.data_ptr(), saved.data_ptr(), dout.data_ptr(), dx.data_ptr(),
-                                            scratch.data_ptr(), scratch.numel(), main, main if side_stream is None else side_stream)
+    rc = lib.bb_block_half_bwd(ctypes.byref(desc), half, x.data_ptr(), saved.data_ptr(), dout.data_ptr(), dx.data_ptr(),
+                               scratch.data_ptr(), scratch.numel(), main, main if side_stream is None else side_stream)
     if rc < 0:
         check(rc, "bb_block_half_bwd")
     return dx
@@ -487,20 +490,20 @@ def avgpool_bwd(dy, dx):
     return dx
 
 
-def _conv_route(desc):
-    """(direct, implicit_x, implicit_dx) as bb_conv_bn_fwd / bb_conv_bn_bwd choose it (launch accounting)."""
-    direct = desc.k == 1 and desc.stride == 1
-    small = desc.k <= 64 and desc.pad < desc.k
-    return direct, not direct and small and desc.Cin % 64 == 0 and desc.stride <= 8, \
-        not direct and small and desc.Cout % 64 == 0 and desc.stride == 1
+def _conv_launches(desc, backward, need_dx):
+    """Kernels behind one call (launch accounting), asked once per descriptor."""
+    counts = desc.__dict__.setdefault("_launches", {})
+    key = (backward, need_dx)
+    if key not in counts:
+        counts[key] = max(0, load().bb_conv_bn_launches(ctypes.byref(desc), _I(backward), _I(need_dx)))
+    return counts[key]
 
 
 def conv_bn_fwd(desc, x, residual, y, z, mean, rstd, scratch, affine=None):
     """``mean`` / ``rstd`` / ``affine``: fp32 tensors, or their device addresses.  ``affine`` [2, Cout] (without a residual
     only) keeps the scale and shift for ``conv_bn_bwd``."""
     global LAUNCHES
-    direct, implicit_x, _ = _conv_route(desc)
-    LAUNCHES += 4 + (0 if direct or implicit_x else 1)
+    LAUNCHES += _conv_launches(desc, 0, 0)
     lib = _lib or load()
     tail = (scratch.data_ptr(), scratch.numel(), _raw_stream())
     if affine is None:
@@ -518,8 +521,7 @@ def conv_bn_bwd(desc, x, y, z, mean, rstd, dz, dx, dres, scratch, residual=True,
     """``residual=False``: the forward call added none.  ``affine``: what that call kept; the ReLU mask then comes from y and
     not from z.  ``mean`` / ``rstd`` / ``affine``: fp32 tensors, or their device addresses."""
     global LAUNCHES
-    direct, implicit_x, implicit_dx = _conv_route(desc)
-    LAUNCHES += 4 + (0 if direct or implicit_x else 1) + (0 if dx is None else (1 if direct or implicit_dx else 2))
+    LAUNCHES += _conv_launches(desc, 1, int(dx is not None))
     lib = _lib or load()
     tail = (scratch.data_ptr(), scratch.numel(), _raw_stream())
     if affine is not None:

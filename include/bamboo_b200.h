@@ -154,6 +154,8 @@ int bb_attention_fwd(const void* q, const void* k, const void* v, void* out, flo
  * from run to run (the order of a row's additions is not fixed); dk and dv do not.
  * BB_ATTENTION_BWD=split in the environment selects kernels that keep every sum in a fixed order. */
 long long bb_attention_bwd_workspace_bytes(int B, int H, int S);
+/* Kernels that bb_attention_bwd launches for a packed projection (launch accounting). */
+int bb_attention_bwd_launches(int H, int D);
 int bb_attention_bwd(const void* q, const void* k, const void* v, const void* out, const void* d_out, const float* lse,
                      void* dq, void* dk, void* dv, void* workspace, long long workspace_bytes, int B, int H, int S,
                      int D, long long stride_qkv, long long stride_o, long long stride_dqkv, int causal, float scale,
@@ -256,6 +258,8 @@ typedef struct bb_conv_desc {
   float *g_w, *g_gamma, *g_beta;      /* fp32 gradient accumulators (backward only) */
 } bb_conv_desc;
 long long bb_conv_bn_scratch_bytes(const bb_conv_desc* d, int backward, int need_dx);
+/* Kernels that the calls below launch (launch accounting); -1: a geometry that they refuse. */
+int bb_conv_bn_launches(const bb_conv_desc* d, int backward, int need_dx);
 int bb_conv_bn_fwd(const bb_conv_desc* d, const void* x, const void* residual, void* y, void* z, float* mean, float* rstd,
                    void* scratch, long long scratch_bytes, void* stream);
 int bb_conv_bn_bwd(const bb_conv_desc* d, const void* x, const void* y, const void* z, const float* mean, const float* rstd,

@@ -24,25 +24,37 @@ def _block(heads, head_dim):
     return layers.TransformerBlock(heads * head_dim, heads, 4 * heads * head_dim, causal=True)
 
 
-def _conv(cin, cout, k):
+def _conv(cin, cout, k, stride=1):
     from bamboo_b200 import resnet
-    return resnet.ConvBN(cin, cout, k, relu=True, generator=torch.Generator().manual_seed(3))
+    return resnet.ConvBN(cin, cout, k, stride=stride, relu=True, generator=torch.Generator().manual_seed(3))
 
 
-def _programmatic_edges(fn):
-    """Edges of the captured call along which a kernel may start before the one in front of it has ended."""
+def captured(fn):
+    """The call as a graph that is not run (its caches and attributes are set up by a call before)."""
     from cuda.bindings import runtime as rt
     fn()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         fn()
-    handle = rt.cudaGraph_t(graph.raw_cuda_graph())
+    return graph, rt.cudaGraph_t(graph.raw_cuda_graph()), rt
+
+
+def _programmatic_edges(fn):
+    """Edges of the captured call along which a kernel may start before the one in front of it has ended."""
+    graph, handle, rt = captured(fn)
     err, *_, n = rt.cudaGraphGetEdges_v2(handle)
     assert err == rt.cudaError_t.cudaSuccess
     err, _from, _to, data, n = rt.cudaGraphGetEdges_v2(handle, n)
     assert err == rt.cudaError_t.cudaSuccess and n > 0
     return sum(int(d.type) == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for d in data[:n])
+
+
+def kernel_nodes(handle, rt):
+    err, _nodes, n = rt.cudaGraphGetNodes(handle)
+    err, nodes, n = rt.cudaGraphGetNodes(handle, n)
+    assert err == rt.cudaError_t.cudaSuccess
+    return [v for v in nodes[:n] if rt.cudaGraphNodeGetType(v)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel]
 
 
 @pytest.mark.parametrize("layer", ["block", "conv"])
@@ -109,3 +121,26 @@ def test_a_convolution_gives_the_same_bits_with_and_without_overlap(cin, cout, k
         for a, b in zip(step(0), want):
             assert torch.equal(a, b)
     assert lib.read_status() == 0
+
+
+@pytest.mark.parametrize("make,shape", [(lambda: _block(4, 64), (2, 100, 256)), (lambda: _block(2, 128), (3, 70, 256)),
+                                        (lambda: _conv(64, 64, 3), (3, 15, 15, 64)), (lambda: _conv(64, 64, 3, 2), (3, 15, 15, 64)),
+                                        (lambda: _conv(16, 64, 1), (3, 15, 15, 16)), (lambda: _conv(64, 16, 3), (3, 15, 15, 64)),
+                                        (lambda: _conv(8, 32, 7, 2), (3, 15, 15, 8))])
+def test_launch_accounting_is_that_of_the_captured_call(make, shape):
+    """lib.LAUNCHES grows by the kernels that a layer's forward and backward call launch, on whichever route."""
+    from bamboo_b200 import layers, lib
+    m = make()
+    _arena([m])
+    x = torch.randn(*shape, device="cuda").bfloat16().requires_grad_(True)
+    dout, counted = torch.ones_like(m(x)), []
+
+    def fn():
+        before = lib.LAUNCHES
+        torch.autograd.grad(m(x), x, dout)
+        if isinstance(m, layers.TransformerBlock):
+            layers.wgrad_sync(x.device)              # (a convolution layer has no work on that stream to join)
+        counted.append(lib.LAUNCHES - before)
+    graph, handle, rt = captured(fn)
+    nodes = len(kernel_nodes(handle, rt))
+    assert counted == [nodes, nodes]

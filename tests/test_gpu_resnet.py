@@ -203,8 +203,9 @@ def test_relu_mask_is_that_of_the_forward_pass(L, residual):
 
 
 # (channels in / out, window, stride, image side): reductions of one to several 64-channel blocks, output rows that no
-# 128-row tile divides, images smaller than the window, an even window (asymmetric turned padding), both tile widths and
-# CTA pairs (256 x 256 outputs with reductions of 2048 and more), channel counts that only one direction can gather
+# 128-row tile divides, images smaller than the window, an even window (asymmetric turned padding), both tile widths (and
+# CTA pairs for the weight gradient of 128 -> 512; the other two products: next test), channel counts that only one direction
+# can gather
 @pytest.mark.parametrize("cin,cout,k,stride,hw", [(64, 64, 3, 1, 1), (64, 64, 3, 1, 2), (64, 16, 3, 1, 5), (192, 64, 3, 1, 11),
                                                   (64, 64, 2, 1, 6), (64, 64, 7, 1, 9), (64, 128, 7, 2, 13), (128, 64, 3, 2, 15),
                                                   (64, 128, 1, 2, 7), (256, 256, 3, 1, 14), (256, 256, 3, 2, 29), (512, 128, 3, 1, 7),
@@ -244,6 +245,23 @@ def test_convolution_with_gathered_patches(L, cin, cout, k, stride, hw):
     assert _rel(m.weight.main_grad.view(cout, k, k, cin).permute(0, 3, 1, 2), w.grad) <= 1e-4
     torch.cuda.synchronize()
     assert L.read_status() == 0
+
+
+def test_convolution_with_gathered_patches_on_cta_pairs(L):
+    """256 -> 256, 3 x 3, nine images of 53 x 53: forward product and input gradient are planned to CTA pairs (two waves of
+    99 tiles of 256 x 256 are expected to take 39.6 us, 128 x 256 tiles 40.4, 128 x 128 44), seen in the captured call's cluster sizes."""
+    from bamboo_b200 import resnet
+    from bamboo_b200.arena import ParamArena
+    from test_gpu_overlap import captured, kernel_nodes
+    m = resnet.ConvBN(256, 256, 3, relu=False, generator=torch.Generator().manual_seed(11))
+    ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
+    x = torch.randn(9, 53, 53, 256, device="cuda").bfloat16().requires_grad_(True)
+    dz = torch.ones_like(m(x))
+    graph, handle, rt = captured(lambda: torch.autograd.grad(m(x), x, dz))
+    clusters = [rt.cudaGraphKernelNodeGetAttribute(n, rt.cudaLaunchAttributeID.cudaLaunchAttributeClusterDimension)[1].clusterDim.x
+                for n in kernel_nodes(handle, rt)]
+    assert sum(c == 2 for c in clusters) >= 2, clusters
+    test_convolution_with_gathered_patches(L, 256, 256, 3, 1, 53)
 
 
 def _block_params(blk, prefix):

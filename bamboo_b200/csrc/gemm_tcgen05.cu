@@ -952,13 +952,12 @@ AccumPlan plan_accum(int M, int N, int K) {
 // within a tenth of the measured times; what the choice gained where it changed (us, with a fixed rule before):
 // 513 x 2048 x 2048 26.6 -> 20.5 (128 wide instead of a quarter-filled wave of pairs), 999 x 1024 x 4096 34.8 -> 28.7,
 // 4096 x 1024 x 1024 20.4 -> 16.4 and 8192 x 512 x 1536 24.6 -> 20.5 (one wave of 256 wide tiles instead of two).
-struct StorePlan { int bn; bool pair; };
-StorePlan plan_store(int M, int N, int K, int max_ctas, bool pairs_allowed) {
+struct StorePlan { int bn; bool pair; double us; };
+StorePlan plan_store(long long M, long long N, long long K, int max_ctas, bool pairs_allowed) {
   static const struct { int bn; bool pair; double kblock, wave, once; } kinds[3] = {
       {256, true, 0.34, 2.3, 10.5}, {256, false, 0.41, 1.2, 8.5}, {128, false, 0.30, 1.2, 8.0}};
   const double kb = (double)((K + BK - 1) / BK);
-  StorePlan best = {128, false};
-  double best_us = -1;
+  StorePlan best = {128, false, -1};
   for (const auto& k : kinds) {
     if ((k.bn == 256 && N <= 128) || (k.pair && (!pairs_allowed || M <= BM))) continue;
     const long long tm = k.pair ? 2 * BM : BM;
@@ -967,7 +966,7 @@ StorePlan plan_store(int M, int N, int K, int max_ctas, bool pairs_allowed) {
     if (max_ctas > 0 && max_ctas < workers) workers = max_ctas;
     if (k.pair) workers = workers > 1 ? workers / 2 : 1;
     const double us = (double)((tiles + workers - 1) / workers) * (kb * k.kblock + k.wave) + k.once;
-    if (best_us < 0 || us < best_us) { best_us = us; best = {k.bn, k.pair}; }
+    if (best.us < 0 || us < best.us) best = {k.bn, k.pair, us};
   }
   return best;
 }
@@ -1039,6 +1038,8 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   bb_set_last_error_msg("bb_gemm_bf16: tile_n must be 0, 128 or 256");
   return BB_ERR_INVALID_ARG;
 }
+
+double bb_gemm_store_us(long long M, long long N, long long K) { return plan_store(M, N, K, 0, true).us; }
 
 bool bb_conv_gemm_supported(int C, int k, int stride, int pad) {
   // tensor map limits of a rank-4 im2col load: window corners in [-128, 127], traversal stride <= 8

@@ -2,6 +2,7 @@
 patch gather and its adjoint, batch norm with batch statistics, pooling, one bottleneck block at
 ResNet-152's own dimensions, and a small bottleneck ResNet through the public API (loss and every
 gradient tensor against the oracle)."""
+import ctypes
 import os
 import sys
 
@@ -211,12 +212,24 @@ def test_relu_mask_is_that_of_the_forward_pass(L, residual):
                                                   (64, 128, 1, 2, 7), (256, 256, 3, 1, 14), (256, 256, 3, 2, 29), (512, 128, 3, 1, 7),
                                                   (8, 64, 3, 1, 10), (64, 8, 3, 1, 9), (128, 512, 3, 1, 35)])
 def test_convolution_with_gathered_patches(L, cin, cout, k, stride, hw):
+    check_convolution(L, cin, cout, k, stride, hw, 9)
+
+
+# enough images that the input gradient is gathered as well: images smaller than the window, an even window, rows that no tile
+# divides, fewer input channels than a tile has columns, one of two tile widths
+@pytest.mark.parametrize("cin,cout,k,hw,N", [(64, 64, 3, 1, 30001), (64, 64, 3, 2, 7003), (32, 64, 5, 5, 2001), (192, 64, 3, 11, 201),
+                                             (64, 64, 2, 6, 701), (64, 64, 7, 9, 301), (512, 128, 3, 7, 211)])
+def test_convolution_with_gathered_input_gradient(L, cin, cout, k, hw, N):
+    d = check_convolution(L, cin, cout, k, 1, hw, N)
+    assert L.load().bb_conv_bn_launches(ctypes.byref(d), 1, 1) == (5 if cin % 64 == 0 else 6)
+
+
+def check_convolution(L, cin, cout, k, stride, hw, N):
     """The convolution alone (what the layer feeds into batch norm, and the gradients that come out of it) against
     conv2d in fp32 on the same bf16 operands.  One bf16 rounding of each result: 2^-9 of the value, so 4e-3 in the
     2-norm; the weight gradient is summed and kept in fp32 (1e-4: order of the sums)."""
     from bamboo_b200 import resnet
     from bamboo_b200.arena import ParamArena
-    N = 9
     m = resnet.ConvBN(cin, cout, k, stride=stride, relu=False, generator=torch.Generator().manual_seed(11))
     ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
     g = torch.Generator(device="cuda").manual_seed(12)
@@ -245,6 +258,7 @@ def test_convolution_with_gathered_patches(L, cin, cout, k, stride, hw):
     assert _rel(m.weight.main_grad.view(cout, k, k, cin).permute(0, 3, 1, 2), w.grad) <= 1e-4
     torch.cuda.synchronize()
     assert L.read_status() == 0
+    return d
 
 
 def test_convolution_with_gathered_patches_on_cta_pairs(L):
@@ -261,7 +275,7 @@ def test_convolution_with_gathered_patches_on_cta_pairs(L):
     clusters = [rt.cudaGraphKernelNodeGetAttribute(n, rt.cudaLaunchAttributeID.cudaLaunchAttributeClusterDimension)[1].clusterDim.x
                 for n in kernel_nodes(handle, rt)]
     assert sum(c == 2 for c in clusters) >= 2, clusters
-    test_convolution_with_gathered_patches(L, 256, 256, 3, 1, 53)
+    check_convolution(L, 256, 256, 3, 1, 53, 9)
 
 
 def _block_params(blk, prefix):

@@ -36,7 +36,7 @@ struct TcParams {
   float* dq_acc;                // [B, H, S, 64] fp32 sums of dQ (fused backward), or null
   long long stride_o, stride_dqkv;
   int B, H, S;
-  int hidden;                   // H * 64: column offset between q, k and v in the packed projection
+  int hidden;                   // H * D: column offset between q, k and v in the packed projection
   int causal;
   float scale;
   int* status;
@@ -122,7 +122,7 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const float* v, 
   }
 }
 
-// shared-memory bookkeeping common to the three kernels
+// shared-memory bookkeeping common to the tcgen05 kernels
 struct Ctl {
   uint64_t bars[32];
   uint32_t tmem_slot;
@@ -984,14 +984,15 @@ attn_tc_dq_convert_kernel(const TcParams p) {
 // fp32 / bf16 range; the final division by the row sum makes the choice of reference immaterial.
 // smem: Q_0, Q_1 [128 x D] | K, V sub-tiles [64 x D] x NKV stages | P_g,b [128 x 64] x 4
 // TMEM: S_g,b at 128 g + 64 b | O_g at 256 + 128 g (D columns)
-// (The template also fits D = 64, where the kernel after this one is faster.)  A [rows x 128] operand lies in shared memory as two [rows x 64] atoms of
+// A [rows x 128] operand lies in shared memory as two [rows x 64] atoms of
 // 128-byte rows, one after the other (two TMA boxes): the score product walks its eight 16-column k-steps
 // through both atoms; V as the B operand of P V (N = D, its columns) names the distance between the atoms in
-// the descriptor's leading-dimension field.  The whole tensor memory is in use at D = 128 (2 x 2 score
-// buffers of 64 columns, 2 outputs of 128), and the sub-tile ring is 3 deep instead of 6.
-template <int D> struct Fwd2 {
+// the descriptor's leading-dimension field.  The whole tensor memory is in use (2 x 2 score
+// buffers of 64 columns, 2 outputs of 128).
+struct Fwd2 {
+  static constexpr int D = 128;
   static constexpr int NA = D / 64;                            // 64-column atoms per row
-  static constexpr int NKV = (D == 64) ? 6 : 3;                // sub-tile ring depth
+  static constexpr int NKV = 3;                                // sub-tile ring depth
   static constexpr int Q_BYTES = NA * TILE_BYTES;              // one query tile
   static constexpr int KV_BYTES = NA * SUB_BYTES;              // one key (or value) sub-tile
   static constexpr int SMEM = 2 * Q_BYTES + 2 * NKV * KV_BYTES + 4 * TILE_BYTES + (int)sizeof(Ctl) + 1024;
@@ -1013,11 +1014,10 @@ __device__ __forceinline__ void atom_store_row64(uint8_t* atom, int row, const f
   }
 }
 
-template <int D>
 __global__ void __launch_bounds__(FWD2_THREADS, 1)
 attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv, const TcParams p) {
-  using C = Fwd2<D>;
-  constexpr int NA = C::NA, NKV = C::NKV, Q_BYTES = C::Q_BYTES, KV_BYTES = C::KV_BYTES;
+  using C = Fwd2;
+  constexpr int D = C::D, NA = C::NA, NKV = C::NKV, Q_BYTES = C::Q_BYTES, KV_BYTES = C::KV_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                          // 2 tiles
@@ -1475,11 +1475,11 @@ template <typename K> int set_smem(K kernel, int bytes) {
 
 }  // namespace
 
-// Entry points used by attention.cu's dispatch: forward for head dimensions 64 and 128, backward for 64.
-namespace {
-template <int D>
-int launch_fwd2(const void* qkv_q, void* out, float* lse, int B, int H, int S, long long stride_qkv, long long stride_o,
-                int causal, float scale, cudaStream_t stream) {
+// Entry points used by attention.cu's dispatch, head dimensions 64 and 128.
+int bb_attention_tc_fwd(const void* qkv_q, void* out, float* lse, int B, int H, int S, int D, long long stride_qkv,
+                        long long stride_o, int causal, float scale, cudaStream_t stream) {
+  if (D != 64 && D != 128) return BB_ERR_UNSUPPORTED;
+  if (int rc = bbhost::bind_context()) return rc;
   CUtensorMap tm_q, tm_kv;
   // the packed projection [B, S, 3*H*D]: q, k, v blocks of H*D columns each; boxes of 64 columns (one
   // 128-byte swizzle atom), 128 rows for the query tiles, 64 rows for the streamed key/value sub-tiles.  A tile past a
@@ -1491,24 +1491,15 @@ int launch_fwd2(const void* qkv_q, void* out, float* lse, int B, int H, int S, l
   p.causal = causal; p.scale = scale; p.status = bb_device_status_word();
   // Three CTAs per SM at 64; at 128 a CTA's scores and output take more than a third of tensor memory (S 64 + O 128
   // columns, allocated in powers of two), and the two-tile kernel keeps the softmax groups on the SM instead.
-  if constexpr (D == 64) {
+  if (D == 64) {
     BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_fwd3_kernel, FWD3_SMEM)) return rc; });
     bb_launch(attn_tc_fwd3_kernel, (S + TQ - 1) / TQ * H * B, FWD3_THREADS, FWD3_SMEM, stream, tm_q, tm_kv, p);
   } else {
-    BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_fwd2_kernel<D>, Fwd2<D>::SMEM)) return rc; });
-    bb_launch(attn_tc_fwd2_kernel<D>, (S + 2 * TQ - 1) / (2 * TQ) * H * B, FWD2_THREADS, Fwd2<D>::SMEM, stream, tm_q, tm_kv, p);
+    BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_fwd2_kernel, Fwd2::SMEM)) return rc; });
+    bb_launch(attn_tc_fwd2_kernel, (S + 2 * TQ - 1) / (2 * TQ) * H * B, FWD2_THREADS, Fwd2::SMEM, stream, tm_q, tm_kv, p);
   }
   BB_CUDA_CHECK(cudaGetLastError());
   return BB_OK;
-}
-}  // namespace
-
-int bb_attention_tc_fwd(const void* qkv_q, void* out, float* lse, int B, int H, int S, int D, long long stride_qkv,
-                        long long stride_o, int causal, float scale, cudaStream_t stream) {
-  if (int rc = bbhost::bind_context()) return rc;
-  if (D == 64) return launch_fwd2<64>(qkv_q, out, lse, B, H, S, stride_qkv, stride_o, causal, scale, stream);
-  if (D == 128) return launch_fwd2<128>(qkv_q, out, lse, B, H, S, stride_qkv, stride_o, causal, scale, stream);
-  return BB_ERR_UNSUPPORTED;
 }
 
 namespace {

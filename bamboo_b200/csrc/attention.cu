@@ -479,8 +479,8 @@ int bb_attention_tc_bwd_launches(int D);
 namespace {
 // The tcgen05 kernels (attention_tc.cu) read q, k, v through one tensor map over the packed
 // projection [tokens, 3*H*D] and are the default at both head dimensions.  Measured on B200
-// (B8 H16 S1024 D64 causal): forward 70 us, backward 180 us, against 120 us and 593 us for the
-// warp-level kernels above; B2 H32 S2048 D128 causal: forward 121 us, backward 552 us against
+// (B8 H16 S1024 D64 causal, L2 flushed between calls): forward 51 us, backward 171 us, against 120 us and
+// 593 us for the warp-level kernels above; B2 H32 S2048 D128 causal: forward 111 us, backward 503 us against
 // 1474 us.  The warp-level kernels remain for q, k, v that are not slices of one packed
 // projection; BB_ATTENTION_IMPL=mma in the environment forces them.
 bool use_tc_path(const void* q, const void* k, const void* v, int H, int D, long long stride_qkv) {

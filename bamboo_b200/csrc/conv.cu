@@ -281,8 +281,8 @@ bn_reduce_kernel(const uint4* a, const uint4* zz, const uint4* yy,
 
 // Column sums over the partial rows: a block owns 32 channels and splits the rows over its 32 warps
 // (coalesced 128-byte reads, four rows in flight per warp), then adds the warps' sums in warp order, so
-// the result does not depend on scheduling.  A thread per channel walking all (up to 592) partial rows is
-// a chain of that many L2 latencies: 26-28 us per call at 592 rows, against about 3 us this way.
+// the result does not depend on scheduling.  A thread per channel walking all partial rows (up to BN_CTAS per SM) is
+// a chain of that many L2 latencies: 26-28 us per call at 592 rows (four blocks per SM), against about 3 us this way.
 // Valid in warp 0 only: t1, t2 of channel blockIdx.x * 32 + lane.
 __device__ __forceinline__ void bn_sum_partials(const float* ws, int parts, int C, float& t1, float& t2) {
   __shared__ float sm1[32][33], sm2[32][33];
@@ -714,8 +714,9 @@ extern "C" int bb_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, vo
 // ---------------------------------------------------------------------------------- one call per layer
 // Convolution + batch norm (+ residual, + ReLU) forward and backward with every kernel issued from
 // one foreign call: a ResNet-152 step has ~2500 such layers-times-micro-batches, and a Python host
-// that pays per kernel becomes the bottleneck.  Same kernels and order as calling the entry points
-// above one by one.
+// that pays per kernel becomes the bottleneck.  Where patches are stored: the same kernels in the same order as the entry
+// points above called one by one.  Gathered products have no entry point of their own; an input gradient is then summed over
+// all taps in fp32 and rounded once, not once per tap.
 namespace {
 
 inline long long up256(long long n) { return (n + 255) & ~255LL; }

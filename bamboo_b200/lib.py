@@ -4,6 +4,7 @@ There is no Python or CPU fallback behind these calls: if the shared library is 
 or a call fails, an exception is raised.
 """
 import ctypes
+import functools
 import os
 import threading
 
@@ -313,10 +314,15 @@ def attention_fwd(qkv, out, lse, B, H, S, D, causal, scale=None):
     return out
 
 
+@functools.lru_cache(maxsize=None)
+def _attention_bwd_launches(H, D):
+    return load().bb_attention_bwd_launches(_I(H), _I(D))
+
+
 def attention_bwd(qkv, out, dout, lse, dqkv, B, H, S, D, causal, scale=None):
     global LAUNCHES
     lib = load()
-    LAUNCHES += lib.bb_attention_bwd_launches(_I(H), _I(D))
+    LAUNCHES += _attention_bwd_launches(H, D)
     hd = H * D
     esz = qkv.element_size()
     base, dbase = qkv.data_ptr(), dqkv.data_ptr()
@@ -392,7 +398,7 @@ def block_half_bwd(desc, half, x, saved, dout, dx, scratch, side_stream=None):
     lib = _lib or load()
     LAUNCHES += HALF_BWD_LAUNCHES[half]
     if half == HALF_ATTENTION:
-        LAUNCHES += lib.bb_attention_bwd_launches(desc.heads, desc.head_dim)
+        LAUNCHES += _attention_bwd_launches(desc.heads, desc.head_dim)
     main = _raw_stream()
     rc = lib.bb_block_half_bwd(ctypes.byref(desc), half, x.data_ptr(), saved.data_ptr(), dout.data_ptr(), dx.data_ptr(),
                                scratch.data_ptr(), scratch.numel(), main, main if side_stream is None else side_stream)

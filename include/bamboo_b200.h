@@ -243,10 +243,12 @@ int bb_bn_apply(const void* y, const float* mean, const float* rstd, const void*
 int bb_bn_bwd(const void* dz, const void* z, const void* y, const float* mean, const float* rstd, const void* gamma,
               void* dy, void* dres, float* dgamma, float* dbeta, long long rows, int C, int relu, void* workspace,
               long long workspace_bytes, void* stream);
-/* One call per layer: convolution + batch norm (+ residual, + ReLU), forward and backward.  Same
- * results as the kernels above in order (patch gather, GEMM, statistics, normalise / batch-norm
- * backward, weight gradient, input gradient); with channels in blocks of 64 the GEMMs gather the
- * patches themselves and no patch matrix exists.  Consecutive kernels of one call overlap at their ends.  y is the
+/* One call per layer: convolution + batch norm (+ residual, + ReLU), forward and backward: patch
+ * gather, GEMM, statistics, normalise / batch-norm backward, weight gradient, input gradient, as the
+ * kernels above in order.  With channels in blocks of 64 the GEMMs gather the patches themselves
+ * (an input gradient only where that is expected to be quicker: it is then summed over all taps in
+ * fp32 and rounded once, where the stored patch gradient rounds every tap) and no patch matrix
+ * exists.  Consecutive kernels of one call overlap at their ends.  y is the
  * convolution output kept for the backward pass, z the layer output; dx / dres may be NULL.
  * `scratch`: bb_conv_bn_scratch_bytes(desc, backward, need_dx).  Replaces one Conv2d + BatchNorm2d
  * (+ add + ReLU) of a bottleneck block and their share of loss.backward(). */

@@ -243,7 +243,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   uint64_t* ds_empty = ds_full + 2;            // [2]
   uint64_t* acc_full = ds_empty + 2;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const int qb = nbx - 1 - id.tile, head = id.head, batch = id.batch;
   const int q0 = qb * TQ;
   const int row_base = batch * p.S;
@@ -277,9 +277,12 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
         bb::tma_load_3d(sQ + a * TILE_BYTES, &tm_q, q_full, colq + 64 * a, q0, batch);
         bb::tma_load_3d(sDO + a * TILE_BYTES, &tm_do, q_full, colq + 64 * a, q0, batch);
       }
-      for (int j = 0; j < nblk; ++j) {
-        const int s = j % NST;
-        if (!bb::mbar_wait(&kv_empty[s], ((j / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+    }
+    __syncwarp();
+    for (int j = 0; j < nblk; ++j) {
+      const int s = j % NST;
+      if (!bb::mbar_wait_warp(&kv_empty[s], ((j / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      if (bb::elect_one()) {
         bb::mbar_arrive_expect_tx(&kv_full[s], 2 * G::STREAM_BYTES);
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -287,6 +290,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
           bb::tma_load_3d(sV + s * G::STREAM_BYTES + a * SUB_BYTES, &tm_kv, &kv_full[s], colv + 64 * a, j * SUB, batch);
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));
@@ -429,7 +433,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   uint64_t* p_empty = p_full + 2;              // [2]
   uint64_t* acc_full = p_empty + 2;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const int kb = id.tile, head = id.head, batch = id.batch;
   const int k0 = kb * TQ;
   const int row_base = batch * p.S;
@@ -464,9 +468,12 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         bb::tma_load_3d(sK + a * TILE_BYTES, &tm128, kv_full, colk + 64 * a, k0, batch);
         bb::tma_load_3d(sV + a * TILE_BYTES, &tm128, kv_full, colv + 64 * a, k0, batch);
       }
-      for (int i = 0; i < nblk; ++i) {
-        const int s = i % NST;
-        if (!bb::mbar_wait(&q_empty[s], ((i / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+    }
+    __syncwarp();
+    for (int i = 0; i < nblk; ++i) {
+      const int s = i % NST;
+      if (!bb::mbar_wait_warp(&q_empty[s], ((i / NST) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      if (bb::elect_one()) {
         bb::mbar_arrive_expect_tx(&q_full[s], 2 * G::STREAM_BYTES);
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -474,6 +481,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
           bb::tma_load_3d(sDO + s * G::STREAM_BYTES + a * SUB_BYTES, &tm_do64, &q_full[s], colq + 64 * a, (qstart + i) * SUB, batch);
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));
@@ -686,7 +694,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
   uint64_t* acc_full = dq_empty + 2;
   uint64_t* st_full = acc_full + 1;            // [NSTAT] statistics of a sub-block's queries
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const TileId id = tile_id(p);
   const int kb = id.tile, head = id.head, batch = id.batch;
   const int k0 = kb * TQ;
@@ -728,13 +736,17 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       bb::mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
       bb::tma_load_3d(sK, &tm128, kv_full, colk, k0, batch);
       bb::tma_load_3d(sV, &tm128, kv_full, colv, k0, batch);
-      for (int i = 0; i < nblk; ++i) {
-        const int s = i % NST3;
-        if (!bb::mbar_wait(&q_empty[s], ((i / NST3) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+    }
+    __syncwarp();
+    for (int i = 0; i < nblk; ++i) {
+      const int s = i % NST3;
+      if (!bb::mbar_wait_warp(&q_empty[s], ((i / NST3) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      if (bb::elect_one()) {
         bb::mbar_arrive_expect_tx(&q_full[s], 2 * SUB_BYTES);
         bb::tma_load_3d(sQ + s * SUB_BYTES, &tm64, &q_full[s], colq, (qstart + i) * SUB, batch);
         bb::tma_load_3d(sDO + s * SUB_BYTES, &tm_do64, &q_full[s], colq, (qstart + i) * SUB, batch);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // score products: one thread issues S^T = K . Q^T and dP^T = V . dO^T for every sub-block, as soon as its
@@ -1036,7 +1048,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // the waiter can never find it two phases on (p_full can be: the other issuing warp moves that one along)
   uint64_t* s_free = pv_full + 2;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const TileId id = tile_id(p);
   const int cb = (p.S + 2 * TQ - 1) / (2 * TQ) - 1 - id.tile, head = id.head, batch = id.batch;   // long CTAs first
   const int row_base = batch * p.S;
@@ -1073,9 +1085,12 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         bb::tma_load_3d(sQ + a * TILE_BYTES, &tm_q, q_full, colq + 64 * a, qa, batch);
         bb::tma_load_3d(sQ + Q_BYTES + a * TILE_BYTES, &tm_q, q_full, colq + 64 * a, qb, batch);
       }
-      for (int jj = 0; jj <= jmax; ++jj) {
-        const int s = jj % NKV;
-        if (!bb::mbar_wait(&kv_empty[s], ((jj / NKV) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+    }
+    __syncwarp();
+    for (int jj = 0; jj <= jmax; ++jj) {
+      const int s = jj % NKV;
+      if (!bb::mbar_wait_warp(&kv_empty[s], ((jj / NKV) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      if (bb::elect_one()) {
         bb::mbar_arrive_expect_tx(&kv_full[s], 2 * KV_BYTES);
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -1083,6 +1098,7 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           bb::tma_load_3d(sV + s * KV_BYTES + a * SUB_BYTES, &tm_kv, &kv_full[s], colv + 64 * a, jj * SUB, batch);
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ));
@@ -1289,7 +1305,7 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* p_full = s_free + 1;               // probabilities in shared memory
   uint64_t* pv_full = p_full + 1;              // P V product retired
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const TileId id = tile_id(p);
   const int q0 = ((p.S + TQ - 1) / TQ - 1 - id.tile) * TQ;       // long CTAs first
   const int row_base = id.batch * p.S;

@@ -124,6 +124,11 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// This thread's warp, as a value that the compiler knows to be the same for the whole warp: branches on it are then uniform,
+// and inside them loop counters and addresses stay in uniform registers, which TMA and tcgen05 instructions take their
+// operands from.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Called by every thread before its first access to global memory (see bb_launch).  A kernel that calls it may be
 // resident while its predecessor still writes, so what a kernel may have written is not constant for its successor's
 // lifetime and must not be read through the read-only path: no __ldg and no `const T* __restrict__` (which lets the

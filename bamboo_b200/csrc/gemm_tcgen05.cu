@@ -1,12 +1,12 @@
 // bf16 GEMM on the 5th-generation tensor cores: D[M,N] = op(A)[M,K] * op(B)[N,K]^T with a
-// fused epilogue.  One persistent CTA per SM; warp 0 feeds shared memory with TMA
+// fused epilogue.  One persistent CTA per SM; warps 0 and 2 feed shared memory with TMA
 // (128-byte swizzle, no cluster multicast), warp 1 issues tcgen05.mma into two TMEM
-// accumulators, warps 2-9 drain TMEM (tcgen05.ld) and run the epilogue (coalesced global
+// accumulators, warps 3-10 drain TMEM (tcgen05.ld) and run the epilogue (coalesced global
 // stores from warp-private staging slabs) while the next tile's main loop is already running.
 //
 // Work units are handed out dynamically: the first unit of a CTA is its own index, every further
 // one comes from a per-launch ticket counter in global memory (one atomicAdd per unit, issued a
-// whole unit ahead of its use), and the producer thread passes it to the MMA and epilogue warps
+// whole unit ahead of its use), and the first producer passes it to the other warps
 // (and to the second CTA of a pair) through a four-entry ring in shared memory.  A CTA that
 // starts late - because a kernel of another stream still held its SM - therefore takes fewer
 // units instead of stretching the launch by its fixed share.
@@ -36,8 +36,11 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 64;        // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-// threads: TMA warp, MMA warp and EW epilogue warps per TMEM lane quarter (EW = 2: 320, EW = 4: 576)
-constexpr int num_threads(int ew) { return 64 + 128 * ew; }
+// threads: two TMA warps, the MMA warp and EW epilogue warps per TMEM lane quarter (EW = 2: 352, EW = 4: 608).
+// Two TMA warps take the stages in turn: one iteration of a producer (wait for the stage, announce the bytes, two copies) is
+// a chain of about 430 cycles, the MMAs of a k-block of a 128 x 128 tile take 256.
+constexpr int TMA_WARP_0 = 0, MMA_WARP = 1, TMA_WARP_1 = 2, EPI_WARP = 3;
+constexpr int num_threads(int ew) { return 32 * EPI_WARP + 128 * ew; }
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 // Epilogue staging: one 4 KiB slab (32 rows x 128 bytes = 64 bf16 or 32 fp32 columns) per
 // epilogue warp; shared memory is better spent on main-loop stages.
@@ -64,6 +67,8 @@ struct GemmParams {
   int dynamic;                // 1: work units after a CTA's first come from the ticket counter
   unsigned int* ticket;       // this launch's ticket counter (global memory)
   unsigned int ticket_base;   // its value before this launch's first ticket
+  unsigned tiles_in, tiles_mn;                     // output tiles along the fast dimension, and in all
+  unsigned long long magic_in, magic_mn;           // ... as divisors
   void* D; void* D2; const void* bias; const void* aux;
   long long ldd, ld_aux;
   int* status;
@@ -111,6 +116,11 @@ __device__ __forceinline__ void panel_store_row_f32(uint8_t* panel, int row, con
 // complete 128-byte row segments.
 __device__ __forceinline__ uint32_t slab_off(int row, int chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); }
 
+// Whether the 32 rows from r0 and `width` columns from nb all lie inside the matrix (the same for a whole warp): then the
+// addresses are one base and a constant step and the accesses go out back to back.  With a test per row and chunk the
+// eight stores of a panel took 950 cycles, the longest part of its epilogue.
+__device__ __forceinline__ bool inside(int r0, int nb, int width, int M, int N) { return r0 + 32 <= M && nb + width <= N; }
+
 __device__ __forceinline__ void slab_put(uint8_t* slab, int lane, const uint4* ax) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(slab + slab_off(4 * i + (lane >> 3), lane & 7)) = ax[i];
@@ -118,6 +128,12 @@ __device__ __forceinline__ void slab_put(uint8_t* slab, int lane, const uint4* a
 // rows r0.., columns nb.. of a bf16 matrix -> ax (zero outside the matrix)
 __device__ __forceinline__ void slab_fetch_bf16(const __nv_bfloat16* src, long long ld, int r0, int nb, int M, int N, int lane, uint4* ax) {
   const int c = nb + (lane & 7) * 8;
+  if (inside(r0, nb, 64, M, N)) {
+    const __nv_bfloat16* g = src + (long long)(r0 + (lane >> 3)) * ld + c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, g += 4 * ld) ax[i] = __ldca(reinterpret_cast<const uint4*>(g));
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = r0 + 4 * i + (lane >> 3);
@@ -139,6 +155,15 @@ __device__ __forceinline__ void slab_fetch_bf16(const __nv_bfloat16* src, long l
 }
 __device__ __forceinline__ void slab_flush_bf16(const uint8_t* slab, __nv_bfloat16* dst, long long ld, int r0, int nb, int M, int N, int lane) {
   const int c = nb + (lane & 7) * 8;
+  if (inside(r0, nb, 64, M, N)) {
+    __nv_bfloat16* g = dst + (long long)(r0 + (lane >> 3)) * ld + c;
+    uint4 q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const uint4*>(slab + slab_off(4 * i + (lane >> 3), lane & 7));
+#pragma unroll
+    for (int i = 0; i < 8; ++i, g += 4 * ld) *reinterpret_cast<uint4*>(g) = q[i];
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int rl = 4 * i + (lane >> 3);
@@ -159,6 +184,18 @@ __device__ __forceinline__ void slab_flush_bf16(const uint8_t* slab, __nv_bfloat
 template <bool ACCUM>
 __device__ __forceinline__ void slab_flush_f32(const uint8_t* slab, float* dst, long long ld, int r0, int nb, int M, int N, int lane) {
   const int c = nb + (lane & 7) * 4;
+  if (inside(r0, nb, 32, M, N)) {
+    float* g = dst + (long long)(r0 + (lane >> 3)) * ld + c;
+    float4 q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const float4*>(slab + slab_off(4 * i + (lane >> 3), lane & 7));
+#pragma unroll
+    for (int i = 0; i < 8; ++i, g += 4 * ld) {
+      if (ACCUM) asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(q[i].x), "f"(q[i].y), "f"(q[i].z), "f"(q[i].w) : "memory");
+      else *reinterpret_cast<float4*>(g) = q[i];
+    }
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int rl = 4 * i + (lane >> 3);
@@ -199,6 +236,14 @@ __device__ __forceinline__ void slab64_store_row(uint8_t* slab, int row, const f
 __device__ __forceinline__ void slab64_fetch(uint8_t* slab, const __nv_bfloat16* src, long long ld, int r0, int nb, int M, int N, int lane) {
   const int c = nb + (lane & 3) * 8;
   uint4 q[4];
+  if (inside(r0, nb, 32, M, N)) {
+    const __nv_bfloat16* g = src + (long long)(r0 + (lane >> 2)) * ld + c;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, g += 8 * ld) q[i] = __ldca(reinterpret_cast<const uint4*>(g));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(slab + slab64_off(8 * i + (lane >> 2), lane & 3)) = q[i];
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = r0 + 8 * i + (lane >> 2);
@@ -221,6 +266,15 @@ __device__ __forceinline__ void slab64_fetch(uint8_t* slab, const __nv_bfloat16*
 }
 __device__ __forceinline__ void slab64_flush(const uint8_t* slab, __nv_bfloat16* dst, long long ld, int r0, int nb, int M, int N, int lane) {
   const int c = nb + (lane & 3) * 8;
+  if (inside(r0, nb, 32, M, N)) {
+    __nv_bfloat16* g = dst + (long long)(r0 + (lane >> 2)) * ld + c;
+    uint4 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint4*>(slab + slab64_off(8 * i + (lane >> 2), lane & 3));
+#pragma unroll
+    for (int i = 0; i < 4; ++i, g += 8 * ld) *reinterpret_cast<uint4*>(g) = q[i];
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int rl = 8 * i + (lane >> 2);
@@ -257,6 +311,183 @@ __device__ __forceinline__ void add_bias(const GemmParams& p, int n0, float* v) 
   }
 }
 
+// (m tile, n tile, split) of a work unit
+__device__ __forceinline__ void unit_coords(const GemmParams& p, int unit, int& mi, int& ni, int& ks) {
+  const unsigned split = bb::fast_div((unsigned)unit, p.magic_mn), mn = (unsigned)unit - split * p.tiles_mn;
+  const unsigned slow = bb::fast_div(mn, p.magic_in), fast = mn - slow * p.tiles_in;
+  mi = (int)(p.n_fast ? slow : fast); ni = (int)(p.n_fast ? fast : slow); ks = (int)split;
+}
+
+// Operand loads of one work unit: k-blocks [kb0, kb1) of the A rows from m0 and the B rows (output columns) from n0 into the
+// stage ring (s, phase), by a whole warp: the waits are warp-wide, one elected lane issues.  `turn`: which of the two producer
+// warps this is; it serves the stages of its parity.  `rank`: which CTA of its pair
+// this is; `lead`: cluster rank of the pair's first CTA, on whose barriers both CTAs' copies complete and where the MMA
+// issuer waits.  False when a wait ran out.
+template <int BN, bool PAIR, bool CONV>
+__device__ __forceinline__ bool load_operands(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
+                                              const typename ConvArg<CONV>::type& cv, uint8_t* sA, uint8_t* sB, uint64_t* full_bar,
+                                              uint64_t* empty_bar, volatile int* abort_flag, uint32_t rank, uint32_t lead, int m0, int n0,
+                                              int kb0, int kb1, int turn, int& s, uint32_t& phase) {
+  using C = Cfg<BN, PAIR>;
+  static_assert(C::STAGES % 2 == 0, "the producers take the stages in turn");
+  if constexpr (CONV) {
+    // Patches of a convolution: a stage's patch tile is 64 channels of one tap for a run of windows, one
+    // im2col load (the hardware walks the windows, applies the stride and fills with zeros outside the
+    // image).  FWD / DGRAD gather A (windows = output rows, k-blocks run over taps x channel blocks),
+    // WGRAD gathers B (windows = the reduction, columns = taps x channels).
+    auto window = [&](unsigned px, int& w, int& h, int& n) {
+      const unsigned row = bb::fast_div(px, cv.magic_w), img = bb::fast_div(row, cv.magic_h);
+      w = (int)(px - row * cv.Wo) * cv.stride - cv.pad;
+      h = (int)(row - img * cv.Ho) * cv.stride - cv.pad;
+      n = (int)img;
+    };
+    auto patches = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int c, int w, int h, int n, int ow, int oh) {
+      if constexpr (PAIR) bb::tma_load_im2col_pair(dst, tm, fb, c, w, h, n, (uint16_t)ow, (uint16_t)oh);
+      else bb::tma_load_im2col(dst, tm, &full_bar[s], c, w, h, n, (uint16_t)ow, (uint16_t)oh);
+    };
+    auto plain = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int x, int y) {
+      if constexpr (PAIR) bb::tma_load_2d_pair(dst, tm, fb, x, y);
+      else bb::tma_load_2d(dst, tm, &full_bar[s], x, y);
+    };
+    constexpr int BJ = C::B_ROWS / 64;
+    int w, h, n;
+    int cj[BJ], rj[BJ], sj[BJ];          // WGRAD: channel and tap of each 64-column block of B
+    if (cv.mode == BB_CONV_WGRAD) {
+#pragma unroll
+      for (int j = 0; j < BJ; ++j) {
+        const int cb = min((n0 >> 6) + j, cv.k * cv.k * cv.cblocks - 1);     // past the last tap: never stored
+        const int tap = cb / cv.cblocks;
+        cj[j] = (cb - tap * cv.cblocks) * 64; rj[j] = tap / cv.k; sj[j] = tap - rj[j] * cv.k;
+      }
+    } else {
+      window((unsigned)m0, w, h, n);
+    }
+    int tap = kb0 / cv.cblocks, cb = kb0 - tap * cv.cblocks;
+    int tr = tap / cv.k, ts = tap - tr * cv.k;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if ((s & 1) == turn) {
+        if (!bb::mbar_wait_warp(&empty_bar[s], phase ^ 1, abort_flag, p.status)) return false;
+        uint8_t* a = sA + s * A_STAGE_BYTES;
+        uint8_t* b = sB + s * C::B_STAGE_BYTES;
+        uint32_t fb = 0;
+        if constexpr (PAIR) fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), lead);
+        if (cv.mode == BB_CONV_WGRAD) window((unsigned)kb * BK, w, h, n);
+        const int col = ((cv.k - 1 - tr) * cv.k + (cv.k - 1 - ts)) * cv.wcols + n0;       // the tap turned by 180 degrees
+        if (bb::elect_one()) {
+          if constexpr (PAIR) {
+            if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+          } else {
+            bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
+          }
+          if (cv.mode == BB_CONV_WGRAD) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) plain(a + j * 8192, &tmA, fb, m0 + 64 * j, kb * BK);
+#pragma unroll
+            for (int j = 0; j < BJ; ++j) patches(b + j * 8192, &tmB, fb, cj[j], w, h, n, sj[j], rj[j]);
+          } else {
+            patches(a, &tmA, fb, cb * 64, w, h, n, ts, tr);
+            if (cv.mode == BB_CONV_FWD) {
+              plain(b, &tmB, fb, kb * BK, n0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BJ; ++j) plain(b + j * 8192, &tmB, fb, col + 64 * j, cb * 64);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (cv.mode != BB_CONV_WGRAD && ++cb == cv.cblocks) { cb = 0; if (++ts == cv.k) { ts = 0; ++tr; } }
+      if (++s == C::STAGES) { s = 0; phase ^= 1; }
+    }
+  } else {
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if ((s & 1) == turn) {
+        if (!bb::mbar_wait_warp(&empty_bar[s], phase ^ 1, abort_flag, p.status)) return false;
+        uint8_t* a = sA + s * A_STAGE_BYTES;
+        uint8_t* b = sB + s * C::B_STAGE_BYTES;
+        const int k0 = kb * BK;
+        if (bb::elect_one()) {
+          if constexpr (PAIR) {
+            // both CTAs' copies complete on rank 0's barrier, where the MMA issuer waits
+            if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+            const uint32_t fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), lead);
+            if (!p.a_mn) {
+              bb::tma_load_2d_pair(a, &tmA, fb, k0, m0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d_pair(a + j * 8192, &tmA, fb, m0 + 64 * j, k0);
+            }
+            if (!p.b_mn) {
+              bb::tma_load_2d_pair(b, &tmB, fb, k0, n0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < C::B_ROWS / 64; ++j) bb::tma_load_2d_pair(b + j * 8192, &tmB, fb, n0 + 64 * j, k0);
+            }
+          } else {
+            bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
+            if (!p.a_mn) {
+              bb::tma_load_2d(a, &tmA, &full_bar[s], k0, m0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d(a + j * 8192, &tmA, &full_bar[s], m0 + 64 * j, k0);
+            }
+            if (!p.b_mn) {
+              bb::tma_load_2d(b, &tmB, &full_bar[s], k0, n0);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BN / 64; ++j) bb::tma_load_2d(b + j * 8192, &tmB, &full_bar[s], n0 + 64 * j, k0);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (++s == C::STAGES) { s = 0; phase ^= 1; }
+    }
+  }
+  return true;
+}
+
+// The MMAs of one work unit's k-blocks into the accumulator at d_tmem, issued by one warp; the last commit signals acc_full.
+// `ctas`: cluster ranks of the pair as a mask.  False when a wait ran out.
+template <int BN, bool PAIR>
+__device__ __forceinline__ bool issue_mmas(const GemmParams& p, uint8_t* sA, uint8_t* sB, uint64_t* full_bar, uint64_t* empty_bar,
+                                           uint64_t* acc_full, volatile int* abort_flag, uint16_t ctas, uint32_t d_tmem, int num_kb, int& s,
+                                           uint32_t& phase) {
+  using C = Cfg<BN, PAIR>;
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
+                         ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(C::TILE_M >> 4) << 24);
+  // K-major: 8-row groups 1024 B apart (LBO unused); MN-major: 64-wide column groups are
+  // separate 8 KiB TMA boxes (LBO), 8 k-rows are 1024 B (SBO).
+  const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+  const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+  for (int kb = 0; kb < num_kb; ++kb) {
+    if (!bb::mbar_wait_warp(&full_bar[s], phase, abort_flag, p.status)) return false;
+    bb::tc_fence_after_sync();
+    if (bb::elect_one()) {
+      // one descriptor per stage; a k-step only adds to its address field (16-byte units)
+      const uint64_t ad0 = bb::make_smem_desc_sw128(bb::smem_u32(sA + s * A_STAGE_BYTES), a_lbo, 1024u);
+      const uint64_t bd0 = bb::make_smem_desc_sw128(bb::smem_u32(sB + s * C::B_STAGE_BYTES), b_lbo, 1024u);
+#pragma unroll
+      for (int k = 0; k < BK / UMMA_K; ++k) {
+        const uint64_t ad = ad0 + (uint64_t)(k * (a_kstep >> 4));
+        const uint64_t bd = bd0 + (uint64_t)(k * (b_kstep >> 4));
+        if (PAIR) bb::umma_f16_pair(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        else bb::umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+      }
+      if (PAIR) {
+        bb::umma_commit_pair(&empty_bar[s], ctas);           // frees the stage in both CTAs
+        if (kb == num_kb - 1) bb::umma_commit_pair(acc_full, ctas);
+      } else {
+        bb::umma_commit(&empty_bar[s]);
+        if (kb == num_kb - 1) bb::umma_commit(acc_full);
+      }
+    }
+    __syncwarp();
+    if (++s == C::STAGES) { s = 0; phase ^= 1; }
+  }
+  return true;
+}
+
 template <int BN, bool PAIR, int EW, bool CONV>
 __global__ void __launch_bounds__(num_threads(EW), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -279,16 +510,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* sched_tile = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [SCHED_RING]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = bb::warp_index();
   const int lane = threadIdx.x & 31;
   // work units go to CTAs (pairs: to clusters; both CTAs of a pair walk the same units)
   const uint32_t rank = PAIR ? bb::cluster_ctarank() : 0u;
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int num_workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int num_m = (p.M + C::TILE_M - 1) / C::TILE_M;
-  const int num_n = (p.N + BN - 1) / BN;
-  const int num_mn = num_m * num_n;
-  const int num_tiles = num_mn * p.ksplit;        // work units: (m, n, k-split)
+  const int num_tiles = (int)p.tiles_mn * p.ksplit;   // work units: (m, n, k-split)
   const int total_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -296,14 +524,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     for (int s = 0; s < C::STAGES; ++s) { bb::mbar_init(&full_bar[s], 1); bb::mbar_init(&empty_bar[s], 1); }
     // accumulator hand-back: one arrival per epilogue warp (of both CTAs for a pair, on rank 0's barrier)
     for (int a = 0; a < 2; ++a) { bb::mbar_init(&tmem_full[a], 1); bb::mbar_init(&tmem_empty[a], (PAIR ? 2 : 1) * 4 * EW); }
-    // work-unit ring: one announcement per entry; read by the MMA warp and the epilogue warps of
-    // this CTA and, for a pair, by the producer and the epilogue warps of the second CTA
-    for (int r = 0; r < SCHED_RING; ++r) { bb::mbar_init(&sched_full[r], 1); bb::mbar_init(&sched_empty[r], (PAIR ? 2 : 1) * (1 + 4 * EW)); }
+    // work-unit ring: one announcement per entry; read by the second producer, the MMA warp and the epilogue warps of
+    // this CTA and, for a pair, by both producers and the epilogue warps of the second CTA
+    for (int r = 0; r < SCHED_RING; ++r) { bb::mbar_init(&sched_full[r], 1); bb::mbar_init(&sched_empty[r], (PAIR ? 2 : 1) * (2 + 4 * EW)); }
     bb::fence_barrier_init();
     bb::tma_prefetch_desc(&tmA);
     bb::tma_prefetch_desc(&tmB);
   }
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     if (PAIR) { bb::tmem_alloc_pair(tmem_slot, C::TMEM_COLS); bb::tmem_relinquish_pair(); }
     else { bb::tmem_alloc(tmem_slot, C::TMEM_COLS); bb::tmem_relinquish(); }
   }
@@ -314,177 +542,80 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   bb::pdl_sync();
 
-  // Next work unit of this CTA as announced by the scheduling thread (-1: no more).  Called by a
-  // whole warp (`warp_wide`) or by a single thread; the entry is handed back once it has been read.
-  auto next_unit = [&](uint32_t it, int& tile, bool warp_wide) -> bool {
+  // Work unit number `it` of this CTA: the first is its own index, the others as announced by the scheduling warp (-1: no
+  // more).  Called by a whole warp; the entry is handed back once it has been read.
+  auto next_unit = [&](uint32_t it, int& tile) -> bool {
+    if (it == 0) { tile = worker; return true; }
+    --it;
     const int r = (int)(it & (SCHED_RING - 1));
     const uint32_t ph = (it / SCHED_RING) & 1u;
     const bool got = PAIR ? bb::mbar_wait_cluster(&sched_full[r], ph, abort_flag, p.status)
                           : bb::mbar_wait(&sched_full[r], ph, abort_flag, p.status);
-    if (warp_wide) { if (!__all_sync(0xffffffffu, got)) return false; }
-    else if (!got) return false;
-    tile = sched_tile[r];
-    if (warp_wide) __syncwarp();
-    if (!warp_wide || lane == 0) {
+    if (!__all_sync(0xffffffffu, got)) return false;
+    tile = __shfl_sync(0xffffffffu, sched_tile[r], 0);
+    if (lane == 0) {
       if (PAIR) bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&sched_empty[r]), 0));
       else bb::mbar_arrive(&sched_empty[r]);
     }
     return true;
   };
 
-  if (warp == 0) {
-    // ------------------------------------------------ TMA producer
-    if (bb::elect_one()) {
+  if (warp == TMA_WARP_0 || warp == TMA_WARP_1) {
+    // ------------------------------------------------ TMA producers
+    // The whole warp walks the units and waits, one elected lane issues: the compiler then knows that loop counters, barrier
+    // addresses and coordinates are the same for the warp, which is what TMA instructions take (see bb::warp_index).
+    {
+      const int turn = warp == TMA_WARP_1 ? 1 : 0;
       int s = 0; uint32_t phase = 0;
       bool alive = true;
       // operand loads of one work unit
       auto load_unit = [&](int tile) {
-        const int mn = tile % num_mn, ks = tile / num_mn;
-        const int mi = p.n_fast ? mn / num_n : mn % num_m, ni = p.n_fast ? mn % num_n : mn / num_m;
-        const int m0 = mi * C::TILE_M + (int)rank * BM;                    // this CTA's A rows
-        const int n0 = ni * BN + (int)rank * C::B_ROWS;                    // this CTA's share of B (pairs: half)
+        int mi, ni, ks;
+        unit_coords(p, tile, mi, ni, ks);
         const int kb0 = ks * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
-        if constexpr (CONV) {
-          // Patches of a convolution: a stage's patch tile is 64 channels of one tap for a run of windows, one
-          // im2col load (the hardware walks the windows, applies the stride and fills with zeros outside the
-          // image).  FWD / DGRAD gather A (windows = output rows, k-blocks run over taps x channel blocks),
-          // WGRAD gathers B (windows = the reduction, columns = taps x channels).
-          auto window = [&](unsigned px, int& w, int& h, int& n) {
-            const unsigned row = bb::fast_div(px, cv.magic_w), img = bb::fast_div(row, cv.magic_h);
-            w = (int)(px - row * cv.Wo) * cv.stride - cv.pad;
-            h = (int)(row - img * cv.Ho) * cv.stride - cv.pad;
-            n = (int)img;
-          };
-          auto patches = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int c, int w, int h, int n, int ow, int oh) {
-            if constexpr (PAIR) bb::tma_load_im2col_pair(dst, tm, fb, c, w, h, n, (uint16_t)ow, (uint16_t)oh);
-            else bb::tma_load_im2col(dst, tm, &full_bar[s], c, w, h, n, (uint16_t)ow, (uint16_t)oh);
-          };
-          auto plain = [&](uint8_t* dst, const CUtensorMap* tm, uint32_t fb, int x, int y) {
-            if constexpr (PAIR) bb::tma_load_2d_pair(dst, tm, fb, x, y);
-            else bb::tma_load_2d(dst, tm, &full_bar[s], x, y);
-          };
-          constexpr int BJ = C::B_ROWS / 64;
-          int w, h, n;
-          int cj[BJ], rj[BJ], sj[BJ];          // WGRAD: channel and tap of each 64-column block of B
-          if (cv.mode == BB_CONV_WGRAD) {
-#pragma unroll
-            for (int j = 0; j < BJ; ++j) {
-              const int cb = min((n0 >> 6) + j, cv.k * cv.k * cv.cblocks - 1);     // past the last tap: never stored
-              const int tap = cb / cv.cblocks;
-              cj[j] = (cb - tap * cv.cblocks) * 64; rj[j] = tap / cv.k; sj[j] = tap - rj[j] * cv.k;
-            }
-          } else {
-            window((unsigned)m0, w, h, n);
-          }
-          int tap = kb0 / cv.cblocks, cb = kb0 - tap * cv.cblocks;
-          int tr = tap / cv.k, ts = tap - tr * cv.k;
-          for (int kb = kb0; kb < kb1; ++kb) {
-            if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) { alive = false; break; }
-            uint8_t* a = sA + s * A_STAGE_BYTES;
-            uint8_t* b = sB + s * C::B_STAGE_BYTES;
-            uint32_t fb = 0;
-            if constexpr (PAIR) {
-              if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
-              fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), 0);
-            } else {
-              bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-            }
-            if (cv.mode == BB_CONV_WGRAD) {
-              window((unsigned)kb * BK, w, h, n);
-#pragma unroll
-              for (int j = 0; j < BM / 64; ++j) plain(a + j * 8192, &tmA, fb, m0 + 64 * j, kb * BK);
-#pragma unroll
-              for (int j = 0; j < BJ; ++j) patches(b + j * 8192, &tmB, fb, cj[j], w, h, n, sj[j], rj[j]);
-            } else {
-              patches(a, &tmA, fb, cb * 64, w, h, n, ts, tr);
-              if (cv.mode == BB_CONV_FWD) {
-                plain(b, &tmB, fb, kb * BK, n0);
-              } else {
-                const int col = ((cv.k - 1 - tr) * cv.k + (cv.k - 1 - ts)) * cv.wcols + n0;   // the tap turned by 180 degrees
-#pragma unroll
-                for (int j = 0; j < BJ; ++j) plain(b + j * 8192, &tmB, fb, col + 64 * j, cb * 64);
-              }
-              if (++cb == cv.cblocks) { cb = 0; if (++ts == cv.k) { ts = 0; ++tr; } }
-            }
-            if (++s == C::STAGES) { s = 0; phase ^= 1; }
-          }
-        } else {
-          for (int kb = kb0; kb < kb1; ++kb) {
-            if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) { alive = false; break; }
-            uint8_t* a = sA + s * A_STAGE_BYTES;
-            uint8_t* b = sB + s * C::B_STAGE_BYTES;
-            const int k0 = kb * BK;
-            if constexpr (PAIR) {
-              // both CTAs' copies complete on rank 0's barrier, where the MMA issuer waits
-              if (rank == 0) bb::mbar_arrive_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
-              const uint32_t fb = bb::mapa_shared(bb::smem_u32(&full_bar[s]), 0);
-              if (!p.a_mn) {
-                bb::tma_load_2d_pair(a, &tmA, fb, k0, m0);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d_pair(a + j * 8192, &tmA, fb, m0 + 64 * j, k0);
-              }
-              if (!p.b_mn) {
-                bb::tma_load_2d_pair(b, &tmB, fb, k0, n0);
-              } else {
-#pragma unroll
-                for (int j = 0; j < C::B_ROWS / 64; ++j) bb::tma_load_2d_pair(b + j * 8192, &tmB, fb, n0 + 64 * j, k0);
-              }
-            } else {
-              bb::mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-              if (!p.a_mn) {
-                bb::tma_load_2d(a, &tmA, &full_bar[s], k0, m0);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BM / 64; ++j) bb::tma_load_2d(a + j * 8192, &tmA, &full_bar[s], m0 + 64 * j, k0);
-              }
-              if (!p.b_mn) {
-                bb::tma_load_2d(b, &tmB, &full_bar[s], k0, n0);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BN / 64; ++j) bb::tma_load_2d(b + j * 8192, &tmB, &full_bar[s], n0 + 64 * j, k0);
-              }
-            }
-            if (++s == C::STAGES) { s = 0; phase ^= 1; }
-          }
-        }
+        alive = load_operands<BN, PAIR, CONV>(tmA, tmB, p, cv, sA, sB, full_bar, empty_bar, abort_flag, rank, 0u, mi * C::TILE_M + (int)rank * BM,
+                                              ni * BN + (int)rank * C::B_ROWS, kb0, kb1, turn, s, phase);
       };
-      if (rank == 0) {
-        // ---- scheduling thread: announces every work unit of this CTA (pair) to its consumers
+      if (rank == 0 && turn == 0) {
+        // ---- scheduling warp: announces every work unit of this CTA (pair) but the first to its consumers
         auto announce = [&](uint32_t it, int tile) -> bool {
           const int r = (int)(it & (SCHED_RING - 1));
           const uint32_t ph = (it / SCHED_RING) & 1u;
           const bool free_ = PAIR ? bb::mbar_wait_cluster(&sched_empty[r], ph ^ 1, abort_flag, p.status)
                                   : bb::mbar_wait(&sched_empty[r], ph ^ 1, abort_flag, p.status);
-          if (!free_) return false;
-          sched_tile[r] = tile;
-          if (PAIR) {
-            bb::st_shared_cluster_u32(bb::mapa_shared(bb::smem_u32(const_cast<int*>(&sched_tile[r])), 1), (uint32_t)tile);
-            bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&sched_full[r]), 1));
+          if (!__all_sync(0xffffffffu, free_)) return false;
+          if (lane == 0) {
+            sched_tile[r] = tile;
+            if (PAIR) {
+              bb::st_shared_cluster_u32(bb::mapa_shared(bb::smem_u32(const_cast<int*>(&sched_tile[r])), 1), (uint32_t)tile);
+              bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&sched_full[r]), 1));
+            }
+            bb::mbar_arrive(&sched_full[r]);
           }
-          bb::mbar_arrive(&sched_full[r]);
+          __syncwarp();
           return true;
         };
         // ticket t of this launch stands for work unit num_workers + t (units below num_workers are
-        // the CTAs' first ones); every scheduling thread draws until its first ticket past the
+        // the CTAs' first ones); every scheduling warp draws until its first ticket past the
         // end, so a launch consumes exactly num_tiles tickets - the host relies on that count
-        auto draw = [&]() -> int { return num_workers + (int)(atomicAdd(p.ticket, 1u) - p.ticket_base); };
+        // (valid in lane 0; broadcast where it is used, so that the atomic is in flight while the unit's loads are issued)
+        auto draw = [&]() -> int { return lane == 0 ? num_workers + (int)(atomicAdd(p.ticket, 1u) - p.ticket_base) : 0; };
         uint32_t it = 0;
         int cur = worker, nxt = worker;
         while (cur < num_tiles) {
-          nxt = p.dynamic ? draw() : cur + num_workers;     // in flight while this unit's loads are issued
-          if (!announce(it++, cur)) { alive = false; break; }
+          nxt = p.dynamic ? draw() : cur + num_workers;
+          if (cur != worker && !announce(it++, cur)) { alive = false; break; }
           load_unit(cur);
           if (!alive) break;
-          cur = nxt;
+          cur = __shfl_sync(0xffffffffu, nxt, 0);
         }
         if (alive) { if (!announce(it++, -1)) alive = false; }
-        else if (p.dynamic) { while (nxt < num_tiles) nxt = draw(); }
+        else if (p.dynamic && lane == 0) { while (nxt < num_tiles) nxt = draw(); }
       } else {
-        // second CTA of a pair: follows rank 0's announcements
+        // second producer, second CTA of a pair: follow the announcements
         for (uint32_t it = 0; alive; ++it) {
           int tile;
-          if (!next_unit(it, tile, false)) { alive = false; break; }
+          if (!next_unit(it, tile)) { alive = false; break; }
           if (tile < 0) break;
           load_unit(tile);
         }
@@ -493,7 +624,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         // rank 0's MMA commits arrive on this CTA's barriers too: wait until the last one of every
         // stage has landed, so that none is still on its way when the CTA leaves
         for (int i = 0; i < C::STAGES && alive; ++i) {
-          if (!bb::mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, p.status)) alive = false;
+          if ((s & 1) == turn && !bb::mbar_wait_warp(&empty_bar[s], phase ^ 1, abort_flag, p.status)) alive = false;
           if (++s == C::STAGES) { s = 0; phase ^= 1; }
         }
       }
@@ -504,52 +635,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         while (bb::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == MMA_WARP) {
     // ------------------------------------------------ MMA issuer
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
-                           ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(C::TILE_M >> 4) << 24);
-    // K-major: 8-row groups 1024 B apart (LBO unused); MN-major: 64-wide column groups are
-    // separate 8 KiB TMA boxes (LBO), 8 k-rows are 1024 B (SBO).
-    const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
-    const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
     int s = 0; uint32_t phase = 0;
     int acc = 0; uint32_t acc_phase = 0;
     bool alive = true;
     // pairs: rank 0 issues for both CTAs; the other CTA's MMA warp only allocates and frees TMEM
     for (uint32_t it = 0; alive && rank == 0; ++it) {
       int tile;
-      if (!next_unit(it, tile, true)) { alive = false; break; }
+      if (!next_unit(it, tile)) { alive = false; break; }
       if (tile < 0) break;
       if (!bb::mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status)) { alive = false; break; }
       bb::tc_fence_after_sync();
       const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-      const int ks = tile / num_mn;
+      int mi, ni, ks;
+      unit_coords(p, tile, mi, ni, ks);
       const int num_kb = min(total_kb, (ks + 1) * p.kb_per_split) - ks * p.kb_per_split;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if (!bb::mbar_wait_warp(&full_bar[s], phase, abort_flag, p.status)) { alive = false; break; }
-        bb::tc_fence_after_sync();
-        if (bb::elect_one()) {
-          // one descriptor per stage; a k-step only adds to its address field (16-byte units)
-          const uint64_t ad0 = bb::make_smem_desc_sw128(bb::smem_u32(sA + s * A_STAGE_BYTES), a_lbo, 1024u);
-          const uint64_t bd0 = bb::make_smem_desc_sw128(bb::smem_u32(sB + s * C::B_STAGE_BYTES), b_lbo, 1024u);
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t ad = ad0 + (uint64_t)(k * (a_kstep >> 4));
-            const uint64_t bd = bd0 + (uint64_t)(k * (b_kstep >> 4));
-            if (PAIR) bb::umma_f16_pair(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            else bb::umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
-          if (PAIR) {
-            bb::umma_commit_pair(&empty_bar[s], 3);            // frees the stage in both CTAs
-            if (kb == num_kb - 1) bb::umma_commit_pair(&tmem_full[acc], 3);
-          } else {
-            bb::umma_commit(&empty_bar[s]);
-            if (kb == num_kb - 1) bb::umma_commit(&tmem_full[acc]);
-          }
-        }
-        __syncwarp();
-        if (++s == C::STAGES) { s = 0; phase ^= 1; }
-      }
+      if (!issue_mmas<BN, PAIR>(p, sA, sB, full_bar, empty_bar, &tmem_full[acc], abort_flag, 3, d_tmem, num_kb, s, phase)) { alive = false; break; }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else {
@@ -559,7 +661,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     // fused math -> the warp's private 4 KiB staging slab in shared memory -> coalesced 16-byte
     // global stores (fp32 add-reduction: vector red) by the same warp.  Nothing here waits on
     // another warp or on the TMA queue, which the producer keeps full of operand loads.
-    const int eg = (warp - 2) >> 2;                // which of the quarter's EW warps
+    const int eg = (warp - EPI_WARP) >> 2;         // which of the quarter's EW warps
     const int quarter = warp & 3;
     const int epi = p.epi;
     const bool f32 = (epi == BB_EPI_ACCUM_F32 || epi == BB_EPI_STORE_F32);
@@ -571,13 +673,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       // Narrow variant for the epilogues with the most arithmetic per element (GeLU and its
       // derivative) on short reductions, where eight warps cannot finish a tile's epilogue
       // within the next tile's main loop: sixteen warps, 32 bf16 columns per pass (bf16 outputs only).
-      uint8_t* slab = panels + (warp - 2) * (SLAB_BYTES / 2);
+      uint8_t* slab = panels + (warp - EPI_WARP) * (SLAB_BYTES / 2);
       for (uint32_t it = 0; alive; ++it) {
         int tile;
-        if (!next_unit(it, tile, true)) { alive = false; break; }
+        if (!next_unit(it, tile)) { alive = false; break; }
         if (tile < 0) break;
-        const int mn = tile % num_mn;
-        const int mi = p.n_fast ? mn / num_n : mn % num_m, ni = p.n_fast ? mn % num_n : mn / num_m;
+        int mi, ni, ks;
+        unit_coords(p, tile, mi, ni, ks);
         const int m0 = mi * C::TILE_M + (int)rank * BM, n0 = ni * BN;
         const int r0 = m0 + quarter * 32;
         const bool got = bb::mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status);
@@ -588,8 +690,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll 1
         for (int pn = eg; pn < npanels; pn += 4) {
           const int nb = n0 + pn * 32;
-          const bool inside = (nb < p.N) && (r0 < p.M);
-          if (has_aux && inside) slab64_fetch(slab, reinterpret_cast<const __nv_bfloat16*>(p.aux), p.ld_aux, r0, nb, p.M, p.N, lane);
+          const bool some = (nb < p.N) && (r0 < p.M);
+          if (has_aux && some) slab64_fetch(slab, reinterpret_cast<const __nv_bfloat16*>(p.aux), p.ld_aux, r0, nb, p.M, p.N, lane);
           float v[32];
           {
             uint32_t r[32];
@@ -606,7 +708,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
               else bb::mbar_arrive(&tmem_empty[acc]);
             }
           }
-          if (!inside) continue;
+          if (!some) continue;
           if (epi == BB_EPI_BIAS || dual || epi == BB_EPI_BIAS_RESIDUAL) add_bias<32>(p, nb, v);
           if (dual) {
             slab64_store_row(slab, lane, v);           // pre-activation first
@@ -637,13 +739,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     } else {
-    uint8_t* slab = panels + (warp - 2) * SLAB_BYTES;
+    uint8_t* slab = panels + (warp - EPI_WARP) * SLAB_BYTES;
     for (uint32_t it = 0; alive; ++it) {
       int tile;
-      if (!next_unit(it, tile, true)) { alive = false; break; }
+      if (!next_unit(it, tile)) { alive = false; break; }
       if (tile < 0) break;
-      const int mn = tile % num_mn;
-      const int mi = p.n_fast ? mn / num_n : mn % num_m, ni = p.n_fast ? mn % num_n : mn / num_m;
+      int mi, ni, ks;
+      unit_coords(p, tile, mi, ni, ks);
       const int m0 = mi * C::TILE_M + (int)rank * BM, n0 = ni * BN;
       const int r0 = m0 + quarter * 32;            // first output row of this warp
       const bool got = bb::mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status);
@@ -655,8 +757,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll 1
       for (int pn = eg; pn < npanels; pn += 2) {
         const int nb = n0 + pn * width;
-        const bool inside = (nb < p.N) && (r0 < p.M);   // warp-uniform
-        if (has_aux && inside) {
+        const bool some = (nb < p.N) && (r0 < p.M);     // warp-uniform
+        if (has_aux && some) {
           // the aux tile comes in coalesced (rows spread over lanes) and is turned through the
           // slab, so that every lane can pick up its own row after the accumulator arrived
           uint4 ax[8];
@@ -686,7 +788,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             else bb::mbar_arrive(&tmem_empty[acc]);
           }
         }
-        if (!inside) continue;                     // panel entirely outside the matrix
+        if (!some) continue;                     // panel entirely outside the matrix
         if (f32) {
           panel_store_row_f32(slab, lane, v);
           __syncwarp();
@@ -736,10 +838,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   if (PAIR) {
     // neither CTA leaves (or frees TMEM) while the other may still signal its barriers
     bb::cluster_sync();
-    if (warp == 1) bb::tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
+    if (warp == MMA_WARP) bb::tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
   } else {
     __syncthreads();
-    if (warp == 1) bb::tmem_dealloc(tmem_base, C::TMEM_COLS);
+    if (warp == MMA_WARP) bb::tmem_dealloc(tmem_base, C::TMEM_COLS);
   }
 }
 
@@ -825,6 +927,9 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   // The CTAs that run at the same time share one operand and stream the other: walk along the
   // dimension of the SMALLER operand, so that the larger one passes through L2 once.
   p.n_fast = (long long)g->M > (long long)g->N ? 1 : 0;
+  const int num_m = (g->M + C::TILE_M - 1) / C::TILE_M, num_n = (g->N + BN - 1) / BN;
+  p.tiles_in = p.n_fast ? num_n : num_m; p.tiles_mn = (unsigned)num_m * (unsigned)num_n;
+  p.magic_in = bb_div_magic((int)p.tiles_in); p.magic_mn = bb_div_magic((int)p.tiles_mn);
   const int total_kb = (g->K + BK - 1) / BK;
   const int mn_tiles = ((g->M + C::TILE_M - 1) / C::TILE_M) * ((g->N + BN - 1) / BN);
   const int workers_max = PAIR ? bb_num_sms() / 2 : bb_num_sms();

@@ -373,6 +373,12 @@ __device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uin
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same without release: for hand-backs of what the thread has finished reading (values in registers).  A release at
+// cluster scope waits until all of the thread's earlier global stores have been performed - a microsecond per tile where an
+// epilogue warp hands an accumulator back between two panels.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // TMA tile load into this CTA's shared memory whose completion is signalled on an mbarrier of
 // either CTA of the pair (given as a shared::cluster address); no multicast.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int c0, int c1) {

@@ -554,7 +554,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     if (!__all_sync(0xffffffffu, got)) return false;
     tile = __shfl_sync(0xffffffffu, sched_tile[r], 0);
     if (lane == 0) {
-      if (PAIR) bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&sched_empty[r]), 0));
+      if (PAIR) bb::mbar_arrive_cluster_relaxed(bb::mapa_shared(bb::smem_u32(&sched_empty[r]), 0));
       else bb::mbar_arrive(&sched_empty[r]);
     }
     return true;
@@ -603,8 +603,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         uint32_t it = 0;
         int cur = worker, nxt = worker;
         while (cur < num_tiles) {
-          nxt = p.dynamic ? draw() : cur + num_workers;
+          // the announcement's release at cluster scope waits for the thread's outstanding global operations: it comes
+          // before the draw, whose result has a whole unit's time to arrive
           if (cur != worker && !announce(it++, cur)) { alive = false; break; }
+          nxt = p.dynamic ? draw() : cur + num_workers;
           load_unit(cur);
           if (!alive) break;
           cur = __shfl_sync(0xffffffffu, nxt, 0);
@@ -704,7 +706,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             bb::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-              if (PAIR) bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&tmem_empty[acc]), 0));
+              if (PAIR) bb::mbar_arrive_cluster_relaxed(bb::mapa_shared(bb::smem_u32(&tmem_empty[acc]), 0));
               else bb::mbar_arrive(&tmem_empty[acc]);
             }
           }
@@ -784,7 +786,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           bb::tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            if (PAIR) bb::mbar_arrive_cluster(bb::mapa_shared(bb::smem_u32(&tmem_empty[acc]), 0));
+            if (PAIR) bb::mbar_arrive_cluster_relaxed(bb::mapa_shared(bb::smem_u32(&tmem_empty[acc]), 0));
             else bb::mbar_arrive(&tmem_empty[acc]);
           }
         }

@@ -425,18 +425,45 @@ __device__ __forceinline__ float tanh_fast(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu_tanh(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  return 0.5f * x * (1.0f + tanh_fast(u));
+// Two-wide fp32 arithmetic (each half rounded like the scalar instruction): half the issue slots, which is what the fused
+// epilogues of short reductions run out of.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
+  return d;
 }
-__device__ __forceinline__ float gelu_tanh_grad(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  float t = tanh_fast(u);
-  float du = k0 * (1.0f + 3.0f * k1 * x * x);
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * du;
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+// tanh GeLU: x/2 (1 + t), t = tanh(k0 x + k0 k1 x^3), and its derivative (1 + t)/2 + x/2 (1 - t^2) (k0 + 3 k0 k1 x^2)
+constexpr float GELU_K0 = 0.7978845608028654f, GELU_K01 = 0.7978845608028654f * 0.044715f;
+__device__ __forceinline__ float2 gelu_tanh2(float2 x) {
+  const float2 u = mul2(fma2(mul2(x, x), make_float2(GELU_K01, GELU_K01), make_float2(GELU_K0, GELU_K0)), x);
+  const float2 h = mul2(x, make_float2(0.5f, 0.5f));
+  return fma2(h, make_float2(tanh_fast(u.x), tanh_fast(u.y)), h);
+}
+__device__ __forceinline__ float2 gelu_tanh_grad2(float2 x) {
+  const float2 x2 = mul2(x, x), k0 = make_float2(GELU_K0, GELU_K0), half = make_float2(0.5f, 0.5f);
+  const float2 u = mul2(fma2(x2, make_float2(GELU_K01, GELU_K01), k0), x);
+  const float2 du = fma2(x2, make_float2(3.f * GELU_K01, 3.f * GELU_K01), k0);
+  const float2 t = make_float2(tanh_fast(u.x), tanh_fast(u.y));
+  const float2 s = fma2(make_float2(-t.x, -t.y), t, make_float2(1.f, 1.f));
+  return fma2(mul2(mul2(x, half), s), du, fma2(half, t, half));
+}
+__device__ __forceinline__ float gelu_tanh_grad(float x) { return gelu_tanh_grad2(make_float2(x, x)).x; }
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

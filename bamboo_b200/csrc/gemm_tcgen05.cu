@@ -293,6 +293,27 @@ __device__ __forceinline__ void slab64_flush(const uint8_t* slab, __nv_bfloat16*
   }
 }
 
+__device__ __forceinline__ float2 get2(const float* v) { return make_float2(v[0], v[1]); }
+__device__ __forceinline__ void set2(float* v, float2 a) { v[0] = a.x; v[1] = a.y; }
+// GeLU of the bf16-rounded pre-activation: forward and backward (which re-reads the stored pre-activation) see the same argument
+template <int W> __device__ __forceinline__ void gelu_rounded(float* v) {
+#pragma unroll
+  for (int i = 0; i < W; i += 2) {
+    const uint32_t q = bb::pack_bf16x2(v[i], v[i + 1]);
+    set2(v + i, bb::gelu_tanh2(make_float2(bb::bf16_lo(q), bb::bf16_hi(q))));
+  }
+}
+// v *= gelu'(x) or v += x
+template <int W> __device__ __forceinline__ void apply_aux(int epi, float* v, const float* x) {
+  if (epi == BB_EPI_MUL_DGELU) {
+#pragma unroll
+    for (int i = 0; i < W; i += 2) set2(v + i, bb::mul2(get2(v + i), bb::gelu_tanh_grad2(get2(x + i))));
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; i += 2) set2(v + i, bb::add2(get2(v + i), get2(x + i)));
+  }
+}
+
 // bias[n0 .. n0+W) added to v; columns past N read as zero
 template <int W>
 __device__ __forceinline__ void add_bias(const GemmParams& p, int n0, float* v) {
@@ -302,7 +323,7 @@ __device__ __forceinline__ void add_bias(const GemmParams& p, int n0, float* v) 
     for (int i = 0; i < W; i += 8) {
       float f[8]; unpack8(__ldg(reinterpret_cast<const uint4*>(b + i)), f);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[i + k] += f[k];
+      for (int k = 0; k < 8; k += 2) set2(v + i + k, bb::add2(get2(v + i + k), make_float2(f[k], f[k + 1])));
     }
   } else {
     // fully unrolled with predicates: a dynamically indexed v[] would live in local memory
@@ -716,21 +737,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             slab64_store_row(slab, lane, v);           // pre-activation first
             __syncwarp();
             slab64_flush(slab, reinterpret_cast<__nv_bfloat16*>(p.D2), p.ldd, r0, nb, p.M, p.N, lane);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = bb::gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
+            gelu_rounded<32>(v);
             __syncwarp();
           } else if (has_aux) {
             __syncwarp();
             float x[32];
 #pragma unroll
             for (int c = 0; c < 4; ++c) unpack8(*reinterpret_cast<const uint4*>(slab + slab64_off(lane, c)), x + 8 * c);
-            if (epi == BB_EPI_MUL_DGELU) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] *= bb::gelu_tanh_grad(x[i]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] += x[i];
-            }
+            apply_aux<32>(epi, v, x);
             __syncwarp();
           }
           slab64_store_row(slab, lane, v);
@@ -804,10 +818,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           panel_store_row_bf16(slab, lane, v);     // pre-activation first
           __syncwarp();
           slab_flush_bf16(slab, reinterpret_cast<__nv_bfloat16*>(p.D2), p.ldd, r0, nb, p.M, p.N, lane);
-          // GeLU of the bf16-rounded pre-activation: forward and backward (which re-reads the
-          // stored pre-activation) see the same argument
-#pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = bb::gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
+          gelu_rounded<64>(v);
           __syncwarp();
         } else if (has_aux) {
           __syncwarp();
@@ -816,13 +827,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             float x[32];
 #pragma unroll
             for (int c = 0; c < 4; ++c) unpack8(*reinterpret_cast<const uint4*>(slab + slab_off(lane, 4 * h + c)), x + 8 * c);
-            if (epi == BB_EPI_MUL_DGELU) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[32 * h + i] *= bb::gelu_tanh_grad(x[i]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[32 * h + i] += x[i];
-            }
+            apply_aux<32>(epi, v + 32 * h, x);
           }
           __syncwarp();
         }
@@ -1055,14 +1060,14 @@ AccumPlan plan_accum(int M, int N, int K) {
 // Products that are stored: tile width and pairing by the time that they are expected to take, in microseconds.  A tile
 // costs a rate per k-block (128 x 128, 128 x 256, and 128 x 256 for each CTA of a pair, the cheapest per output because
 // it loads least) and, wave after wave, what its epilogue leaves uncovered; once per launch its start and its last
-// epilogue.  Fitted on 8 shapes each of 12 problem sizes between 512 x 256 x 256 and 4096 x 16384 x 4096, where it is
-// within a tenth of the measured times; what the choice gained where it changed (us, with a fixed rule before):
-// 513 x 2048 x 2048 26.6 -> 20.5 (128 wide instead of a quarter-filled wave of pairs), 999 x 1024 x 4096 34.8 -> 28.7,
-// 4096 x 1024 x 1024 20.4 -> 16.4 and 8192 x 512 x 1536 24.6 -> 20.5 (one wave of 256 wide tiles instead of two).
+// epilogue.  Fitted on 57 products of 512 x 256 x 256 to 8192 x 50304 x 1024 with every epilogue, where the times are met within a
+// tenth on average and the choice is the quickest of the three every time.  Constants from before the pairs' hand-backs became
+// cheap kept 8192 x 4096 x 1024 (bias + GeLU 66.5 us, as pairs 57.2), 8192 x 3072 x 1024 (47.4, 42.7), 2331 x 4096 x 1024 (31.1, 27.8)
+// and 8192 x 50304 x 1024 (648, 564) on single CTAs.
 struct StorePlan { int bn; bool pair; double us; };
 StorePlan plan_store(long long M, long long N, long long K, int max_ctas, bool pairs_allowed) {
   static const struct { int bn; bool pair; double kblock, wave, once; } kinds[3] = {
-      {256, true, 0.34, 2.3, 10.5}, {256, false, 0.41, 1.2, 8.5}, {128, false, 0.30, 1.2, 8.0}};
+      {256, true, 0.32, 1.9, 5.0}, {256, false, 0.375, 1.8, 3.7}, {128, false, 0.283, 1.0, 3.7}};
   const double kb = (double)((K + BK - 1) / BK);
   StorePlan best = {128, false, -1};
   for (const auto& k : kinds) {
@@ -1088,11 +1093,10 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     *pair_out = pl.pair;
     return pl.bn;
   }
-  // sixteen epilogue warps for the GeLU epilogues on short reductions (see the narrow variant), and for the residual add,
-  // whose operand comes from memory: twice the warps have twice the loads in flight
-  // (2331 x 1024 x 1024 16.1 -> 14.9 us, 4096 x 1024 x 1024 16.9 -> 15.1 us, 8192 x 1024 x 4096 56.7 -> 55.8 us; none slower)
-  *wide_out = g->epi_warps == 4 || (g->epi_warps == 0 && (e == BB_EPI_BIAS_RESIDUAL ||
-                                                          ((e == BB_EPI_BIAS_GELU || e == BB_EPI_MUL_DGELU) && g->K <= 2048)));
+  // eight epilogue warps unless sixteen are asked for: with two-wide arithmetic and panels stored without a test per row they
+  // finish a tile within the next one's main loop (8192 x 4096 x 1024 as pairs, bias + GeLU 57.2 us with eight, 57.5 with sixteen;
+  // residual 8192 x 1024 x 1024 21.2 and 22.2)
+  *wide_out = g->epi_warps == 4;
   *pair_out = g->cta_pair > 0;
   if (g->cta_pair > 0) return 256;
   if (g->tile_n != 0) return g->tile_n;

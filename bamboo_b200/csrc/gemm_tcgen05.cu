@@ -1002,16 +1002,18 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   return BB_OK;
 }
 
-// Whether a weight gradient of the widest tile would run as CTA pairs
+// Whether a weight gradient may run as CTA pairs.  It runs beside the input gradients of its layer, and a pair needs both SMs of
+// a processing cluster free: beside an input gradient of few single CTAs short reductions starve as pairs (vocabulary head on
+// 999 tokens: the weight gradient alone 122 -> 107 us, the case 475 -> 628 us).
 bool pairs_pay(int M, int N, int K) {
   const long long tiles_single = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);
   return M > BM && N > 128 && (K >= 2048 || tiles_single >= 16LL * bb_num_sms());
 }
 
 // Weight gradients (fp32 add-reduction): few output tiles and a long reduction, so tile, pairing and the split of the
-// reduction are chosen together.  A unit's time is counted in 16 KiB operand loads: two per k-block for a 128 x 128
-// tile, three for 128 x 256, a little less for each CTA of a 256 x 256 pair, plus a tile's start and its add-reduction
-// (EPI per 128 columns); a plan costs waves x that.  Splits go as far as one wave of the machine (or 16, as more
+// reduction are chosen together, by the time in microseconds: waves x (k-blocks x rate + a tile's start and add-reduction) +
+// once per launch (fitted on 35 products with up to 24 splits each, within a tenth; 1024 x 1024 x 2331
+// 11.8 -> 10.3 us, 1024 x 256 x 8192 12.4 -> 10.9 against a plan that counted operand loads).  Splits go as far as one wave of the machine (or 16, as more
 // than one wave evens out ragged ones) and leave at least eight k-blocks per unit (short reductions stay whole, with one
 // order of additions).  No unit sums more k-blocks than wave_split gives the widest tile: the accumulator's rounding
 // grows with their number (256 x 2304 x 6272 against fp64: 13 k-blocks 7.8e-7, 25 k-blocks 1.6e-6).
@@ -1020,7 +1022,8 @@ bool pairs_pay(int M, int N, int K) {
 // 14.3 -> 12.3; 1024 x 1024 x 8192 and larger as before.
 struct AccumPlan { int bn; bool pair; int ksplit; };
 AccumPlan plan_accum(int M, int N, int K) {
-  constexpr double EPI = 14.0;
+  static const struct { int bn; bool pair; double kblock, tile, once; } kinds[3] = {
+      {256, true, 0.316, 4.6, 3.2}, {256, false, 0.365, 4.6, 1.9}, {128, false, 0.282, 1.75, 3.1}};
   const long long kb = (K + BK - 1) / BK;
   long long longest;
   {
@@ -1031,15 +1034,13 @@ AccumPlan plan_accum(int M, int N, int K) {
   }
   AccumPlan best = {128, false, 1};
   double best_cost = -1;
-  for (int c = 0; c < 3; ++c) {
-    const bool pair = c == 0;
-    const int bn = c == 2 ? 128 : 256;
-    if (bn == 256 && N <= 128) continue;
-    if (pair && !pairs_pay(M, N, K)) continue;
+  for (const auto& k : kinds) {
+    const int bn = k.bn;
+    const bool pair = k.pair;
+    if ((bn == 256 && N <= 128) || (pair && !pairs_pay(M, N, K))) continue;
     const long long tm = pair ? 2 * BM : BM;
     const long long tiles = ((M + tm - 1) / tm) * ((N + bn - 1) / bn);
     const long long workers = pair ? bb_num_sms() / 2 : bb_num_sms();
-    const double per_kb = pair ? 2.9 : (bn == 256 ? 3.0 : 2.0), fixed = bn == 256 ? 2 * EPI : EPI;
     // up to 16, then the largest that stays within one wave: between the two a larger split only shortens the units
     long long widest = workers / tiles;
     if (widest > (kb - 1) / 7) widest = (kb - 1) / 7;        // (the largest with eight k-blocks per unit)
@@ -1050,7 +1051,7 @@ AccumPlan plan_accum(int M, int N, int K) {
       if (s > 1 && kbs < 8) break;
       if (kbs > longest) continue;
       const long long units = tiles * ((kb + kbs - 1) / kbs);
-      const double cost = (double)((units + workers - 1) / workers) * ((double)kbs * per_kb + fixed);
+      const double cost = (double)((units + workers - 1) / workers) * ((double)kbs * k.kblock + k.tile) + k.once;
       if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, pair, (int)s}; }
     }
   }

@@ -184,6 +184,35 @@ attn_tc_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const TcP
   }
 }
 
+// 32 scores of one key row against 32 queries -> P^T and dS^T as bf16 pairs: p = 2^(s c - L), dS = p (dP - delta), with -L (log2
+// units) and -delta per query column in shared memory.  The element-wise work fills the issue slots of these kernels (2300 of the
+// 2600 cycles that a sub-block took with scalar instructions and a mask test per element), so the arithmetic is two elements
+// wide and only sub-blocks that touch an edge test columns: visible are first..last.
+template <bool MASK>
+__device__ __forceinline__ void dkv_math(const float* s, const float* dp, const float* nl, const float* nd, float sl, int first, int last,
+                                         uint32_t* pkP, uint32_t* pkDS) {
+  const float2 c2 = make_float2(sl, sl);
+#pragma unroll
+  for (int e = 0; e < 32; e += 4) {
+    const float4 l4 = *reinterpret_cast<const float4*>(nl + e);
+    const float4 d4 = *reinterpret_cast<const float4*>(nd + e);
+    const float2 ls[2] = {make_float2(l4.x, l4.y), make_float2(l4.z, l4.w)}, ds[2] = {make_float2(d4.x, d4.y), make_float2(d4.z, d4.w)};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = e + 2 * u;
+      const float2 x = bb::fma2(make_float2(s[i], s[i + 1]), c2, ls[u]);
+      float2 pv = make_float2(ex2(x.x), ex2(x.y));
+      if (MASK) {
+        if (i < first || i > last) pv.x = 0.f;
+        if (i + 1 < first || i + 1 > last) pv.y = 0.f;
+      }
+      const float2 g = bb::mul2(pv, bb::add2(make_float2(dp[i], dp[i + 1]), ds[u]));
+      pkP[i >> 1] = bb::pack_bf16x2(pv.x, pv.y);
+      pkDS[i >> 1] = bb::pack_bf16x2(g.x, g.y);
+    }
+  }
+}
+
 // =====================================================================================
 // Pipelined backward kernels: 64-wide sub-blocks, every hand-off double-buffered, two compute
 // groups (warps 2-5 and 6-9) that take alternate sub-blocks, so the tensor core always has the
@@ -652,12 +681,13 @@ attn_tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
 // but S^T and dP^T are computed once: the staged dS^T tiles of two consecutive sub-blocks
 // ([128 keys x 64 queries] each, adjacent in shared memory) also serve, read with the queries as
 // the M dimension, as the A operand of dQ[128 queries x 64] = dS . K for that pair of sub-blocks.
-// The pair's dQ [128 x 64] fp32 leaves tensor memory through a shared-memory staging tile and two
-// bulk tensor add-reductions (one per 32-column half) into a [B, H, S, 64] accumulator: each query
-// row receives one contribution per key tile, in no fixed order; a small kernel scales and converts
-// the sums once all CTAs are done.  Five contractions instead of seven, one
+// The pair's dQ [128 x 64] fp32 leaves tensor memory through staging tiles and bulk tensor add-reductions
+// into a [B, H, S, 64] accumulator: each of the sixteen compute warps moves 32 rows x 16 columns through a tile of its own,
+// so nothing here waits for another warp; each query row receives one contribution per key tile, in no fixed order; a small
+// kernel scales and converts the sums once all CTAs are done.  Five contractions instead of seven, one
 // exponential pass instead of two, half the CTAs.
-// smem: K, V [128 x 64] | Q, dO sub-tiles x NST3 | P^T x 2 | dS^T x 2 pair slots x 2 groups | dQ staging 2 x 16 KiB | lse / delta
+// A compute warp that gave up on a wait goes on through the loop (its waits return at once then) and stores nothing.
+// smem: K, V [128 x 64] | Q, dO sub-tiles x NST3 | P^T x 2 | dS^T x 2 pair slots x 2 groups | dQ staging 16 x 2 KiB | lse / delta
 // TMEM: S^T 2 x 64 | dP^T 2 x 64 | dV 64 | dK 64 | dQ 2 x 64
 constexpr int NST3 = 4;
 constexpr int NSTAT = 3;                         // depth of the ring of query statistics
@@ -677,8 +707,8 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
   uint8_t* sDO = sQ + NST3 * SUB_BYTES;        // NST3 stages x 8 KiB
   uint8_t* sP = sDO + NST3 * SUB_BYTES;        // [group] x 16 KiB
   uint8_t* sDS = sP + 2 * TILE_BYTES;          // [pair slot][group] x 16 KiB
-  uint8_t* sDQ = sDS + 4 * TILE_BYTES;         // [column half] x 16 KiB: [128 queries x 32] fp32, 128-byte rows
-  float* s_lse = reinterpret_cast<float*>(sDQ + 2 * TILE_BYTES);   // [NSTAT][64]: log-sum-exp and delta of a sub-block's queries
+  uint8_t* sDQ = sDS + 4 * TILE_BYTES;         // [compute warp] x 2 KiB: [32 queries x 16] fp32, 64-byte rows, 64-byte swizzle
+  float* s_lse = reinterpret_cast<float*>(sDQ + 2 * TILE_BYTES);   // [NSTAT][64]: negated log-sum-exp (log2 units) and delta of a sub-block's queries
   float* s_delta = s_lse + NSTAT * SUB;                            // [NSTAT][64]
   Ctl* ctl = reinterpret_cast<Ctl*>(s_delta + NSTAT * SUB);
   uint64_t* kv_full = &ctl->bars[0];
@@ -715,7 +745,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       bb::mbar_init(&s_full[i], 1); bb::mbar_init(&s_empty[i], GROUP_THREADS / 32);
       bb::mbar_init(&p_full[i], GROUP_THREADS / 32); bb::mbar_init(&p_empty[i], 1);
       bb::mbar_init(&ds_empty[i], 1);
-      bb::mbar_init(&dq_full[i], 1); bb::mbar_init(&dq_empty[i], GROUP_THREADS / 32);
+      bb::mbar_init(&dq_full[i], 1); bb::mbar_init(&dq_empty[i], 2 * GROUP_THREADS / 32);
     }
     bb::mbar_init(acc_full, 1);
     for (int i = 0; i < NSTAT; ++i) bb::mbar_init(&st_full[i], 1);
@@ -825,8 +855,8 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int q = (qstart + i) * SUB + lane + 32 * u;
-        l2[u] = (q < p.S) ? lse_g[q] * LOG2E : 0.f;
-        d2[u] = (q < p.S) ? delta_g[q] : 0.f;
+        l2[u] = (q < p.S) ? -(lse_g[q] * LOG2E) : 0.f;
+        d2[u] = (q < p.S) ? -delta_g[q] : 0.f;
       }
       if (i >= NSTAT && !bb::mbar_wait_warp(&q_empty[(i - NSTAT) % NST3], ((i - NSTAT) / NST3) & 1, &ctl->abort_flag, p.status)) break;
       const int st = i % NSTAT;
@@ -840,61 +870,56 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
     const int hf = ((warp - 4) >> 2) & 1;                  // which 32 of the sub-block's 64 query columns
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;                   // key row inside the tile / query row inside a pair
-    const int gt = threadIdx.x - 128 - GROUP_THREADS * g;  // thread index inside the group
     const int krow = k0 + row;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const float sl = p.scale * LOG2E;
     uint8_t* myP = sP + g * TILE_BYTES;
-    bool alive = true;
-    int n = 0;
-    int next_drain = 0;                                     // group 1 drains every pair
+    uint8_t* myDQ = sDQ + (warp - 4) * 2048;
+    const int dq_col = g * 32 + hf * 16;                   // this warp's columns of a pair's dQ
     const long long acc_row0 = ((long long)batch * p.H + head) * p.S;
-    // one pair's dQ: tensor memory -> staging tile -> add-reduction into the accumulator rows of its 128
-    // queries.  Rows past the sequence end belong to the next (batch, head): they add zeros, also where a key is Inf or NaN
-    // (a tensor map with a sequence dimension, which leaves such rows out, costs every reduction: B8 H16 S1024 non-causal 222 -> 228 us)
-    auto drain = [&](int pair) -> bool {
-      const bool ok = bb::mbar_wait(&dq_full[pair & 1], (pair >> 1) & 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) return false;
+    bool alive = true;
+    // This warp's part of one pair's dQ: tensor memory -> staging tile -> add-reduction into the accumulator.  Rows past the
+    // sequence end belong to the next (batch, head): they add zeros, also where a key is Inf or NaN (a tensor map with a
+    // sequence dimension, which leaves such rows out, costs every reduction: B8 H16 S1024 non-causal 222 -> 228 us).
+    auto drain = [&](int pair) {
+      if (!bb::mbar_wait_warp(&dq_full[pair & 1], (pair >> 1) & 1, &ctl->abort_flag, p.status)) alive = false;
       bb::tc_fence_after_sync();
-      float v[32];
-      ld32(tDQ + 64 * (pair & 1) + lane_addr + hf * 32, v);
-      const int q0 = (qstart + 2 * pair) * SUB;
-      if (q0 + row >= p.S) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0.f;
-      }
+      uint32_t r[16];
+      bb::tmem_ld_32x32b_x16(tDQ + 64 * (pair & 1) + lane_addr + dq_col, r);
+      bb::tmem_ld_wait();
       bb::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) bb::mbar_arrive(&dq_empty[pair & 1]);
-      // the staging tile is free once the previous pair's reductions have read it
-      if (gt == 0) bb::bulk_wait_group_read<0>();
-      bb::named_bar_sync(3 + g, GROUP_THREADS);
-      uint8_t* dst = sDQ + hf * TILE_BYTES + row * 128;
+      if (lane == 0) {
+        bb::mbar_arrive(&dq_empty[pair & 1]);
+        bb::bulk_wait_group_read<0>();                     // the staging tile: the previous pair's reduction has read it
+      }
+      __syncwarp();
+      const int q0 = (qstart + 2 * pair) * SUB + quarter * 32;
+      if (q0 >= p.S) return;
+      if (q0 + lane >= p.S) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<float4*>(dst + ((c ^ (row & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        for (int i = 0; i < 16; ++i) r[i] = 0u;
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(myDQ + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
       bb::fence_proxy_async();
-      bb::named_bar_sync(3 + g, GROUP_THREADS);
-      if (gt == 0) {
-        const int r0 = (int)(acc_row0 + q0);
-        bb::tma_reduce_add_2d(&tm_acc, sDQ, 0, r0);
-        bb::tma_reduce_add_2d(&tm_acc, sDQ + TILE_BYTES, 32, r0);
+      __syncwarp();
+      if (lane == 0) {
+        bb::tma_reduce_add_2d(&tm_acc, myDQ, dq_col, (int)(acc_row0 + q0));
         bb::bulk_commit_group();
       }
-      return true;
     };
-    for (int i = g; i < nblk && alive; i += 2, ++n) {
-      const int qc0 = (qstart + i) * SUB;
+    int n = 0;
+    for (int i = g; i < nblk; i += 2, ++n) {
+      const int q0 = (qstart + i) * SUB + hf * 32;           // first query of this thread's columns
       const int ps = n & 1;                                  // sub-block i belongs to pair n
-      const float* my_lse = s_lse + (i % NSTAT) * SUB;
-      const float* my_delta = s_delta + (i % NSTAT) * SUB;
+      const float* my_lse = s_lse + (i % NSTAT) * SUB + hf * 32;
+      const float* my_delta = s_delta + (i % NSTAT) * SUB + hf * 32;
       const uint32_t tS = tmem + 64 * g, tDP = tmem + 128 + 64 * g;
-      const bool ok = bb::mbar_wait(&st_full[i % NSTAT], (i / NSTAT) & 1, &ctl->abort_flag, p.status) &&
-                      bb::mbar_wait(&s_full[g], n & 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&st_full[i % NSTAT], (i / NSTAT) & 1, &ctl->abort_flag, p.status) ||
+          !bb::mbar_wait_warp(&s_full[g], n & 1, &ctl->abort_flag, p.status)) alive = false;
       bb::tc_fence_after_sync();
-      // (keys past the sequence end must not reach dQ: their rows of dK / dV are simply not stored)
-      const bool need_mask = (qc0 + SUB > p.S) || (k0 + TQ > p.S) || (p.causal && k0 + TQ - 1 > qc0);
       uint32_t pkP[16], pkDS[16];                            // this thread's 32 P^T and dS^T values as bf16 pairs
       {
         float sv[32], dp[32];
@@ -903,49 +928,27 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
         bb::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) bb::mbar_arrive(&s_empty[g]);
-#pragma unroll
-        for (int e4 = 0; e4 < 32; e4 += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(my_lse + hf * 32 + e4);
-          const float4 d4 = *reinterpret_cast<const float4*>(my_delta + hf * 32 + e4);
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, ds[4] = {d4.x, d4.y, d4.z, d4.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int e = e4 + u;
-            float pv = ex2(fmaf(sv[e], sl, -ls[u]));
-            if (need_mask) {
-              const int q = qc0 + hf * 32 + e;
-              if (q >= p.S || krow >= p.S || (p.causal && krow > q)) pv = 0.f;
-            }
-            sv[e] = pv;
-            dp[e] = pv * (dp[e] - ds[u]);
-          }
-        }
-        pack32(sv, pkP);
-        pack32(dp, pkDS);
+        // (keys past the sequence end must not reach dQ: their rows of dK / dV are simply not stored)
+        if (q0 + 32 > p.S || k0 + TQ > p.S || (p.causal && k0 + TQ - 1 > q0))
+          dkv_math<true>(sv, dp, my_lse, my_delta, sl, p.causal ? krow - q0 : 0, krow < p.S ? p.S - 1 - q0 : -1, pkP, pkDS);
+        else
+          dkv_math<false>(sv, dp, my_lse, my_delta, sl, 0, 0, pkP, pkDS);
       }
       // P^T's buffer is free once the dV update that read it retired; the pair slot's dS^T buffers once
       // the dK updates and the dQ product of the pair that used the slot before have
-      const bool ok2 = bb::mbar_wait(&p_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status) &&
-                       bb::mbar_wait(&ds_empty[ps], ((n >> 1) & 1) ^ 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok2)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&p_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status) ||
+          !bb::mbar_wait_warp(&ds_empty[ps], ((n >> 1) & 1) ^ 1, &ctl->abort_flag, p.status)) alive = false;
       atom_store_half_row(myP, row, hf, pkP);
       atom_store_half_row(sDS + (ps * 2 + g) * TILE_BYTES, row, hf, pkDS);
       bb::fence_proxy_async();
       __syncwarp();
       if (lane == 0) bb::mbar_arrive(&p_full[g]);
-      // group 1 drains the previous pair, whose second half it staged one iteration ago: certainly complete
-      if (g == 1 && next_drain < n) {
-        if (!drain(next_drain)) { alive = false; break; }
-        ++next_drain;
-      }
+      // the previous pair, whose second half was staged one iteration ago
+      if (n > 0) drain(n - 1);
     }
-    while (g == 1 && alive && next_drain < npairs) {
-      if (!drain(next_drain)) { alive = false; break; }
-      ++next_drain;
-    }
-    if (g == 1 && gt == 0) bb::bulk_wait_group<0>();       // the reductions read this CTA's shared memory
-    const bool fin = alive && nblk > 0 && bb::mbar_wait(acc_full, 0, &ctl->abort_flag, p.status);
-    if (bb::named_bar_all(3 + g, GROUP_THREADS, fin)) {
+    drain(npairs - 1);
+    if (!bb::mbar_wait_warp(acc_full, 0, &ctl->abort_flag, p.status)) alive = false;
+    if (alive) {
       bb::tc_fence_after_sync();
       float v[32];
       // the two groups split the final stores: group 0 writes dV, group 1 writes dK
@@ -954,6 +957,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       __nv_bfloat16* dst = (g == 0) ? p.dv : p.dk;
       if (krow < p.S) store_row32(dst + (long long)(row_base + krow) * p.stride_dqkv + colq + hf * 32, v, g == 0 ? 1.f : p.scale);
     }
+    if (lane == 0) bb::bulk_wait_group_read<0>();          // the reductions read this CTA's shared memory
   }
   bb::tc_fence_before_sync();
   __syncthreads();
@@ -1570,9 +1574,9 @@ int bb_attention_tc_bwd(const void* qkv_q, const void* out, const void* d_out, c
   BB_ONCE_PER_DEVICE({ if (int rc = set_smem(attn_tc_bwd3_kernel, BWD3_SMEM)) return rc; });
   bb_launch(attn_tc_delta_kernel<64>, (int)dgrid, 256, 0, stream, (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, p);
   const int grid = (S + TQ - 1) / TQ * H * B;
-  // the accumulator as [B * H * S rows, 64] fp32; a reduction moves [128 rows x 32 columns]
+  // the accumulator as [B * H * S rows, 64] fp32; a reduction moves [32 rows x 16 columns]
   CUtensorMap tm_acc;
-  if (int rc = bbhost::encode_2d(&tm_acc, dq_acc, (long long)B * H * S, HD, HD, 32, TQ, 1)) return rc;
+  if (int rc = bbhost::encode_2d(&tm_acc, dq_acc, (long long)B * H * S, HD, HD, 16, 32, 1, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
   bb_launch(attn_tc_bwd3_kernel, grid, NT3, BWD3_SMEM, stream, tm_qkv, tm_qkv64, tm_do64, tm_acc, p);
   long long cgrid = (chunks + 255) / 256;
   bb_launch(attn_tc_dq_convert_kernel, (int)(cgrid < cap ? cgrid : cap), 256, 0, stream, p);

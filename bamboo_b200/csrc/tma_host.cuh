@@ -36,15 +36,15 @@ inline int bind_context() {
   return BB_OK;
 }
 
-// Tensor map of `rank` dimensions (innermost first, 128-byte swizzle) over bf16, or fp32 when f32 != 0; `pitch`: bytes
+// Tensor map of `rank` dimensions (innermost first, 128-byte swizzle unless named) over bf16, or fp32 when f32 != 0; `pitch`: bytes
 // between neighbours of every dimension but the innermost.
 inline int encode_tiled(CUtensorMap* tm, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* pitch,
-                        const cuuint32_t* box, int f32) {
+                        const cuuint32_t* box, int f32, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) { bb_set_last_error_msg("cuTensorMapEncodeTiled entry point not available"); return BB_ERR_CUDA; }
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base),
-                  dims, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  dims, pitch, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     char msg[256];
@@ -59,10 +59,10 @@ inline int encode_tiled(CUtensorMap* tm, const void* base, int rank, const cuuin
 
 // 2-D tensor map over a row-major [rows, cols] matrix with leading dimension ld (elements); box = box_cols x box_rows.
 inline int encode_2d(CUtensorMap* tm, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows,
-                     int f32 = 0) {
+                     int f32 = 0, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, pitch[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
   const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  return encode_tiled(tm, base, 2, dims, pitch, box, f32);
+  return encode_tiled(tm, base, 2, dims, pitch, box, f32, swizzle);
 }
 
 // 3-D tensor map over `seqs` sequences of `rows` bf16 rows each, one after the other in a [seqs * rows, cols] matrix.  A box

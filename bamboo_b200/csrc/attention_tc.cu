@@ -225,7 +225,9 @@ constexpr int SUB_BYTES = SUB * HD * 2;          // 8 KiB: [64 x 64] bf16
 // reductions here, and four compute warps per scheduler hide the TMEM-load and ALU latencies that
 // two could not (issue slots were 35 % busy with 4-warp groups).
 constexpr int GROUP_THREADS = 256;
-constexpr int NT2 = 64 + 2 * GROUP_THREADS;
+constexpr int NT2 = 64 + 2 * GROUP_THREADS + 32;     // the last warp stages the queries' statistics (dK / dV role)
+constexpr int STAT_WARP = 2 + 2 * GROUP_THREADS / 32;
+constexpr int NSTAT = 3;                         // depth of the ring of query statistics
 
 // Geometry of the two-role backward at head dimension D.  A [rows x 128] operand is two [rows x 64] atoms of
 // 128-byte rows, one after the other (two TMA boxes), exactly as in the forward kernel.
@@ -360,7 +362,7 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
         __syncwarp();
       }
     }
-  } else {
+  } else if (warp != STAT_WARP) {
     const int g = (warp - 2) >> 3;                           // compute group = buffer index
     const int hf = ((warp - 2) >> 2) & 1;                    // which 32 of the sub-block's 64 columns
     const int quarter = warp & 3;
@@ -373,49 +375,51 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
     const float dl = (qrow < p.S) ? delta_g[qrow] : 0.f;
     const float sl = p.scale * LOG2E;
     uint8_t* myDS = sDS + g * TILE_BYTES;
+    // every warp waits for itself; one that gave up goes on (its waits return at once then) and stores nothing
     bool alive = true;
     int n = 0;                                               // this group's iteration count
-    for (int j = g; j < nblk && alive; j += 2, ++n) {
+    const float2 sl2 = make_float2(sl, sl), nlse2 = make_float2(-lse, -lse), ndl2 = make_float2(-dl, -dl);
+    for (int j = g; j < nblk; j += 2, ++n) {
       const int sb = j % NSB;
       const uint32_t tS = tmem + 64 * sb, tDP = tmem + 64 * (NSB + sb);
-      const bool ok = bb::mbar_wait(&s_full[sb], (j / NSB) & 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&s_full[sb], (j / NSB) & 1, &ctl->abort_flag, p.status)) alive = false;
       bb::tc_fence_after_sync();
       const int c0 = j * SUB + hf * 32;
-      // only sub-blocks that touch the sequence end or the causal diagonal need per-element masks
-      const bool need_mask = (c0 + 32 > p.S) || (p.causal && c0 + 32 - 1 > q0);
-      const float nlse = -lse;
       uint32_t pk[16];                                       // this thread's 32 dS values as bf16 pairs
       {
         float sv[32], dp[32];
         ld32x2(tS + lane_addr + hf * 32, tDP + lane_addr + hf * 32, sv, dp);
-        if (!need_mask) {
+        bb::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) bb::mbar_arrive(&s_empty[sb]);        // scores in registers: the MMA warp may refill
+        // only sub-blocks that touch the sequence end or the causal diagonal test columns
+        if (c0 + 32 > p.S || (p.causal && c0 + 32 - 1 > q0)) {
+          const int last = min(p.S - 1, p.causal ? qrow : p.S - 1) - c0;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) dp[i] = ex2(fmaf(sv[i], sl, nlse)) * (dp[i] - dl);
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = bb::fma2(make_float2(sv[i], sv[i + 1]), sl2, nlse2);
+            const float2 pv = make_float2(i > last ? 0.f : ex2(x.x), i + 1 > last ? 0.f : ex2(x.y));
+            const float2 d = bb::mul2(pv, bb::add2(make_float2(dp[i], dp[i + 1]), ndl2));
+            pk[i >> 1] = bb::pack_bf16x2(d.x, d.y);
+          }
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int col = c0 + i;
-            float pv = ex2(fmaf(sv[i], sl, nlse));
-            if (col >= p.S || (p.causal && col > qrow)) pv = 0.f;
-            dp[i] = pv * (dp[i] - dl);
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = bb::fma2(make_float2(sv[i], sv[i + 1]), sl2, nlse2);
+            const float2 d = bb::mul2(make_float2(ex2(x.x), ex2(x.y)), bb::add2(make_float2(dp[i], dp[i + 1]), ndl2));
+            pk[i >> 1] = bb::pack_bf16x2(d.x, d.y);
           }
         }
-        pack32(dp, pk);
       }
-      bb::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) bb::mbar_arrive(&s_empty[sb]);          // scores consumed: the MMA warp may refill
       // the staging buffer is free once the dQ update that read it two sub-blocks ago retired
-      const bool ok2 = bb::mbar_wait(&ds_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok2)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&ds_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status)) alive = false;
       atom_store_half_row(myDS, row, hf, pk);
       bb::fence_proxy_async();
       __syncwarp();
       if (lane == 0) bb::mbar_arrive(&ds_full[g]);
     }
-    const bool fin = alive && bb::mbar_wait(acc_full, 0, &ctl->abort_flag, p.status);
-    if (bb::named_bar_all(3 + g, GROUP_THREADS, fin) && g < NA) {
+    if (!bb::mbar_wait_warp(acc_full, 0, &ctl->abort_flag, p.status)) alive = false;
+    if (alive && g < NA) {
       // group g stores the g-th 64 columns
       bb::tc_fence_after_sync();
       float v[32];
@@ -435,7 +439,7 @@ template <int D> constexpr int dq2_smem() {
 
 // ------------------------------------------------------------------ dK, dV (pipelined)
 // smem: K, V [128 x D] | Q, dO sub-tiles [64 x D] x NST stages | P^T, dS^T [128 kv x 64 q] x 2 each
-//       | per-group lse / delta of the sub-block's 64 query columns
+//       | lse / delta of a sub-block's 64 query columns, x NSTAT
 // TMEM: S^T NSB x 64 | dP^T NSB x 64 | dV D | dK D
 template <int D>
 __device__ __forceinline__ void
@@ -450,9 +454,9 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   uint8_t* sDO = sQ + NST * G::STREAM_BYTES;   // NST stages
   uint8_t* sP = sDO + NST * G::STREAM_BYTES;   // 2 x 16 KiB
   uint8_t* sDS = sP + 2 * TILE_BYTES;          // 2 x 16 KiB
-  float* s_lse = reinterpret_cast<float*>(sDS + 2 * TILE_BYTES);   // [2][64]
-  float* s_delta = s_lse + 2 * SUB;                                // [2][64]
-  Ctl* ctl = reinterpret_cast<Ctl*>(s_delta + 2 * SUB);
+  float* s_lse = reinterpret_cast<float*>(sDS + 2 * TILE_BYTES);   // [NSTAT][64]: negated log-sum-exp (log2 units) and delta
+  float* s_delta = s_lse + NSTAT * SUB;                            // [NSTAT][64]
+  Ctl* ctl = reinterpret_cast<Ctl*>(s_delta + NSTAT * SUB);
   uint64_t* kv_full = &ctl->bars[0];
   uint64_t* q_full = &ctl->bars[1];            // [NST]
   uint64_t* q_empty = &ctl->bars[1 + NST];     // [NST]
@@ -461,6 +465,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   uint64_t* p_full = s_empty + NSB;            // [2]
   uint64_t* p_empty = p_full + 2;              // [2]
   uint64_t* acc_full = p_empty + 2;
+  uint64_t* st_full = acc_full + 1;            // [NSTAT] statistics of a sub-block's queries
 
   const int warp = bb::warp_index(), lane = threadIdx.x & 31;
   const int kb = id.tile, head = id.head, batch = id.batch;
@@ -478,6 +483,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
     for (int i = 0; i < NSB; ++i) { bb::mbar_init(&s_full[i], 1); bb::mbar_init(&s_empty[i], GROUP_THREADS / 32); }
     for (int i = 0; i < 2; ++i) { bb::mbar_init(&p_full[i], GROUP_THREADS / 32); bb::mbar_init(&p_empty[i], 1); }
     bb::mbar_init(acc_full, 1);
+    for (int i = 0; i < NSTAT; ++i) bb::mbar_init(&st_full[i], 1);
     bb::fence_barrier_init();
     bb::tma_prefetch_desc(&tm128); bb::tma_prefetch_desc(&tm64); bb::tma_prefetch_desc(&tm_do64);
   }
@@ -556,84 +562,67 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         __syncwarp();
       }
     }
+  } else if (warp == STAT_WARP) {
+    const float* lse_g = p.lse + ((long long)batch * p.H + head) * p.S;
+    const float* delta_g = p.delta + ((long long)batch * p.H + head) * p.S;
+    for (int i = 0; i < nblk; ++i) {
+      // two queries per lane; the updates of the sub-block that had the slot before have retired
+      float l2[2], d2[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int q = (qstart + i) * SUB + lane + 32 * u;
+        l2[u] = (q < p.S) ? -(lse_g[q] * LOG2E) : 0.f;
+        d2[u] = (q < p.S) ? -delta_g[q] : 0.f;
+      }
+      if (i >= NSTAT && !bb::mbar_wait_warp(&q_empty[(i - NSTAT) % NST], ((i - NSTAT) / NST) & 1, &ctl->abort_flag, p.status)) break;
+      const int st = i % NSTAT;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) { s_lse[st * SUB + lane + 32 * u] = l2[u]; s_delta[st * SUB + lane + 32 * u] = d2[u]; }
+      __syncwarp();
+      if (lane == 0) bb::mbar_arrive(&st_full[st]);
+    }
   } else {
     const int g = (warp - 2) >> 3;
     const int hf = ((warp - 2) >> 2) & 1;                  // which 32 of the sub-block's 64 query columns
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;                   // key row inside the tile
-    const int gt = threadIdx.x - 64 - GROUP_THREADS * g;   // thread index inside the group
     const int krow = k0 + row;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const float* lse_g = p.lse + ((long long)batch * p.H + head) * p.S;
-    const float* delta_g = p.delta + ((long long)batch * p.H + head) * p.S;
     const float sl = p.scale * LOG2E;
     uint8_t* myP = sP + g * TILE_BYTES;
     uint8_t* myDS = sDS + g * TILE_BYTES;
-    float* my_lse = s_lse + g * SUB;
-    float* my_delta = s_delta + g * SUB;
+    // every warp waits for itself; one that gave up goes on (its waits return at once then) and stores nothing
     bool alive = true;
     int n = 0;
-    // per-column statistics are fetched one sub-block ahead so their latency is off the critical path
-    float nx_lse = 0.f, nx_delta = 0.f;
-    if (gt < SUB && g < nblk) {
-      const int q = (qstart + g) * SUB + gt;
-      if (q < p.S) { nx_lse = lse_g[q] * LOG2E; nx_delta = delta_g[q]; }
-    }
-    for (int i = g; i < nblk && alive; i += 2, ++n) {
-      const int qc0 = (qstart + i) * SUB;
-      // (the group's previous readers are past their last use once everybody is through this barrier)
-      bb::named_bar_sync(1 + g, GROUP_THREADS);
-      if (gt < SUB) { my_lse[gt] = nx_lse; my_delta[gt] = nx_delta; }
-      bb::named_bar_sync(1 + g, GROUP_THREADS);
-      if (gt < SUB && i + 2 < nblk) {
-        const int q = (qstart + i + 2) * SUB + gt;
-        nx_lse = (q < p.S) ? lse_g[q] * LOG2E : 0.f;
-        nx_delta = (q < p.S) ? delta_g[q] : 0.f;
-      }
-      const int sb = i % NSB;
+    for (int i = g; i < nblk; i += 2, ++n) {
+      const int qc0 = (qstart + i) * SUB + hf * 32;          // first query of this thread's columns
+      const int sb = i % NSB, st = i % NSTAT;
       const uint32_t tS = tmem + 64 * sb, tDP = tmem + 64 * (NSB + sb);
-      const bool ok = bb::mbar_wait(&s_full[sb], (i / NSB) & 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok)) { alive = false; break; }
+      if (!bb::mbar_wait2_warp(&st_full[st], (i / NSTAT) & 1, &s_full[sb], (i / NSB) & 1, &ctl->abort_flag, p.status)) alive = false;
       bb::tc_fence_after_sync();
-      const bool need_mask = (qc0 + SUB > p.S) || (p.causal && k0 + TQ - 1 > qc0);
+      const float *my_lse = s_lse + st * SUB + hf * 32, *my_delta = s_delta + st * SUB + hf * 32;
       uint32_t pkP[16], pkDS[16];                            // this thread's 32 P^T and dS^T values as bf16 pairs
       {
         float sv[32], dp[32];
         ld32x2(tS + lane_addr + hf * 32, tDP + lane_addr + hf * 32, sv, dp);
-#pragma unroll
-        for (int e4 = 0; e4 < 32; e4 += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(my_lse + hf * 32 + e4);
-          const float4 d4 = *reinterpret_cast<const float4*>(my_delta + hf * 32 + e4);
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, ds[4] = {d4.x, d4.y, d4.z, d4.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int e = e4 + u;
-            float pv = ex2(fmaf(sv[e], sl, -ls[u]));
-            if (need_mask) {
-              const int q = qc0 + hf * 32 + e;
-              if (q >= p.S || (p.causal && krow > q)) pv = 0.f;
-            }
-            sv[e] = pv;
-            dp[e] = pv * (dp[e] - ds[u]);
-          }
-        }
-        pack32(sv, pkP);
-        pack32(dp, pkDS);
+        bb::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) bb::mbar_arrive(&s_empty[sb]);
+        if (qc0 + 32 > p.S || (p.causal && k0 + TQ - 1 > qc0))
+          dkv_math<true>(sv, dp, my_lse, my_delta, sl, p.causal ? krow - qc0 : 0, p.S - 1 - qc0, pkP, pkDS);
+        else
+          dkv_math<false>(sv, dp, my_lse, my_delta, sl, 0, 0, pkP, pkDS);
       }
-      bb::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) bb::mbar_arrive(&s_empty[sb]);
       // the staging buffers are free once the dV / dK update that read them retired
-      const bool ok2 = bb::mbar_wait(&p_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status);
-      if (!bb::named_bar_all(3 + g, GROUP_THREADS, ok2)) { alive = false; break; }
+      if (!bb::mbar_wait_warp(&p_empty[g], (n & 1) ^ 1, &ctl->abort_flag, p.status)) alive = false;
       atom_store_half_row(myP, row, hf, pkP);
       atom_store_half_row(myDS, row, hf, pkDS);
       bb::fence_proxy_async();
       __syncwarp();
       if (lane == 0) bb::mbar_arrive(&p_full[g]);
     }
-    const bool fin = alive && nblk > 0 && bb::mbar_wait(acc_full, 0, &ctl->abort_flag, p.status);
-    if (bb::named_bar_all(3 + g, GROUP_THREADS, fin)) {
+    if (!bb::mbar_wait_warp(acc_full, 0, &ctl->abort_flag, p.status)) alive = false;
+    if (alive) {
       bb::tc_fence_after_sync();
       // the two groups split the final stores: group 0 writes dV, group 1 writes dK
       const uint32_t src = (g == 0) ? tDV : tDK;
@@ -653,7 +642,7 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
 }
 
 template <int D> constexpr int dkv2_smem() {
-  return 2 * Bwd2<D>::OWN_BYTES + 2 * Bwd2<D>::NST * Bwd2<D>::STREAM_BYTES + 4 * TILE_BYTES + 4 * SUB * (int)sizeof(float) + (int)sizeof(Ctl) + 1024;
+  return 2 * Bwd2<D>::OWN_BYTES + 2 * Bwd2<D>::NST * Bwd2<D>::STREAM_BYTES + 4 * TILE_BYTES + 2 * NSTAT * SUB * (int)sizeof(float) + (int)sizeof(Ctl) + 1024;
 }
 
 // Both backward roles in one launch: of the 2 * nbx CTAs of a (batch, head), the first nbx own a
@@ -690,7 +679,6 @@ attn_tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
 // smem: K, V [128 x 64] | Q, dO sub-tiles x NST3 | P^T x 2 | dS^T x 2 pair slots x 2 groups | dQ staging 16 x 2 KiB | lse / delta
 // TMEM: S^T 2 x 64 | dP^T 2 x 64 | dV 64 | dK 64 | dQ 2 x 64
 constexpr int NST3 = 4;
-constexpr int NSTAT = 3;                         // depth of the ring of query statistics
 // warps: 0 TMA, 1 score products (S^T, dP^T), 2 updates (dV, dK, dQ), 3 the queries' log-sum-exp and delta, 4..19 the two
 // compute groups (compute warp w must sit at w % 4 == its tensor-memory lane quarter).  Fetched and staged by the compute
 // groups themselves, the statistics cost two group-wide barriers per sub-block: B8 H16 S1024 causal 175 -> 171 us,

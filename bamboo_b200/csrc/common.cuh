@@ -197,6 +197,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, status));
 }
 
+// The same for two barriers: their first tests are in flight together.
+__device__ __forceinline__ bool mbar_wait2_warp(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, volatile int* abort, int* status) {
+  const bool oa = mbar_try_wait(a, pa), ob = mbar_try_wait(b, pb);
+  if (__all_sync(0xffffffffu, oa && ob)) return true;
+  const bool ra = mbar_wait(a, pa, abort, status), rb = mbar_wait(b, pb, abort, status);
+  return __all_sync(0xffffffffu, ra && rb);
+}
+
 // Bounded wait with cluster-scope acquire: for barriers that another CTA of the cluster arrives on
 // after writing this CTA's shared memory with plain stores (st.shared::cluster).
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort, int* status) {

@@ -225,8 +225,10 @@ constexpr int SUB_BYTES = SUB * HD * 2;          // 8 KiB: [64 x 64] bf16
 // reductions here, and four compute warps per scheduler hide the TMEM-load and ALU latencies that
 // two could not (issue slots were 35 % busy with 4-warp groups).
 constexpr int GROUP_THREADS = 256;
-constexpr int NT2 = 64 + 2 * GROUP_THREADS + 32;     // the last warp stages the queries' statistics (dK / dV role)
-constexpr int STAT_WARP = 2 + 2 * GROUP_THREADS / 32;
+// warps: 0 TMA, 1 score products, 2..17 compute, 18 the queries' statistics (dK / dV role), 19 updates (a second issuing thread, so
+// that the scores of the next sub-blocks never queue behind a wait for staged operands)
+constexpr int NT2 = 64 + 2 * GROUP_THREADS + 64;
+constexpr int STAT_WARP = 2 + 2 * GROUP_THREADS / 32, UPD_WARP = STAT_WARP + 1;
 constexpr int NSTAT = 3;                         // depth of the ring of query statistics
 
 // Geometry of the two-role backward at head dimension D.  A [rows x 128] operand is two [rows x 64] atoms of
@@ -326,41 +328,40 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
   } else if (warp == 1) {
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));     // stage 0; stage s: + s * STREAM_BYTES / 16
-    const uint64_t dKm0 = desc_mn0(bb::smem_u32(sK)), dDS0 = desc_k0(bb::smem_u32(sDS));
-    const uint32_t i_s = idesc(64, 0, 0), i_dq = idesc(D, 0, 1);
+    const uint32_t i_s = idesc(64, 0, 0);
     bool alive = bb::mbar_wait_warp(q_full, 0, &ctl->abort_flag, p.status);
-    // software pipeline: the scores run two sub-blocks ahead of the dQ updates
-    for (int j = 0; j < nblk + 2 && alive; ++j) {
-      if (j < nblk) {
-        const int s = j % NST, b = j % NSB;
-        if (!bb::mbar_wait_warp(&kv_full[s], (j / NST) & 1, &ctl->abort_flag, p.status)) break;
-        if (!bb::mbar_wait_warp(&s_empty[b], ((j / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
-        bb::tc_fence_after_sync();
-        if (bb::elect_one()) {
-          const uint64_t dK = dK0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dV = dV0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
+    for (int j = 0; j < nblk && alive; ++j) {
+      const int s = j % NST, b = j % NSB;
+      if (!bb::mbar_wait2_warp(&kv_full[s], (j / NST) & 1, &s_empty[b], ((j / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      bb::tc_fence_after_sync();
+      if (bb::elect_one()) {
+        const uint64_t dK = dK0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dV = dV0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
-            bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dQ0, k, TILE_BYTES), desc_kmajor_atoms(dK, k, SUB_BYTES), i_s, k > 0);
-            bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dDO0, k, TILE_BYTES), desc_kmajor_atoms(dV, k, SUB_BYTES), i_s, k > 0);
-          }
-          bb::umma_commit(&s_full[b]);
+        for (int k = 0; k < D / 16; ++k) {
+          bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dQ0, k, TILE_BYTES), desc_kmajor_atoms(dK, k, SUB_BYTES), i_s, k > 0);
+          bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dDO0, k, TILE_BYTES), desc_kmajor_atoms(dV, k, SUB_BYTES), i_s, k > 0);
         }
-        __syncwarp();
+        bb::umma_commit(&s_full[b]);
       }
-      if (j >= 2) {
-        const int jj = j - 2, s2 = jj % NST, b2 = jj & 1;
-        if (!bb::mbar_wait_warp(&ds_full[b2], (jj >> 1) & 1, &ctl->abort_flag, p.status)) break;
-        bb::tc_fence_after_sync();
-        if (bb::elect_one()) {
-          const uint64_t dK2 = dKm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
+      __syncwarp();
+    }
+  } else if (warp == UPD_WARP) {
+    const uint64_t dKm0 = desc_mn0(bb::smem_u32(sK)), dDS0 = desc_k0(bb::smem_u32(sDS));
+    const uint32_t i_dq = idesc(D, 0, 1);
+    for (int jj = 0; jj < nblk; ++jj) {
+      const int s2 = jj % NST, b2 = jj & 1;
+      // (the sub-tiles landed long ago - the score products read them; the wait makes them visible to this thread)
+      if (!bb::mbar_wait2_warp(&kv_full[s2], (jj / NST) & 1, &ds_full[b2], (jj >> 1) & 1, &ctl->abort_flag, p.status)) break;
+      bb::tc_fence_after_sync();
+      if (bb::elect_one()) {
+        const uint64_t dK2 = dKm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) bb::umma_f16(tDQ, desc_kmajor(dDS, k), desc_mnmajor64(dK2, k), i_dq, (jj > 0 || k > 0));
-          bb::umma_commit(&ds_empty[b2]);
-          bb::umma_commit(&kv_empty[s2]);
-          if (jj == nblk - 1) bb::umma_commit(acc_full);
-        }
-        __syncwarp();
+        for (int k = 0; k < 4; ++k) bb::umma_f16(tDQ, desc_kmajor(dDS, k), desc_mnmajor64(dK2, k), i_dq, (jj > 0 || k > 0));
+        bb::umma_commit(&ds_empty[b2]);
+        bb::umma_commit(&kv_empty[s2]);
+        if (jj == nblk - 1) bb::umma_commit(acc_full);
       }
+      __syncwarp();
     }
   } else if (warp != STAT_WARP) {
     const int g = (warp - 2) >> 3;                           // compute group = buffer index
@@ -521,46 +522,45 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
   } else if (warp == 1) {
     const uint64_t dK0 = desc_k0(bb::smem_u32(sK)), dV0 = desc_k0(bb::smem_u32(sV));
     const uint64_t dQ0 = desc_k0(bb::smem_u32(sQ)), dDO0 = desc_k0(bb::smem_u32(sDO));   // stage 0; stage s: + s * STREAM_BYTES / 16
+    const uint32_t i_s = idesc(64, 0, 0);
+    bool alive = bb::mbar_wait_warp(kv_full, 0, &ctl->abort_flag, p.status);
+    for (int i = 0; i < nblk && alive; ++i) {
+      const int s = i % NST, b = i % NSB;
+      if (!bb::mbar_wait2_warp(&q_full[s], (i / NST) & 1, &s_empty[b], ((i / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
+      bb::tc_fence_after_sync();
+      if (bb::elect_one()) {
+        const uint64_t dQ = dQ0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dK0, k, TILE_BYTES), desc_kmajor_atoms(dQ, k, SUB_BYTES), i_s, k > 0);
+          bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dV0, k, TILE_BYTES), desc_kmajor_atoms(dDO, k, SUB_BYTES), i_s, k > 0);
+        }
+        bb::umma_commit(&s_full[b]);
+      }
+      __syncwarp();
+    }
+  } else if (warp == UPD_WARP) {
     const uint64_t dQm0 = desc_mn0(bb::smem_u32(sQ)), dDOm0 = desc_mn0(bb::smem_u32(sDO));
     const uint64_t dP0 = desc_k0(bb::smem_u32(sP)), dDS0 = desc_k0(bb::smem_u32(sDS));
-    const uint32_t i_s = idesc(64, 0, 0), i_acc = idesc(D, 0, 1);
-    bool alive = bb::mbar_wait_warp(kv_full, 0, &ctl->abort_flag, p.status);
-    // the score products run two sub-blocks ahead of the dV / dK updates
-    for (int i = 0; i < nblk + 2 && alive; ++i) {
-      if (i < nblk) {
-        const int s = i % NST, b = i % NSB;
-        if (!bb::mbar_wait_warp(&q_full[s], (i / NST) & 1, &ctl->abort_flag, p.status)) break;
-        if (!bb::mbar_wait_warp(&s_empty[b], ((i / NSB) & 1) ^ 1, &ctl->abort_flag, p.status)) break;
-        bb::tc_fence_after_sync();
-        if (bb::elect_one()) {
-          const uint64_t dQ = dQ0 + (uint64_t)(s * (G::STREAM_BYTES >> 4)), dDO = dDO0 + (uint64_t)(s * (G::STREAM_BYTES >> 4));
+    const uint32_t i_acc = idesc(D, 0, 1);
+    for (int ii = 0; ii < nblk; ++ii) {
+      const int s2 = ii % NST, b2 = ii & 1;
+      // (the sub-tiles landed long ago - the score products read them; the wait makes them visible to this thread)
+      if (!bb::mbar_wait2_warp(&q_full[s2], (ii / NST) & 1, &p_full[b2], (ii >> 1) & 1, &ctl->abort_flag, p.status)) break;
+      bb::tc_fence_after_sync();
+      if (bb::elect_one()) {
+        const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4));
+        const uint64_t dP = dP0 + (uint64_t)(b2 * (TILE_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
-            bb::umma_f16(tmem + 64 * b, desc_kmajor_atoms(dK0, k, TILE_BYTES), desc_kmajor_atoms(dQ, k, SUB_BYTES), i_s, k > 0);
-            bb::umma_f16(tmem + 64 * (NSB + b), desc_kmajor_atoms(dV0, k, TILE_BYTES), desc_kmajor_atoms(dDO, k, SUB_BYTES), i_s, k > 0);
-          }
-          bb::umma_commit(&s_full[b]);
+        for (int k = 0; k < 4; ++k) {
+          bb::umma_f16(tDV, desc_kmajor(dP, k), desc_mnmajor64(dDO2, k), i_acc, (ii > 0 || k > 0));
+          bb::umma_f16(tDK, desc_kmajor(dDS, k), desc_mnmajor64(dQ2, k), i_acc, (ii > 0 || k > 0));
         }
-        __syncwarp();
+        bb::umma_commit(&p_empty[b2]);
+        bb::umma_commit(&q_empty[s2]);
+        if (ii == nblk - 1) bb::umma_commit(acc_full);
       }
-      if (i >= 2) {
-        const int ii = i - 2, s2 = ii % NST, b2 = ii & 1;
-        if (!bb::mbar_wait_warp(&p_full[b2], (ii >> 1) & 1, &ctl->abort_flag, p.status)) break;
-        bb::tc_fence_after_sync();
-        if (bb::elect_one()) {
-          const uint64_t dQ2 = dQm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4)), dDO2 = dDOm0 + (uint64_t)(s2 * (G::STREAM_BYTES >> 4));
-          const uint64_t dP = dP0 + (uint64_t)(b2 * (TILE_BYTES >> 4)), dDS = dDS0 + (uint64_t)(b2 * (TILE_BYTES >> 4));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            bb::umma_f16(tDV, desc_kmajor(dP, k), desc_mnmajor64(dDO2, k), i_acc, (ii > 0 || k > 0));
-            bb::umma_f16(tDK, desc_kmajor(dDS, k), desc_mnmajor64(dQ2, k), i_acc, (ii > 0 || k > 0));
-          }
-          bb::umma_commit(&p_empty[b2]);
-          bb::umma_commit(&q_empty[s2]);
-          if (ii == nblk - 1) bb::umma_commit(acc_full);
-        }
-        __syncwarp();
-      }
+      __syncwarp();
     }
   } else if (warp == STAT_WARP) {
     const float* lse_g = p.lse + ((long long)batch * p.H + head) * p.S;
@@ -649,6 +649,8 @@ template <int D> constexpr int dkv2_smem() {
 // key tile (dK, dV) and the rest a query tile (dQ), each role's longest first.  The two roles are independent, so the
 // tail of one fills with CTAs of the other instead of leaving SMs idle between two launches.  (Roles taken in turn
 // were slower: 538 us against 503 us at B2 H32 S2048 D128 causal.)
+// B2 H32 S2048 D128 causal, step by step: 479 us with one issuing warp, group barriers around every hand-off and scalar arithmetic;
+// 447 with two-wide arithmetic and warps that wait for themselves; 331 with a second issuing warp.
 template <int D> constexpr int bwd2_smem() { return dkv2_smem<D>() > dq2_smem<D>() ? dkv2_smem<D>() : dq2_smem<D>(); }
 static_assert(bwd2_smem<64>() <= 232448 && bwd2_smem<128>() <= 232448, "227 KiB of shared memory per CTA");
 template <int D>

@@ -509,6 +509,32 @@ __device__ __forceinline__ bool issue_mmas(const GemmParams& p, uint8_t* sA, uin
   return true;
 }
 
+// Fused math and stores of 32 rows x 32 columns of a bf16 output, one accumulator row per lane; the aux operand, where the
+// epilogue has one, is in the slab already.
+__device__ __forceinline__ void narrow_panel(const GemmParams& p, uint8_t* slab, int r0, int nb, int lane, float* v) {
+  const int epi = p.epi;
+  const bool dual = (epi == BB_EPI_BIAS_GELU), has_aux = (epi == BB_EPI_MUL_DGELU || epi == BB_EPI_BIAS_RESIDUAL);
+  if (epi == BB_EPI_BIAS || dual || epi == BB_EPI_BIAS_RESIDUAL) add_bias<32>(p, nb, v);
+  if (dual) {
+    slab64_store_row(slab, lane, v);           // pre-activation first
+    __syncwarp();
+    slab64_flush(slab, reinterpret_cast<__nv_bfloat16*>(p.D2), p.ldd, r0, nb, p.M, p.N, lane);
+    gelu_rounded<32>(v);
+    __syncwarp();
+  } else if (has_aux) {
+    __syncwarp();
+    float x[32];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) unpack8(*reinterpret_cast<const uint4*>(slab + slab64_off(lane, c)), x + 8 * c);
+    apply_aux<32>(epi, v, x);
+    __syncwarp();
+  }
+  slab64_store_row(slab, lane, v);
+  __syncwarp();
+  slab64_flush(slab, reinterpret_cast<__nv_bfloat16*>(p.D), p.ldd, r0, nb, p.M, p.N, lane);
+  __syncwarp();
+}
+
 template <int BN, bool PAIR, int EW, bool CONV>
 __global__ void __launch_bounds__(num_threads(EW), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -732,25 +758,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             }
           }
           if (!some) continue;
-          if (epi == BB_EPI_BIAS || dual || epi == BB_EPI_BIAS_RESIDUAL) add_bias<32>(p, nb, v);
-          if (dual) {
-            slab64_store_row(slab, lane, v);           // pre-activation first
-            __syncwarp();
-            slab64_flush(slab, reinterpret_cast<__nv_bfloat16*>(p.D2), p.ldd, r0, nb, p.M, p.N, lane);
-            gelu_rounded<32>(v);
-            __syncwarp();
-          } else if (has_aux) {
-            __syncwarp();
-            float x[32];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) unpack8(*reinterpret_cast<const uint4*>(slab + slab64_off(lane, c)), x + 8 * c);
-            apply_aux<32>(epi, v, x);
-            __syncwarp();
-          }
-          slab64_store_row(slab, lane, v);
-          __syncwarp();
-          slab64_flush(slab, reinterpret_cast<__nv_bfloat16*>(p.D), p.ldd, r0, nb, p.M, p.N, lane);
-          __syncwarp();
+          narrow_panel(p, slab, r0, nb, lane, v);
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
@@ -852,6 +860,177 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
 }
 
+// ---------------------------------------------------------------- reduction split inside a cluster
+// Products of few output tiles and a long reduction: S CTAs (or CTA pairs) of one cluster share a tile's reduction, each over its
+// own k-blocks.  What bounds such a product is the latency of its operands: six stages in flight give an SM about 80 bytes a
+// clock, a k-block of a 128 x 256 tile takes 0.3 us however idle the rest of the GPU is - so the reduction goes to SMs that would
+// be idle.  The partial sums meet in fp32 through distributed shared memory: the tile's 32-column panels are dealt out to
+// the splits, each split writes its sums of the others' panels into their (by then unused) operand stages and adds what it
+// received to its own panels in the order of the splits: a fixed order, no global scratch, no counters.  One tile per cluster.
+// Receive buffers: [owned panel][other split] x 16 KiB = [quarter][16-byte chunk of the row][row], so that a warp's store
+// is 512 contiguous bytes.
+constexpr int SPLIT_EW = 4;                       // epilogue warps per TMEM lane quarter
+constexpr int split_limit(bool pair) { return pair ? 4 : 8; }        // a cluster of eight CTAs
+// receive buffers of the split that owns most panels
+constexpr int split_buffers(int bn, bool pair) {
+  int most = 0;
+  for (int s = 2; s <= split_limit(pair); ++s) {
+    const int n = (bn / 32 + s - 1) / s * (s - 1);
+    if (n > most) most = n;
+  }
+  return most;
+}
+static_assert(split_buffers(128, false) * (BM * 32 * 4) <= Cfg<128, false>::STAGES * Cfg<128, false>::STAGE_BYTES &&
+              split_buffers(256, false) * (BM * 32 * 4) <= Cfg<256, false>::STAGES * Cfg<256, false>::STAGE_BYTES &&
+              split_buffers(256, true) * (BM * 32 * 4) <= Cfg<256, true>::STAGES * Cfg<256, true>::STAGE_BYTES,
+              "receive buffers fit the operand stages");
+
+template <int BN, bool PAIR, bool CONV>
+__global__ void __launch_bounds__(num_threads(SPLIT_EW), 1)
+gemm_cluster_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                          const GemmParams p, const typename ConvArg<CONV>::type cv) {
+  using C = Cfg<BN, PAIR>;
+  constexpr int PC = PAIR ? 2 : 1;                // CTAs per split
+  constexpr int NP = BN / 32;                     // panels of a tile
+  constexpr int PANEL_BYTES = BM * 32 * 4;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + C::STAGES * A_STAGE_BYTES;
+  uint8_t* panels = smem + C::STAGES * C::STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(panels + NUM_SLABS * SLAB_BYTES);
+  uint64_t* full_bar = bars;                      // [STAGES]
+  uint64_t* empty_bar = bars + C::STAGES;         // [STAGES]
+  uint64_t* tmem_full = bars + 2 * C::STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = bb::warp_index();
+  const int lane = threadIdx.x & 31;
+  const uint32_t crank = bb::cluster_ctarank();
+  const uint32_t rank = PAIR ? (crank & 1u) : 0u, lead = crank - rank;
+  const int S = p.ksplit, ks = (int)crank / PC;
+  const int total_kb = (p.K + BK - 1) / BK;
+  int mi, ni, unused;
+  unit_coords(p, (int)bb::cluster_id(), mi, ni, unused);
+  const int m0 = mi * C::TILE_M + (int)rank * BM, n0 = ni * BN;
+  const int kb0 = ks * p.kb_per_split, kb1 = min(total_kb, kb0 + p.kb_per_split);
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < C::STAGES; ++s) { bb::mbar_init(&full_bar[s], 1); bb::mbar_init(&empty_bar[s], 1); }
+    bb::mbar_init(tmem_full, 1);
+    bb::fence_barrier_init();
+    bb::tma_prefetch_desc(&tmA);
+    bb::tma_prefetch_desc(&tmB);
+  }
+  if (warp == MMA_WARP) {
+    if (PAIR) { bb::tmem_alloc_pair(tmem_slot, BN); bb::tmem_relinquish_pair(); }
+    else { bb::tmem_alloc(tmem_slot, BN); bb::tmem_relinquish(); }
+  }
+  bb::tc_fence_before_sync();
+  if (PAIR) bb::cluster_sync();     // the peer's barriers are initialised before anything signals them
+  else __syncthreads();
+  bb::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  bb::pdl_sync();
+
+  const int eg = (warp - EPI_WARP) >> 2, quarter = warp & 3;
+  const int r0 = m0 + quarter * 32;
+  const bool has_aux = (p.epi == BB_EPI_MUL_DGELU || p.epi == BB_EPI_BIAS_RESIDUAL);
+  const int first = ks + eg * S;                            // this warp's first own panel; the next is SPLIT_EW * S further
+  uint8_t* slab = panels + (warp - EPI_WARP) * (SLAB_BYTES / 2);
+  bool summed = false;
+  if (warp == TMA_WARP_0 || warp == TMA_WARP_1) {
+    const int turn = warp == TMA_WARP_1 ? 1 : 0;
+    int s = 0; uint32_t phase = 0;
+    bool alive = load_operands<BN, PAIR, CONV>(tmA, tmB, p, cv, sA, sB, full_bar, empty_bar, abort_flag, rank, lead, m0,
+                                               n0 + (int)rank * C::B_ROWS, kb0, kb1, turn, s, phase);
+    if constexpr (PAIR) {
+      // the commits that free a stage arrive in both CTAs: none may still be on its way when the CTA leaves
+      for (int i = 0; i < C::STAGES && alive; ++i) {
+        if ((s & 1) == turn && !bb::mbar_wait_warp(&empty_bar[s], phase ^ 1, abort_flag, p.status)) alive = false;
+        if (++s == C::STAGES) { s = 0; phase ^= 1; }
+      }
+    }
+    if (!alive) {
+      // copies still in flight get time to land (bounded)
+      uint64_t t0 = bb::globaltimer_ns();
+      while (bb::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    }
+  } else if (warp == MMA_WARP) {
+    if (rank == 0) {
+      int s = 0; uint32_t phase = 0;
+      issue_mmas<BN, PAIR>(p, sA, sB, full_bar, empty_bar, tmem_full, abort_flag, (uint16_t)(3u << lead), tmem_base, kb1 - kb0, s, phase);
+    }
+  } else {
+    // the aux operand of the first own panel is fetched under the main loop
+    if (has_aux && first < NP && n0 + first * 32 < p.N && r0 < p.M)
+      slab64_fetch(slab, reinterpret_cast<const __nv_bfloat16*>(p.aux), p.ld_aux, r0, n0 + first * 32, p.M, p.N, lane);
+    summed = bb::mbar_wait_warp(tmem_full, 0, abort_flag, p.status);
+    bb::tc_fence_after_sync();
+  }
+  __syncwarp();
+  // every CTA's MMAs have retired, so its operand stages can receive (and all of its copies have landed)
+  bb::cluster_sync();
+  const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
+  if (summed && r0 < p.M) {
+    int turn = 0;
+    for (int i = 1; i < S; ++i) {                           // the splits start with different owners
+      const int owner = ks + i < S ? ks + i : ks + i - S;
+      int slot = ks < owner ? ks : ks - 1;
+      for (int pn = owner; pn < NP; pn += S, slot += S - 1) {
+        if ((turn++ & (SPLIT_EW - 1)) != eg || n0 + pn * 32 >= p.N) continue;
+        uint32_t r[32];
+        bb::tmem_ld_32x32b_x32(t_row + pn * 32, r);
+        bb::tmem_ld_wait();
+        const uint32_t dst = bb::mapa_shared(bb::smem_u32(smem) + slot * PANEL_BYTES + quarter * 4096 + lane * 16, owner * PC + rank);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bb::st_shared_cluster_v4(dst + j * 512, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+      }
+    }
+  }
+  __syncwarp();
+  bb::cluster_sync();
+  if (summed && r0 < p.M) {
+    const uint8_t* part = smem + eg * (S - 1) * PANEL_BYTES + quarter * 4096 + lane * 16;
+    for (int pn = first; pn < NP; pn += SPLIT_EW * S, part += SPLIT_EW * (S - 1) * PANEL_BYTES) {
+      const int nb = n0 + pn * 32;
+      if (nb >= p.N) break;
+      if (has_aux && pn != first) slab64_fetch(slab, reinterpret_cast<const __nv_bfloat16*>(p.aux), p.ld_aux, r0, nb, p.M, p.N, lane);
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0.f;
+      for (int t = 0; t < S; ++t) {
+        if (t == ks) {
+          uint32_t r[32];
+          bb::tmem_ld_32x32b_x32(t_row + pn * 32, r);
+          bb::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r[i]);
+        } else {
+          const uint8_t* q0 = part + (t < ks ? t : t - 1) * PANEL_BYTES;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 q = *reinterpret_cast<const float4*>(q0 + j * 512);
+            v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+          }
+        }
+      }
+      narrow_panel(p, slab, r0, nb, lane, v);
+    }
+  }
+  bb::tc_fence_before_sync();
+  __syncwarp();
+  if (PAIR) {
+    bb::cluster_sync();
+    if (warp == MMA_WARP) bb::tmem_dealloc_pair(tmem_base, BN);
+  } else {
+    __syncthreads();
+    if (warp == MMA_WARP) bb::tmem_dealloc(tmem_base, BN);
+  }
+}
+
 // ---------------------------------------------------------------- host side
 using bbhost::encode_2d;
 
@@ -904,11 +1083,12 @@ int wave_split(int mn_tiles, int workers, int total_kb) {
   return ksplit;
 }
 
+// Tensor maps and launch parameters of a product, except for the split of its reduction and the ticket counter.
 // `cv`: convolution product (CONV); the descriptor then holds the sizes and the operand that is no patch matrix
-template <int BN, bool PAIR, int EW, bool CONV>
-int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* cv = nullptr) {
+template <int BN, bool PAIR, bool CONV>
+int operands(const bb_gemm_desc* g, const bb_conv_gemm_args* cv, CUtensorMap& tmA, CUtensorMap& tmB, GemmParams& p,
+             typename ConvArg<CONV>::type& cp) {
   using C = Cfg<BN, PAIR>;
-  CUtensorMap tmA, tmB;
   int rc;
   if (CONV && cv->mode != BB_CONV_WGRAD) rc = bbhost::encode_im2col(&tmA, cv->x, cv->N, cv->H, cv->W, cv->C, cv->k, cv->stride, cv->pad, BM);
   else if (!g->a_mn_major) rc = encode_2d(&tmA, g->A, g->M, g->K, g->lda, BK, BM);
@@ -919,7 +1099,6 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   else if (!g->b_mn_major) rc = encode_2d(&tmB, g->B, g->N, g->K, g->ldb, BK, C::B_ROWS);
   else rc = encode_2d(&tmB, g->B, g->K, g->N, g->ldb, 64, BK);
   if (rc) return rc;
-  typename ConvArg<CONV>::type cp;
   if constexpr (CONV) {
     cp.mode = cv->mode; cp.k = cv->k; cp.stride = cv->stride; cp.pad = cv->pad; cp.cblocks = cv->C / 64;
     cp.wcols = cv->mode == BB_CONV_DGRAD ? cv->other_channels : cv->C;
@@ -927,7 +1106,6 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
     cp.magic_w = bb_div_magic(cv->Wo);
     cp.magic_h = bb_div_magic(cv->Ho);
   }
-  GemmParams p;
   p.M = g->M; p.N = g->N; p.K = g->K; p.a_mn = g->a_mn_major; p.b_mn = g->b_mn_major; p.epi = g->epilogue;
   p.D = g->D; p.D2 = g->D2; p.bias = g->bias; p.aux = g->aux; p.ldd = g->ldd; p.ld_aux = g->ld_aux ? g->ld_aux : g->ldd;
   p.status = bb_device_status_word();
@@ -937,6 +1115,17 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   const int num_m = (g->M + C::TILE_M - 1) / C::TILE_M, num_n = (g->N + BN - 1) / BN;
   p.tiles_in = p.n_fast ? num_n : num_m; p.tiles_mn = (unsigned)num_m * (unsigned)num_n;
   p.magic_in = bb_div_magic((int)p.tiles_in); p.magic_mn = bb_div_magic((int)p.tiles_mn);
+  p.dynamic = 0; p.ticket = nullptr; p.ticket_base = 0;
+  return BB_OK;
+}
+
+template <int BN, bool PAIR, int EW, bool CONV>
+int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* cv = nullptr) {
+  using C = Cfg<BN, PAIR>;
+  CUtensorMap tmA, tmB;
+  GemmParams p;
+  typename ConvArg<CONV>::type cp;
+  if (int rc = operands<BN, PAIR, CONV>(g, cv, tmA, tmB, p, cp)) return rc;
   const int total_kb = (g->K + BK - 1) / BK;
   const int mn_tiles = ((g->M + C::TILE_M - 1) / C::TILE_M) * ((g->N + BN - 1) / BN);
   const int workers_max = PAIR ? bb_num_sms() / 2 : bb_num_sms();
@@ -963,7 +1152,6 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   // of the main stream launched meanwhile waits for that SM with a fixed share of the tiles.
   if (g->max_ctas < 0) workers = tiles;
   // more units than CTAs: every unit after a CTA's first is drawn from this launch's ticket counter
-  p.dynamic = 0; p.ticket = nullptr; p.ticket_base = 0;
   unsigned slot = 0;
   TicketTable* tt = nullptr;
   if (tiles > workers && !g_static_schedule) {
@@ -999,6 +1187,40 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
       return BB_ERR_CUDA;
     }
   }
+  return BB_OK;
+}
+
+template <int BN, bool PAIR, bool CONV>
+cudaLaunchConfig_t split_config(int splits, int tiles, cudaLaunchAttribute* attr) {
+  const int cluster = splits * (PAIR ? 2 : 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster * tiles); cfg.blockDim = dim3(num_threads(SPLIT_EW)); cfg.dynamicSmemBytes = Cfg<BN, PAIR>::SMEM_BYTES;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cfg;
+}
+
+// The same product with its reduction split over the CTAs of a cluster (gemm_cluster_split_kernel)
+template <int BN, bool PAIR, bool CONV>
+int launch_split(const bb_gemm_desc* g, cudaStream_t stream, int splits, const bb_conv_gemm_args* cv = nullptr) {
+  using C = Cfg<BN, PAIR>;
+  CUtensorMap tmA, tmB;
+  GemmParams p;
+  typename ConvArg<CONV>::type cp;
+  if (int rc = operands<BN, PAIR, CONV>(g, cv, tmA, tmB, p, cp)) return rc;
+  const int total_kb = (g->K + BK - 1) / BK;
+  if (splits > split_limit(PAIR)) splits = split_limit(PAIR);
+  if (splits > total_kb) splits = total_kb;
+  p.kb_per_split = (total_kb + splits - 1) / splits;
+  p.ksplit = (total_kb + p.kb_per_split - 1) / p.kb_per_split;   // no empty splits
+  BB_ONCE_PER_DEVICE(BB_CUDA_CHECK(cudaFuncSetAttribute(gemm_cluster_split_kernel<BN, PAIR, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES)));
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = split_config<BN, PAIR, CONV>(p.ksplit, (int)p.tiles_mn, attr);
+  cfg.stream = stream;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
+  if (bb_back_to_back > 0) cfg.numAttrs = 2;
+  BB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_cluster_split_kernel<BN, PAIR, CONV>, tmA, tmB, p, cp));
   return BB_OK;
 }
 
@@ -1065,7 +1287,7 @@ AccumPlan plan_accum(int M, int N, int K) {
 // tenth on average and the choice is the quickest of the three every time.  Constants from before the pairs' hand-backs became
 // cheap kept 8192 x 4096 x 1024 (bias + GeLU 66.5 us, as pairs 57.2), 8192 x 3072 x 1024 (47.4, 42.7), 2331 x 4096 x 1024 (31.1, 27.8)
 // and 8192 x 50304 x 1024 (648, 564) on single CTAs.
-struct StorePlan { int bn; bool pair; double us; };
+struct StorePlan { int bn; bool pair; double us; int splits = 0; };
 StorePlan plan_store(long long M, long long N, long long K, int max_ctas, bool pairs_allowed) {
   static const struct { int bn; bool pair; double kblock, wave, once; } kinds[3] = {
       {256, true, 0.32, 1.9, 5.0}, {256, false, 0.375, 1.8, 3.7}, {128, false, 0.283, 1.0, 3.7}};
@@ -1080,6 +1302,54 @@ StorePlan plan_store(long long M, long long N, long long K, int max_ctas, bool p
     if (k.pair) workers = workers > 1 ? workers / 2 : 1;
     const double us = (double)((tiles + workers - 1) / workers) * (kb * k.kblock + k.wave) + k.once;
     if (best.us < 0 || us < best.us) best = {k.bn, k.pair, us};
+  }
+  return best;
+}
+
+// Clusters of `cluster` CTAs of the split kernel that the device holds at the same time (GPCs are not multiples of every cluster
+// size); 0 when it cannot be asked.
+template <int BN, bool PAIR>
+int clusters_at_once(int splits) {
+  static std::atomic<int> cache[64][9];
+  const int dev = bb_current_device();
+  if (dev < 0) return 0;
+  int n = cache[dev][splits].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = split_config<BN, PAIR, false>(splits, 1, attr);
+    if (cudaFuncSetAttribute(gemm_cluster_split_kernel<BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, PAIR>::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_cluster_split_kernel<BN, PAIR, false>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    if (n <= 0) n = -1;
+    cache[dev][splits].store(n, std::memory_order_relaxed);
+  }
+  return n > 0 ? n : 0;
+}
+
+// The plan with the reduction split over a cluster where that is expected to be quicker by a twentieth: one wave of clusters, every
+// split with four k-blocks or more.  The exchange costs about half a microsecond per split on top of a launch
+// (once + step x splits; us, unsplit / split: 513 x 2048 x 8192 41.7 / 25.5 as three splits of 256 columns, 128 x 1024 x 4096
+// 20.9 / 9.9 as six of 128, 1000 x 512 x 2048 12.9 / 9.0 as four, 1568 x 512 x 4608 24.8 / 16.0, 512 x 256 x 1024 8.2 / 7.1; with K = 512
+// and less, or tiles for more than half of the SMs, nothing is gained).
+StorePlan plan_split(long long M, long long N, long long K) {
+  static const struct { int bn; bool pair; double kblock, once, step; } kinds[3] = {
+      {256, true, 0.32, 7.2, 0.95}, {256, false, 0.375, 6.2, 0.6}, {128, false, 0.283, 4.7, 0.45}};
+  const StorePlan whole = plan_store(M, N, K, 0, true);
+  StorePlan best = whole;
+  const long long kb = (K + BK - 1) / BK;
+  for (const auto& k : kinds) {
+    if ((k.bn == 256 && N <= 128) || (k.pair && M <= BM)) continue;
+    const long long tm = k.pair ? 2 * BM : BM;
+    const long long tiles = ((M + tm - 1) / tm) * ((N + k.bn - 1) / k.bn);
+    for (int sp = 2; sp <= split_limit(k.pair) && kb / sp >= 4; ++sp) {
+      if (tiles * sp * (k.pair ? 2 : 1) > bb_num_sms()) break;
+      const int at_once = k.pair ? clusters_at_once<256, true>(sp) : k.bn == 256 ? clusters_at_once<256, false>(sp) : clusters_at_once<128, false>(sp);
+      if (tiles > at_once) continue;
+      const double us = (double)((kb + sp - 1) / sp) * k.kblock + k.once + k.step * sp;
+      if (us < best.us && us * 1.05 < whole.us) best = {k.bn, k.pair, us, sp};
+    }
   }
   return best;
 }
@@ -1106,7 +1376,10 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     *pair_out = g->cta_pair == 0 && pairs_pay(g->M, g->N, g->K);
     return g->N > 128 ? 256 : 128;
   }
-  const StorePlan pl = plan_store(g->M, g->N, g->K, g->max_ctas, g->cta_pair == 0);
+  const bool bf16_out = e != BB_EPI_STORE_F32;
+  const StorePlan pl = bf16_out && (g->max_ctas == 0 || g->max_ctas >= bb_num_sms()) && g->split_k == 0 && g->cta_pair == 0 && g->epi_warps == 0
+                           ? plan_split(g->M, g->N, g->K) : plan_store(g->M, g->N, g->K, g->max_ctas, g->cta_pair == 0);
+  if (pl.splits) g->split_k = pl.splits;
   *pair_out = pl.pair;
   return pl.bn;
 }
@@ -1144,6 +1417,10 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   bb_gemm_desc planned = *g;
   const int bn = choose_tile(&planned, &pair, &wide_epi);
   g = &planned;
+  if (!f32 && g->split_k > 0) {
+    if (pair) return launch_split<256, true, false>(g, s, g->split_k);
+    return bn == 256 ? launch_split<256, false, false>(g, s, g->split_k) : launch_split<128, false, false>(g, s, g->split_k);
+  }
   if (pair) return wide_epi ? launch<256, true, 4, false>(g, s) : launch<256, true, 2, false>(g, s);
   if (bn == 256) return wide_epi ? launch<256, false, 4, false>(g, s) : launch<256, false, 2, false>(g, s);
   if (bn == 128) return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);
@@ -1184,6 +1461,10 @@ int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   bool pair, wide_epi;
   const int bn = choose_tile(&g, &pair, &wide_epi);
+  if (g.epilogue == BB_EPI_STORE && g.split_k > 0) {
+    if (pair) return launch_split<256, true, true>(&g, s, g.split_k, a);
+    return bn == 256 ? launch_split<256, false, true>(&g, s, g.split_k, a) : launch_split<128, false, true>(&g, s, g.split_k, a);
+  }
   if (pair) return launch<256, true, 2, true>(&g, s, a);
   return bn == 256 ? launch<256, false, 2, true>(&g, s, a) : launch<128, false, 2, true>(&g, s, a);
 }

@@ -583,3 +583,48 @@ def test_attention_non_finite_values_stay_in_their_sequence(L, D, causal, S):
             else:
                 assert ((g0[b, :, 0, h].float() - g1[b, :, 0, h].float()).abs().max() <= 2 ** -8 * g0[b, :, 0, h].float().abs().max()).item(), (b, h)
     assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("tile_n,cta_pair", [(128, -1), (256, -1), (0, 1)])
+@pytest.mark.parametrize("shape", [(8, 8, 8), (128, 128, 64), (136, 264, 200), (304, 520, 1000), (520, 1032, 2048)])
+def test_gemm_reduction_split_inside_a_cluster(L, a_mn, b_mn, tile_n, cta_pair, shape):
+    """Every number of splits (more than panels or k-blocks among them) with every bf16 epilogue, operand layout and a leading
+    dimension of its own.  Operands of -1, 0 and 1: sums are whole numbers below 2^24, the same in any order, so the stored value is
+    the bf16 rounding of the fp32 result bit for bit."""
+    torch.manual_seed(21)
+    M, N, K = shape
+    A = torch.randint(-1, 2, (M, K), device="cuda").bfloat16()
+    B = torch.randint(-1, 2, (N, K), device="cuda").bfloat16()
+    a, b = A.t().contiguous() if a_mn else A, B.t().contiguous() if b_mn else B
+    bias = torch.randint(-4, 5, (N,), device="cuda").bfloat16()
+    aux = torch.randint(-4, 5, (M, N + 8), device="cuda").bfloat16()[:, :N]
+    ref = A.float() @ B.float().t()
+    wide = torch.empty(M, N + 8, device="cuda", dtype=torch.bfloat16)
+    out, pre = wide[:, :N], torch.empty(M, N + 8, device="cuda", dtype=torch.bfloat16)[:, :N]
+    for split in (1, 2, 3, 4, 5, 6, 7, 8, 40):
+        kw = dict(a_mn=a_mn, b_mn=b_mn, M=M, N=N, K=K, tile_n=tile_n, cta_pair=cta_pair, split_k=split)
+        wide.fill_(7)
+        L.gemm(a, b, out, **kw)
+        assert torch.equal(out, ref.bfloat16()) and torch.all(wide[:, N:] == 7)
+        L.gemm(a, b, out, epilogue=L.EPI_BIAS_RESIDUAL, bias=bias, aux=aux, **kw)
+        assert torch.equal(out, (ref + bias.float() + aux.float()).bfloat16())
+        L.gemm(a, b, out, epilogue=L.EPI_BIAS_GELU, bias=bias, out2=pre, **kw)
+        assert torch.equal(pre, (ref + bias.float()).bfloat16())
+        close(out, gelu(pre.float()))
+    assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(520, 2048, 4096), (64, 2048, 2048), (1000, 512, 2048), (136, 1032, 4104)])
+def test_gemm_planned_split_is_as_exact_as_the_whole_reduction(L, shape):
+    """Shapes whose plan splits the reduction: the distance from 64 bits is that of one chain of additions, or less (both end in
+    one bf16 rounding, which dominates: the larger of the two may exceed the other by the fp32 part, 2^-24 sqrt(K) relative)."""
+    torch.manual_seed(22)
+    M, N, K = shape
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref = A.double() @ B.double().t()
+    out, whole = (torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    L.gemm(A, B, out)
+    L.gemm(A, B, whole, tile_n=128, cta_pair=-1)
+    err = [float((o.double() - ref).norm() / ref.norm()) for o in (out, whole)]
+    assert err[0] <= err[1] + 2 ** -24 * K ** 0.5

@@ -60,11 +60,41 @@ def _wgrad_stream(device):
     return st
 
 
+# Layers up to this size keep their weight gradients on the launching stream: tokens x hidden^2 of a transformer half,
+# eighths of the multiply-adds of any other layer.  Their kernels are shorter than their launches, so there is nothing to run
+# beside, while the fork, the stream's claim on three buffers and the allocator's events behind it cost 25 us per half block.
+# Forward + backward of one block (us, beside / in line): 512 tokens x 256 253 / 225, 1024 x 1024 258 / 234, 4096 x 512 258 / 256
+# (the line), 2048 x 1024 299 / 315, 1024 x 2048 452 / 455, 4096 x 1024 436 / 455.
+WGRAD_INLINE = 1 << 30
+
+
+def _beside(device, size, weight):
+    """Whether the weight-gradient work of a layer of this size goes to the side stream.  A weight's gradients are added to in
+    stream order: work in line waits for what earlier calls (on more tokens) left on the side stream, which itself
+    waits for the launching stream at every fork."""
+    if not WGRAD_SIDE_STREAM:
+        return False
+    if size > WGRAD_INLINE:
+        weight._wgrad_beside = True
+        return True
+    if getattr(weight, "_wgrad_beside", False):
+        wgrad_sync(device)
+    return False
+
+
 def wgrad_sync(device):
-    """Make the current stream wait for all weight-gradient work issued so far on ``device``."""
+    """Make the current stream wait for all weight-gradient work issued so far on ``device``.  In a stream capture: for what
+    the capture has put on the side stream - possibly nothing, with small layers only; earlier work there is no part of the graph,
+    and whoever captures joins it before."""
     st = _side_streams.get(device.index if device.index is not None else torch.cuda.current_device())
-    if st is not None:
-        torch.cuda.current_stream(device).wait_stream(st)
+    if st is None:
+        return
+    current = torch.cuda.current_stream(device)
+    if torch.cuda.is_current_stream_capturing():
+        with torch.cuda.stream(st):
+            if not torch.cuda.is_current_stream_capturing():
+                return
+    current.wait_stream(st)
 
 
 def _wgrad(dy2d, x2d, weight, bias, stream=None):
@@ -78,14 +108,15 @@ def _wgrad(dy2d, x2d, weight, bias, stream=None):
 def flush_wgrads(pending):
     """Launch the deferred weight-gradient work `[(dy, x, weight, bias), ...]`: on the side stream
     (one fork per call, all operands already produced on the current stream), or in place when
-    the side stream is switched off."""
+    the side stream is switched off or the layer is small."""
     if not pending:
         return
-    if not WGRAD_SIDE_STREAM:
+    dev = pending[0][0].device
+    size = max(dy.shape[0] * dy.shape[1] * x.shape[1] for dy, x, _, _ in pending) // 8
+    if not any([_beside(dev, size, weight) for _, _, weight, _ in pending]):
         for item in pending:
             _wgrad(*item)
         return
-    dev = pending[0][0].device
     side = _wgrad_stream(dev)
     side.wait_stream(torch.cuda.current_stream(dev))
     raw = side.cuda_stream
@@ -361,7 +392,8 @@ class _HalfFn(torch.autograd.Function):
         scratch = torch.empty(d._scratch_bytes, dtype=torch.uint8, device=x.device)
         dx = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
         side = None
-        if WGRAD_SIDE_STREAM:
+        weight = getattr(ctx.mod, _HALF_PARAMS[ctx.half][2])
+        if _beside(x.device, ctx.geom[0] * weight.shape[1] ** 2, weight):
             st = _wgrad_stream(x.device)
             side = st.cuda_stream
             # operands of the weight-gradient kernels: not to be handed out again before that stream is done

@@ -205,3 +205,34 @@ def test_checkpoint_round_trip_on_cuda_arena(tmp_path):
     assert got == want
     for name in ("master", "exp_avg", "exp_avg_sq", "lp"):
         assert torch.equal(getattr(a.arenas[0], name), getattr(b.arenas[0], name)), name
+
+
+def test_small_and_large_micro_batches_share_a_weight_gradient():
+    """A layer's weight gradients run in line for few tokens and beside the input gradients for many: the sums of both land in
+    the arena in either order of calls, as when everything stays on one stream."""
+    from bamboo_b200 import layers
+    from bamboo_b200.arena import ParamArena
+    h, line = 128, layers.WGRAD_INLINE
+    torch.manual_seed(5)
+    blk = layers.TransformerBlock(h, 2, 4 * h, causal=True)
+    head = layers.Linear(h, 256, bias=True)
+    arena = ParamArena([p for m in (blk, head) for p in m.parameters()], torch.device("cuda"), torch.bfloat16)
+    xs = [torch.randn(1, s, h, device="cuda").bfloat16() for s in (640, 64, 640, 64)]
+
+    def grads(limit):
+        layers.WGRAD_INLINE = limit
+        try:
+            arena.grad.zero_()
+            for x in xs:
+                y = head(blk(x.clone().requires_grad_(True)))
+                y.backward(torch.ones_like(y) * 0.01)
+            layers.wgrad_sync(xs[0].device)
+        finally:
+            layers.WGRAD_INLINE = line
+        return arena.grad.clone()
+    want = grads(1 << 60)                       # everything in line
+    for _ in range(10):
+        got = grads(200 * h * h)                # 640 tokens beside, 64 in line
+        # two orders of fp32 additions of the same bf16 products, at most 640 of them and four calls
+        assert float((got - want).norm() / want.norm()) < 1e-5
+    assert float((grads(0) - want).norm() / want.norm()) < 1e-5

@@ -399,3 +399,20 @@ def test_small_resnet_training_steps_match_oracle():
     from bamboo_b200 import lib
     torch.cuda.synchronize()
     assert lib.read_status() == 0
+
+
+# (k, stride, pad): one to four taps along a dimension at strides 1 and 2, and what stays with the general kernel
+@pytest.mark.parametrize("k,stride,pad", [(1, 2, 0), (2, 2, 0), (3, 2, 1), (4, 2, 1), (5, 2, 2), (7, 2, 3), (1, 1, 0), (2, 1, 1), (3, 1, 1),
+                                          (4, 1, 0), (5, 1, 2), (3, 3, 1), (9, 2, 4), (1, 2, 1)])
+@pytest.mark.parametrize("n,size,c", [(1, 9, 8), (3, 14, 24), (2, 33, 64)])
+def test_patch_adjoint_sums_every_tap_once(L, k, stride, pad, n, size, c):
+    """Whole numbers whose sums (at most 81 of magnitude 3) are exact in bf16's eight bits: equal to the fold bit for bit."""
+    torch.manual_seed(9)
+    out = (size + 2 * pad - k) // stride + 1
+    cols = torch.randint(-3, 4, (n, out, out, k * k, c), device="cuda")
+    col = torch.full((n * out * out, k * k * c + 8), 5.0, device="cuda", dtype=torch.bfloat16)
+    col[:, :k * k * c] = cols.reshape(n * out * out, -1).bfloat16()
+    dx = torch.empty(n, size, size, c, device="cuda", dtype=torch.bfloat16)
+    L.col2im(col[:, :k * k * c], dx, k, stride, pad, out, out)
+    folded = F.fold(cols.permute(0, 4, 3, 1, 2).reshape(n, c * k * k, out * out).float(), size, k, padding=pad, stride=stride)
+    assert torch.equal(dx.float(), folded.permute(0, 2, 3, 1))

@@ -1354,13 +1354,34 @@ StorePlan plan_split(long long M, long long N, long long K) {
   return best;
 }
 
+// The plans of a thread's recent problem sizes (a plan depends on nothing else but the device): going through up to seventeen
+// splits of three kinds of tile costs the host half a microsecond to two per product, as much as its tensor maps.
+struct PlanMemo { int M = 0, N = 0, K = 0, dev = -1, accum = 0, bn = 0, splits = 0; bool pair = false; };
+const PlanMemo& memoised_plan(int M, int N, int K, bool accum) {
+  static thread_local PlanMemo memo[256];
+  unsigned h = (unsigned)M * 2654435761u ^ (unsigned)N * 2246822519u ^ (unsigned)K * 3266489917u ^ (accum ? 1u : 0u);
+  PlanMemo& e = memo[(h ^ (h >> 16)) & 255u];
+  const int dev = bb_current_device();
+  if (e.M != M || e.N != N || e.K != K || e.accum != (accum ? 1 : 0) || e.dev != dev || dev < 0) {
+    e.M = M; e.N = N; e.K = K; e.dev = dev; e.accum = accum ? 1 : 0;
+    if (accum) {
+      const AccumPlan pl = plan_accum(M, N, K);
+      e.bn = pl.bn; e.pair = pl.pair; e.splits = pl.ksplit;
+    } else {
+      const StorePlan pl = plan_split(M, N, K);
+      e.bn = pl.bn; e.pair = pl.pair; e.splits = pl.splits;
+    }
+  }
+  return e;
+}
+
 // Tile width (0: the descriptor names none that exists), pairing, epilogue warps, and the split of a weight gradient
 int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
   const int e = g->epilogue;
   *wide_out = false;
   if (e == BB_EPI_ACCUM_F32 && g->split_k <= 0 && g->tile_n == 0 && g->cta_pair == 0) {
-    const AccumPlan pl = plan_accum(g->M, g->N, g->K);
-    g->split_k = pl.ksplit;
+    const PlanMemo& pl = memoised_plan(g->M, g->N, g->K, true);
+    g->split_k = pl.splits;
     *pair_out = pl.pair;
     return pl.bn;
   }
@@ -1376,10 +1397,13 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     *pair_out = g->cta_pair == 0 && pairs_pay(g->M, g->N, g->K);
     return g->N > 128 ? 256 : 128;
   }
-  const bool bf16_out = e != BB_EPI_STORE_F32;
-  const StorePlan pl = bf16_out && (g->max_ctas == 0 || g->max_ctas >= bb_num_sms()) && g->split_k == 0 && g->cta_pair == 0 && g->epi_warps == 0
-                           ? plan_split(g->M, g->N, g->K) : plan_store(g->M, g->N, g->K, g->max_ctas, g->cta_pair == 0);
-  if (pl.splits) g->split_k = pl.splits;
+  if (e != BB_EPI_STORE_F32 && (g->max_ctas == 0 || g->max_ctas >= bb_num_sms()) && g->split_k == 0 && g->cta_pair == 0 && g->epi_warps == 0) {
+    const PlanMemo& pl = memoised_plan(g->M, g->N, g->K, false);
+    g->split_k = pl.splits;
+    *pair_out = pl.pair;
+    return pl.bn;
+  }
+  const StorePlan pl = plan_store(g->M, g->N, g->K, g->max_ctas, g->cta_pair == 0);
   *pair_out = pl.pair;
   return pl.bn;
 }

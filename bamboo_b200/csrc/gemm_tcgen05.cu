@@ -719,9 +719,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     int acc = 0; uint32_t acc_phase = 0;
     bool alive = true;
     if constexpr (EW == 4) {
-      // Narrow variant for the epilogues with the most arithmetic per element (GeLU and its
-      // derivative) on short reductions, where eight warps cannot finish a tile's epilogue
-      // within the next tile's main loop: sixteen warps, 32 bf16 columns per pass (bf16 outputs only).
+      // Narrow variant: sixteen warps, 32 bf16 columns per pass (bf16 outputs only), when the descriptor asks for it.
       uint8_t* slab = panels + (warp - EPI_WARP) * (SLAB_BYTES / 2);
       for (uint32_t it = 0; alive; ++it) {
         int tile;

@@ -100,26 +100,26 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// one row of 64 fp32 values -> bf16 in global memory (128 contiguous bytes)
-__device__ __forceinline__ void store_row64(__nv_bfloat16* dst, const float* v, float mul) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 q;
-    q.x = bb::pack_bf16x2(v[8 * c + 0] * mul, v[8 * c + 1] * mul); q.y = bb::pack_bf16x2(v[8 * c + 2] * mul, v[8 * c + 3] * mul);
-    q.z = bb::pack_bf16x2(v[8 * c + 4] * mul, v[8 * c + 5] * mul); q.w = bb::pack_bf16x2(v[8 * c + 6] * mul, v[8 * c + 7] * mul);
-    reinterpret_cast<uint4*>(dst)[c] = q;
-  }
-}
-
-// 32 fp32 values of one row -> bf16 in global memory (64 contiguous bytes)
-__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const float* v, float mul) {
+// 32 rows x 32 columns of results, one row per lane, -> bf16 in global memory through 2 KiB of shared memory of the warp's own: an
+// instruction then writes 64 bytes of each of eight rows.  Stored by the rows' own lanes, every instruction touched 32
+// lines and the stores of a CTA's end took 1800 cycles.  `rows`: how many of the 32 exist.
+__device__ __forceinline__ void store_tile32(uint8_t* tile, __nv_bfloat16* dst, long long stride, int rows, int lane, const float* v, float mul) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     uint4 q;
     q.x = bb::pack_bf16x2(v[8 * c + 0] * mul, v[8 * c + 1] * mul); q.y = bb::pack_bf16x2(v[8 * c + 2] * mul, v[8 * c + 3] * mul);
     q.z = bb::pack_bf16x2(v[8 * c + 4] * mul, v[8 * c + 5] * mul); q.w = bb::pack_bf16x2(v[8 * c + 6] * mul, v[8 * c + 7] * mul);
-    reinterpret_cast<uint4*>(dst)[c] = q;
+    *reinterpret_cast<uint4*>(tile + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = q;
   }
+  __syncwarp();
+  const int c = lane & 3;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 8 * i + (lane >> 2);
+    const uint4 q = *reinterpret_cast<const uint4*>(tile + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+    if (r < rows) *reinterpret_cast<uint4*>(dst + r * stride + c * 8) = q;
+  }
+  __syncwarp();
 }
 
 // shared-memory bookkeeping common to the tcgen05 kernels
@@ -426,7 +426,8 @@ attn_tc_dq2_body(const CUtensorMap& tm_q, const CUtensorMap& tm_kv, const CUtens
       float v[32];
       const int c = 64 * g + hf * 32;
       ld32(tDQ + lane_addr + c, v);
-      if (qrow < p.S) store_row32(p.dq + (long long)(row_base + qrow) * p.stride_dqkv + colq + c, v, p.scale);
+      const int w0 = q0 + quarter * 32;
+      store_tile32(myDS + (hf * 4 + quarter) * 2048, p.dq + (long long)(row_base + w0) * p.stride_dqkv + colq + c, p.stride_dqkv, p.S - w0, lane, v, p.scale);
     }
   }
   bb::tc_fence_before_sync();
@@ -632,7 +633,9 @@ attn_tc_dkv2_body(const CUtensorMap& tm128, const CUtensorMap& tm64, const CUten
         float v[32];
         const int c = 64 * a + hf * 32;
         ld32(src + lane_addr + c, v);
-        if (krow < p.S) store_row32(dst + (long long)(row_base + krow) * p.stride_dqkv + colq + c, v, g == 0 ? 1.f : p.scale);
+        const int w0 = k0 + quarter * 32;
+        store_tile32(myP + (hf * 4 + quarter) * 2048, dst + (long long)(row_base + w0) * p.stride_dqkv + colq + c, p.stride_dqkv, p.S - w0, lane, v,
+                     g == 0 ? 1.f : p.scale);
       }
     }
   }
@@ -945,7 +948,8 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       const uint32_t src = (g == 0) ? tDV : tDK;
       ld32(src + lane_addr + hf * 32, v);
       __nv_bfloat16* dst = (g == 0) ? p.dv : p.dk;
-      if (krow < p.S) store_row32(dst + (long long)(row_base + krow) * p.stride_dqkv + colq + hf * 32, v, g == 0 ? 1.f : p.scale);
+      const int w0 = k0 + quarter * 32;
+      store_tile32(myP + (hf * 4 + quarter) * 2048, dst + (long long)(row_base + w0) * p.stride_dqkv + colq + hf * 32, p.stride_dqkv, p.S - w0, lane, v, g == 0 ? 1.f : p.scale);
     }
     if (lane == 0) bb::bulk_wait_group_read<0>();          // the reductions read this CTA's shared memory
   }
@@ -1244,11 +1248,15 @@ attn_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (__all_sync(0xffffffffu, fin)) {
         bb::tc_fence_after_sync();
         const float inv = l_i > 0.f ? 1.f / l_i : 0.f;
+        const int w0 = q0 + quarter * 32;
+        uint8_t* tile = sP + 2 * g * TILE_BYTES + quarter * 4096;              // (the group's P buffers: every product has retired)
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
           float o[64];
           ld32x2(tO + 64 * a, tO + 64 * a + 32, o, o + 32);
-          if (qrow < p.S) store_row64(p.out + (long long)(row_base + qrow) * p.stride_o + colq + 64 * a, o, inv);
+          __nv_bfloat16* dst = p.out + (long long)(row_base + w0) * p.stride_o + colq + 64 * a;
+          store_tile32(tile, dst, p.stride_o, p.S - w0, lane, o, inv);
+          store_tile32(tile + 2048, dst + 32, p.stride_o, p.S - w0, lane, o + 32, inv);
         }
         if (qrow < p.S) {
           p.lse[((long long)batch * p.H + head) * p.S + qrow] = (l_i > 0.f) ? (m_ref + log2f(l_i)) / LOG2E : -INFINITY;
@@ -1466,7 +1474,8 @@ attn_tc_fwd3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int h = 0; h < 2; ++h) {
         float o[32];
         ld32(tO + 32 * h, o);
-        if (qrow < p.S) store_row32(p.out + (long long)(row_base + qrow) * p.stride_o + colq + 32 * h, o, inv);
+        const int w0 = q0 + quarter * 32;                      // (P is free: its last product has retired)
+        store_tile32(sP + quarter * 4096 + h * 2048, p.out + (long long)(row_base + w0) * p.stride_o + colq + 32 * h, p.stride_o, p.S - w0, lane, o, inv);
       }
       if (qrow < p.S) {
         p.lse[((long long)id.batch * p.H + id.head) * p.S + qrow] = (l_i > 0.f) ? (m_ref + log2f(l_i)) / LOG2E : -INFINITY;

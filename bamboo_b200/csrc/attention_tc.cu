@@ -653,7 +653,8 @@ template <int D> constexpr int dkv2_smem() {
 // tail of one fills with CTAs of the other instead of leaving SMs idle between two launches.  (Roles taken in turn
 // were slower: 538 us against 503 us at B2 H32 S2048 D128 causal.)
 // B2 H32 S2048 D128 causal, step by step: 479 us with one issuing warp, group barriers around every hand-off and scalar arithmetic;
-// 447 with two-wide arithmetic and warps that wait for themselves; 331 with a second issuing warp.
+// 447 with two-wide arithmetic and warps that wait for themselves; 331 with a second issuing warp; 304 with results stored through
+// shared memory.
 template <int D> constexpr int bwd2_smem() { return dkv2_smem<D>() > dq2_smem<D>() ? dkv2_smem<D>() : dq2_smem<D>(); }
 static_assert(bwd2_smem<64>() <= 232448 && bwd2_smem<128>() <= 232448, "227 KiB of shared memory per CTA");
 template <int D>

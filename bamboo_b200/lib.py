@@ -188,26 +188,21 @@ _workspaces = {}
 
 
 def workspace(nbytes, tag="default", stream=None):
-    """A per-device scratch buffer that only ever grows (allocated through torch so it is
-    accounted in the caching allocator; the native side never allocates).  ``stream`` is the raw
-    handle of the stream the buffer's kernels run on when that is not the current one: a
-    buffer that is replaced by a larger one is first marked as in use on every stream that
-    consumed it, so the caching allocator cannot hand its block to another tensor while
-    kernels queued there still read and write it."""
+    """A scratch buffer of one stream that only ever grows (allocated through torch so it is accounted
+    in the caching allocator; the native side never allocates).  ``stream`` is the raw handle of the
+    stream that the buffer's kernels run on when that is not the current one.  Kernels of
+    different streams may overlap, so no two streams share a buffer, whatever their tags; on one stream
+    calls with one tag follow each other.  The buffer is allocated on its own stream: when a
+    larger one replaces it, the caching allocator hands its block out again behind the kernels queued there."""
     import torch
     dev = torch.cuda.current_device()
-    key = (dev, tag)
-    entry = _workspaces.get(key)
-    buf = entry[0] if entry is not None else None
-    users = entry[1] if entry is not None else set()
-    if stream is not None:
-        users.add(int(stream))
+    raw = torch._C._cuda_getCurrentRawStream(dev) if stream is None else int(stream)
+    key = (dev, raw, tag)
+    buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
-        if buf is not None:
-            for raw in users:
-                buf.record_stream(torch.cuda.ExternalStream(raw, device=f"cuda:{dev}"))
-        buf = torch.empty(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=f"cuda:{dev}")
-    _workspaces[key] = (buf, users)
+        with torch.cuda.stream(torch.cuda.ExternalStream(raw, device=f"cuda:{dev}")):
+            buf = torch.empty(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=f"cuda:{dev}")
+        _workspaces[key] = buf
     return buf
 
 
@@ -262,8 +257,7 @@ def layernorm_bwd_static(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta):
 
 
 def colsum_accum(dy, out, tag="rowwise", stream=None):
-    """out(fp32)[n] += dy(bf16)[rows, n].sum(0); ``tag`` names the scratch buffer (calls that may
-    overlap on the GPU, e.g. on different streams, need different ones)"""
+    """out(fp32)[n] += dy(bf16)[rows, n].sum(0); ``tag`` names the scratch buffer among those of the call's stream"""
     global LAUNCHES
     LAUNCHES += 1
     rows, n = dy.shape

@@ -236,3 +236,41 @@ def test_small_and_large_micro_batches_share_a_weight_gradient():
         # two orders of fp32 additions of the same bf16 products, at most 640 of them and four calls
         assert float((got - want).norm() / want.norm()) < 1e-5
     assert float((grads(0) - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("behind", ["linear", "transform", "block"])
+def test_bias_gradients_in_line_behind_others_beside(behind, monkeypatch):
+    """A layer whose weight gradients run beside, followed in the backward pass by one whose run in line: column sums of both are in
+    flight together.  Column sums have one order, so every bias gradient has the bits of everything on one stream."""
+    from bamboo_b200 import layers
+    from bamboo_b200.arena import ParamArena
+    h, rows = 256, 4096
+    torch.manual_seed(6)
+    if behind == "block":
+        # (the per-kernel path, whose halves fall on either side of the line; one key tile per sequence: dQ has one order too)
+        monkeypatch.setattr(layers, "NATIVE_BLOCKS", False)
+        mods = [layers.AttentionHalf(h, 4, 4 * h), layers.MLPHalf(h, 4, 4 * h)]
+        inline = {mods[0].qkv_w, mods[0].proj_w}
+    else:
+        first = layers.Linear(h, h) if behind == "linear" else layers.MLMTransform(h)
+        mods = [first, layers.Linear(h, 4096)]
+        inline = {first.weight}
+    arena = ParamArena([p for m in mods for p in m.parameters()], torch.device("cuda"), torch.bfloat16)
+    biases = [p for m in mods for n, p in m.named_parameters() if p.dim() == 1 and not n.startswith("ln")]
+    x = torch.randint(-1, 2, (rows // 128, 128, h), device="cuda").bfloat16()
+
+    def grads(beside):
+        monkeypatch.setattr(layers, "_beside", lambda device, size, weight: beside and weight not in inline)
+        arena.grad.zero_()
+        for _ in range(8):
+            y = x.clone().requires_grad_(True)
+            for m in mods:
+                y = m(y)
+            y.backward(torch.randint(-1, 2, y.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).bfloat16())
+        layers.wgrad_sync(x.device)
+        return [p.main_grad.clone() for p in biases]
+    want = grads(False)
+    assert len(want) in (2, 4) and all(float(w.abs().max()) > 0 for w in want)
+    for _ in range(3):
+        for got, w in zip(grads(True), want):
+            assert torch.equal(got, w)

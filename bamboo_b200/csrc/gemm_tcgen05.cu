@@ -1035,7 +1035,8 @@ using bbhost::encode_2d;
 // Ticket counters of the dynamic work distribution: a launch takes the next slot of a ring of
 // counters in device memory and draws exactly `units` tickets from it (see the scheduling
 // thread), so the host knows every counter's value without reading it back and nothing is ever
-// reset.  A slot is reused 65536 launches later, long after the launch that held it retired.
+// reset.  A slot is reused 65536 launches later, long after the launch that held it retired.  A launch that is being captured takes
+// no slot: the host cannot know how often, or whether, the graph runs, and every replay would start from another count.
 constexpr unsigned TICKET_SLOTS = 1u << 16;
 __device__ unsigned int g_gemm_tickets[TICKET_SLOTS];
 
@@ -1064,6 +1065,14 @@ TicketTable* ticket_table() {
   t->dev = static_cast<unsigned int*>(ptr);
   tables[dev] = t;
   return t;
+}
+
+// (a stream that cannot be asked belongs to a capture that the launch itself will report)
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus st;
+  if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
 }
 
 // Too few output tiles to fill the machine: split the reduction; partial sums meet in the fp32 add-reduction of the
@@ -1149,10 +1158,11 @@ int launch(const bb_gemm_desc* g, cudaStream_t stream, const bb_conv_gemm_args* 
   // persistent CTA that found a free SM keeps it for its whole tile loop, and a persistent kernel
   // of the main stream launched meanwhile waits for that SM with a fixed share of the tiles.
   if (g->max_ctas < 0) workers = tiles;
-  // more units than CTAs: every unit after a CTA's first is drawn from this launch's ticket counter
+  // more units than CTAs: every unit after a CTA's first is drawn from this launch's ticket counter (in a graph: unit i of a CTA
+  // is its index + i x CTAs)
   unsigned slot = 0;
   TicketTable* tt = nullptr;
-  if (tiles > workers && !g_static_schedule) {
+  if (tiles > workers && !g_static_schedule && !capturing(stream)) {
     tt = ticket_table();
     if (!tt) { bb_set_last_error_msg("bb_gemm_bf16: ticket counters unavailable on this device"); return BB_ERR_CUDA; }
     slot = tt->next.fetch_add(1u) & (TICKET_SLOTS - 1);

@@ -628,3 +628,29 @@ def test_gemm_planned_split_is_as_exact_as_the_whole_reduction(L, shape):
     L.gemm(A, B, whole, tile_n=128, cta_pair=-1)
     err = [float((o.double() - ref).norm() / ref.norm()) for o in (out, whole)]
     assert err[0] <= err[1] + 2 ** -24 * K ** 0.5
+
+
+@pytest.mark.parametrize("tile_n,cta_pair", [(128, -1), (256, -1), (0, 1)])
+@pytest.mark.parametrize("accum", [False, True])
+def test_gemm_of_several_waves_in_a_graph(L, tile_n, cta_pair, accum):
+    """More work units than CTAs, captured once and replayed on new operands, with calls outside the graph in between: every
+    replay computes every tile.  Whole numbers: sums are exact in any order."""
+    torch.manual_seed(23)
+    M, N, K = (4168, 2312, 136) if not accum else (2312, 2056, 1032)
+    A, B = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16), torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.zeros(M, N, device="cuda", dtype=torch.float32 if accum else torch.bfloat16)
+    kw = dict(tile_n=tile_n, cta_pair=cta_pair, epilogue=L.EPI_ACCUM_F32 if accum else L.EPI_STORE, split_k=2 if accum else 0)
+    L.gemm(A, B, out, **kw)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        L.gemm(A, B, out, **kw)
+    for _ in range(3):
+        for t in (A, B):
+            t.copy_(torch.randint(-1, 2, t.shape, device="cuda"))
+        ref = A.float() @ B.float().t()
+        ref = ref if accum else ref.bfloat16()
+        for run in (graph.replay, lambda: L.gemm(A, B, out, **kw)):
+            out.zero_()
+            run()
+            assert torch.equal(out, ref)
+    assert L.read_status() == 0

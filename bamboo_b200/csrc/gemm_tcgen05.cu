@@ -62,7 +62,7 @@ struct GemmParams {
   int M, N, K;
   int a_mn, b_mn;
   int epi;
-  int ksplit, kb_per_split;   // split-K work units (fp32 add-reduction epilogue only)
+  int ksplit, kb_per_split;   // parts of a tile's reduction: work units (fp32 add-reductions), or CTAs of a cluster (bf16 outputs)
   int n_fast;                 // tile order: consecutive work units walk along N (else along M)
   int dynamic;                // 1: work units after a CTA's first come from the ticket counter
   unsigned int* ticket;       // this launch's ticket counter (global memory)
@@ -1383,10 +1383,13 @@ const PlanMemo& memoised_plan(int M, int N, int K, bool accum) {
   return e;
 }
 
-// Tile width (0: the descriptor names none that exists), pairing, epilogue warps, and the split of a weight gradient
+// Tile width, pairing, epilogue warps, and the split of the reduction (bf16 outputs: 0 for none)
 int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
   const int e = g->epilogue;
+  const bool all_sms = g->max_ctas == 0 || g->max_ctas >= bb_num_sms();
   *wide_out = false;
+  // a split over a cluster takes CTAs and epilogue warps of its own: a descriptor that names either keeps the reduction whole
+  if (e != BB_EPI_ACCUM_F32 && (!all_sms || g->epi_warps != 0 || g->split_k < 0)) g->split_k = 0;
   if (e == BB_EPI_ACCUM_F32 && g->split_k <= 0 && g->tile_n == 0 && g->cta_pair == 0) {
     const PlanMemo& pl = memoised_plan(g->M, g->N, g->K, true);
     g->split_k = pl.splits;
@@ -1405,7 +1408,7 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     *pair_out = g->cta_pair == 0 && pairs_pay(g->M, g->N, g->K);
     return g->N > 128 ? 256 : 128;
   }
-  if (e != BB_EPI_STORE_F32 && (g->max_ctas == 0 || g->max_ctas >= bb_num_sms()) && g->split_k == 0 && g->cta_pair == 0 && g->epi_warps == 0) {
+  if (e != BB_EPI_STORE_F32 && all_sms && g->split_k == 0 && g->cta_pair == 0 && g->epi_warps == 0) {
     const PlanMemo& pl = memoised_plan(g->M, g->N, g->K, false);
     g->split_k = pl.splits;
     *pair_out = pl.pair;
@@ -1441,6 +1444,10 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
     bb_set_last_error_msg("bb_gemm_bf16: epi_warps must be 0, 2 or 4 (4 only with bf16 outputs)");
     return BB_ERR_INVALID_ARG;
   }
+  if (g->cta_pair <= 0 && g->tile_n != 0 && g->tile_n != 128 && g->tile_n != 256) {
+    bb_set_last_error_msg("bb_gemm_bf16: tile_n must be 0, 128 or 256");
+    return BB_ERR_INVALID_ARG;
+  }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // cuTensorMapEncodeTiled is a driver call and needs a context bound to the calling thread;
   // a thread that has only ever set its device (autograd worker threads) has none yet.
@@ -1455,9 +1462,7 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   }
   if (pair) return wide_epi ? launch<256, true, 4, false>(g, s) : launch<256, true, 2, false>(g, s);
   if (bn == 256) return wide_epi ? launch<256, false, 4, false>(g, s) : launch<256, false, 2, false>(g, s);
-  if (bn == 128) return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);
-  bb_set_last_error_msg("bb_gemm_bf16: tile_n must be 0, 128 or 256");
-  return BB_ERR_INVALID_ARG;
+  return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);
 }
 
 double bb_gemm_store_us(long long M, long long N, long long K) { return plan_store(M, N, K, 0, true).us; }

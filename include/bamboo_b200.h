@@ -61,7 +61,8 @@ typedef struct bb_gemm_desc {
   int max_ctas;                     /* 0 = one persistent CTA per SM; > 0 = cap (leaves SMs to a concurrent stream);
                                        < 0 = one tile per CTA (short CTAs for a low-priority stream) */
   int split_k;                      /* 0 = choose; else number of K splits: add-reductions into D for BB_EPI_ACCUM_F32, CTAs of a
-                                       cluster that share a tile's reduction for bf16 outputs (as far as clusters allow) */
+                                       cluster that share a tile's reduction for bf16 outputs (as far as clusters allow; the
+                                       reduction stays whole under a cap on the CTAs or with epi_warps named) */
   int cta_pair;                     /* 0 = choose, 1 = CTA pairs (cta_group::2, 256 x 256 tiles), -1 = single CTAs */
   int epi_warps;                    /* epilogue warps per TMEM lane quarter: 0 = choose, 2, or 4 (bf16 outputs only) */
 } bb_gemm_desc;

@@ -4,6 +4,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -39,3 +41,13 @@ def test_argument_errors_do_not_need_a_gpu():
     handle = lib.load()
     rc = handle.bb_gemm_bf16(None, None)
     assert rc == -1 and b"bb_gemm_bf16" in handle.bb_last_error()
+
+
+@pytest.mark.parametrize("tile_n", [64, 96, 512, -1])
+@pytest.mark.parametrize("split_k", [0, 1, 4])
+def test_a_tile_that_does_not_exist_is_refused_with_and_without_a_split(tile_n, split_k):
+    from bamboo_b200 import lib
+    handle, fake = lib.load(), 1 << 20
+    d = lib.GemmDesc(M=128, N=128, K=1024, A=fake, lda=1024, B=fake, ldb=1024, D=fake, ldd=128, tile_n=tile_n, split_k=split_k)
+    assert handle.bb_gemm_bf16(ctypes.byref(d), None) == -1
+    assert b"tile_n" in handle.bb_last_error()

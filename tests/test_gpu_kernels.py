@@ -654,3 +654,26 @@ def test_gemm_of_several_waves_in_a_graph(L, tile_n, cta_pair, accum):
             run()
             assert torch.equal(out, ref)
     assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("limit", [dict(max_ctas=16), dict(max_ctas=-1), dict(epi_warps=2), dict(max_ctas=6, cta_pair=1), dict(max_ctas=100000)])
+def test_gemm_budget_goes_before_a_split_of_the_reduction(L, limit):
+    """A descriptor that names a split of a bf16 product together with a cap on its CTAs keeps the cap: the same launch, and the same
+    bits, as without the split.  (A cap above the number of SMs is none.)"""
+    from cuda.bindings import driver
+    from test_gpu_overlap import captured, kernel_nodes
+    torch.manual_seed(24)
+    M, N, K = 520, 1032, 2048
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    out = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    shapes = []
+    for split in (0, 4):
+        graph, handle, rt = captured(lambda: L.gemm(A, B, out[split > 0], split_k=split, **limit))
+        node, = kernel_nodes(handle, rt)
+        cluster = rt.cudaGraphKernelNodeGetAttribute(node, rt.cudaLaunchAttributeID.cudaLaunchAttributeClusterDimension)[1].clusterDim.x
+        shapes.append((driver.cuGraphKernelNodeGetParams(driver.CUgraphNode(int(node)))[1].gridDimX, cluster))
+    if limit.get("max_ctas", 0) > 1000:
+        assert shapes[1][1] >= 4
+    else:
+        assert shapes[0] == shapes[1] and (limit.get("max_ctas", 0) <= 0 or shapes[1][0] <= limit["max_ctas"])
+        assert torch.equal(*out)

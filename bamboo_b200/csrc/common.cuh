@@ -86,8 +86,8 @@ struct bb_conv_gemm_args {
 // tensor map's limits).
 bool bb_conv_gemm_supported(int C, int k, int stride, int pad);
 int bb_conv_gemm(const bb_conv_gemm_args* a, void* stream);
-// Time that a stored product of M x N over K is expected to take on the whole GPU.
-double bb_gemm_store_us(long long M, long long N, long long K);
+// Time that a stored product of M x N over K is expected to take on the whole GPU, as it is planned for that CTA budget.
+double bb_gemm_store_us(long long M, long long N, long long K, int max_ctas);
 
 // Division by a number known at launch: n / d = high word of n * magic with magic = floor(2^64 / d) + 1 (0 stands for
 // d = 1); for n < 2^32 the error n * d / 2^64 stays below 1.

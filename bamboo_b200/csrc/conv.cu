@@ -821,9 +821,11 @@ struct ConvSizes {
   // of k * k * Cout, where the patch-gradient product has k * k * Cin columns and reduces over Cout.  Backward pass (us),
   // patch matrix / gathered: 8 -> 1024 channels, 7 x 7, 32 images of 56 x 56: 587 / 1776; 256 -> 1024, 7 x 7, 8 of 14 x 14
   // (8 output tiles): 153 / 348; 64 -> 64, 3 x 3, 32 of 56 x 56: 142 / 68; 256 -> 256, 3 x 3, 32 of 56 x 56: 437 / 243.
-  // The adjoint gather is counted as 1.5 TB/s of patch matrix, the gathered product as 1.2 of its plan: over 213 layers (8 to 256
-  // -> 64 to 1024 channels, windows 2 to 7, 1568 to 100352 pixels) none is slower than with the patch matrix, and the pass is
-  // within 2 % of the quicker route on average.
+  // Few pixels and a long reduction split it over clusters, and the product is priced as it runs: 256 -> 1024, 7 x 7, 32 images
+  // of 14 x 14 304 / 260, 512 -> 256, 7 x 7, one of 28 x 28 71 / 51, 64 -> 64, 7 x 7, 32 of 7 x 7 44 / 28, all gathered.
+  // The adjoint gather is counted as 1.5 TB/s of patch matrix, the gathered product as 1.2 of its plan: over 130 layers (8 to 512
+  // -> 64 to 1024 channels, windows 3 to 7, 98 to 166012 pixels) one is slower than with the patch matrix (44.0 / 46.7), and the pass
+  // is within 4 % of the quicker route on average (5 % with the gathered product priced whole).
   // A 3 x 3 layer's patch matrix is nine times its input, written and read once per product: 128 channels, 32 images
   // of 28 x 28, forward + backward 181 -> 89 us of device time (gathers 80 us, GEMMs 63 -> 55 us) without it.
   bool implicit_x, implicit_dx;
@@ -844,8 +846,8 @@ bool conv_sizes(const bb_conv_desc* d, ConvSizes* s) {
   s->implicit_x = !s->direct && bb_conv_gemm_supported(d->Cin, d->k, d->stride, d->pad) &&
                   (d->H < d->W ? d->H : d->W) + 2 * d->pad >= d->k;
   s->implicit_dx = !s->direct && d->stride == 1 && d->pad < d->k && bb_conv_gemm_supported(d->Cout, d->k, 1, d->k - 1 - d->pad) &&
-                   1.2 * bb_gemm_store_us((long long)d->N * d->H * d->W, d->Cin, (long long)d->k * d->k * d->Cout) <
-                       bb_gemm_store_us(s->P, s->K, d->Cout) + (double)s->P * s->K * 2 / 1.5e6;
+                   1.2 * bb_gemm_store_us((long long)d->N * d->H * d->W, d->Cin, (long long)d->k * d->k * d->Cout, d->max_ctas) <
+                       bb_gemm_store_us(s->P, s->K, d->Cout, d->max_ctas) + (double)s->P * s->K * 2 / 1.5e6;
   s->bn_bytes = bb_bn_workspace_bytes(s->P, d->Cout);
   if (s->bn_bytes < 0) return false;
   s->col_bytes = s->direct || s->implicit_x ? 0 : up256(s->P * s->K * 2);

@@ -1364,7 +1364,7 @@ StorePlan plan_split(long long M, long long N, long long K) {
 
 // The plans of a thread's recent problem sizes (a plan depends on nothing else but the device): going through up to seventeen
 // splits of three kinds of tile costs the host half a microsecond to two per product, as much as its tensor maps.
-struct PlanMemo { int M = 0, N = 0, K = 0, dev = -1, accum = 0, bn = 0, splits = 0; bool pair = false; };
+struct PlanMemo { int M = 0, N = 0, K = 0, dev = -1, accum = 0, bn = 0, splits = 0; bool pair = false; double us = 0; };
 const PlanMemo& memoised_plan(int M, int N, int K, bool accum) {
   static thread_local PlanMemo memo[256];
   unsigned h = (unsigned)M * 2654435761u ^ (unsigned)N * 2246822519u ^ (unsigned)K * 3266489917u ^ (accum ? 1u : 0u);
@@ -1377,7 +1377,7 @@ const PlanMemo& memoised_plan(int M, int N, int K, bool accum) {
       e.bn = pl.bn; e.pair = pl.pair; e.splits = pl.ksplit;
     } else {
       const StorePlan pl = plan_split(M, N, K);
-      e.bn = pl.bn; e.pair = pl.pair; e.splits = pl.splits;
+      e.bn = pl.bn; e.pair = pl.pair; e.splits = pl.splits; e.us = pl.us;
     }
   }
   return e;
@@ -1465,7 +1465,11 @@ extern "C" int bb_gemm_bf16(const bb_gemm_desc* g, void* stream) {
   return wide_epi ? launch<128, false, 4, false>(g, s) : launch<128, false, 2, false>(g, s);
 }
 
-double bb_gemm_store_us(long long M, long long N, long long K) { return plan_store(M, N, K, 0, true).us; }
+double bb_gemm_store_us(long long M, long long N, long long K, int max_ctas) {
+  if (max_ctas != 0 && max_ctas < bb_num_sms()) return plan_store(M, N, K, 0, true).us;      // (a budget keeps the reduction whole)
+  if (M > INT_MAX || N > INT_MAX || K > INT_MAX) return plan_split(M, N, K).us;
+  return memoised_plan((int)M, (int)N, (int)K, false).us;
+}
 
 bool bb_conv_gemm_supported(int C, int k, int stride, int pad) {
   // tensor map limits of a rank-4 im2col load: window corners in [-128, 127], traversal stride <= 8

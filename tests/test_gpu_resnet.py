@@ -416,3 +416,12 @@ def test_patch_adjoint_sums_every_tap_once(L, k, stride, pad, n, size, c):
     L.col2im(col[:, :k * k * c], dx, k, stride, pad, out, out)
     folded = F.fold(cols.permute(0, 4, 3, 1, 2).reshape(n, c * k * k, out * out).float(), size, k, padding=pad, stride=stride)
     assert torch.equal(dx.float(), folded.permute(0, 2, 3, 1))
+
+
+# few pixels and a reduction of k * k * Cout: the gathered input gradient is split over clusters; the last on a budget, which keeps it whole
+@pytest.mark.parametrize("n,hw,cin,cout,k,max_ctas,kernels", [(32, 7, 64, 64, 7, 0, 5), (1, 28, 512, 256, 7, 0, 5), (8, 14, 128, 256, 5, 0, 5),
+                                                              (6, 14, 256, 2048, 3, 0, 6), (32, 7, 64, 64, 7, -1, 6)])
+def test_input_gradient_is_priced_as_it_is_planned(L, monkeypatch, n, hw, cin, cout, k, max_ctas, kernels):
+    monkeypatch.setattr(L, "GEMM_MAX_CTAS", max_ctas)
+    d = check_convolution(L, cin, cout, k, 1, hw, n)
+    assert L._conv_launches(d, 1, 1) == kernels

@@ -889,7 +889,7 @@ attn_tc_bwd3_kernel(const __grid_constant__ CUtensorMap tm128, const __grid_cons
       }
       __syncwarp();
       const int q0 = (qstart + 2 * pair) * SUB + quarter * 32;
-      if (q0 >= p.S) return;
+      if (!alive || q0 >= p.S) return;                     // (a warp that gave up adds nothing to the accumulator)
       if (q0 + lane >= p.S) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) r[i] = 0u;

@@ -397,9 +397,12 @@ __device__ __forceinline__ void st_shared_cluster_v4(uint32_t cluster_addr, uint
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same without release: for hand-backs of what the thread has finished reading (values in registers).  A release at
-// cluster scope waits until all of the thread's earlier global stores have been performed - a microsecond per tile where an
-// epilogue warp hands an accumulator back between two panels.
+// The same without release, for hand-backs of what the warp has finished reading.  It orders nothing by itself, so the reads have to be
+// over when it is issued: an accumulator's by tcgen05.wait::ld and tcgen05.fence::before_thread_sync, which orders the tensor
+// core's accesses before a barrier operation of any kind (the taker answers with fence::after_thread_sync); a word of shared
+// memory's by a branch on its value (a value cannot be the one that its own hand-back brings about).  A release at cluster scope
+// waits until all of the thread's earlier global stores have been performed - a microsecond per tile where an epilogue
+// warp hands an accumulator back between two panels.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

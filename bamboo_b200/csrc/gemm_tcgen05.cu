@@ -590,7 +590,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   bb::pdl_sync();
 
   // Work unit number `it` of this CTA: the first is its own index, the others as announced by the scheduling warp (-1: no
-  // more).  Called by a whole warp; the entry is handed back once it has been read.
+  // more).  Called by a whole warp; the entry is handed back once it has been read: the hand-back of a pair, which is not a
+  // release, branches on the value, so that it cannot be on its way before the value is there.
   auto next_unit = [&](uint32_t it, int& tile) -> bool {
     if (it == 0) { tile = worker; return true; }
     --it;
@@ -601,8 +602,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     if (!__all_sync(0xffffffffu, got)) return false;
     tile = __shfl_sync(0xffffffffu, sched_tile[r], 0);
     if (lane == 0) {
-      if (PAIR) bb::mbar_arrive_cluster_relaxed(bb::mapa_shared(bb::smem_u32(&sched_empty[r]), 0));
-      else bb::mbar_arrive(&sched_empty[r]);
+      if (!PAIR) bb::mbar_arrive(&sched_empty[r]);
+      else if (tile >= -1) bb::mbar_arrive_cluster_relaxed(bb::mapa_shared(bb::smem_u32(&sched_empty[r]), 0));
     }
     return true;
   };

@@ -60,11 +60,15 @@ def _wgrad_stream(device):
     return st
 
 
-# Layers up to this size keep their weight gradients on the launching stream: tokens x hidden^2 of a transformer half,
-# eighths of the multiply-adds of any other layer.  Their kernels are shorter than their launches, so there is nothing to run
-# beside, while the fork, the stream's claim on three buffers and the allocator's events behind it cost 25 us per half block.
-# Forward + backward of one block (us, beside / in line): 512 tokens x 256 253 / 225, 1024 x 1024 258 / 234, 4096 x 512 258 / 256
-# (the line), 2048 x 1024 299 / 315, 1024 x 2048 452 / 455, 4096 x 1024 436 / 455.
+# Layers up to this size keep their weight gradients on the launching stream: their kernels are shorter than their launches, so
+# there is nothing to run beside, while the fork, the stream's claim on the operands and the allocator's events behind it cost
+# host time.  The size is an eighth of the multiply-adds of a layer's largest weight gradient where kernels are launched
+# one by one, and twice tokens x hidden^2 for a half block, whose kernels follow each other without the host: there the line lies
+# lower.  Forward + backward (us, beside / in line): Linear 512 x 256 -> 256 168 / 135, 8192 x 1024 -> 1024 152 / 136 (the line),
+# 4096 x 2048 -> 2048 152 / 136, 8192 x 2048 -> 2048 168 / 203; MLMTransform 8192 x 1024 219 / 196; blocks of separate launches,
+# 1024 tokens x 1024 554 / 464 and 2331 x 1024 567 / 490.  Four blocks in a row, two native calls each way: 4 x 128 tokens x 256
+# 790 / 689, 2 x 512 x 512 829 / 744, 4 x 512 x 512 881 / 798, 512 x 1024 793 / 793 and 4 x 128 x 1024 796 / 801 (the line), 8 x 512 x 512
+# 945 / 1042, 2 x 512 x 1024 903 / 954, 4 x 512 x 1024 1180 / 1257.
 WGRAD_INLINE = 1 << 30
 
 
@@ -393,7 +397,7 @@ class _HalfFn(torch.autograd.Function):
         dx = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
         side = None
         weight = getattr(ctx.mod, _HALF_PARAMS[ctx.half][2])
-        if _beside(x.device, ctx.geom[0] * weight.shape[1] ** 2, weight):
+        if _beside(x.device, 2 * ctx.geom[0] * weight.shape[1] ** 2, weight):
             st = _wgrad_stream(x.device)
             side = st.cuda_stream
             # operands of the weight-gradient kernels: not to be handed out again before that stream is done

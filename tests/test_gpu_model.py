@@ -274,3 +274,25 @@ def test_bias_gradients_in_line_behind_others_beside(behind, monkeypatch):
     for _ in range(3):
         for got, w in zip(grads(True), want):
             assert torch.equal(got, w)
+
+
+# (tokens x hidden^2 of a block at 2^29 and above it; a layer of separate launches at 2^33 multiply-adds and above it)
+@pytest.mark.parametrize("layer,rows,h,beside", [("block", 2048, 512, False), ("block", 2176, 512, True), ("block", 4096, 512, True),
+                                                 ("transform", 8192, 1024, False), ("linear", 8192, 1024, False), ("linear", 8320, 1024, True)])
+def test_where_weight_gradients_leave_the_launching_stream(layer, rows, h, beside, monkeypatch):
+    from bamboo_b200 import layers
+    from bamboo_b200 import lib as L
+    from bamboo_b200.arena import ParamArena
+    mod = {"block": lambda: layers.TransformerBlock(h, h // 64, 4 * h), "transform": lambda: layers.MLMTransform(h),
+           "linear": lambda: layers.Linear(h, h)}[layer]()
+    arena = ParamArena(list(mod.parameters()), torch.device("cuda"), torch.bfloat16)
+    seen = []
+    gemm, half = L.gemm, L.block_half_bwd
+    monkeypatch.setattr(L, "gemm", lambda *a, **k: (seen.append(k.get("stream")) if k.get("epilogue") == L.EPI_ACCUM_F32 else None, gemm(*a, **k))[1])
+    monkeypatch.setattr(L, "block_half_bwd", lambda *a: (seen.append(a[-1]), half(*a))[1])
+    x = torch.randn(rows // 128, 128, h, device="cuda").bfloat16().requires_grad_(True)
+    y = mod(x)
+    y.backward(torch.ones_like(y))
+    layers.wgrad_sync(x.device)
+    assert seen and [s is not None for s in seen] == [beside] * len(seen)
+    assert torch.isfinite(arena.grad).all()

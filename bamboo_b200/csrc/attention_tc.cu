@@ -67,10 +67,6 @@ __device__ __forceinline__ uint64_t desc_kmajor(uint64_t d0, int kstep) { return
 // [rows x 64] tile, reduction over its rows (N or M = the 64 columns): k-step = 16 rows = 2 KiB
 __device__ __forceinline__ uint64_t desc_mn0(uint32_t tile) { return bb::make_smem_desc_sw128(tile, 8192, 1024); }
 __device__ __forceinline__ uint64_t desc_mnmajor64(uint64_t d0, int kstep) { return d0 + (uint64_t)(kstep * (2048 >> 4)); }
-__device__ __forceinline__ void pack32(const float* v, uint32_t* out16) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) out16[i] = bb::pack_bf16x2(v[2 * i], v[2 * i + 1]);
-}
 // half a row (64 bytes: chunks 4*half .. 4*half+3) of a [128 x 64] bf16 atom from 16 packed registers
 __device__ __forceinline__ void atom_store_half_row(uint8_t* atom, int row, int half, const uint32_t* pk) {
   uint8_t* base = atom + row * 128;

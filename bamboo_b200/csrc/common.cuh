@@ -252,11 +252,7 @@ __device__ __forceinline__ void tma_load_im2col(void* smem_dst, const void* tmap
       : : "r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
       : "memory");
 }
-// shared -> global tile store / fp32 add-reduction through a tensor map (clips at the edges)
-__device__ __forceinline__ void tma_store_2d(const void* tmap, const void* smem_src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               : : "l"(tmap), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1) : "memory");
-}
+// shared -> global fp32 add-reduction of a tile through a tensor map (clips at the edges)
 __device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* smem_src, int c0, int c1) {
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
                : : "l"(tmap), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1) : "memory");
@@ -267,20 +263,6 @@ template <int N> __device__ __forceinline__ void bulk_wait_group_read() {
 }
 template <int N> __device__ __forceinline__ void bulk_wait_group() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-// barrier + AND-reduction of a predicate over the participating threads (uniform result)
-__device__ __forceinline__ bool named_bar_all(int id, int threads, bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 q, %3, 0;\n\t"
-      "bar.red.and.pred p, %1, %2, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r) : "r"(id), "r"(threads), "r"((uint32_t)pred) : "memory");
-  return r != 0;
 }
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");

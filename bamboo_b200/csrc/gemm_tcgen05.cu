@@ -1398,8 +1398,10 @@ int choose_tile(bb_gemm_desc* g, bool* pair_out, bool* wide_out) {
     return pl.bn;
   }
   // eight epilogue warps unless sixteen are asked for: with two-wide arithmetic and panels stored without a test per row they
-  // finish a tile within the next one's main loop (8192 x 4096 x 1024 as pairs, bias + GeLU 57.2 us with eight, 57.5 with sixteen;
-  // residual 8192 x 1024 x 1024 21.2 and 22.2)
+  // finish a tile within the next one's main loop (us, eight / sixteen: 8192 x 4096 x 1024 bias + GeLU 65.7 / 69.8, residual
+  // 66.0 / 70.3; 8192 x 1024 x 1024 plain 18.6 / 20.5).  Sixteen are the quicker only for x gelu' on tiles that nothing follows
+  // (4096 x 1024 x 1024 20.5 / 16.8-19.5, 2331 x 1024 x 1024 15.6 / 14.5) and on the shortest reductions (16384 x 1024 x 256 27.6 /
+  // 26.9, 100352 x 256 x 64 47.7 / 43.5).
   *wide_out = g->epi_warps == 4;
   *pair_out = g->cta_pair > 0;
   if (g->cta_pair > 0) return 256;

@@ -181,10 +181,15 @@ __device__ __forceinline__ void slab_flush_bf16(const uint8_t* slab, __nv_bfloat
     }
   }
 }
+// Add-reductions go out back to back only into outputs of less than 16 MiB.  A large output is read and written in memory, and bursts
+// of reductions slow that down: 4096 x 16384 x 333 141 us in bursts and 135 row by row, 8192 x 2048 x 333 35.3 and 33.5, 2048 x 2048 x 513
+// 13.2 and 12.5 (outputs not in L2; from 2000 k on no difference); a small one of many splits stays in L2: 64 x 576 x 100352
+// 25.7 and 26.9.
+__device__ __forceinline__ bool small_output(int M, int N) { return (long long)M * N < (1LL << 22); }
 template <bool ACCUM>
 __device__ __forceinline__ void slab_flush_f32(const uint8_t* slab, float* dst, long long ld, int r0, int nb, int M, int N, int lane) {
   const int c = nb + (lane & 7) * 4;
-  if (inside(r0, nb, 32, M, N)) {
+  if ((!ACCUM || small_output(M, N)) && inside(r0, nb, 32, M, N)) {
     float* g = dst + (long long)(r0 + (lane >> 3)) * ld + c;
     float4 q[8];
 #pragma unroll

@@ -677,3 +677,20 @@ def test_gemm_budget_goes_before_a_split_of_the_reduction(L, limit):
     else:
         assert shapes[0] == shapes[1] and (limit.get("max_ctas", 0) <= 0 or shapes[1][0] <= limit["max_ctas"])
         assert torch.equal(*out)
+
+
+# outputs just below and at 2^22 elements, with panels inside the matrix and across its edges; 4 bytes a column in a longer row
+@pytest.mark.parametrize("M,N", [(2040, 2048), (2048, 2048), (2056, 2060), (130, 32268)])
+@pytest.mark.parametrize("tile_n,cta_pair", [(128, -1), (256, -1), (0, 1)])
+def test_gemm_add_reduction_into_small_and_large_outputs(L, M, N, tile_n, cta_pair):
+    """Whole numbers: sums are exact in any order, and what lies beside the matrix is not touched."""
+    torch.manual_seed(25)
+    K = 200
+    A, B = (torch.randint(-1, 2, (K, n + (-n) % 8), device="cuda").bfloat16() for n in (M, N))
+    wide = torch.full((M + 1, N + 4), 3.0, device="cuda")
+    for split in (1, 2):
+        L.gemm(A, B, wide[:M, :N], a_mn=True, b_mn=True, epilogue=L.EPI_ACCUM_F32, M=M, N=N, K=K, tile_n=tile_n, cta_pair=cta_pair, split_k=split)
+    want = torch.full_like(wide, 3.0)
+    want[:M, :N] += 2 * (A[:, :M].float().t() @ B[:, :N].float())
+    assert torch.equal(wide, want)
+    assert L.read_status() == 0

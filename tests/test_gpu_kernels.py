@@ -694,3 +694,56 @@ def test_gemm_add_reduction_into_small_and_large_outputs(L, M, N, tile_n, cta_pa
     want[:M, :N] += 2 * (A[:, :M].float().t() @ B[:, :N].float())
     assert torch.equal(wide, want)
     assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("tile_n,cta_pair", [(128, -1), (256, -1), (0, 1)])
+@pytest.mark.parametrize("shape", [(8, 8, 72), (136, 264, 200), (520, 1032, 2048)])
+def test_gemm_split_inside_a_cluster_with_bias_and_gelu_derivative(L, tile_n, cta_pair, shape):
+    """The two bf16 epilogues that the test of all splits leaves out.  Sums of whole numbers are the same in any order, and what is done to
+    them is the same code: the bits of the whole reduction."""
+    torch.manual_seed(26)
+    M, N, K = shape
+    A, B = torch.randint(-1, 2, (M, K), device="cuda").bfloat16(), torch.randint(-1, 2, (N, K), device="cuda").bfloat16()
+    bias, aux = torch.randint(-4, 5, (N,), device="cuda").bfloat16(), (2 * torch.randn(M, N + 8, device="cuda")).bfloat16()[:, :N]
+    want = (A.float() @ B.float().t() + bias.float()).bfloat16()
+    out, whole = (torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    kw = dict(tile_n=tile_n, cta_pair=cta_pair)
+    L.gemm(A, B, whole, epilogue=L.EPI_MUL_DGELU, aux=aux, **kw)
+    for split in (1, 2, 3, 4, 5, 6, 7, 8, 40):
+        L.gemm(A, B, out.fill_(7), epilogue=L.EPI_BIAS, bias=bias, split_k=split, **kw)
+        assert torch.equal(out, want)
+        L.gemm(A, B, out.fill_(7), epilogue=L.EPI_MUL_DGELU, aux=aux, split_k=split, **kw)
+        assert torch.equal(out, whole)
+    assert L.read_status() == 0
+
+
+def split_launch(call):
+    """Whether the call's one product runs with its reduction split over clusters: that kernel has 608 threads, the other 352."""
+    from cuda.bindings import driver
+    from test_gpu_overlap import captured, kernel_nodes
+    graph, handle, rt = captured(call)
+    node, = kernel_nodes(handle, rt)
+    return driver.cuGraphKernelNodeGetParams(driver.CUgraphNode(int(node)))[1].blockDimX == 608
+
+
+@pytest.mark.parametrize("shape", [(520, 2048, 4096), (64, 2048, 2048), (1000, 512, 2048), (136, 1032, 4104)])
+@pytest.mark.parametrize("budget", [-1, 64])
+def test_gemm_own_and_redundant_routes_agree(L, shape, budget):
+    """The stage's own product splits its reduction, the same product on the CTA budget of redundant work keeps it whole: sums that are
+    exact in any order give the same bits; others are as far from 64 bits either way (one bf16 rounding, and the fp32
+    part of 2^-24 sqrt(K))."""
+    torch.manual_seed(27)
+    M, N, K = shape
+    out = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    for exact in (True, False):
+        A, B = ((torch.randint(-1, 2, (n, K), device="cuda") if exact else torch.randn(n, K, device="cuda")).bfloat16() for n in (M, N))
+        calls = [lambda: L.gemm(A, B, out[0]), lambda: L.gemm(A, B, out[1], max_ctas=budget)]
+        assert [split_launch(c) for c in calls] == [True, False]
+        for c in calls:
+            c()
+        ref = A.double() @ B.double().t()
+        if exact:
+            assert torch.equal(out[0], ref.bfloat16()) and torch.equal(*out)
+        else:
+            err = [float((o.double() - ref).norm() / ref.norm()) for o in out]
+            assert abs(err[0] - err[1]) <= 2 ** -24 * K ** 0.5

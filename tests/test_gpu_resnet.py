@@ -425,3 +425,20 @@ def test_input_gradient_is_priced_as_it_is_planned(L, monkeypatch, n, hw, cin, c
     monkeypatch.setattr(L, "GEMM_MAX_CTAS", max_ctas)
     d = check_convolution(L, cin, cout, k, 1, hw, n)
     assert L._conv_launches(d, 1, 1) == kernels
+
+
+@pytest.mark.parametrize("n,hw,cin,cout,k", [(32, 7, 512, 512, 3), (5, 9, 64, 64, 7)])
+def test_gathered_products_split_inside_a_cluster(L, n, hw, cin, cout, k):
+    """Few pixels and a long reduction: forward product and, where it is gathered, input gradient as clusters (kernels of 608 threads)."""
+    from bamboo_b200 import resnet
+    from bamboo_b200.arena import ParamArena
+    from cuda.bindings import driver
+    from test_gpu_overlap import captured, kernel_nodes
+    d = check_convolution(L, cin, cout, k, 1, hw, n)
+    m = resnet.ConvBN(cin, cout, k, relu=False, generator=torch.Generator().manual_seed(11))
+    ParamArena(list(m.parameters()), torch.device("cuda"), torch.bfloat16)
+    x = torch.randn(n, hw, hw, cin, device="cuda").bfloat16().requires_grad_(True)
+    dz = torch.ones_like(m(x))
+    graph, handle, rt = captured(lambda: torch.autograd.grad(m(x), x, dz))
+    threads = [driver.cuGraphKernelNodeGetParams(driver.CUgraphNode(int(v)))[1].blockDimX for v in kernel_nodes(handle, rt)]
+    assert threads.count(608) >= (2 if L._conv_launches(d, 1, 1) == 5 else 1), threads

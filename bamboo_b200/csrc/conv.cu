@@ -117,9 +117,10 @@ col2im_kernel(const uint4* dcol, uint4* __restrict__ dx, const ConvGeom g, const
 }
 
 // The same for strides 1 and 2 and up to T taps along each dimension that reach a pixel (T = ceil(k / S)): a thread owns an input
-// column's chunk over `rows` image rows, so what depends on the column is computed once and by shifts, and all of a pixel's
-// taps are requested before the first is added - in the same order (r, then s).  With four divisions by the stride and a chain
-// of loads per 16-byte result the general kernel ran at a third of the memory rate (us): 32 x 56 x 56 x 128, 3 x 3 / 2 36.8,
+// column's chunk over `rows` image rows, so what depends on the column is computed once and by shifts, and no load waits for an
+// address or a branch; taps are added in the same order (r, then s).  How many of them are in flight is the compiler's choice (32
+// registers for nine taps do not hold all).  With four divisions by the stride and a chain of loads per 16-byte
+// result the general kernel ran at a third of the memory rate (us): 32 x 56 x 56 x 128, 3 x 3 / 2 36.8,
 // 32 x 56 x 56 x 256, 1 x 1 / 2 28.4, 32 x 56 x 56 x 64, 3 x 3 45.3, 32 x 224 x 224 x 8, 7 x 7 / 2 141.6; this one 17.2,
 // 13.7, 21.0 and 65.1.
 template <typename I, int S, int T>

@@ -1347,6 +1347,13 @@ int clusters_at_once(int splits) {
 // (once + step x splits; us, unsplit / split: 513 x 2048 x 8192 41.7 / 25.5 as three splits of 256 columns, 128 x 1024 x 4096
 // 20.9 / 9.9 as six of 128, 1000 x 512 x 2048 12.9 / 9.0 as four, 1568 x 512 x 4608 24.8 / 16.0, 512 x 256 x 1024 8.2 / 7.1; with K = 512
 // and less, or tiles for more than half of the SMs, nothing is gained).
+// The constants come from an idle GPU; beside other work the split holds up (us, whole / split): forward + backward of one block with
+// its weight gradients on the side stream 513 x 2048 413 / 376, 1000 x 2048 503 / 468, 300 x 4096 834 / 764, 513 x 4096 982 / 991,
+// 1100 x 1024 260 / 278; a projection of 999 x 1024 to 50264 357 / 305, 513 x 2048 to 30528 257 / 243; twelve blocks forward
+// beside redundant work of one tile per CTA 513 x 2048 2106 / 1924, 300 x 4096 3347 / 2910, 512 x 1024 1274 / 1284.
+// A split sums in another order than the whole reduction, in fp32 either way and as close to 64 bits.  So the bf16 rounding of a product may
+// depend on how many rows ride along and on the budget: the stage's own forward and a redundant one, whose budget of CTAs
+// keeps reductions whole, agree within one rounding and not bit for bit.
 StorePlan plan_split(long long M, long long N, long long K) {
   static const struct { int bn; bool pair; double kblock, once, step; } kinds[3] = {
       {256, true, 0.32, 7.2, 0.95}, {256, false, 0.375, 6.2, 0.6}, {128, false, 0.283, 4.7, 0.45}};
